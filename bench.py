@@ -705,7 +705,7 @@ def batched_vs_plain(args, rank, torch):
 
     # The same points one after another: the plain kernels launched pass by
     # pass ("fused", the comparison the batched launch is measured against),
-    # and the library's default form per point ("auto": the resident cluster
+    # and the library's default form per point ("auto": the resident
     # launch for the 32^3 points, the fused passes for the others).
     t_seq = {"fused": float("nan"), "auto": float("nan")}
     for kind, sp in [(k, sp) for k in t_seq for sp in ([] if args.no_plain_grid else specs)]:

@@ -137,6 +137,19 @@ struct GraphEntry {
   uint64_t last_use = 0;
 };
 
+// Makes a device current for a scope.
+struct DeviceGuard {
+  int before = -1;
+  explicit DeviceGuard(int device) {
+    cudaGetDevice(&before);
+    if (before == device) before = -1;
+    else cudaSetDevice(device);
+  }
+  ~DeviceGuard() {
+    if (before >= 0) cudaSetDevice(before);
+  }
+};
+
 struct chll_lattice {
   int ni = 0, nj = 0, nk = 0, hx = 0, periodic = 0;
   long long nsites = 0;
@@ -146,6 +159,7 @@ struct chll_lattice {
   Control* ctl = nullptr;
   double* partials = nullptr;
   unsigned int* tickets = nullptr;  // [0] observables, [1] gradient
+  unsigned long long* words = nullptr;  // meeting words of the resident sweeps
   double* rows = nullptr;
   int rows_cap = 0;
   double* out4 = nullptr;
@@ -221,8 +235,8 @@ void drop_graphs(chll_lattice* L) {
 }
 
 // Returns an executable graph of `nsweeps` steps for this coupling and key,
-// capturing it on first use: 2 fused passes per step plus a closing flip
-// pass, or the reference's 4 half-sweeps per step.
+// capturing it on first use: the launches of 2 fused passes per step plus a
+// closing flip pass, or the reference's 4 half-sweeps per step.
 int get_graph(chll_lattice* L, const Coupling& cp, uint32_t k0, uint32_t k1, uint32_t rep,
               int nsweeps, cudaGraphExec_t* out) {
   for (auto& g : L->graphs) {
@@ -234,26 +248,9 @@ int get_graph(chll_lattice* L, const Coupling& cp, uint32_t k0, uint32_t k1, uin
     }
   }
   const LatticeView v = L->view();
-  // auto: the resident cluster launch where its threads hold at most one
-  // unit per pass (a pass is then mostly latency: up to 32^3), else the fused
-  // passes (decided before the capture, which the cluster query must not
-  // meet)
-  const bool resident =
-      L->kernel == chll::kSweepResident ||
-      (L->kernel == chll::kSweepAuto && chll::resident_cluster() > 0 &&
-       chll::resident_units_per_thread(v) <= 1);
   cudaGraph_t graph = nullptr;
   CHLL_CUDA_TRY(cudaStreamBeginCapture(L->capture_stream, cudaStreamCaptureModeThreadLocal));
-  if (resident) {
-    // the whole chunk in one cluster launch
-    if (chll::launch_resident_sweeps(v, cp, k0, k1, rep, L->ctl, nsweeps, L->capture_stream)) {
-      cudaGraph_t g = nullptr;
-      cudaStreamEndCapture(L->capture_stream, &g);
-      if (g) cudaGraphDestroy(g);
-      cudaGetLastError();
-      return fail(CHLL_ECUDA, "resident sweep launch failed");
-    }
-  } else if (L->kernel == chll::kSweepAuto || L->kernel == chll::kSweepFused) {
+  if (L->kernel != chll::kSweepDirect && L->kernel != chll::kSweepStaged) {
     // A0 B (A B)... F: the fused two-pass sweep, flips completed at the end
     for (int s = 0; s < nsweeps; ++s) {
       chll::launch_fused_pass(v, cp, k0, k1, rep, L->ctl, s ? chll::kFusedA : chll::kFusedA0,
@@ -297,10 +294,30 @@ int get_graph(chll_lattice* L, const Coupling& cp, uint32_t k0, uint32_t k1, uin
 }
 
 constexpr int kGraphChunk = 100;
+constexpr int kResidentChunk = 1000;
+
+// Whether the lattice's sweeps run as resident launches (with the lattice's
+// device current).
+bool runs_resident(const chll_lattice* L) {
+  if (L->slab || !chll::resident_fits(L->view())) return false;
+  return L->kernel == chll::kSweepResident ||
+         (L->kernel == chll::kSweepAuto && chll::resident_pays(L->view()));
+}
 
 int sweep_impl(chll_lattice* L, const Coupling& cp, uint64_t seed, uint32_t rep, int nsweeps) {
   if (nsweeps <= 0) return CHLL_OK;
   const uint32_t k0 = seed_lo(seed), k1 = seed_hi(seed);
+  const DeviceGuard on(L->device);
+  if (runs_resident(L)) {
+    for (int done = 0; done < nsweeps; done += kResidentChunk) {
+      const cudaError_t e = chll::launch_resident_sweeps(
+          L->view(), cp, k0, k1, rep, L->ctl, L->words, std::min(kResidentChunk, nsweeps - done),
+          L->stream);
+      if (e != cudaSuccess)
+        return fail(CHLL_ECUDA, "resident sweep launch: %s", cudaGetErrorString(e));
+    }
+    return CHLL_OK;
+  }
   const int chunk = std::min(nsweeps, kGraphChunk);
   const int full = nsweeps / chunk, rest = nsweeps % chunk;
   cudaGraphExec_t exec = nullptr;
@@ -372,6 +389,8 @@ int set_control_impl(chll_lattice* L, double d, long long step, long long adapt_
   c.nsites = L->ctl_sites;
   c.deferred = L->slab;
   CHLL_CUDA_TRY(cudaMemcpyAsync(L->ctl, &c, sizeof(c), cudaMemcpyHostToDevice, L->stream));
+  // the new block's status is clear: so are the words a failed wait left
+  CHLL_CUDA_TRY(cudaMemsetAsync(L->words, 0, chll::kResidentWordBytes, L->stream));
   CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
   return CHLL_OK;
 }
@@ -457,6 +476,8 @@ int create_impl(int ni, int nj, int nk, int boundary, chll_lattice** out, int sl
     return bail(e, "partials");
   if ((e = cudaMalloc(&L->tickets, 2 * sizeof(unsigned int))) != cudaSuccess)
     return bail(e, "tickets");
+  if ((e = cudaMalloc(&L->words, chll::kResidentWordBytes)) != cudaSuccess)
+    return bail(e, "meeting words");
   if ((e = cudaMalloc(&L->out4, 4 * sizeof(double) + chll::kRowLen * sizeof(double))) !=
       cudaSuccess)
     return bail(e, "result buffer");
@@ -715,6 +736,7 @@ void chll_lattice_destroy(chll_lattice* L) {
   cudaFree(L->ctl);
   cudaFree(L->partials);
   cudaFree(L->tickets);
+  cudaFree(L->words);
   cudaFree(L->rows);
   cudaFree(L->out4);
   cudaFree(L->staging);
@@ -730,8 +752,6 @@ int chll_lattice_set_kernel(chll_lattice* L, int kernel) {
     return fail(CHLL_EINVAL, "set_kernel: kernel must be 0, 1, 2, 3 or 4");
   if (kernel == chll::kSweepResident && L->slab)
     return fail(CHLL_EINVAL, "set_kernel: a slab cannot run the resident form");
-  if (kernel == chll::kSweepResident && chll::resident_cluster() <= 0)
-    return fail(CHLL_ECUDA, "set_kernel: no thread-block cluster fits on this device");
   if (kernel == chll::kSweepStaged && !chll::staged_fits(L->view()))
     return fail(CHLL_EINVAL, "set_kernel: rows of %d sites are too long for the staged kernel",
                 L->ni);

@@ -190,15 +190,12 @@ __device__ __forceinline__ bool metropolis(float dE, float u, float inv_kT) {
 // side by side and only their acceptance depends on v0, v1, so the two
 // independent chains interleave; a missing (padding) site's arithmetic is
 // discarded.
-template <int C, bool FLIP_BEFORE, bool DIR, bool FLIP_AFTER, class KEY>
-__device__ __forceinline__ void unit_trials(float4& n0, float4& n1, const Nbrs& nb0,
-                                            const Nbrs& nb1, bool v0, bool v1, uint32_t g,
-                                            uint32_t step, float d, const Coupling& cp,
-                                            const KEY& key, uint32_t replica,
-                                            unsigned int& nacc, unsigned int& nflip) {
-  constexpr bool kNextStep = FLIP_AFTER && !DIR && C == 0;
-  const UnitRandoms u = unit_randoms(
-      philox4x32_10({{g, kNextStep ? step + 1u : step, replica, (uint32_t)C}}, key));
+template <bool FLIP_BEFORE, bool DIR, bool FLIP_AFTER>
+__device__ __forceinline__ void unit_trials_drawn(float4& n0, float4& n1, const Nbrs& nb0,
+                                                  const Nbrs& nb1, bool v0, bool v1,
+                                                  const UnitRandoms& u, float d,
+                                                  const Coupling& cp, unsigned int& nacc,
+                                                  unsigned int& nflip) {
   // The trial directors depend only on n's direction, which the flips before
   // them leave alone, so both bond sums of a site come from one paired pass.
   float mx0, my0, mz0, mx1, my1, mz1;
@@ -243,6 +240,18 @@ __device__ __forceinline__ void unit_trials(float4& n0, float4& n1, const Nbrs& 
     if (a1) n1.w = -n1.w;
     nflip += (unsigned int)a0 + (unsigned int)a1;
   }
+}
+
+template <int C, bool FLIP_BEFORE, bool DIR, bool FLIP_AFTER, class KEY>
+__device__ __forceinline__ void unit_trials(float4& n0, float4& n1, const Nbrs& nb0,
+                                            const Nbrs& nb1, bool v0, bool v1, uint32_t g,
+                                            uint32_t step, float d, const Coupling& cp,
+                                            const KEY& key, uint32_t replica,
+                                            unsigned int& nacc, unsigned int& nflip) {
+  constexpr bool kNextStep = FLIP_AFTER && !DIR && C == 0;
+  const UnitRandoms u = unit_randoms(
+      philox4x32_10({{g, kNextStep ? step + 1u : step, replica, (uint32_t)C}}, key));
+  unit_trials_drawn<FLIP_BEFORE, DIR, FLIP_AFTER>(n0, n1, nb0, nb1, v0, v1, u, d, cp, nacc, nflip);
 }
 
 }  // namespace chll

@@ -1,31 +1,37 @@
-// Resident sweeps: a whole chunk of fused sweeps of one small lattice in ONE
-// launch of ONE thread-block cluster.
+// Resident sweeps: a whole chunk of fused sweeps of one lattice in ONE
+// cooperative launch whose CTAs stay on the SMs and meet at a grid barrier
+// between passes.
 //
-// A small lattice's fused pass is latency-bound: at 32^3 a pass holds 8,192
-// units, one per thread, and takes ~3.3 us from one launch to the next, most
-// of it the grid's start, drain, count epilogue and completion rather than
-// its work.  Here
-// the cluster's CTAs (up to 16, one per SM) stay resident for the whole
-// chunk and meet at the hardware cluster barrier between passes
-// (barrier.cluster.arrive.release / wait.acquire): no launch, no grid drain,
-// no software barrier in global memory.  Each CTA adds its pass counts into
-// every CTA's shared memory through distributed shared memory
-// (red.shared::cluster), and every CTA derives the next d and step from the
-// same totals with the plain kernels' control arithmetic
-// (fused_control_update), so the chain -- units, counters, arithmetic,
-// control block -- is the fused form's bit for bit.
+// What bounds a small lattice's sweep is latency: at 32^3 a pass holds 8,192
+// units, and as a launch of its own it takes 3.3 us, most of it the grid's
+// start and drain, the read of the control block and the count epilogue.
+// Here a pass is its loads (L2: the lattice was written by other SMs a pass
+// earlier), one unit's serial trial arithmetic, and the barrier: about 0.75 us
+// for the barrier of 128 CTAs and 1.1 us for the arithmetic of a single warp
+// per scheduler (8^3 in one CTA, where the barrier is the CTA's own, runs a
+// sweep in 2.3 us; 16^3 on 32 CTAs in 4.5).  So the units are spread over all
+// SMs, as few warps on each as there can be: threads per CTA come from
+// units / SMs.  The form that this one replaces kept the chunk in one cluster
+// of 16 CTAs with the hardware cluster barrier: its barrier was cheaper, but 16
+// SMs had to issue every instruction of the pass.  us per sweep on one B200
+// (periodic, kT 0.5, K 0.5):
 //
-// The other colour is read through the coherent path (sweep_unit.cuh
-// kLoadCoherentOrdered): it was written by other CTAs of the cluster earlier
-// in the launch, and the barrier's release/acquire orders those stores
-// before the loads; the loads carry a memory clobber, so the compiler cannot
-// move them across a barrier either.
+//   edge                    8     16    24    32    48    64    96    128   200
+//   passes launched each   5.4   6.3   6.4   6.5   6.9   8.1   15.0  26.6  85.2
+//   one cluster            3.5   5.4   5.5   5.6  14.5
+//   this form              2.3   4.5   4.6   4.7   5.1   6.5   13.6  24.6  79.9
 //
-// Launched without a programmatic-dependent attribute: a chunk is one launch.
+// The barrier and the counts are one 64-bit word per pass: a CTA adds its
+// accept counts and its arrival with one release reduction and polls the
+// word (acquire) until every CTA has arrived, so the wait already holds the
+// pass's total; every CTA then derives the next d and step from it with the
+// control update's arithmetic (fused_close), and the chain -- units, counters,
+// arithmetic, control block -- is the fused form's bit for bit.  Every wait is
+// bounded; one that runs out sets the control block's status word, and
+// launches do nothing until set_control clears it.
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <cstdlib>
 #include <mutex>
 
 #include "sweep.cuh"
@@ -34,7 +40,18 @@
 namespace chll {
 namespace {
 
-constexpr int kResThreads = 512;
+constexpr int kResThreads = 512;  // most threads per CTA, and per SM (128 registers each)
+constexpr uint32_t kWaitLimit = 1u << 22;  // polls of the word before a wait gives up
+
+// One word per pass, three in rotation, 128 bytes apart: director accepts in
+// bits 0-25, flips in bits 26-51, arrived CTAs in bits 52-63.  The word of pass
+// q is cleared by the first CTA once the barrier of pass q + 1 is through --
+// every CTA has then read it for the last time -- and that CTA's release at
+// pass q + 2 puts the clear before any arrival at pass q + 3, its next use.
+constexpr int kWordStride = 16;
+constexpr int kCountBits = 26;
+constexpr unsigned long long kCountMask = (1ull << kCountBits) - 1;
+constexpr int kArriveShift = 2 * kCountBits;
 
 struct ResidentArgs {
   LatticeView L;
@@ -43,321 +60,401 @@ struct ResidentArgs {
   Coupling cp;
   PhiloxKeys keys;
   uint32_t replica;
-  uint32_t nct;  // CTAs in the cluster (= the grid)
   Control* ctl;
+  unsigned long long* words;
   int nsweeps;
+  uint32_t wait_limit;
 };
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-
-// Every thread of every CTA of the cluster: this thread's earlier writes
-// (global and shared) are released, the others' acquired.
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile(
-      "barrier.cluster.arrive.release.aligned;\n\t"
-      "barrier.cluster.wait.acquire.aligned;" ::
-          : "memory");
-}
-
-// Address of this CTA's shared variable `p` in CTA `rank` of the cluster.
-__device__ __forceinline__ uint32_t dsmem_addr(const void* p, uint32_t rank) {
-  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-  return r;
-}
-
-__device__ __forceinline__ void dsmem_add(uint32_t addr, unsigned long long v) {
-  asm volatile("red.shared::cluster.add.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
-}
-
-// The control block's running state, kept by thread 0 of every CTA (all the
-// same) and written back by the first CTA at the end.
-struct ResControl {
+struct ResidentShared {
+  unsigned int cnt[2][kResThreads / 32];
   double d;
-  long long step;
-  unsigned long long nacc, nflip;
-  float paccept, faccept;
-  long long nacc_last, nflip_last;
-  float n3;                // site count as FP32 (chll_mod.f90:83,93)
-  long long adapt_until;
+  int ok;
 };
 
-// One fused pass (sweep.cuh FusedPhase) over the lattice by the cluster's
-// threads: the plain kernels' column walk or unit loop, with coherent loads
-// that the compiler keeps between the barriers around the pass.
-template <int PHASE, int BMODE, int FORM>
-__device__ __forceinline__ void resident_pass(const ResidentArgs& A, uint32_t rank, uint32_t step,
-                                           float d, unsigned int& nacc, unsigned int& nflip) {
-  constexpr int C = PHASE == kFusedB ? 1 : 0;
-  constexpr bool FLIP_BEFORE = PHASE == kFusedA || PHASE == kFusedF;
-  constexpr bool DIR = PHASE != kFusedF;
-  constexpr bool FLIP_AFTER = PHASE == kFusedB;
-  constexpr bool P = BMODE == kBoundPeriodic;
-  constexpr bool FULL = FORM != 0;
-  const LatticeView L = A.L;
-  const Coupling cp = A.cp;
-  const PhiloxKeys key = A.keys;
-  const uint32_t replica = A.replica;
-  const uint32_t stride = A.nct * kResThreads;
-  unsigned int na = 0, nf = 0;
-  if (FORM == 2) {
-    const WalkGeom W = A.W;
-    for (uint32_t t = rank * kResThreads + threadIdx.x; t < W.ntasks; t += stride)
-      walk_task<C, P, P, FLIP_BEFORE, DIR, FLIP_AFTER, kLoadCoherentOrdered>(
-          L, W, t, step, d, cp, key, replica, na, nf);
-  } else {
-    const SweepGeom G = A.G;
-    const uint32_t plane = (uint32_t)L.hx * (uint32_t)L.nj;
-    const uint32_t per_colour = plane * (uint32_t)L.nk;
-    for (uint32_t g = rank * kResThreads + threadIdx.x; g < G.units; g += stride) {
-      if (g + stride < G.units) prefetch_unit<C>(L, g + stride, plane, per_colour);
-      unit_step<C, P, P, FLIP_BEFORE, DIR, FLIP_AFTER, FULL, kLoadCoherentOrdered>(
-          L, G, g, step, d, cp, key, replica, na, nf);
+// Which trials a phase runs, of which colour (sweep.cuh FusedPhase).
+template <int PHASE>
+struct PhaseOf {
+  static constexpr int C = PHASE == kFusedB ? 1 : 0;
+  static constexpr bool flip_before = PHASE == kFusedA || PHASE == kFusedF;
+  static constexpr bool dir = PHASE != kFusedF;
+  static constexpr bool flip_after = PHASE == kFusedB;
+};
+
+// Lattices of more units than threads: the plain kernels' column walk or
+// unit loop, with coherent loads that the compiler keeps between the barriers
+// around a pass.
+template <bool P, int FORM>
+struct SharedUnits {
+  const ResidentArgs& A;
+  __device__ __forceinline__ explicit SharedUnits(const ResidentArgs& a) : A(a) {}
+
+  template <int C>
+  __device__ __forceinline__ void draw(uint32_t) {}
+
+  template <int PHASE>
+  __device__ __forceinline__ void pass(uint32_t step, float d, unsigned int& nacc,
+                                       unsigned int& nflip) {
+    using T = PhaseOf<PHASE>;
+    const uint32_t stride = gridDim.x * blockDim.x;
+    const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned int na = 0, nf = 0;
+    if (FORM == 2) {
+      for (uint32_t t = first; t < A.W.ntasks; t += stride)
+        walk_task<T::C, P, P, T::flip_before, T::dir, T::flip_after, kLoadCoherentOrdered>(
+            A.L, A.W, t, step, d, A.cp, A.keys, A.replica, na, nf);
+    } else {
+      const uint32_t plane = (uint32_t)A.L.hx * (uint32_t)A.L.nj;
+      const uint32_t per_colour = plane * (uint32_t)A.L.nk;
+      for (uint32_t g = first; g < A.G.units; g += stride) {
+        if (g + stride < A.G.units) prefetch_unit<T::C>(A.L, g + stride, plane, per_colour);
+        unit_step<T::C, P, P, T::flip_before, T::dir, T::flip_after, FORM != 0,
+                  kLoadCoherentOrdered>(A.L, A.G, g, step, d, A.cp, A.keys, A.replica, na, nf);
+      }
+    }
+    nacc = na;
+    nflip = nf;
+  }
+};
+
+// Lattices of at most one unit per thread (48^3 5.1 against 5.4 us per sweep
+// with the unit loop, 64^3 6.5 against 7.1): the thread keeps both colours'
+// unit g (the 4-site x-block q of row (j, k)) in registers for the whole
+// chunk.  The other colour's pair then is the x-row pair of walk_task, so a
+// pass loads the +-y and +-z pairs and one x neighbour, at addresses fixed for
+// the launch, and the pass's random words are drawn while the barrier before
+// it is waited for.  ni a multiple of 4, or open boundaries (a padding slot
+// reads as the zero of a missing neighbour).
+template <bool P>
+struct OwnUnit {
+  const ResidentArgs& A;
+  uint32_t g, u, o0;             // unit, its slot, parity of colour 0's sites in the row
+  uint32_t yp, ym, zp, zm;       // slots of the neighbour pairs
+  uint32_t xm, xp;               // the x neighbours outside the block: below, above
+  bool has, hyp, hym, hzp, hzm, hxm, hxp;
+  bool v[4];                     // sites 4q .. 4q+3 inside the lattice
+  float4 n[2][2];
+  Ctr4 words;
+
+  __device__ __forceinline__ explicit OwnUnit(const ResidentArgs& a) : A(a) {
+    const LatticeView& L = A.L;
+    g = blockIdx.x * blockDim.x + threadIdx.x;
+    has = g < A.G.units;
+    const uint32_t hx = (uint32_t)L.hx, nj = (uint32_t)L.nj, nk = (uint32_t)L.nk;
+    const uint32_t plane = hx * nj;
+    const uint32_t row = A.G.by_Q.div(g), q = g - row * A.G.Q;
+    const uint32_t k = A.G.by_nj.div(row), j = row - k * nj;
+    o0 = (j + k) & 1u;
+    u = 2 * g;
+    hyp = P || j + 1 < nj;
+    hym = P || j > 0;
+    hzp = P || k + 1 < nk;
+    hzm = P || k > 0;
+    hxm = P || q > 0;
+    hxp = P || q + 1 < A.G.Q;
+    yp = j + 1 < nj ? u + hx : u - (nj - 1) * hx;
+    ym = j > 0 ? u - hx : u + (nj - 1) * hx;
+    zp = k + 1 < nk ? u + plane : u - (nk - 1) * plane;
+    zm = k > 0 ? u - plane : u + (nk - 1) * plane;
+    xm = q > 0 ? u - 1 : u + hx - 1;
+    xp = q + 1 < A.G.Q ? u + 2 : u - 2 * q;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) v[t] = has && 4 * q + t < (uint32_t)L.ni;
+    n[0][0] = n[0][1] = n[1][0] = n[1][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (has) {
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const UnitSlots s = ld_unit(L.col[c] + u);
+        n[c][0] = s.a;
+        n[c][1] = s.b;
+      }
     }
   }
-  nacc = na;
-  nflip = nf;
-}
 
-// Pass q and its counts: summed over the CTA, then added by CTA-many threads
-// into slot q % 3 of EVERY CTA's counters (director accepts in the low, flips
-// in the high 32 bits of one word), so that after the barrier each CTA reads
-// the cluster's totals from its own shared memory.  Each CTA clears its own
-// slot (q + 1) % 3 before it arrives at barrier q: it read that slot last,
-// for pass q - 2, before arriving at barrier q (program order), and the next
-// additions to it come from pass q + 1, after barrier q.
-template <int PHASE, int BMODE, int FORM>
-__device__ __forceinline__ void resident_pass_counted(const ResidentArgs& A, uint32_t rank,
-                                                      uint32_t q, uint32_t step, float d,
-                                                      unsigned long long* s_tot,
-                                                      unsigned int* s_part) {
-  unsigned int na = 0, nf = 0;
-  resident_pass<PHASE, BMODE, FORM>(A, rank, step, d, na, nf);
+  // The random words of the next pass (colour C, step): independent of the
+  // lattice, so they are drawn before the wait.
+  template <int C>
+  __device__ __forceinline__ void draw(uint32_t step) {
+    words = philox4x32_10({{g, step, A.replica, (uint32_t)C}}, A.keys);
+    asm volatile("" : "+r"(words.v[0]), "+r"(words.v[1]), "+r"(words.v[2]), "+r"(words.v[3]));
+  }
+
+  template <int PHASE>
+  __device__ __forceinline__ void pass(uint32_t, float d, unsigned int& nacc,
+                                       unsigned int& nflip) {
+    using T = PhaseOf<PHASE>;
+    constexpr int C = T::C;
+    nacc = nflip = 0;
+    if (!has) return;
+    const float4* oth = A.L.col[C ^ 1];
+    const bool odd = (o0 ^ C) != 0;  // sites 4q+1, 4q+3 rather than 4q, 4q+2
+    Nbrs nb0, nb1;
+    nbr_units<kLoadCoherentOrdered>(hyp, oth + yp, nb0.b[2], nb1.b[2]);
+    nbr_units<kLoadCoherentOrdered>(hym, oth + ym, nb0.b[3], nb1.b[3]);
+    nbr_units<kLoadCoherentOrdered>(hzp, oth + zp, nb0.b[4], nb1.b[4]);
+    nbr_units<kLoadCoherentOrdered>(hzm, oth + zm, nb0.b[5], nb1.b[5]);
+    float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (odd ? hxp : hxm) e = ld4_other<kLoadCoherentOrdered>(oth + (odd ? xp : xm));
+    const float4 xa = n[C ^ 1][0], xb = n[C ^ 1][1];
+    nb0.b[0] = odd ? xb : xa;
+    nb0.b[1] = odd ? xa : e;
+    nb1.b[0] = odd ? e : xb;
+    nb1.b[1] = odd ? xb : xa;
+    unit_trials_drawn<T::flip_before, T::dir, T::flip_after>(
+        n[C][0], n[C][1], nb0, nb1, odd ? v[1] : v[0], odd ? v[3] : v[2], unit_randoms(words), d,
+        A.cp, nacc, nflip);
+    st_unit(A.L.col[C] + u, n[C][0], n[C][1]);
+  }
+};
+
+// The CTA's counts of a pass (thread 0): director accepts, and flips where
+// they are wanted.  Ends with the CTA's stores ordered before thread 0's
+// release.
+__device__ __forceinline__ unsigned long long cta_counts(ResidentShared& S, unsigned int na,
+                                                         unsigned int nf, bool flips) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   na = __reduce_add_sync(0xffffffffu, na);
-  nf = __reduce_add_sync(0xffffffffu, nf);
-  if ((threadIdx.x & 31) == 0) {
-    if (na) atomicAdd(&s_part[0], na);
-    if (nf) atomicAdd(&s_part[1], nf);
+  if (flips) nf = __reduce_add_sync(0xffffffffu, nf);
+  if (lane == 0) {
+    S.cnt[0][warp] = na;
+    if (flips) S.cnt[1][warp] = nf;
   }
   __syncthreads();
-  const unsigned long long v = (unsigned long long)s_part[0] |
-                               ((unsigned long long)s_part[1] << 32);
-  if (threadIdx.x < A.nct && v) dsmem_add(dsmem_addr(&s_tot[q % 3], threadIdx.x), v);
-  __syncthreads();  // s_part read by every sender before it is cleared
+  unsigned long long v = 0;
   if (threadIdx.x == 0) {
-    s_part[0] = s_part[1] = 0;
-    s_tot[(q + 1) % 3] = 0;
+    unsigned int a = 0, f = 0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
+      a += S.cnt[0][w];
+      if (flips) f += S.cnt[1][w];
+    }
+    v = (unsigned long long)a | ((unsigned long long)f << kCountBits);
   }
-  cluster_barrier();
+  return v;
 }
 
-// The control updates of fused_control_update for the counts of pass q
-// (thread 0; the totals in this CTA's slot q % 3).
-template <int PHASE>
-__device__ __forceinline__ void resident_update(ResControl& S, const unsigned long long* s_tot,
-                                                uint32_t q) {
-  const unsigned long long t = s_tot[q % 3];
-  S.nacc += t & 0xffffffffull;
-  S.nflip += t >> 32;
-  if (PHASE == kFusedB) {
-    const float pa = (float)S.nacc / S.n3;
-    S.paccept = pa;
-    S.nacc_last = (long long)S.nacc;
-    S.nacc = 0;
-    if (S.step < S.adapt_until) S.d = adapt_d(S.d, pa);
-    S.step = S.step + 1;
-  } else if (PHASE == kFusedA || PHASE == kFusedF) {
-    S.faccept = (float)S.nflip / S.n3;
-    S.nflip_last = (long long)S.nflip;
-    S.nflip = 0;
-  }
+// Thread 0 of every CTA adds the CTA's counts and arrival to the pass's word
+// (release: the CTA's stores, ordered before it by the CTA barrier, are
+// visible to whoever acquires the word) ...
+__device__ __forceinline__ void grid_arrive(unsigned long long* w, unsigned long long counts,
+                                            uint32_t nct) {
+  if (nct == 1) return;
+  const unsigned long long add = counts + (1ull << kArriveShift);
+  asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(w), "l"(add) : "memory");
 }
 
-// A sweep is pass A (A0 first) and pass B with a cluster barrier after each;
-// the counts of both close after B's barrier (A's update first, as the fused
-// passes apply them), and only B changes d and step, which thread 0 then
-// hands to the CTA.  Passes A and F only need the lattice ordered by their
-// barrier.
-template <int BMODE, int FORM>
-__global__ void __launch_bounds__(kResThreads, 1)
-    resident_sweeps_kernel(const __grid_constant__ ResidentArgs A) {
-  __shared__ unsigned long long s_tot[3];
-  __shared__ unsigned int s_part[2];
-  __shared__ double s_d;
-  __shared__ long long s_step;
-  const uint32_t rank = cluster_rank();
+// ... and waits until every CTA has (acquire).  Returns the word, or the CTA's
+// own counts of a grid of one CTA; ok = false if the wait ran out.
+__device__ __forceinline__ unsigned long long grid_wait(unsigned long long* w,
+                                                        unsigned long long counts, uint32_t nct,
+                                                        uint32_t limit, bool& ok) {
+  if (nct == 1) return counts;
+  unsigned long long v;
+  uint32_t polls = 0;
+  do {
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(w) : "memory");
+    if ((uint32_t)(v >> kArriveShift) == nct) return v;
+  } while (++polls < limit);
+  ok = false;
+  return v;
+}
+
+// The chunk: A0 B (A B)... F with the grid barrier after every pass but the
+// last.
+template <class UNITS>
+__device__ __forceinline__ void resident_sweeps(const ResidentArgs& A, ResidentShared& S) {
   Control* ctl = A.ctl;
-  if (threadIdx.x < 3) s_tot[threadIdx.x] = 0;
-  if (threadIdx.x < 2) s_part[threadIdx.x] = 0;
+  if (ctl->status) return;  // an earlier wait ran out: the words are not to be trusted
+  const uint32_t nct = gridDim.x;
+  const bool lead = threadIdx.x == 0;
   double d = ctl->d;
   long long step = ctl->step;
-  ResControl S;
-  if (threadIdx.x == 0) {
-    S.d = d;
-    S.step = step;
-    S.nacc = ctl->nacc;
-    S.nflip = ctl->nflip;
-    S.paccept = ctl->paccept;
-    S.faccept = ctl->faccept;
-    S.nacc_last = ctl->nacc_last;
-    S.nflip_last = ctl->nflip_last;
-    S.n3 = (float)ctl->nsites;
-    S.adapt_until = ctl->adapt_until;
-  }
-  cluster_barrier();  // counters cleared in every CTA, the control block read
-  uint32_t q = 0;
+  const long long adapt_until = ctl->adapt_until;
+  const float n3 = (float)ctl->nsites;  // chll_mod.f90:83,93
+  unsigned long long nacc = ctl->nacc, nflip = ctl->nflip;  // left open by single passes
+  float paccept = 0.f;
+  bool ok = true;
+  uint32_t slot = 0;  // word of the pass
+  unsigned int na, nf;
+  UNITS units(A);
+  units.template draw<0>((uint32_t)step);
   for (int s = 0; s < A.nsweeps; ++s) {
+    const bool last = s == A.nsweeps - 1;
     if (s)
-      resident_pass_counted<kFusedA, BMODE, FORM>(A, rank, q, (uint32_t)step, (float)d, s_tot,
-                                                  s_part);
+      units.template pass<kFusedA>((uint32_t)step, (float)d, na, nf);
     else
-      resident_pass_counted<kFusedA0, BMODE, FORM>(A, rank, q, (uint32_t)step, (float)d, s_tot,
-                                                   s_part);
-    resident_pass_counted<kFusedB, BMODE, FORM>(A, rank, q + 1, (uint32_t)step, (float)d, s_tot,
-                                                s_part);
-    if (threadIdx.x == 0) {
-      if (s)
-        resident_update<kFusedA>(S, s_tot, q);
-      else
-        resident_update<kFusedA0>(S, s_tot, q);
-      resident_update<kFusedB>(S, s_tot, q + 1);
-      s_d = S.d;
-      s_step = S.step;
+      units.template pass<kFusedA0>((uint32_t)step, (float)d, na, nf);
+    unsigned long long v = cta_counts(S, na, nf, false);
+    if (lead) grid_arrive(A.words + slot * kWordStride, v, nct);
+    units.template draw<1>((uint32_t)step);
+    if (lead) {
+      v = grid_wait(A.words + slot * kWordStride, v, nct, A.wait_limit, ok);
+      nacc += v & kCountMask;
+      if (blockIdx.x == 0) A.words[(slot == 0 ? 2 : slot - 1) * kWordStride] = 0;
+      S.ok = ok;
     }
+    slot = slot == 2 ? 0 : slot + 1;
     __syncthreads();
-    d = s_d;
-    step = s_step;
-    q += 2;
+    if (!S.ok) break;
+    units.template pass<kFusedB>((uint32_t)step, (float)d, na, nf);
+    v = cta_counts(S, na, nf, last);
+    if (lead) grid_arrive(A.words + slot * kWordStride, v, nct);
+    units.template draw<0>((uint32_t)step + 1u);
+    if (lead) {
+      // both outcomes of adapt_d ahead of the wait
+      double dn = adapt_d(d, 0.f), up = adapt_d(d, 1.f);
+      asm volatile("" : "+d"(dn), "+d"(up));
+      v = grid_wait(A.words + slot * kWordStride, v, nct, A.wait_limit, ok);
+      nacc += v & kCountMask;
+      if (blockIdx.x == 0) A.words[(slot == 0 ? 2 : slot - 1) * kWordStride] = 0;
+      // the control update that closes the director count (fused_close)
+      paccept = (float)nacc / n3;
+      if (step < adapt_until) {
+        if ((double)paccept < 0.4) d = dn;
+        else if ((double)paccept > 0.6) d = up;
+      }
+      if (last) {
+        if (s) nflip = 0;  // closed by this sweep's pass A
+        nflip += v >> kCountBits & kCountMask;
+      } else {
+        nacc = 0;
+      }
+      S.d = d;
+      S.ok = ok;
+    }
+    slot = slot == 2 ? 0 : slot + 1;
+    ++step;
+    __syncthreads();
+    if (!S.ok) break;
+    d = S.d;
   }
-  if (A.nsweeps > 0) {
-    resident_pass_counted<kFusedF, BMODE, FORM>(A, rank, q, (uint32_t)step, (float)d, s_tot,
-                                                s_part);
-    if (threadIdx.x == 0) resident_update<kFusedF>(S, s_tot, q);
+  if (!S.ok) {
+    if (lead) atomicOr(&ctl->status, 4u);
+    return;
   }
-  if (rank == 0 && threadIdx.x == 0) {
-    ctl->d = S.d;
-    ctl->step = S.step;
-    ctl->nacc = S.nacc;
-    ctl->nflip = S.nflip;
-    ctl->paccept = S.paccept;
-    ctl->faccept = S.faccept;
-    ctl->nacc_last = S.nacc_last;
-    ctl->nflip_last = S.nflip_last;
+  units.template pass<kFusedF>((uint32_t)step, (float)d, na, nf);
+  unsigned long long v = cta_counts(S, 0, nf, true);
+  if (!lead) return;
+  // the CTA that completes the closing pass's word has the flip count and
+  // writes the control block; nobody waits for this word, so it also clears
+  // all three for the next launch
+  if (nct > 1) {
+    const unsigned long long old =
+        atomicAdd(A.words + slot * kWordStride, v + (1ull << kArriveShift));
+    if ((uint32_t)(old >> kArriveShift) != nct - 1) return;
+    v += old;
+    for (int w = 0; w < 3; ++w) A.words[w * kWordStride] = 0;
   }
+  nflip += v >> kCountBits & kCountMask;
+  ctl->d = d;
+  ctl->step = step;
+  ctl->paccept = paccept;
+  ctl->nacc_last = (long long)nacc;
+  ctl->nacc = 0;
+  ctl->faccept = (float)nflip / n3;
+  ctl->nflip_last = (long long)nflip;
+  ctl->nflip = 0;
+}
+
+template <bool P, int FORM>
+__global__ void __launch_bounds__(kResThreads, 1)
+    resident_sweeps_kernel(const __grid_constant__ ResidentArgs A) {
+  __shared__ ResidentShared S;
+  if (FORM == 3)
+    resident_sweeps<OwnUnit<P>>(A, S);
+  else
+    resident_sweeps<SharedUnits<P, FORM>>(A, S);
 }
 
 using ResidentKernel = void (*)(const ResidentArgs);
-// [periodic][form]
-const ResidentKernel kResident[2][3] = {
-    {resident_sweeps_kernel<kBoundOpen, 0>, resident_sweeps_kernel<kBoundOpen, 1>,
-     resident_sweeps_kernel<kBoundOpen, 2>},
-    {resident_sweeps_kernel<kBoundPeriodic, 0>, resident_sweeps_kernel<kBoundPeriodic, 1>,
-     resident_sweeps_kernel<kBoundPeriodic, 2>}};
+// [periodic][form]: 0 unit loop with padding checks, 1 unit loop, 2 column
+// walk, 3 one unit per thread
+const ResidentKernel kResident[2][4] = {
+    {resident_sweeps_kernel<false, 0>, resident_sweeps_kernel<false, 1>,
+     resident_sweeps_kernel<false, 2>, resident_sweeps_kernel<false, 3>},
+    {resident_sweeps_kernel<true, 0>, resident_sweeps_kernel<true, 1>,
+     resident_sweeps_kernel<true, 2>, resident_sweeps_kernel<true, 3>}};
 
-// The largest cluster (16, 8, 4, 2 or 1 CTAs) of which one can be resident
-// on this device, per device; 0 if none.
 std::mutex g_res_mutex;
-int g_res_cluster[64];
-bool g_res_known[64];
+int g_res_sms[64];
 
-// CHLL_RESIDENT_CLUSTER caps the cluster size (for measurements).
-int query_cluster() {
-  int best = 0;
-  const char* env = std::getenv("CHLL_RESIDENT_CLUSTER");
-  const int cap = env ? std::atoi(env) : 16;
-  for (int p = 0; p < 2; ++p)
-    for (int f = 0; f < 3; ++f)
-      cudaFuncSetAttribute(kResident[p][f], cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  for (int c : {16, 8, 4, 2, 1}) {
-    if (c > cap) continue;
-    bool all = true;
-    for (int p = 0; p < 2 && all; ++p)
-      for (int f = 0; f < 3 && all; ++f) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)c);
-        cfg.blockDim = dim3(kResThreads);
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)c;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, (const void*)kResident[p][f], &cfg) !=
-                cudaSuccess ||
-            n < 1)
-          all = false;
-      }
-    if (all) {
-      best = c;
-      break;
-    }
-  }
-  cudaGetLastError();
-  return best;
-}
-
-}  // namespace
-
-int resident_cluster() {
+int resident_sms() {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) dev = 0;
   std::lock_guard<std::mutex> lk(g_res_mutex);
-  if (!g_res_known[dev]) {
-    g_res_cluster[dev] = query_cluster();
-    g_res_known[dev] = true;
+  if (!g_res_sms[dev]) {
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    g_res_sms[dev] = sms > 0 ? sms : 148;
   }
-  return g_res_cluster[dev];
+  return g_res_sms[dev];
 }
 
-uint32_t resident_units_per_thread(const LatticeView& L) {
-  const int c = resident_cluster();
-  if (c <= 0) return 0xffffffffu;
-  const SweepGeom G = make_geom(L);
-  const uint32_t threads = (uint32_t)c * kResThreads;
-  return (G.units + threads - 1) / threads;
+}  // namespace
+
+// Lattice of a pass's counts in 26 bits (fewer than 2^27 sites).
+bool resident_fits(const LatticeView& L) {
+  return 2 * (uint64_t)make_geom(L).units < (1ull << kCountBits);
 }
 
-int launch_resident_sweeps(const LatticeView& L, const Coupling& cp, uint32_t key0,
-                           uint32_t key1, uint32_t replica, Control* ctl, int nsweeps,
-                           cudaStream_t stream) {
-  const int c = resident_cluster();
-  if (c <= 0) return -1;
+namespace {
+
+// One unit per thread: see OwnUnit.
+bool one_unit_each(const LatticeView& L, uint32_t units) {
+  return units <= (uint32_t)resident_sms() * kResThreads && (L.ni % 4 == 0 || !L.periodic);
+}
+
+}  // namespace
+
+// Against a launch per pass: always where a thread holds one unit.  Beyond
+// that the barrier still saves about 1 us per pass, but the loops' coherent
+// loads cost the units more than the read-only ones do: with periodic
+// boundaries and unpadded rows it pays up to 200^3 (2 M units; 79.9 against
+// 85.2 us, but 174.7 against 164.6 at 256^3), with open boundaries or padded
+// rows it does not (128^3 open 28.4 against 27.1, 102^3 open 19.5 against 17.7).
+bool resident_pays(const LatticeView& L) {
+  const uint32_t units = make_geom(L).units;
+  return one_unit_each(L, units) || (L.periodic && L.ni % 4 == 0 && units <= (1u << 21));
+}
+
+cudaError_t launch_resident_sweeps(const LatticeView& L, const Coupling& cp, uint32_t key0,
+                                   uint32_t key1, uint32_t replica, Control* ctl,
+                                   unsigned long long* words, int nsweeps, cudaStream_t stream) {
   ResidentArgs A;
   A.L = L;
   A.G = make_geom(L);
-  const uint32_t threads = (uint32_t)c * kResThreads;
+  const uint32_t sms = (uint32_t)resident_sms();
   const bool full = L.ni % 4 == 0;
+  const bool own = one_unit_each(L, A.G.units);
+  // Up to 256 units (two warps per scheduler) one CTA, whose barrier is its
+  // own; else the units spread over the SMs in CTAs of whole warps.
+  const uint32_t share = A.G.units <= 256 ? A.G.units : (A.G.units + sms - 1) / sms;
+  const uint32_t block = std::min<uint32_t>(kResThreads, (share + 31) / 32 * 32);
+  const uint32_t ctas =
+      std::min((A.G.units + block - 1) / block, sms * (uint32_t)(kResThreads / block));
   const uint32_t ncols = A.G.Q * (uint32_t)L.nj;
   uint32_t seg = 0;
-  if (full) walk_pass_cost(A.G.units, ncols, (uint32_t)L.nk, true, threads, -1, &seg);
+  if (full && !own)
+    walk_pass_cost(A.G.units, ncols, (uint32_t)L.nk, true, ctas * block, -1, &seg);
   A.W = make_walk(A.G, L, seg ? seg : 1);
-  const int form = seg ? 2 : (full ? 1 : 0);
+  const int form = own ? 3 : (seg ? 2 : (full ? 1 : 0));
   A.cp = cp;
   A.keys = philox_keys(key0, key1);
   A.replica = replica;
-  A.nct = (uint32_t)c;
   A.ctl = ctl;
+  A.words = words;
   A.nsweeps = nsweeps;
+  A.wait_limit = kWaitLimit;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)c);
-  cfg.blockDim = dim3(kResThreads);
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(block);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)c;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kResident[L.periodic ? 1 : 0][form], A) == cudaSuccess ? 0 : -1;
+  return cudaLaunchKernelEx(&cfg, kResident[L.periodic ? 1 : 0][form], A);
 }
 
 }  // namespace chll

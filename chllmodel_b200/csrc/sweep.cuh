@@ -10,8 +10,8 @@ namespace chll {
 // stream capture) and one half-sweep (pass = kPassDir0..kPassSpin1).
 void sweep_prepare();
 // Sweep form: the two-pass fused sweep, the fused passes of a chunk in one
-// cluster launch (resident.cu; auto picks it where each of its threads walks
-// at most one unit per pass, else the fused sweep), or the reference's four
+// cooperative launch (resident.cu; auto picks it where resident_pays, else the
+// fused sweep), or the reference's four
 // half-sweeps with the direct kernel or the staged kernel (shared-memory
 // tiles by bulk copies).  All give the same chain.  Single half-sweeps
 // (chll_lattice_pass) use the direct kernel unless staged is chosen.
@@ -46,16 +46,17 @@ void launch_fused_pass(const LatticeView& L, const SweepGeom& G, int bmode, cons
 void launch_control_update(Control* ctl, int phase, cudaStream_t stream);
 
 // resident.cu: nsweeps fused sweeps of a whole lattice (A0 B (A B)... F, the
-// same chain and control block as the fused passes) in one launch of one
-// thread-block cluster whose CTAs meet at the cluster barrier between passes.
-// resident_cluster: CTAs of that cluster on this device (0: none fits);
-// resident_units_per_thread: units each of its threads walks per pass.
-// The launcher returns 0, or -1 if the launch failed.
-int resident_cluster();
-uint32_t resident_units_per_thread(const LatticeView& L);
-int launch_resident_sweeps(const LatticeView& L, const Coupling& cp, uint32_t key0,
-                           uint32_t key1, uint32_t replica, Control* ctl, int nsweeps,
-                           cudaStream_t stream);
+// same chain and control block as the fused passes) in one cooperative launch
+// whose CTAs meet at a grid barrier between passes.  words: kResidentWordBytes
+// of device memory, zero before the first launch (a launch leaves them zero).
+// resident_fits: the lattice's counts fit the words; resident_pays: the form
+// is faster than the fused passes' launches.
+constexpr size_t kResidentWordBytes = 3 * 128;
+bool resident_fits(const LatticeView& L);
+bool resident_pays(const LatticeView& L);
+cudaError_t launch_resident_sweeps(const LatticeView& L, const Coupling& cp, uint32_t key0,
+                                   uint32_t key1, uint32_t replica, Control* ctl,
+                                   unsigned long long* words, int nsweeps, cudaStream_t stream);
 
 // layout.cu: natural-order (F-order, i fastest) <-> red/black float4.
 void launch_pack_f64(const LatticeView& L, const double* nx, const double* ny, const double* nz,

@@ -69,12 +69,14 @@ class Lattice:
         check(self._L.chll_lattice_set_stream(self._h, ct.c_void_p(stream_ptr or 0)))
 
     def set_kernel(self, kind: str) -> None:
-        """Sweep form: 'auto' ('resident' up to about 32^3, else 'fused'),
+        """Sweep form: 'auto' ('resident' where it is the faster one: up to
+        one unit of two sites per GPU thread, about 66^3, and periodic lattices
+        up to 200^3; else 'fused'),
         'fused' (two passes per sweep),
         'direct' (the reference's four half-sweeps, neighbours from global
         memory), 'staged' (four half-sweeps from shared-memory row tiles) or
-        'resident' (the fused passes of a whole chunk in one thread-block
-        cluster launch, for small lattices).  All give the same chain bit for
+        'resident' (the fused passes of a whole chunk in one cooperative
+        launch; lattices of 2^27 sites and more take the fused passes).  All give the same chain bit for
         bit."""
         code = {"auto": 0, "direct": 1, "staged": 2, "fused": 3, "resident": 4}[kind]
         check(self._L.chll_lattice_set_kernel(self._h, code))
