@@ -18,6 +18,7 @@ LIB_PATH = os.path.join(HERE, "libchll_mod.so")
 CHLL_OK, CHLL_EINVAL, CHLL_ECUDA, CHLL_ENOMEM, CHLL_EDEVICE, CHLL_ERANGE = range(6)
 CHLL_OPEN, CHLL_PERIODIC = 0, 1
 ROW_LEN = 16
+GRAD_WORK = 2368  # CHLL_GRAD_WORK
 ROW_ETOT, ROW_ETA, ROW_PACCEPT, ROW_FACCEPT, ROW_D = 0, 1, 2, 3, 4
 ROW_ENERGY, ROW_SUM_S, ROW_QXX, ROW_ETOT_SUM, ROW_STEP, ROW_NSITES = 5, 6, 7, 13, 14, 15
 
@@ -30,7 +31,8 @@ EXPORTS = (
     "chll_lattice_storage", "chll_lattice_set_control", "chll_lattice_get_control",
     "chll_lattice_sweep", "chll_lattice_pass", "chll_lattice_observe",
     "chll_lattice_energy_grad", "chll_lattice_reserve_rows", "chll_lattice_measure",
-    "chll_lattice_read_rows", "chll_energy_grad_noalloc", "chll_lattice_quench",
+    "chll_lattice_read_rows", "chll_energy_grad_noalloc",
+    "chll_energy_grad_natural", "chll_lattice_quench",
     "chll_lattice_set_kernel", "chll_lattice_shell_corr", "chll_lattice_projection",
     "chll_lattice_create_slab", "chll_lattice_slab_plane", "chll_lattice_counters",
     "chll_lattice_control_update", "chll_lattice_slab_set_peers", "chll_lattice_slab_push",
@@ -190,6 +192,9 @@ def _declare(L: ct.CDLL) -> None:
     L.chll_energy_grad_noalloc.argtypes = [vp, vp, i32, i32, i32, i32, P(Coupling), i32, vp, vp,
                                            vp]
     L.chll_energy_grad_noalloc.restype = i32
+    L.chll_energy_grad_natural.argtypes = [vp, vp, i32, i32, i32, i32, P(Coupling), i32, vp, vp,
+                                           vp, vp, vp]
+    L.chll_energy_grad_natural.restype = i32
     L.chll_batch_create.argtypes = [P(ReplicaSpec), i32, P(vp)]
     L.chll_batch_create.restype = i32
     L.chll_batch_destroy.argtypes = [vp]

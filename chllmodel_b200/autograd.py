@@ -3,10 +3,10 @@
 ``lattice_energy(n, s, eps, K, h, shape, boundary)`` returns the FP64 total
 energy of a lattice whose directors ``n`` (N x 3, FP32, CUDA, natural order
 i fastest) and chiralities ``s`` (N, +-1) are torch tensors; its backward
-pass comes from the adjoint kernel (``energy_grad_unit_kernel``: dE/dn for every site, plus
-dE/deps, dE/dK, dE/dh in FP64), not from autograd tracing.  The Metropolis
-sweep itself is not differentiated: acceptance stays exactly the reference's
-rule (chll_mod.f90:188-200).
+pass comes from the adjoint kernel (``natural_grad_kernel``, on the tensors as
+they are: dE/dn for every site, plus dE/deps, dE/dK, dE/dh in FP64), not from
+autograd tracing.  The Metropolis sweep itself is not differentiated:
+acceptance stays exactly the reference's rule (chll_mod.f90:188-200).
 
 ``quench`` runs the zero-temperature gradient descent on the device, and
 ``coupling_sensitivities`` returns dE/d(eps, K, h) of a lattice state.
@@ -14,31 +14,36 @@ This module is the only place the package uses torch on the compute side.
 """
 from __future__ import annotations
 
+import ctypes as ct
+
 import torch
 
 from . import _lib
+from ._lib import Coupling
 from .lattice import Lattice, coupling
 
-_cache: dict = {}
 
-
-def _lattice(shape, boundary, device) -> Lattice:
-    key = (tuple(int(x) for x in shape), boundary, int(device))
-    lat = _cache.get(key)
-    if lat is None:
-        with torch.cuda.device(device):
-            lat = Lattice(*key[0], boundary=boundary)
-        _cache[key] = lat
-    return lat
-
-
-def _stream_handle() -> int:
-    return _lib.torch_stream_handle()
-
-
-def _pack(n: torch.Tensor, s: torch.Tensor) -> torch.Tensor:
-    return torch.cat([n.detach().to(torch.float32), s.detach().to(torch.float32).reshape(-1, 1)],
-                     dim=1).contiguous()
+def _natural(n, s, eps, K, h, shape, boundary, project, want_grad, energy, derivs):
+    """The adjoint of CUDA tensors n (N, 3) and s (N,) on n's device, enqueued
+    on its current stream: E into energy, dE/d(eps, K, h) into derivs (FP64),
+    and the gradient (N, 3), FP32, returned if wanted."""
+    ni, nj, nk = (int(x) for x in shape)
+    if boundary not in ("open", "periodic"):
+        raise ValueError("boundary must be 'open' or 'periodic'")
+    if s.device != n.device:
+        raise RuntimeError(f"n and s must be on one device (got {n.device} and {s.device})")
+    n32 = n.detach().to(torch.float32).contiguous()
+    s32 = s.detach().to(torch.float32).contiguous()
+    grad = torch.empty_like(n32) if want_grad else None
+    work = torch.empty(_lib.GRAD_WORK, dtype=torch.float64, device=n.device)
+    cp = Coupling(0.0, float(K), float(h), float(eps))
+    with torch.cuda.device(n.device):
+        _lib.check(_lib.load().chll_energy_grad_natural(
+            n32.data_ptr(), s32.data_ptr(), ni, nj, nk,
+            _lib.CHLL_PERIODIC if boundary == "periodic" else _lib.CHLL_OPEN, ct.byref(cp),
+            int(bool(project)), grad.data_ptr() if want_grad else None, energy.data_ptr(),
+            derivs.data_ptr(), work.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    return grad
 
 
 class LatticeEnergy(torch.autograd.Function):
@@ -49,26 +54,26 @@ class LatticeEnergy(torch.autograd.Function):
         N = int(shape[0]) * int(shape[1]) * int(shape[2])
         if n.shape != (N, 3) or s.numel() != N:
             raise ValueError(f"n must be ({N}, 3) and s ({N},) for lattice {tuple(shape)}")
-        lat = _lattice(shape, boundary, n.device.index or 0)
-        lat.set_stream(_stream_handle())
-        packed = _pack(n, s)
-        lat.upload_f4(packed.data_ptr())
-        grad = torch.empty((N, 4), dtype=torch.float32, device=n.device)
-        cp = coupling(0.0, float(K), float(h), float(eps))
-        _, out4 = lat.energy_grad(cp, project=False, grad_ptr=grad.data_ptr())
-        dev = n.device
-        ctx.save_for_backward(grad[:, :3].to(n.dtype),
-                              torch.tensor(out4[1:], dtype=torch.float64, device=dev))
-        return torch.tensor(out4[0], dtype=torch.float64, device=dev)
+        energy = torch.empty((), dtype=torch.float64, device=n.device)
+        derivs = torch.empty(3, dtype=torch.float64, device=n.device)
+        grad = _natural(n, s, eps, K, h, shape, boundary, False, ctx.needs_input_grad[0], energy,
+                        derivs)
+        ctx.on_host = not (eps.is_cuda or K.is_cuda or h.is_cuda)
+        ctx.save_for_backward(grad.to(n.dtype) if grad is not None else None, derivs)
+        return energy
 
     @staticmethod
     def backward(ctx, g_out):
         grad_n, d_couplings = ctx.saved_tensors
         g = g_out.to(torch.float64)
         gn = (g.to(grad_n.dtype) * grad_n) if ctx.needs_input_grad[0] else None
-        ge = g * d_couplings[0] if ctx.needs_input_grad[2] else None
-        gk = g * d_couplings[1] if ctx.needs_input_grad[3] else None
-        gh = g * d_couplings[2] if ctx.needs_input_grad[4] else None
+        ge = gk = gh = None
+        if any(ctx.needs_input_grad[2:5]):
+            gc = g * d_couplings
+            if ctx.on_host:
+                gc = gc.cpu()  # one copy for the three
+            ge, gk, gh = (v if need else None
+                          for v, need in zip(gc.unbind(), ctx.needs_input_grad[2:5]))
         return gn, None, ge, gk, gh, None, None
 
 
@@ -81,25 +86,30 @@ def lattice_energy(n, s, eps, K, h, shape, boundary="periodic"):
     return LatticeEnergy.apply(n, s, as_t(eps), as_t(K), as_t(h), tuple(shape), boundary)
 
 
+def _on_gpu(n: torch.Tensor, s: torch.Tensor, shape):
+    """n and s checked against the lattice, on a GPU (host tensors are copied)."""
+    N = int(shape[0]) * int(shape[1]) * int(shape[2])
+    if n.ndim != 2 or n.shape[1] != 3 or n.shape[0] < N or s.numel() != n.shape[0]:
+        raise ValueError(f"n must be ({N}, 3) and s ({N},) for lattice {tuple(shape)}")
+    if not n.is_cuda and not s.is_cuda:
+        return n.to("cuda:0"), s.to("cuda:0")
+    return n, s
+
+
 def tangent_gradient(n, s, eps, K, h, shape, boundary="periodic") -> torch.Tensor:
     """(I - n n^T) dE/dn: the torque direction on every director."""
-    N = n.shape[0]
-    lat = _lattice(shape, boundary, n.device.index or 0)
-    lat.set_stream(_stream_handle())
-    lat.upload_f4(_pack(n, s).data_ptr())
-    grad = torch.empty((N, 4), dtype=torch.float32, device=n.device)
-    lat.energy_grad(coupling(0.0, float(K), float(h), float(eps)), project=True,
-                    grad_ptr=grad.data_ptr())
-    return grad[:, :3]
+    gn, gs = _on_gpu(n, s, shape)
+    out = torch.empty(4, dtype=torch.float64, device=gn.device)
+    return _natural(gn, gs, eps, K, h, shape, boundary, True, True, out, out[1:]).to(n.device)
 
 
 def coupling_sensitivities(n, s, eps, K, h, shape, boundary="periodic") -> dict:
     """E and dE/d(eps, K, h) of a lattice state, FP64."""
-    lat = _lattice(shape, boundary, n.device.index or 0)
-    lat.set_stream(_stream_handle())
-    lat.upload_f4(_pack(n, s).data_ptr())
-    _, out4 = lat.energy_grad(coupling(0.0, float(K), float(h), float(eps)))
-    return {"E": out4[0], "dE_deps": out4[1], "dE_dK": out4[2], "dE_dh": out4[3]}
+    gn, gs = _on_gpu(n, s, shape)
+    out = torch.empty(4, dtype=torch.float64, device=gn.device)
+    _natural(gn, gs, eps, K, h, shape, boundary, False, False, out, out[1:])
+    E, de, dk, dh = out.cpu().numpy()
+    return {"E": E, "dE_deps": de, "dE_dK": dk, "dE_dh": dh}
 
 
 def quench(lat: Lattice, eps: float, K: float, h: float, eta: float, nsteps: int,

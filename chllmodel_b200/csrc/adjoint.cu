@@ -263,6 +263,179 @@ __global__ void __launch_bounds__(kGradThreads)
   finish_sums(acc, partials, ticket, out4);
 }
 
+// ---------------------------------------------------------------------------
+// The adjoint of caller arrays in natural order (i fastest): directors n
+// (N x 3) and chiralities s (N), FP32, as the autograd wrapper has them.
+//
+// The path through a red/black lattice read and wrote the state five more times
+// (records packed together, a cleared lattice, the red/black copy, the
+// gradient unpacked and its fourth column cut off); here a call reads each
+// array once and writes the (N x 3) gradient once: 28 B per site.
+//
+// A thread walks one column (i, j) over a run of planes and carries its site
+// and the two z neighbours in registers, with the FP64 forms of its site from
+// the step before (the conversions are a quarter-rate pipe: 12 per site instead
+// of 16).  A warp holds 32 consecutive columns of the flattened plane, so a
+// load of a component is three whole lines per warp whatever ni is, and the x
+// neighbours come from the lanes beside; the ends of a warp or a row load
+// theirs.
+// ---------------------------------------------------------------------------
+struct NaturalGeom {
+  uint32_t ni, nj, nk;
+  uint32_t plane;      // ni * nj, columns
+  uint32_t cols;       // columns rounded up to whole warps
+  uint32_t seg, nseg;  // planes per task, tasks per column
+  int periodic;
+};
+
+struct Site64 {
+  double x, y, z, s;
+};
+
+__device__ __forceinline__ Site64 to64(const float4& v) {
+  return {(double)v.x, (double)v.y, (double)v.z, (double)v.w};
+}
+
+__device__ __forceinline__ float4 natural_site(const float* __restrict__ n,
+                                               const float* __restrict__ s, size_t e) {
+  return make_float4(__ldg(n + 3 * e), __ldg(n + 3 * e + 1), __ldg(n + 3 * e + 2), __ldg(s + e));
+}
+
+// One forward bond's FP64 terms (as site_sums).
+template <int AXIS>
+__device__ __forceinline__ void bond_sums64(const Site64& n, const Site64& b,
+                                            const CouplingD& cd, double acc[4]) {
+  const double c = n.x * b.x + n.y * b.y + n.z * b.z;
+  const double X = AXIS == 0 ? n.y * b.z - n.z * b.y
+                 : AXIS == 1 ? n.z * b.x - n.x * b.z
+                             : n.x * b.y - n.y * b.x;
+  const double sbar = 0.5 * (n.s + b.s);
+  const double nem = 1.0 - c * c;
+  const double chi = -c * X * sbar;
+  acc[0] += cd.eps * nem + cd.K * chi;
+  acc[1] += nem;
+  acc[2] += chi;
+}
+
+template <bool GRAD>
+__global__ void __launch_bounds__(kGradThreads)
+    natural_grad_kernel(NaturalGeom G, const float* __restrict__ n, const float* __restrict__ s,
+                        CouplingD cd, float* __restrict__ grad, int project,
+                        double* __restrict__ partials) {
+  Coupling cp;  // FP32 couplings of the per-site gradient
+  cp.eps = (float)cd.eps;
+  cp.K = (float)cd.K;
+  cp.g = (float)cd.g;
+  cp.inv_kT = 0.f;
+  const bool per = G.periodic;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t ntasks = (uint64_t)G.cols * G.nseg;
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};  // E, dE/deps, dE/dK, dE/dh
+  for (uint64_t t = blockIdx.x * (uint64_t)kGradThreads + threadIdx.x; t < ntasks;
+       t += (uint64_t)gridDim.x * kGradThreads) {
+    // whole warps share a segment: the same planes in every lane
+    const uint32_t sg = (uint32_t)(t / G.cols);
+    const uint32_t p = (uint32_t)(t - (uint64_t)sg * G.cols);
+    const bool has = p < G.plane;
+    const uint32_t j = p / G.ni, i = p - j * G.ni;
+    const uint32_t k0 = sg * G.seg, k1 = min(k0 + G.seg, G.nk);
+    const bool hxp = has && (per || i + 1 < G.ni), hxm = has && (per || i > 0);
+    const bool hyp = has && (per || j + 1 < G.nj), hym = has && (per || j > 0);
+    // columns of the in-plane neighbours
+    const uint32_t pxp = i + 1 < G.ni ? p + 1 : p - i;
+    const uint32_t pxm = i > 0 ? p - 1 : p + (G.ni - 1);
+    const uint32_t pyp = j + 1 < G.nj ? p + G.ni : i;
+    const uint32_t pym = j > 0 ? p - G.ni : p + (G.nj - 1) * G.ni;
+    // whose x neighbours are not in the lanes beside
+    const bool lxp = hxp && (lane == 31 || i + 1 == G.ni);
+    const bool lxm = hxm && (lane == 0 || i == 0);
+    size_t base = (size_t)k0 * G.plane;  // first site of the plane
+    float4 c = has ? natural_site(n, s, base + p) : zero;
+    float4 zm = zero;
+    if (GRAD && has && (per || k0 > 0))
+      zm = natural_site(n, s, (k0 > 0 ? base - G.plane : (size_t)(G.nk - 1) * G.plane) + p);
+    Site64 c64 = to64(c);
+    for (uint32_t k = k0; k < k1; ++k, base += G.plane) {
+      const bool hzp = has && (per || k + 1 < G.nk);
+      const float4 zp =
+          hzp ? natural_site(n, s, (k + 1 < G.nk ? base + G.plane : 0) + p) : zero;
+      const float4 yp = hyp ? natural_site(n, s, base + pyp) : zero;
+      const float4 ym = GRAD && hym ? natural_site(n, s, base + pym) : zero;
+      float4 xp, xm = zero;
+      xp.x = __shfl_down_sync(0xffffffffu, c.x, 1);
+      xp.y = __shfl_down_sync(0xffffffffu, c.y, 1);
+      xp.z = __shfl_down_sync(0xffffffffu, c.z, 1);
+      xp.w = __shfl_down_sync(0xffffffffu, c.w, 1);
+      if (lxp) xp = natural_site(n, s, base + pxp);
+      if (!hxp) xp = zero;
+      if (GRAD) {
+        xm.x = __shfl_up_sync(0xffffffffu, c.x, 1);
+        xm.y = __shfl_up_sync(0xffffffffu, c.y, 1);
+        xm.z = __shfl_up_sync(0xffffffffu, c.z, 1);
+        xm.w = __shfl_up_sync(0xffffffffu, c.w, 1);
+        if (lxm) xm = natural_site(n, s, base + pxm);
+        if (!hxm) xm = zero;
+      }
+      const Site64 zp64 = to64(zp);
+      if (has) {
+        if (GRAD) {
+          const float4 g = site_grad(c, xp, xm, yp, ym, zp, zm, cp, project);
+          float* out = grad + 3 * (base + p);
+          out[0] = g.x;
+          out[1] = g.y;
+          out[2] = g.z;
+        }
+        if (hxp) bond_sums64<0>(c64, to64(xp), cd, acc);
+        if (hyp) bond_sums64<1>(c64, to64(yp), cd, acc);
+        if (hzp) bond_sums64<2>(c64, zp64, cd, acc);
+        acc[0] -= cd.g * c64.s;
+        acc[3] -= c64.s;
+      }
+      zm = c;
+      c = zp;
+      c64 = zp64;
+    }
+  }
+  __shared__ double s_part[kGradThreads / 32][4];
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const double v = warp_sum(acc[m]);
+    if (lane == 0) s_part[threadIdx.x >> 5][m] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    double v = 0.0;
+    for (int w = 0; w < kGradThreads / 32; ++w) v += s_part[w][threadIdx.x];
+    partials[(size_t)blockIdx.x * 4 + threadIdx.x] = v;
+  }
+}
+
+// The CTA partials summed in a fixed order: E, then dE/d(eps, K, h).
+__global__ void __launch_bounds__(kGradThreads)
+    natural_sums_kernel(const double* __restrict__ partials, uint32_t rows,
+                        double* __restrict__ energy, double* __restrict__ derivs) {
+  __shared__ double s_part[kGradThreads / 32][4];
+  double v[4] = {0.0, 0.0, 0.0, 0.0};
+  wait_prerequisite_grids();
+  for (uint32_t b = threadIdx.x; b < rows; b += kGradThreads) {
+#pragma unroll
+    for (int m = 0; m < 4; ++m) v[m] += __ldcg(&partials[(size_t)b * 4 + m]);
+  }
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const double w = warp_sum(v[m]);
+    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5][m] = w;
+  }
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    double t = 0.0;
+    for (int w = 0; w < kGradThreads / 32; ++w) t += s_part[w][threadIdx.x];
+    if (threadIdx.x == 0) *energy = t;
+    else derivs[threadIdx.x - 1] = t;
+  }
+}
+
 // One site of a zero-temperature gradient quench: n moves against its
 // tangent-projected energy gradient, n <- normalise(n - eta (I - n n^T) dE/dn),
 // with the neighbours nb (+x, -x, +y, -y, +z, -z) held fixed.
@@ -348,6 +521,56 @@ void launch_quench_pass(const LatticeView& L, const CouplingD& cd, float eta, in
     if (colour == 0) quench_pass_kernel<0, false><<<nb, kGradThreads, 0, stream>>>(L, G, cp, eta);
     else quench_pass_kernel<1, false><<<nb, kGradThreads, 0, stream>>>(L, G, cp, eta);
   }
+}
+
+cudaError_t launch_natural_grad(int ni, int nj, int nk, int periodic, const float* n,
+                                const float* s, const CouplingD& cd, float* grad, int project,
+                                double* partials, double* energy, double* derivs,
+                                cudaStream_t stream) {
+  static std::atomic<int> resident[2][16];
+  const uint32_t ctas = (uint32_t)std::min(
+      kGradMaxBlocks, grad ? resident_ctas(natural_grad_kernel<true>, resident[1])
+                           : resident_ctas(natural_grad_kernel<false>, resident[0]));
+  NaturalGeom G;
+  G.ni = (uint32_t)ni;
+  G.nj = (uint32_t)nj;
+  G.nk = (uint32_t)nk;
+  G.plane = G.ni * G.nj;
+  G.cols = (G.plane + 31) / 32 * 32;
+  G.periodic = periodic;
+  // Planes per task: the fewest steps on the busiest thread, a task's first
+  // loads counted as half a step.
+  double best = 1e300;
+  for (uint32_t seg = 1; seg <= G.nk; ++seg) {
+    const uint64_t tasks = (uint64_t)G.cols * ((G.nk + seg - 1) / seg);
+    const uint64_t threads = (uint64_t)ctas * kGradThreads;
+    const double cost = (double)((tasks + threads - 1) / threads) * (seg + 0.5);
+    if (cost < best) {
+      best = cost;
+      G.seg = seg;
+    }
+  }
+  G.nseg = (G.nk + G.seg - 1) / G.seg;
+  const uint64_t need = ((uint64_t)G.cols * G.nseg + kGradThreads - 1) / kGradThreads;
+  const uint32_t blocks = (uint32_t)std::min<uint64_t>(need, ctas);
+  if (grad)
+    natural_grad_kernel<true><<<blocks, kGradThreads, 0, stream>>>(G, n, s, cd, grad, project,
+                                                                   partials);
+  else
+    natural_grad_kernel<false><<<blocks, kGradThreads, 0, stream>>>(G, n, s, cd, nullptr, 0,
+                                                                    partials);
+  // scheduled while the kernel before it drains
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1);
+  cfg.blockDim = dim3(kGradThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, natural_sums_kernel, (const double*)partials, blocks, energy,
+                            derivs);
 }
 
 void launch_energy_grad(const LatticeView& L, const CouplingD& cp, float4* grad_rb, int project,

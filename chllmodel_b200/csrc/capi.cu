@@ -405,10 +405,8 @@ int observe_impl(chll_lattice* L, const chll::CouplingD& cp, double* dev_row, lo
   return CHLL_OK;
 }
 
-int create_impl(int ni, int nj, int nk, int boundary, chll_lattice** out, int slab_z0 = -1,
-                int slab_nk = 0) {
-  if (!out) return fail(CHLL_EINVAL, "lattice_create: null output pointer");
-  *out = nullptr;
+// Sizes and boundary of a lattice (or a slab of it).
+int check_lattice(int ni, int nj, int nk, int boundary, int slab_z0 = -1, int slab_nk = 0) {
   if (ni < 1 || nj < 1 || nk < 1)
     return fail(CHLL_EINVAL, "lattice dims must be >= 1 (got %d %d %d)", ni, nj, nk);
   if (boundary != CHLL_OPEN && boundary != CHLL_PERIODIC)
@@ -432,6 +430,14 @@ int create_impl(int ni, int nj, int nk, int boundary, chll_lattice** out, int sl
                 "lattice too large: %lld slots per colour (rows padded to a multiple of 4 "
                 "sites%s); the limit is 2^31",
                 slots, slab_z0 >= 0 ? ", halo planes included" : "");
+  return CHLL_OK;
+}
+
+int create_impl(int ni, int nj, int nk, int boundary, chll_lattice** out, int slab_z0 = -1,
+                int slab_nk = 0) {
+  if (!out) return fail(CHLL_EINVAL, "lattice_create: null output pointer");
+  *out = nullptr;
+  CHLL_TRY(check_lattice(ni, nj, nk, boundary, slab_z0, slab_nk));
   CHLL_TRY(check_device());
   chll::sweep_prepare();
 
@@ -441,8 +447,7 @@ int create_impl(int ni, int nj, int nk, int boundary, chll_lattice** out, int sl
   L->nk = nk;
   L->hx = chll::padded_ni(ni) / 2;
   L->periodic = boundary;
-  L->nsites = n;
-  L->ctl_sites = n;
+  L->nsites = L->ctl_sites = (long long)ni * nj * nk;
   if (slab_z0 >= 0) {
     L->slab = 1;
     L->z0 = slab_z0;
@@ -981,6 +986,29 @@ int chll_lattice_energy_grad(chll_lattice* L, const chll_coupling* c, float* gra
   return ok();
 }
 
+int chll_energy_grad_natural(const float* n, const float* s, int ni, int nj, int nk, int boundary,
+                             const chll_coupling* c, int project, float* grad, double* energy,
+                             double* derivs, double* work, void* stream) {
+  if (!n || !s || !c || !energy || !derivs || !work)
+    return fail(CHLL_EINVAL, "energy_grad_natural: null argument");
+  CHLL_TRY(check_lattice(ni, nj, nk, boundary));
+  CHLL_TRY(check_device());
+  for (const void* p : {(const void*)n, (const void*)s, (const void*)energy, (const void*)derivs,
+                        (const void*)work, (const void*)grad}) {
+    if (p && !is_device_ptr(p))
+      return fail(CHLL_EINVAL, "energy_grad_natural: arrays must be device memory");
+    const uintptr_t size = p == n || p == s || p == grad ? sizeof(float) : sizeof(double);
+    if ((uintptr_t)p % size)
+      return fail(CHLL_EINVAL, "energy_grad_natural: arrays must be aligned to their elements");
+  }
+  const cudaError_t e = chll::launch_natural_grad(ni, nj, nk, boundary, n, s, make_coupling_d(*c),
+                                                  grad, project, work, energy, derivs,
+                                                  (cudaStream_t)stream);
+  if (e != cudaSuccess)
+    return fail(CHLL_ECUDA, "energy_grad_natural: %s", cudaGetErrorString(e));
+  return ok();
+}
+
 int chll_lattice_shell_corr(chll_lattice* L, int nshells, int wrap, double* gn, double* gs,
                             double* counts) {
   if (!L || !gn || !gs || !counts) return fail(CHLL_EINVAL, "shell_corr: null argument");
@@ -1113,6 +1141,7 @@ int chll_lattice_slab_plane(chll_lattice* L, int colour, int which, void** ptr, 
   return ok();
 }
 
+static_assert(CHLL_GRAD_WORK == chll::kGradMaxBlocks * 4, "four sums per adjoint CTA");
 static_assert(offsetof(Control, nflip) == offsetof(Control, nacc) + sizeof(unsigned long long),
               "the two pass counters are read as one array");
 

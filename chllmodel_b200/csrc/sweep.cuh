@@ -82,6 +82,12 @@ void launch_observables(const LatticeView& L, const MomentGeom& M, const Couplin
 void launch_energy_grad(const LatticeView& L, const CouplingD& cp, float4* grad_rb, int project,
                         double* partials, unsigned int* ticket, double* out4,
                         cudaStream_t stream);
+// The same of natural-order arrays n (3 per site), s: the gradient (3 per site,
+// or null) and the sums E and dE/d(eps, K, h); partials: kGradMaxBlocks * 4.
+cudaError_t launch_natural_grad(int ni, int nj, int nk, int periodic, const float* n,
+                                const float* s, const CouplingD& cd, float* grad, int project,
+                                double* partials, double* energy, double* derivs,
+                                cudaStream_t stream);
 // The adjoint kernels run at most kGradMaxBlocks CTAs (grid-stride beyond
 // that), each leaving four FP64 partial sums: the partial-sum buffers of the
 // adjoint hold kGradMaxBlocks * 4 doubles on any GPU.

@@ -361,6 +361,22 @@ int chll_lattice_shell_corr(chll_lattice* lat, int nshells, int wrap, double* gn
 int chll_lattice_projection(chll_lattice* lat, const int* plane, long long* hist,
                             long long* m_min, int* nbins);
 
+/* ---- energy adjoint of arrays in natural order --------------------------- */
+
+/* The total energy of a state in the caller's device arrays, its gradient to
+ * every director and its derivatives to the couplings, without a lattice
+ * handle.  No counterpart in the reference.
+ *   n, s: device, natural order (i fastest): 3 and 1 floats per site;
+ *   grad: device, 3 floats per site (tangent-projected if project), or NULL;
+ *   energy: device, 1 double; derivs: device, 3 doubles dE/d(eps, K, h);
+ *   work: device, CHLL_GRAD_WORK doubles of scratch;
+ *   stream: cudaStream_t the work is enqueued on (asynchronous).
+ * Sizes and boundary as chll_lattice_create. */
+#define CHLL_GRAD_WORK 2368
+int chll_energy_grad_natural(const float* n, const float* s, int ni, int nj, int nk, int boundary,
+                             const chll_coupling* c, int project, float* grad, double* energy,
+                             double* derivs, double* work, void* stream);
+
 /* ---- energy adjoint without device allocation --------------------------- */
 
 /* Same results as chll_lattice_energy_grad, for callers that cannot let a
