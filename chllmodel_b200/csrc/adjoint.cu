@@ -301,20 +301,49 @@ __device__ __forceinline__ float4 natural_site(const float* __restrict__ n,
   return make_float4(__ldg(n + 3 * e), __ldg(n + 3 * e + 1), __ldg(n + 3 * e + 2), __ldg(s + e));
 }
 
-// One forward bond's FP64 terms (as site_sums).
+// One forward bond's FP64 terms: acc[0] the sum of 1 - c^2, acc[1] that of
+// c X (s + s').
 template <int AXIS>
-__device__ __forceinline__ void bond_sums64(const Site64& n, const Site64& b,
-                                            const CouplingD& cd, double acc[4]) {
+__device__ __forceinline__ void bond_sums64(const Site64& n, const Site64& b, double acc[3]) {
   const double c = n.x * b.x + n.y * b.y + n.z * b.z;
   const double X = AXIS == 0 ? n.y * b.z - n.z * b.y
                  : AXIS == 1 ? n.z * b.x - n.x * b.z
                              : n.x * b.y - n.y * b.x;
-  const double sbar = 0.5 * (n.s + b.s);
-  const double nem = 1.0 - c * c;
-  const double chi = -c * X * sbar;
-  acc[0] += cd.eps * nem + cd.K * chi;
-  acc[1] += nem;
-  acc[2] += chi;
+  acc[0] += 1.0 - c * c;
+  acc[1] += c * X * (n.s + b.s);
+}
+
+// One bond's dE/dn_i as coefficients of the neighbour and of b x e_a:
+// (-2 eps c + w X) b + (w c) (b x e_a) with w = sigma K sbar, in half the
+// instructions of bond_grad's term by term form (m2eps = -2 eps, kw = sigma
+// K / 2).  Adds the second part to g and returns the first one's coefficient,
+// so that the smaller parts are summed before the larger ones.
+template <int AXIS>
+__device__ __forceinline__ float bond_grad_part(const float4& n, const float4& b, float m2eps,
+                                                float kw, float& gx, float& gy, float& gz) {
+  const float c = n.x * b.x + n.y * b.y + n.z * b.z;
+  const float X = AXIS == 0 ? n.y * b.z - n.z * b.y
+                : AXIS == 1 ? n.z * b.x - n.x * b.z
+                            : n.x * b.y - n.y * b.x;
+  const float w = kw * (n.w + b.w), q = w * c;
+  if (AXIS == 0) {
+    gy += q * b.z;
+    gz -= q * b.y;
+  } else if (AXIS == 1) {
+    gz += q * b.x;
+    gx -= q * b.z;
+  } else {
+    gx += q * b.y;
+    gy -= q * b.x;
+  }
+  return w * X + m2eps * c;
+}
+
+__device__ __forceinline__ void add_scaled(float p, const float4& b, float& gx, float& gy,
+                                           float& gz) {
+  gx += p * b.x;
+  gy += p * b.y;
+  gz += p * b.z;
 }
 
 template <bool GRAD>
@@ -322,16 +351,12 @@ __global__ void __launch_bounds__(kGradThreads)
     natural_grad_kernel(NaturalGeom G, const float* __restrict__ n, const float* __restrict__ s,
                         CouplingD cd, float* __restrict__ grad, int project,
                         double* __restrict__ partials) {
-  Coupling cp;  // FP32 couplings of the per-site gradient
-  cp.eps = (float)cd.eps;
-  cp.K = (float)cd.K;
-  cp.g = (float)cd.g;
-  cp.inv_kT = 0.f;
+  const float m2eps = -2.f * (float)cd.eps, kw = 0.5f * (float)cd.K;
   const bool per = G.periodic;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t ntasks = (uint64_t)G.cols * G.nseg;
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};  // E, dE/deps, dE/dK, dE/dh
+  double acc[3] = {0.0, 0.0, 0.0};  // bond_sums64's two, then the sum of s
   for (uint64_t t = blockIdx.x * (uint64_t)kGradThreads + threadIdx.x; t < ntasks;
        t += (uint64_t)gridDim.x * kGradThreads) {
     // whole warps share a segment: the same planes in every lane
@@ -343,10 +368,10 @@ __global__ void __launch_bounds__(kGradThreads)
     const bool hxp = has && (per || i + 1 < G.ni), hxm = has && (per || i > 0);
     const bool hyp = has && (per || j + 1 < G.nj), hym = has && (per || j > 0);
     // columns of the in-plane neighbours
-    const uint32_t pxp = i + 1 < G.ni ? p + 1 : p - i;
-    const uint32_t pxm = i > 0 ? p - 1 : p + (G.ni - 1);
-    const uint32_t pyp = j + 1 < G.nj ? p + G.ni : i;
-    const uint32_t pym = j > 0 ? p - G.ni : p + (G.nj - 1) * G.ni;
+    const uint32_t cxp = i + 1 < G.ni ? p + 1 : p - i;
+    const uint32_t cxm = i > 0 ? p - 1 : p + (G.ni - 1);
+    const uint32_t cyp = j + 1 < G.nj ? p + G.ni : i;
+    const uint32_t cym = j > 0 ? p - G.ni : p + (G.nj - 1) * G.ni;
     // whose x neighbours are not in the lanes beside
     const bool lxp = hxp && (lane == 31 || i + 1 == G.ni);
     const bool lxm = hxm && (lane == 0 || i == 0);
@@ -360,54 +385,77 @@ __global__ void __launch_bounds__(kGradThreads)
       const bool hzp = has && (per || k + 1 < G.nk);
       const float4 zp =
           hzp ? natural_site(n, s, (k + 1 < G.nk ? base + G.plane : 0) + p) : zero;
-      const float4 yp = hyp ? natural_site(n, s, base + pyp) : zero;
-      const float4 ym = GRAD && hym ? natural_site(n, s, base + pym) : zero;
+      const float4 yp = hyp ? natural_site(n, s, base + cyp) : zero;
+      const float4 ym = GRAD && hym ? natural_site(n, s, base + cym) : zero;
       float4 xp, xm = zero;
       xp.x = __shfl_down_sync(0xffffffffu, c.x, 1);
       xp.y = __shfl_down_sync(0xffffffffu, c.y, 1);
       xp.z = __shfl_down_sync(0xffffffffu, c.z, 1);
       xp.w = __shfl_down_sync(0xffffffffu, c.w, 1);
-      if (lxp) xp = natural_site(n, s, base + pxp);
+      if (lxp) xp = natural_site(n, s, base + cxp);
       if (!hxp) xp = zero;
       if (GRAD) {
         xm.x = __shfl_up_sync(0xffffffffu, c.x, 1);
         xm.y = __shfl_up_sync(0xffffffffu, c.y, 1);
         xm.z = __shfl_up_sync(0xffffffffu, c.z, 1);
         xm.w = __shfl_up_sync(0xffffffffu, c.w, 1);
-        if (lxm) xm = natural_site(n, s, base + pxm);
+        if (lxm) xm = natural_site(n, s, base + cxm);
         if (!hxm) xm = zero;
       }
       const Site64 zp64 = to64(zp);
       if (has) {
         if (GRAD) {
-          const float4 g = site_grad(c, xp, xm, yp, ym, zp, zm, cp, project);
+          float gx = 0.f, gy = 0.f, gz = 0.f;
+          const float pxp = bond_grad_part<0>(c, xp, m2eps, -kw, gx, gy, gz);
+          const float pxm = bond_grad_part<0>(c, xm, m2eps, kw, gx, gy, gz);
+          const float pyp = bond_grad_part<1>(c, yp, m2eps, -kw, gx, gy, gz);
+          const float pym = bond_grad_part<1>(c, ym, m2eps, kw, gx, gy, gz);
+          const float pzp = bond_grad_part<2>(c, zp, m2eps, -kw, gx, gy, gz);
+          const float pzm = bond_grad_part<2>(c, zm, m2eps, kw, gx, gy, gz);
+          add_scaled(pxp, xp, gx, gy, gz);
+          add_scaled(pxm, xm, gx, gy, gz);
+          add_scaled(pyp, yp, gx, gy, gz);
+          add_scaled(pym, ym, gx, gy, gz);
+          add_scaled(pzp, zp, gx, gy, gz);
+          add_scaled(pzm, zm, gx, gy, gz);
+          if (project) {
+            const float nn = c.x * c.x + c.y * c.y + c.z * c.z;
+            const float gn = (gx * c.x + gy * c.y + gz * c.z) / nn;
+            gx -= gn * c.x;
+            gy -= gn * c.y;
+            gz -= gn * c.z;
+          }
           float* out = grad + 3 * (base + p);
-          out[0] = g.x;
-          out[1] = g.y;
-          out[2] = g.z;
+          out[0] = gx;
+          out[1] = gy;
+          out[2] = gz;
         }
-        if (hxp) bond_sums64<0>(c64, to64(xp), cd, acc);
-        if (hyp) bond_sums64<1>(c64, to64(yp), cd, acc);
-        if (hzp) bond_sums64<2>(c64, zp64, cd, acc);
-        acc[0] -= cd.g * c64.s;
-        acc[3] -= c64.s;
+        if (hxp) bond_sums64<0>(c64, to64(xp), acc);
+        if (hyp) bond_sums64<1>(c64, to64(yp), acc);
+        if (hzp) bond_sums64<2>(c64, zp64, acc);
+        acc[2] += c64.s;
       }
       zm = c;
       c = zp;
       c64 = zp64;
     }
   }
-  __shared__ double s_part[kGradThreads / 32][4];
+  __shared__ double s_part[kGradThreads / 32][3];
 #pragma unroll
-  for (int m = 0; m < 4; ++m) {
+  for (int m = 0; m < 3; ++m) {
     const double v = warp_sum(acc[m]);
     if (lane == 0) s_part[threadIdx.x >> 5][m] = v;
   }
   __syncthreads();
-  if (threadIdx.x < 4) {
-    double v = 0.0;
-    for (int w = 0; w < kGradThreads / 32; ++w) v += s_part[w][threadIdx.x];
-    partials[(size_t)blockIdx.x * 4 + threadIdx.x] = v;
+  if (threadIdx.x == 0) {
+    double v[3] = {0.0, 0.0, 0.0};
+    for (int w = 0; w < kGradThreads / 32; ++w)
+      for (int m = 0; m < 3; ++m) v[m] += s_part[w][m];
+    double* out = partials + (size_t)blockIdx.x * 4;  // E, dE/d(eps, K, h)
+    out[1] = v[0];
+    out[2] = -0.5 * v[1];
+    out[3] = -v[2];
+    out[0] = cd.eps * out[1] + cd.K * out[2] + cd.g * out[3];
   }
 }
 
