@@ -931,10 +931,7 @@ int chll_lattice_read_rows(chll_lattice* L, double* rows16, int first, int count
 int chll_lattice_observe(chll_lattice* L, const chll_coupling* c, double* row16) {
   if (!L || !c || !row16) return fail(CHLL_EINVAL, "observe: null argument");
   double* drow = L->out4 + 4;
-  Control ctl;
-  CHLL_CUDA_TRY(cudaMemcpyAsync(&ctl, L->ctl, sizeof(ctl), cudaMemcpyDeviceToHost, L->stream));
-  CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
-  CHLL_TRY(observe_impl(L, make_coupling_d(*c), drow, ctl.step - 1));
+  CHLL_TRY(observe_impl(L, make_coupling_d(*c), drow, chll::kStepOfControl));
   CHLL_CUDA_TRY(cudaMemcpyAsync(row16, drow, sizeof(double) * chll::kRowLen,
                                 cudaMemcpyDeviceToHost, L->stream));
   CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));

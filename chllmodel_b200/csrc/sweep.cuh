@@ -68,7 +68,9 @@ void launch_unpack_f4(const LatticeView& L, float4* xyzs, cudaStream_t stream);
 void launch_init_random(const LatticeView& L, uint32_t key0, uint32_t key1, uint32_t replica,
                         cudaStream_t stream, uint64_t site0 = 0);
 
-// observables.cu: FP64 moments and the measurement row.
+// observables.cu: FP64 moments and the measurement row.  step: the row's step
+// column, or kStepOfControl for the control block's last completed step.
+constexpr long long kStepOfControl = -0x7fffffffffffffffll;
 int observables_max_blocks();
 void launch_observables(const LatticeView& L, const CouplingD& cp, const Control* ctl,
                         double* partials, unsigned int* ticket, double* row, long long step,
