@@ -331,12 +331,20 @@ int sweep_impl(chll_lattice* L, const Coupling& cp, uint64_t seed, uint32_t rep,
   return CHLL_OK;
 }
 
+// A slab's halo planes, which the kernels that fill its own planes do not
+// reach.
+int clear_halos(chll_lattice* L) {
+  if (L->slab)
+    CHLL_CUDA_TRY(cudaMemsetAsync(L->lat, 0, 2 * L->per_colour * sizeof(float4), L->stream));
+  return CHLL_OK;
+}
+
 int upload_f64_impl(chll_lattice* L, const double* nx, const double* ny, const double* nz,
                     const int* s) {
   if (!nx || !ny || !nz || !s) return fail(CHLL_EINVAL, "upload: null array");
   const size_t n = (size_t)L->nsites;
   const LatticeView v = L->view();
-  CHLL_CUDA_TRY(cudaMemsetAsync(L->lat, 0, 2 * L->per_colour * sizeof(float4), L->stream));
+  CHLL_TRY(clear_halos(L));
   if (is_device_ptr(nx) && is_device_ptr(ny) && is_device_ptr(nz) && is_device_ptr(s)) {
     chll::launch_pack_f64(v, nx, ny, nz, s, L->stream);
   } else {
@@ -779,7 +787,7 @@ int chll_lattice_sync(chll_lattice* L) {
 
 int chll_lattice_init_random(chll_lattice* L, uint64_t seed, uint32_t replica) {
   if (!L) return fail(CHLL_EINVAL, "null lattice");
-  CHLL_CUDA_TRY(cudaMemsetAsync(L->lat, 0, 2 * L->per_colour * sizeof(float4), L->stream));
+  CHLL_TRY(clear_halos(L));
   // a slab draws the values of its global sites
   chll::launch_init_random(L->view(), seed_lo(seed), seed_hi(seed), replica, L->stream,
                            (uint64_t)L->ni * L->nj * L->z0);
@@ -804,7 +812,7 @@ int chll_lattice_download_f64(chll_lattice* L, double* nx, double* ny, double* n
 int chll_lattice_upload_f4(chll_lattice* L, const float* xyzs) {
   if (!L || !xyzs) return fail(CHLL_EINVAL, "upload_f4: null argument");
   const size_t n = (size_t)L->nsites;
-  CHLL_CUDA_TRY(cudaMemsetAsync(L->lat, 0, 2 * L->per_colour * sizeof(float4), L->stream));
+  CHLL_TRY(clear_halos(L));
   const float4* src = (const float4*)xyzs;
   if (!is_device_ptr(xyzs)) {
     CHLL_TRY(ensure_staging(L, n * sizeof(float4)));
