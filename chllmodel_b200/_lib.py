@@ -34,6 +34,7 @@ EXPORTS = (
     "chll_lattice_read_rows", "chll_energy_grad_noalloc",
     "chll_energy_grad_natural", "chll_lattice_quench",
     "chll_lattice_set_kernel", "chll_lattice_shell_corr", "chll_lattice_projection",
+    "chll_lattice_structure_factor",
     "chll_lattice_create_slab", "chll_lattice_slab_plane", "chll_lattice_counters",
     "chll_lattice_control_update", "chll_lattice_slab_set_peers", "chll_lattice_slab_push",
     "chll_lattice_ipc_handle", "chll_ipc_open", "chll_ipc_close",
@@ -179,6 +180,8 @@ def _declare(L: ct.CDLL) -> None:
     L.chll_lattice_shell_corr.restype = i32
     L.chll_lattice_projection.argtypes = [vp, vp, vp, P(ct.c_longlong), P(i32)]
     L.chll_lattice_projection.restype = i32
+    L.chll_lattice_structure_factor.argtypes = [vp, vp, vp, i32, vp]
+    L.chll_lattice_structure_factor.restype = i32
     L.chll_lattice_reserve_rows.argtypes = [vp, i32]
     L.chll_lattice_measure.argtypes = [vp, P(Coupling), i32]
     L.chll_lattice_read_rows.argtypes = [vp, vp, i32, i32]

@@ -11,8 +11,8 @@ The reference computes these in numba on saved configurations:
   notebooks/.ipynb_checkpoints/hero_stripe-checkpoint.py (lines 10-29):
   |sum_x s_x exp(-i kv p.(x+1)) / N|^2 for kv on a grid and an integer
   direction p.  Here the sum over sites is first binned on the device by the
-  integer m = p.(x+1) (exact integer sums), and the transform over the few
-  thousand bins runs on the host in FP64.
+  integer m = p.(x+1) (exact integer sums), then transformed over the few
+  thousand bins in FP64.
 """
 from __future__ import annotations
 
@@ -53,13 +53,9 @@ def projection(lat: Lattice, plane):
 
 def structure_factor(lat: Lattice, bins: int, k_min: float, k_max: float, plane):
     """(sf, kvs) as hero_stripe's structure_factor(s, bins, k_min, k_max, plane)."""
-    m, hist = projection(lat, plane)
     kvs = np.linspace(k_min, k_max, bins)
-    n3 = lat.ni * lat.nj * lat.nk
-    keep = hist != 0
-    mm, hh = m[keep].astype(np.float64), hist[keep].astype(np.float64)
-    sc = np.empty(len(kvs), dtype=complex)
-    for idx, kv in enumerate(kvs):
-        sc[idx] = np.sum(hh * np.exp(-1j * kv * mm)) / n3
-    sf = sc.real * sc.real + sc.imag * sc.imag
+    sf = np.empty(len(kvs), np.float64)
+    p = (ct.c_int * 3)(*[int(v) for v in plane])
+    check(_lib.load().chll_lattice_structure_factor(lat._h, p, kvs.ctypes.data_as(ct.c_void_p),
+                                                    len(kvs), sf.ctypes.data_as(ct.c_void_p)))
     return sf, kvs

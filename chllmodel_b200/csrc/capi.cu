@@ -1085,38 +1085,81 @@ int chll_lattice_shell_corr(chll_lattice* L, int nshells, int wrap, double* gn, 
   return ok();
 }
 
-int chll_lattice_projection(chll_lattice* L, const int* plane, long long* hist,
-                            long long* m_min, int* nbins) {
-  if (!L || !plane || !m_min || !nbins) return fail(CHLL_EINVAL, "projection: null argument");
-  if (L->slab) return fail(CHLL_EINVAL, "projection: not available on a slab (whole lattices only)");
-  const int n[3] = {L->ni, L->nj, L->nk};
-  long long lo = 0, hi = 0;
+}  // extern "C"
+
+namespace {
+
+// Bins of the chirality projection along `plane`: m = lo .. lo + n - 1.
+int projection_bins(chll_lattice* L, const int* plane, long long* lo, int* n) {
+  if (L->slab)
+    return fail(CHLL_EINVAL, "projection: not available on a slab (whole lattices only)");
+  const int dims[3] = {L->ni, L->nj, L->nk};
+  long long hi = 0;
+  *lo = 0;
   for (int d = 0; d < 3; ++d) {
     const long long p = plane[d];
-    lo += p > 0 ? p : p * n[d];
-    hi += p > 0 ? p * n[d] : p;
+    *lo += p > 0 ? p : p * dims[d];
+    hi += p > 0 ? p * dims[d] : p;
   }
-  const long long nb = hi - lo + 1;
+  const long long nb = hi - *lo + 1;
   if (nb > chll::kMaxProjectionBins)
     return fail(CHLL_ERANGE, "projection: %lld bins exceed %d (direction too long)", nb,
                 chll::kMaxProjectionBins);
+  *n = (int)nb;
+  return CHLL_OK;
+}
+
+// The histogram into device memory, enqueued.
+int project(chll_lattice* L, const int* plane, long long lo, int nb, unsigned long long* d_hist) {
+  CHLL_CUDA_TRY(cudaMemsetAsync(d_hist, 0, (size_t)nb * sizeof(unsigned long long), L->stream));
+  chll::launch_projection(L->view(), plane[0], plane[1], plane[2], lo, nb, d_hist, L->stream);
+  CHLL_CUDA_TRY(cudaGetLastError());
+  return CHLL_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int chll_lattice_projection(chll_lattice* L, const int* plane, long long* hist,
+                            long long* m_min, int* nbins) {
+  if (!L || !plane || !m_min || !nbins) return fail(CHLL_EINVAL, "projection: null argument");
+  long long lo = 0;
+  int nb = 0;
+  CHLL_TRY(projection_bins(L, plane, &lo, &nb));
   *m_min = lo;
-  *nbins = (int)nb;
+  *nbins = nb;
   if (!hist) return ok();
-  unsigned long long* d_hist = nullptr;
-  CHLL_CUDA_TRY(cudaMalloc(&d_hist, (size_t)nb * sizeof(unsigned long long)));
-  cudaError_t e = cudaMemsetAsync(d_hist, 0, (size_t)nb * sizeof(unsigned long long), L->stream);
-  if (e == cudaSuccess) {
-    chll::launch_projection(L->view(), plane[0], plane[1], plane[2], lo, (int)nb, d_hist,
-                            L->stream);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(hist, d_hist, (size_t)nb * sizeof(long long), cudaMemcpyDeviceToHost,
-                        L->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(L->stream);
-  cudaFree(d_hist);
-  if (e != cudaSuccess) return fail(CHLL_ECUDA, "projection: %s", cudaGetErrorString(e));
+  CHLL_TRY(ensure_staging(L, (size_t)nb * sizeof(unsigned long long)));
+  CHLL_TRY(project(L, plane, lo, nb, (unsigned long long*)L->staging));
+  CHLL_CUDA_TRY(cudaMemcpyAsync(hist, L->staging, (size_t)nb * sizeof(long long),
+                                cudaMemcpyDeviceToHost, L->stream));
+  CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
+  return ok();
+}
+
+int chll_lattice_structure_factor(chll_lattice* L, const int* plane, const double* kvs, int nkv,
+                                  double* sf) {
+  if (!L || !plane || nkv < 0 || (nkv > 0 && (!kvs || !sf)))
+    return fail(CHLL_EINVAL, "structure_factor: bad argument");
+  long long lo = 0;
+  int nb = 0;
+  CHLL_TRY(projection_bins(L, plane, &lo, &nb));
+  if (nkv == 0) return ok();
+  // scratch: histogram, wave numbers, result
+  CHLL_TRY(ensure_staging(L, (size_t)nb * sizeof(unsigned long long) +
+                                 2 * (size_t)nkv * sizeof(double)));
+  unsigned long long* const d_hist = (unsigned long long*)L->staging;
+  double* const d_kvs = (double*)(d_hist + nb);
+  double* const d_sf = d_kvs + nkv;
+  CHLL_CUDA_TRY(cudaMemcpyAsync(d_kvs, kvs, nkv * sizeof(double), cudaMemcpyHostToDevice,
+                                L->stream));
+  CHLL_TRY(project(L, plane, lo, nb, d_hist));
+  chll::launch_structure_factor(d_hist, lo, nb, d_kvs, nkv, (double)L->nsites, d_sf, L->stream);
+  CHLL_CUDA_TRY(cudaGetLastError());
+  CHLL_CUDA_TRY(cudaMemcpyAsync(sf, d_sf, nkv * sizeof(double), cudaMemcpyDeviceToHost,
+                                L->stream));
+  CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
   return ok();
 }
 

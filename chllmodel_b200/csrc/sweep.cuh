@@ -111,5 +111,9 @@ void launch_shell_corr(const float4* site, int ni, int nj, int nk, const int4* o
                        cudaStream_t stream);
 void launch_projection(const LatticeView& L, int px, int py, int pz, long long m0, int nbins,
                        unsigned long long* hist, cudaStream_t stream);
+// |sum_b hist[b] exp(-i kvs[q] (m0 + b)) / nsites|^2 for nkv wave numbers.
+void launch_structure_factor(const unsigned long long* hist, long long m0, int nbins,
+                             const double* kvs, int nkv, double nsites, double* sf,
+                             cudaStream_t stream);
 
 }  // namespace chll

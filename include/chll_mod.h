@@ -360,6 +360,10 @@ int chll_lattice_shell_corr(chll_lattice* lat, int nshells, int wrap, double* gn
  * Sets *m_min and *nbins (at most 12288); hist may be NULL to ask the size. */
 int chll_lattice_projection(chll_lattice* lat, const int* plane, long long* hist,
                             long long* m_min, int* nbins);
+/* |sum_x s_x exp(-i kvs[q] p.(x+1)) / N|^2 for nkv wave numbers along an integer
+ * direction p (host arrays): the projection above, transformed on the device. */
+int chll_lattice_structure_factor(chll_lattice* lat, const int* plane, const double* kvs, int nkv,
+                                  double* sf);
 
 /* ---- energy adjoint of arrays in natural order --------------------------- */
 
