@@ -11,19 +11,30 @@
 // and one half-space of offsets (the host doubles shells >= 1; shell 0 holds
 // d = 0 only) and the pair counts come from the host in closed form.
 //
-// Work layout: natural-order float4 sites (unpacked once into scratch), one
-// thread per site, grid-stride in whole warps so every lane walks the same
-// offset list (sorted by shell) and the warp reduces a shell's sums together.
-// Per pair: FP32 dot product and FP32 running sums over at most kChunk
-// offsets (the chirality term is exact: +-1 products), then an FP64 warp sum
-// into per-warp shared slots; CTA partials are summed in a fixed order by a
-// second kernel, so results are reproducible bit for bit.
+// Work layout: natural-order float4 sites (unpacked once into scratch).  The
+// offsets, sorted by shell, are cut into chunks of at most kCorrChunk of one
+// shell; a thread holds a strip of eight sites (i, j .. j+7, k) in registers and
+// runs every site's pairs with a chunk's offsets: FP32 dot products and one FP32
+// running sum per site and chunk (the chirality term is exact: +-1 products),
+// then FP64 sums per thread and shell in shared memory.  CTA partials are summed
+// in a fixed order by a second kernel, so results are reproducible bit for bit.
+//
+// What bounds it: a pair loads its other site, four L1 wavefronts of a warp's
+// 512 bytes (offsets of one shell lie on a thin sphere, so a strip's sites share
+// few neighbours while it is walked).  With one thread per site, the offset's
+// load, wrap and bounds tests, the shell test and the 64-bit address were paid
+// per pair: 33 instructions, and 8 wavefronts (96^3, 10 shells: 2460 us, the
+// sum of the partials by one thread per column another 59).  The strip shares
+// them: 14 instructions and 5 wavefronts, 1310 and 3 us (64^3, 20 shells: 7.2 ->
+// 4.3 ms; strips of four sites: 1.72 ms and 4.8).  A site past an open boundary reads as the zero site behind
+// the lattice.  Small lattices give a strip several tasks, chunks in turn.
 //
 // The projection kernel bins s by m = p . (i+1, j+1, k+1) for an integer
 // direction p into an integer histogram (exact, order-free), from which the
 // structure factor of hero_stripe.py's get_sc (a sum of s exp(-i k.(x+1)) for
 // k along p) is a short one-dimensional transform (structure_factor_kernel).
 #include <algorithm>
+#include <atomic>
 
 #include "chll_common.cuh"
 #include "moments.cuh"
@@ -33,104 +44,115 @@ namespace chll {
 
 namespace {
 
-constexpr int kCorrThreads = 256;
-constexpr int kCorrWarps = kCorrThreads / 32;
-constexpr int kChunk = 128;  // FP32 terms per running sum before the FP64 flush
+constexpr int kCorrThreads = 128;
+constexpr int kStrip = 8;
 
-__device__ __forceinline__ void flush_shell(double (*s_n)[kMaxCorrShells],
-                                            double (*s_s)[kMaxCorrShells], int warp, int lane,
-                                            int shell, float an, float as) {
-  const double vn = warp_sum_d((double)an);
-  const double vs = warp_sum_d((double)as);
-  if (lane == 0) {
-    s_n[warp][shell] += vn;
-    s_s[warp][shell] += vs;
-  }
-}
+struct CorrGeom {
+  uint32_t ni, nj, nk;
+  uint32_t strips;  // ni * ceil(nj / kStrip) * nk, rounded up to whole warps
+  uint32_t splits;  // tasks per strip, each every splits-th chunk
+  int nchunks, nshells;
+};
 
-// offs[o] = {di, dj, dk, shell}, sorted by shell.  With WRAP the host has
-// reduced di, dj, dk into [0, n) so one conditional subtraction wraps.
+// offs[o] = {di, dj, dk, 0}, with WRAP reduced into [0, n); chunks[c] = {first
+// offset, end, shell}.  site[ni * nj * nk] is zero.
 template <bool WRAP>
 __global__ void __launch_bounds__(kCorrThreads)
-    shell_corr_kernel(const float4* __restrict__ site, int ni, int nj, int nk,
-                      const int4* __restrict__ offs, int noffs, int nshells,
-                      double* __restrict__ partials) {
-  __shared__ double s_n[kCorrWarps][kMaxCorrShells];
-  __shared__ double s_s[kCorrWarps][kMaxCorrShells];
-  __shared__ double s_sum[kCorrWarps];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int r = lane; r < nshells; r += 32) {
-    s_n[warp][r] = 0.0;
-    s_s[warp][r] = 0.0;
-  }
-  __syncwarp();
-  const uint32_t uni = (uint32_t)ni, unj = (uint32_t)nj, unk = (uint32_t)nk;
-  const uint64_t N = (uint64_t)uni * unj * unk;
-  const uint64_t stride = (uint64_t)gridDim.x * kCorrThreads;
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    shell_corr_kernel(const float4* __restrict__ site, CorrGeom G, const int4* __restrict__ offs,
+                      const int4* __restrict__ chunks, double* __restrict__ partials) {
+  extern __shared__ double s_acc[];  // [2 * nshells][thread]
+  const int R = G.nshells, tid = threadIdx.x;
+  double* const an64 = s_acc + tid;
+  double* const as64 = s_acc + (size_t)R * kCorrThreads + tid;
+  for (int r = 0; r < R; ++r) an64[r * kCorrThreads] = as64[r * kCorrThreads] = 0.0;
+  const uint32_t njs = (G.nj + kStrip - 1) / kStrip;
+  const uint32_t nothing = G.ni * G.nj * G.nk;  // the zero site
+  const uint64_t tasks = (uint64_t)G.strips * G.splits;
   double ssum = 0.0;
-  for (uint64_t x0 = (uint64_t)blockIdx.x * kCorrThreads + (uint64_t)warp * 32; x0 < N;
-       x0 += stride) {
-    const uint64_t x = x0 + (uint64_t)lane;
-    const bool valid = x < N;
-    const uint32_t xi = valid ? (uint32_t)x : 0u;
-    const uint32_t row = xi / uni;
-    const int i = (int)(xi - row * uni);
-    const int k = (int)(row / unj);
-    const int j = (int)(row - (uint32_t)k * unj);
-    const float4 a = valid ? site[xi] : zero;
-    ssum += (double)a.w;
-    int cur = -1, run = 0;
-    float an = 0.f, as = 0.f;
-    for (int o = 0; o < noffs; ++o) {
-      const int4 d = __ldg(offs + o);
-      if (d.w != cur || run == kChunk) {
-        if (cur >= 0) flush_shell(s_n, s_s, warp, lane, cur, an, as);
-        cur = d.w;
-        run = 0;
-        an = 0.f;
-        as = 0.f;
-      }
-      ++run;
-      uint32_t ii = (uint32_t)(i + d.x), jj = (uint32_t)(j + d.y), kk = (uint32_t)(k + d.z);
-      bool in = valid;
-      if (WRAP) {
-        if (ii >= uni) ii -= uni;
-        if (jj >= unj) jj -= unj;
-        if (kk >= unk) kk -= unk;
-      } else {
-        in = in && ii < uni && jj < unj && kk < unk;
-      }
-      if (in) {
-        const float4 b = site[ii + uni * (jj + unj * kk)];
-        const float dt = fmaf(a.z, b.z, fmaf(a.y, b.y, __fmul_rn(a.x, b.x)));
-        an = fmaf(dt, dt, an);
-        as = fmaf(a.w, b.w, as);
-      }
+  for (uint64_t t = (uint64_t)blockIdx.x * kCorrThreads + tid; t < tasks;
+       t += (uint64_t)gridDim.x * kCorrThreads) {
+    const uint32_t split = (uint32_t)(t / G.strips);  // the same in a whole warp
+    const uint32_t x = (uint32_t)(t - (uint64_t)split * G.strips);
+    const uint32_t row = x / G.ni, i = x - row * G.ni;
+    const uint32_t k = row / njs, j0 = (row - k * njs) * kStrip;
+    const bool has = k < G.nk;
+    // the strip's sites; those past its row's end are zero and sit at j = 0
+    float4 a[kStrip];
+    uint32_t j[kStrip];
+#pragma unroll
+    for (int c = 0; c < kStrip; ++c) {
+      const bool v = has && j0 + c < G.nj;
+      j[c] = v ? j0 + c : 0u;
+      a[c] = __ldg(site + (v ? i + G.ni * (j[c] + G.nj * k) : nothing));
+      if (split == 0) ssum += (double)a[c].w;
     }
-    if (cur >= 0) flush_shell(s_n, s_s, warp, lane, cur, an, as);
+    for (int q = (int)split; q < G.nchunks; q += (int)G.splits) {
+      const int4 chunk = __ldg(chunks + q);
+      float an[kStrip], as[kStrip];
+#pragma unroll
+      for (int c = 0; c < kStrip; ++c) an[c] = as[c] = 0.f;
+      int4 after = __ldg(offs + chunk.x);
+      for (int o = chunk.x; o < chunk.y; ++o) {
+        const int4 d = after;
+        after = __ldg(offs + o + 1);  // the chunks follow the offsets
+        uint32_t ii = i + (uint32_t)d.x, kk = k + (uint32_t)d.z;
+        bool in = has;
+        if (WRAP) {
+          if (ii >= G.ni) ii -= G.ni;
+          if (kk >= G.nk) kk -= G.nk;
+        } else {
+          in = in && ii < G.ni && kk < G.nk;
+        }
+        const uint32_t base = ii + G.ni * G.nj * kk;
+#pragma unroll
+        for (int c = 0; c < kStrip; ++c) {
+          uint32_t jj = j[c] + (uint32_t)d.y;
+          if (WRAP && jj >= G.nj) jj -= G.nj;
+          const float4 b = __ldg(site + (in && (WRAP || jj < G.nj) ? base + G.ni * jj : nothing));
+          const float dt = fmaf(a[c].z, b.z, fmaf(a[c].y, b.y, __fmul_rn(a[c].x, b.x)));
+          an[c] = fmaf(dt, dt, an[c]);
+          as[c] = fmaf(a[c].w, b.w, as[c]);
+        }
+      }
+      double vn = 0.0, vs = 0.0;
+#pragma unroll
+      for (int c = 0; c < kStrip; ++c) {
+        vn += (double)an[c];
+        vs += (double)as[c];
+      }
+      an64[chunk.z * kCorrThreads] += vn;
+      as64[chunk.z * kCorrThreads] += vs;
+    }
   }
+  __syncthreads();
+  const int lane = tid & 31, warp = tid >> 5, width = 2 * R + 1;
+  double* const out = partials + (size_t)blockIdx.x * width;
+  for (int c = warp; c < 2 * R; c += kCorrThreads / 32) {
+    double v = 0.0;
+    for (int w = lane; w < kCorrThreads; w += 32) v += s_acc[(size_t)c * kCorrThreads + w];
+    v = warp_sum_d(v);
+    if (lane == 0) out[c] = v;
+  }
+  __shared__ double s_sum[kCorrThreads / 32];
   ssum = warp_sum_d(ssum);
   if (lane == 0) s_sum[warp] = ssum;
   __syncthreads();
-  const int width = 2 * nshells + 1;
-  double* out = partials + (size_t)blockIdx.x * width;
-  for (int t = threadIdx.x; t < width; t += kCorrThreads) {
+  if (tid == 0) {
     double v = 0.0;
-    for (int w = 0; w < kCorrWarps; ++w)
-      v += t < nshells ? s_n[w][t] : (t < 2 * nshells ? s_s[w][t - nshells] : s_sum[w]);
-    out[t] = v;
+    for (int w = 0; w < kCorrThreads / 32; ++w) v += s_sum[w];
+    out[2 * R] = v;
   }
 }
 
-// Column t of the CTA partials summed over CTAs in index order.
-__global__ void sum_partials_kernel(const double* __restrict__ partials, int rows, int width,
-                                    double* __restrict__ out) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= width) return;
+// Column blockIdx.x of the CTA partials summed over the CTAs, one warp per
+// column in a fixed order.
+__global__ void __launch_bounds__(32)
+    sum_partials_kernel(const double* __restrict__ partials, int rows, int width,
+                        double* __restrict__ out) {
   double v = 0.0;
-  for (int r = 0; r < rows; ++r) v += partials[(size_t)r * width + t];
-  out[t] = v;
+  for (int r = threadIdx.x; r < rows; r += 32) v += partials[(size_t)r * width + blockIdx.x];
+  v = warp_sum_d(v);
+  if (threadIdx.x == 0) out[blockIdx.x] = v;
 }
 
 // hist[m - m0] += s over the real sites, m = p . (i+1, j+1, k+1).  A thread
@@ -247,23 +269,71 @@ int device_sms() {
 
 }  // namespace
 
-int shell_corr_blocks(uint64_t nsites) {
-  const uint64_t need = (nsites + kCorrThreads - 1) / kCorrThreads;
-  const uint64_t cap = (uint64_t)device_sms() * 8;
-  return (int)(need < cap ? (need ? need : 1) : cap);
+namespace {
+
+size_t corr_smem(int nshells) { return 2 * (size_t)nshells * kCorrThreads * sizeof(double); }
+
+CorrGeom corr_geom(int ni, int nj, int nk, int nchunks, int nshells, int blocks) {
+  CorrGeom G;
+  G.ni = (uint32_t)ni;
+  G.nj = (uint32_t)nj;
+  G.nk = (uint32_t)nk;
+  const uint64_t strips = (uint64_t)ni * ((nj + kStrip - 1) / kStrip) * nk;
+  G.strips = (uint32_t)((strips + 31) / 32 * 32);
+  // the least work on the busiest thread, a task's start counted as half a
+  // percent of a strip
+  const uint64_t threads = (uint64_t)blocks * kCorrThreads;
+  double best = 1e300;
+  for (uint32_t s = 1; s <= (uint32_t)nchunks; ++s) {
+    const double cost =
+        (double)((G.strips * (uint64_t)s + threads - 1) / threads) * (1.0 / s + 0.005);
+    if (cost < best) {
+      best = cost;
+      G.splits = s;
+    }
+  }
+  G.nchunks = nchunks;
+  G.nshells = nshells;
+  return G;
 }
 
-void launch_shell_corr(const float4* site, int ni, int nj, int nk, const int4* offs, int noffs,
-                       int nshells, bool wrap, double* partials, int blocks, double* out,
-                       cudaStream_t stream) {
+}  // namespace
+
+// Resident CTAs of the kernel with these shells, queried once per device and
+// number of shells.
+int shell_corr_blocks(int nshells) {
+  static std::atomic<int> cache[16][kMaxCorrShells + 1];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::atomic<int>& known = cache[dev & 15][nshells];
+  if (const int n = known.load(std::memory_order_relaxed)) return n;
+  const size_t smem = corr_smem(nshells);
+  int per_sm = 1 << 30;
+  for (auto kernel : {shell_corr_kernel<false>, shell_corr_kernel<true>}) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)corr_smem(kMaxCorrShells));
+    int n = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kCorrThreads, smem);
+    if (n < per_sm) per_sm = n;
+  }
+  const int blocks = device_sms() * (per_sm > 0 ? per_sm : 1);
+  known.store(blocks, std::memory_order_relaxed);
+  return blocks;
+}
+
+void launch_shell_corr(const float4* site, int ni, int nj, int nk, const int4* offs,
+                       const int4* chunks, int nchunks, int nshells, bool wrap, double* partials,
+                       int blocks, double* out, cudaStream_t stream) {
+  const CorrGeom G = corr_geom(ni, nj, nk, nchunks, nshells, blocks);
+  const uint64_t need = ((uint64_t)G.strips * G.splits + kCorrThreads - 1) / kCorrThreads;
+  const int grid = (int)std::min<uint64_t>(need, (uint64_t)blocks);
+  const size_t smem = corr_smem(nshells);
   if (wrap)
-    shell_corr_kernel<true><<<blocks, kCorrThreads, 0, stream>>>(site, ni, nj, nk, offs, noffs,
-                                                                  nshells, partials);
+    shell_corr_kernel<true><<<grid, kCorrThreads, smem, stream>>>(site, G, offs, chunks, partials);
   else
-    shell_corr_kernel<false><<<blocks, kCorrThreads, 0, stream>>>(site, ni, nj, nk, offs,
-                                                                   noffs, nshells, partials);
+    shell_corr_kernel<false><<<grid, kCorrThreads, smem, stream>>>(site, G, offs, chunks, partials);
   const int width = 2 * nshells + 1;
-  sum_partials_kernel<<<(width + 127) / 128, 128, 0, stream>>>(partials, blocks, width, out);
+  sum_partials_kernel<<<width, 32, 0, stream>>>(partials, grid, width, out);
 }
 
 void launch_projection(const LatticeView& L, int px, int py, int pz, long long m0, int nbins,

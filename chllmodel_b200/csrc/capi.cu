@@ -1023,9 +1023,9 @@ int chll_lattice_shell_corr(chll_lattice* L, int nshells, int wrap, double* gn, 
                 nshells);
   const int ni = L->ni, nj = L->nj, nk = L->nk, R = nshells;
   const double N = (double)L->nsites;
-  // d = 0 and one half-space of offsets with |d|^2 < R^2, sorted by shell;
-  // pair counts over all offsets in closed form.
-  std::vector<int4> offs;
+  // d = 0 and one half-space of offsets with |d|^2 < R^2, sorted by shell (w, then
+  // cut into chunks); pair counts over all offsets in closed form.
+  std::vector<int4> offs, chunks;
   std::vector<double> cnt(R, 0.0);
   auto wrapped = [](int d, int n) { return ((d % n) + n) % n; };
   for (int dk = -R + 1; dk < R; ++dk)
@@ -1047,34 +1047,36 @@ int chll_lattice_shell_corr(chll_lattice* L, int nshells, int wrap, double* gn, 
       }
   std::stable_sort(offs.begin(), offs.end(),
                    [](const int4& a, const int4& b) { return a.w < b.w; });
-  const int blocks = chll::shell_corr_blocks((uint64_t)L->nsites);
+  for (int o = 0; o < (int)offs.size(); ++o) {
+    if (chunks.empty() || chunks.back().z != offs[o].w ||
+        o - chunks.back().x == chll::kCorrChunk)
+      chunks.push_back(make_int4(o, o, offs[o].w, 0));
+    chunks.back().y = o + 1;
+  }
+  const int blocks = chll::shell_corr_blocks(R);
   const int width = 2 * R + 1;
-  CHLL_TRY(ensure_staging(L, (size_t)L->nsites * sizeof(float4)));
-  int4* d_offs = nullptr;
-  double* d_part = nullptr;
-  CHLL_CUDA_TRY(cudaMalloc(&d_offs, std::max<size_t>(1, offs.size()) * sizeof(int4)));
-  cudaError_t e = cudaMalloc(&d_part, ((size_t)blocks + 1) * width * sizeof(double));
-  if (e != cudaSuccess) {
-    cudaFree(d_offs);
-    return fail(CHLL_ENOMEM, "shell_corr: %s", cudaGetErrorString(e));
-  }
+  // scratch: the sites in natural order and the zero site, offsets, chunks, CTA
+  // partials and their sums
+  const size_t sites = (size_t)L->nsites + 1;
+  CHLL_TRY(ensure_staging(L, (sites + offs.size() + chunks.size()) * sizeof(float4) +
+                                 ((size_t)blocks + 1) * width * sizeof(double)));
+  float4* const d_site = (float4*)L->staging;
+  int4* const d_offs = (int4*)(d_site + sites);
+  int4* const d_chunks = d_offs + offs.size();
+  double* const d_part = (double*)(d_chunks + chunks.size());
   std::vector<double> out(width, 0.0);
-  e = cudaMemcpyAsync(d_offs, offs.data(), offs.size() * sizeof(int4), cudaMemcpyHostToDevice,
-                      L->stream);
-  if (e == cudaSuccess) {
-    chll::launch_unpack_f4(L->view(), (float4*)L->staging, L->stream);
-    chll::launch_shell_corr((const float4*)L->staging, ni, nj, nk, d_offs, (int)offs.size(), R,
-                            wrap != 0, d_part, blocks, d_part + (size_t)blocks * width,
-                            L->stream);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(out.data(), d_part + (size_t)blocks * width, width * sizeof(double),
-                        cudaMemcpyDeviceToHost, L->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(L->stream);
-  cudaFree(d_offs);
-  cudaFree(d_part);
-  if (e != cudaSuccess) return fail(CHLL_ECUDA, "shell_corr: %s", cudaGetErrorString(e));
+  CHLL_CUDA_TRY(cudaMemsetAsync(d_site + L->nsites, 0, sizeof(float4), L->stream));
+  CHLL_CUDA_TRY(cudaMemcpyAsync(d_offs, offs.data(), offs.size() * sizeof(int4),
+                                cudaMemcpyHostToDevice, L->stream));
+  CHLL_CUDA_TRY(cudaMemcpyAsync(d_chunks, chunks.data(), chunks.size() * sizeof(int4),
+                                cudaMemcpyHostToDevice, L->stream));
+  chll::launch_unpack_f4(L->view(), d_site, L->stream);
+  chll::launch_shell_corr(d_site, ni, nj, nk, d_offs, d_chunks, (int)chunks.size(), R, wrap != 0,
+                          d_part, blocks, d_part + (size_t)blocks * width, L->stream);
+  CHLL_CUDA_TRY(cudaGetLastError());
+  CHLL_CUDA_TRY(cudaMemcpyAsync(out.data(), d_part + (size_t)blocks * width, width * sizeof(double),
+                                cudaMemcpyDeviceToHost, L->stream));
+  CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
   const double s_mean = out[2 * R] / N;
   for (int r = 0; r < R; ++r) {
     const double w = r == 0 ? 1.0 : 2.0;  // shells >= 1 hold d and -d
