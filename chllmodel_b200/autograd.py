@@ -125,6 +125,5 @@ def quench(lat: Lattice, eps: float, K: float, h: float, eta: float, nsteps: int
         step = min(chunk, nsteps - done)
         lat.quench(cp, eta, step)
         done += step
-        _, out4 = lat.energy_grad(cp)
-        energies.append((done, out4[0]))
+        energies.append((done, lat.energy_sums(cp)[0]))
     return energies

@@ -16,7 +16,7 @@ LIB = os.path.join(HERE, "libchll_mod.so")
 SOURCES = ["sweep.cu", "batched.cu", "pooled.cu", "resident.cu", "layout.cu", "observables.cu",
            "adjoint.cu", "analysis.cu", "capi.cu", "noalloc.cu"]
 HEADERS = ["chll_common.cuh", "chll_physics.cuh", "sweep.cuh", "sweep_unit.cuh", "moments.cuh",
-           "staged.cuh", "pooled.cuh"]
+           "staged.cuh", "pooled.cuh", "resident.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

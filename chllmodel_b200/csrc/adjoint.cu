@@ -14,9 +14,11 @@
 // dE/dh = -sum(s), together with E itself.
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "chll_common.cuh"
 #include "moments.cuh"
+#include "resident.cuh"
 #include "sweep.cuh"
 #include "sweep_unit.cuh"
 
@@ -484,27 +486,65 @@ __global__ void __launch_bounds__(kGradThreads)
   }
 }
 
+// Every product and sum of a quench step is an explicit fmaf / __fmul_rn /
+// __fadd_rn, so that the pass kernel and the resident form round alike: a quench
+// amplifies a rounding along the lattice's soft modes, and its energies are
+// compared to ten digits.
+
+// x0 y0 + x1 y1 + x2 y2; SECOND: the second product is the rounded one of the
+// first two.
+template <bool SECOND>
+__device__ __forceinline__ float quench_dot(float x0, float y0, float x1, float y1, float x2,
+                                            float y2) {
+  const float t = SECOND ? fmaf(x0, y0, __fmul_rn(x1, y1)) : fmaf(x1, y1, __fmul_rn(x0, y0));
+  return fmaf(x2, y2, t);
+}
+
+// One bond's dE/dn_i (bond_grad) added to g.
+template <int AXIS, bool SECOND>
+__device__ __forceinline__ void quench_bond(const float4& n, const float4& b, float m2eps, float sk,
+                                            float g[3]) {
+  constexpr int p = (AXIS + 1) % 3, q = (AXIS + 2) % 3;
+  const float nv[3] = {n.x, n.y, n.z}, bv[3] = {b.x, b.y, b.z};
+  const float c = quench_dot<SECOND>(n.x, b.x, n.y, b.y, n.z, b.z);
+  const float X = fmaf(nv[p], bv[q], -__fmul_rn(nv[q], bv[p]));
+  const float a = __fmul_rn(m2eps, c);
+  const float w = __fmul_rn(sk, __fmul_rn(0.5f, __fadd_rn(n.w, b.w)));
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+    // component t of X b + c (b x e_a)
+    const float e = t == p ? bv[q] : -bv[p];
+    const float u = t == AXIS ? __fmul_rn(X, bv[t]) : fmaf(X, bv[t], __fmul_rn(c, e));
+    g[t] = __fadd_rn(g[t], fmaf(a, bv[t], __fmul_rn(w, u)));
+  }
+}
+
 // One site of a zero-temperature gradient quench: n moves against its
 // tangent-projected energy gradient, n <- normalise(n - eta (I - n n^T) dE/dn),
-// with the neighbours nb (+x, -x, +y, -y, +z, -z) held fixed.
+// with the neighbours nb (+x, -x, +y, -y, +z, -z) held fixed.  Which product of a
+// bond's dot product is rounded on its own differs between the boundaries and,
+// for -z, between a unit's sites (SITE 0, 1): the roundings this quench has
+// always had.
+template <bool P, int SITE>
 __device__ __forceinline__ float4 quench_site(float4 n, const Nbrs& nb, const Coupling& cp,
                                               float eta) {
-  float gx = 0.f, gy = 0.f, gz = 0.f;
-  bond_grad<0>(n, nb.b[0], -1.f, cp, gx, gy, gz);
-  bond_grad<0>(n, nb.b[1], +1.f, cp, gx, gy, gz);
-  bond_grad<1>(n, nb.b[2], -1.f, cp, gx, gy, gz);
-  bond_grad<1>(n, nb.b[3], +1.f, cp, gx, gy, gz);
-  bond_grad<2>(n, nb.b[4], -1.f, cp, gx, gy, gz);
-  bond_grad<2>(n, nb.b[5], +1.f, cp, gx, gy, gz);
-  const float nn = n.x * n.x + n.y * n.y + n.z * n.z;
-  const float gn = (gx * n.x + gy * n.y + gz * n.z) / nn;
-  const float x = n.x - eta * (gx - gn * n.x);
-  const float y = n.y - eta * (gy - gn * n.y);
-  const float z = n.z - eta * (gz - gn * n.z);
-  const float rn = rsqrtf(x * x + y * y + z * z);
-  n.x = x * rn;
-  n.y = y * rn;
-  n.z = z * rn;
+  const float m2eps = __fmul_rn(-2.f, cp.eps);
+  float g[3] = {0.f, 0.f, 0.f};
+  quench_bond<0, true>(n, nb.b[0], m2eps, -cp.K, g);
+  quench_bond<0, true>(n, nb.b[1], m2eps, cp.K, g);
+  quench_bond<1, P>(n, nb.b[2], m2eps, -cp.K, g);
+  quench_bond<1, P>(n, nb.b[3], m2eps, cp.K, g);
+  quench_bond<2, P>(n, nb.b[4], m2eps, -cp.K, g);
+  quench_bond<2, P || SITE == 1>(n, nb.b[5], m2eps, cp.K, g);
+  const float nn = quench_dot<true>(n.x, n.x, n.y, n.y, n.z, n.z);
+  const float gn = __fdiv_rn(quench_dot<true>(g[0], n.x, g[1], n.y, g[2], n.z), nn);
+  const float x = fmaf(-eta, fmaf(-gn, n.x, g[0]), n.x);
+  const float y = fmaf(-eta, fmaf(-gn, n.y, g[1]), n.y);
+  const float z = fmaf(-eta, fmaf(-gn, n.z, g[2]), n.z);
+  const float rn = rsqrtf(quench_dot<true>(x, x, y, y, z, z));
+  n.x = __fmul_rn(x, rn);
+  n.y = __fmul_rn(y, rn);
+  n.z = __fmul_rn(z, rn);
   return n;
 }
 
@@ -519,9 +559,78 @@ __global__ void __launch_bounds__(kGradThreads) quench_pass_kernel(LatticeView L
        g += gridDim.x * kGradThreads) {
     UnitNbhd U;
     gather_unit<C, PERIODIC, PERIODIC>(L, G, g, U);
-    if (U.v0) U.n0 = quench_site(U.n0, U.nb0, cp, eta);
-    if (U.v1) U.n1 = quench_site(U.n1, U.nb1, cp, eta);
+    if (U.v0) U.n0 = quench_site<PERIODIC, 0>(U.n0, U.nb0, cp, eta);
+    if (U.v1) U.n1 = quench_site<PERIODIC, 1>(U.n1, U.nb1, cp, eta);
     st_unit(U.cen, U.n0, U.n1);
+  }
+}
+
+// The same steps in one cooperative launch (resident.cuh): a step is a pass of
+// each colour with the grid barrier after it.  A launch per pass costs a small
+// lattice about 4 us, most of it the launch; a pass here takes 2.9 at 64^3.
+struct QuenchArgs {
+  LatticeView L;
+  SweepGeom G;
+  Coupling cp;
+  float eta;
+  Control* ctl;
+  unsigned long long* words;
+  int nsteps;
+};
+
+template <bool P, bool OWN>
+__global__ void __launch_bounds__(kResThreads, 1)
+    quench_resident_kernel(const __grid_constant__ QuenchArgs A) {
+  __shared__ int s_ok;
+  if (A.ctl->status) return;  // an earlier wait ran out: the words are not to be trusted
+  const bool lead = threadIdx.x == 0;
+  OwnBlock<P> B(A.L, A.G);
+  uint32_t slot = 0;
+  auto pass = [&](auto colour) {
+    constexpr int C = decltype(colour)::value;
+    if (OWN) {
+      if (!B.has) return;
+      Nbrs nb0, nb1;
+      B.template neighbours<C>(A.L, nb0, nb1);
+      const bool odd = B.template odd<C>();
+      if (odd ? B.v[1] : B.v[0]) B.n[C][0] = quench_site<P, 0>(B.n[C][0], nb0, A.cp, A.eta);
+      if (odd ? B.v[3] : B.v[2]) B.n[C][1] = quench_site<P, 1>(B.n[C][1], nb1, A.cp, A.eta);
+      st_unit(A.L.col[C] + B.u, B.n[C][0], B.n[C][1]);
+    } else {
+      for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < A.G.units;
+           g += gridDim.x * blockDim.x) {
+        UnitNbhd U;
+        gather_unit<C, P, P, false, kLoadCoherentOrdered>(A.L, A.G, g, U);
+        if (U.v0) U.n0 = quench_site<P, 0>(U.n0, U.nb0, A.cp, A.eta);
+        if (U.v1) U.n1 = quench_site<P, 1>(U.n1, U.nb1, A.cp, A.eta);
+        st_unit(U.cen, U.n0, U.n1);
+      }
+    }
+  };
+  // false in every thread if the wait ran out
+  auto meet = [&]() {
+    __syncthreads();  // the CTA's stores before thread 0's release
+    if (lead) {
+      bool ok = true;
+      grid_arrive(A.words + slot * kWordStride, 0, gridDim.x);
+      grid_wait(A.words + slot * kWordStride, 0, gridDim.x, kWaitLimit, ok);
+      if (blockIdx.x == 0) A.words[(slot == 0 ? 2 : slot - 1) * kWordStride] = 0;
+      if (!ok) atomicOr(&A.ctl->status, 4u);
+      s_ok = ok;
+    }
+    slot = slot == 2 ? 0 : slot + 1;
+    __syncthreads();
+    return s_ok != 0;
+  };
+  for (int s = 0; s < A.nsteps; ++s) {
+    pass(std::integral_constant<int, 0>());
+    if (!meet()) return;
+    pass(std::integral_constant<int, 1>());
+    if (s + 1 < A.nsteps && !meet()) return;
+  }
+  if (lead && gridDim.x > 1) {
+    const unsigned long long old = atomicAdd(A.words + slot * kWordStride, 1ull << kArriveShift);
+    if ((uint32_t)(old >> kArriveShift) == gridDim.x - 1) clear_words(A.words);
   }
 }
 
@@ -569,6 +678,35 @@ void launch_quench_pass(const LatticeView& L, const CouplingD& cd, float eta, in
     if (colour == 0) quench_pass_kernel<0, false><<<nb, kGradThreads, 0, stream>>>(L, G, cp, eta);
     else quench_pass_kernel<1, false><<<nb, kGradThreads, 0, stream>>>(L, G, cp, eta);
   }
+}
+
+// Against a launch per pass, us per step (periodic): 8^3 1.5 and 7.5, 48^3 4.6 and
+// 8.4, 64^3 5.7 and 8.4, 96^3 12.7 and 16.6, 128^3 24.6 and 25.0; from 160^3 on the
+// launches win (45.2 and 41.3: their loads are the read-only ones).
+bool quench_resident_pays(const LatticeView& L) { return make_geom(L).units <= (1u << 19); }
+
+cudaError_t launch_quench_resident(const LatticeView& L, const CouplingD& cd, float eta,
+                                   Control* ctl, unsigned long long* words, int nsteps,
+                                   cudaStream_t stream) {
+  QuenchArgs A;
+  A.L = L;
+  A.G = make_geom(L);
+  A.cp.eps = (float)cd.eps;
+  A.cp.K = (float)cd.K;
+  A.cp.g = (float)cd.g;
+  A.cp.inv_kT = 0.f;
+  A.eta = eta;
+  A.ctl = ctl;
+  A.words = words;
+  A.nsteps = nsteps;
+  uint32_t block, ctas;
+  resident_shape(A.G.units, block, ctas);
+  const bool own = one_unit_each(L, A.G.units);
+  auto kernel = L.periodic ? (own ? quench_resident_kernel<true, true>
+                                  : quench_resident_kernel<true, false>)
+                           : (own ? quench_resident_kernel<false, true>
+                                  : quench_resident_kernel<false, false>);
+  return launch_cooperative(kernel, ctas, block, stream, A);
 }
 
 cudaError_t launch_natural_grad(int ni, int nj, int nk, int periodic, const float* n,

@@ -952,6 +952,15 @@ int chll_lattice_quench(chll_lattice* L, const chll_coupling* c, double eta, int
   if (nsteps < 0 || !(eta >= 0.0)) return fail(CHLL_EINVAL, "quench: need nsteps >= 0, eta >= 0");
   const LatticeView v = L->view();
   const chll::CouplingD cd = make_coupling_d(*c);
+  const DeviceGuard on(L->device);
+  if (chll::quench_resident_pays(v)) {
+    for (int done = 0; done < nsteps; done += kResidentChunk) {
+      const cudaError_t e = chll::launch_quench_resident(
+          v, cd, (float)eta, L->ctl, L->words, std::min(kResidentChunk, nsteps - done), L->stream);
+      if (e != cudaSuccess) return fail(CHLL_ECUDA, "quench launch: %s", cudaGetErrorString(e));
+    }
+    return ok();
+  }
   for (int s = 0; s < nsteps; ++s) {
     chll::launch_quench_pass(v, cd, (float)eta, 0, L->stream);
     chll::launch_quench_pass(v, cd, (float)eta, 1, L->stream);

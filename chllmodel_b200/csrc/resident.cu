@@ -31,27 +31,12 @@
 // launches do nothing until set_control clears it.
 #include <cuda_runtime.h>
 
-#include <algorithm>
-#include <mutex>
-
+#include "resident.cuh"
 #include "sweep.cuh"
 #include "sweep_unit.cuh"
 
 namespace chll {
 namespace {
-
-constexpr int kResThreads = 512;  // most threads per CTA, and per SM (128 registers each)
-constexpr uint32_t kWaitLimit = 1u << 22;  // polls of the word before a wait gives up
-
-// One word per pass, three in rotation, 128 bytes apart: director accepts in
-// bits 0-25, flips in bits 26-51, arrived CTAs in bits 52-63.  The word of pass
-// q is cleared by the first CTA once the barrier of pass q + 1 is through --
-// every CTA has then read it for the last time -- and that CTA's release at
-// pass q + 2 puts the clear before any arrival at pass q + 3, its next use.
-constexpr int kWordStride = 16;
-constexpr int kCountBits = 26;
-constexpr unsigned long long kCountMask = (1ull << kCountBits) - 1;
-constexpr int kArriveShift = 2 * kCountBits;
 
 struct ResidentArgs {
   LatticeView L;
@@ -118,64 +103,22 @@ struct SharedUnits {
 };
 
 // Lattices of at most one unit per thread (48^3 5.1 against 5.4 us per sweep
-// with the unit loop, 64^3 6.5 against 7.1): the thread keeps both colours'
-// unit g (the 4-site x-block q of row (j, k)) in registers for the whole
-// chunk.  The other colour's pair then is the x-row pair of walk_task, so a
-// pass loads the +-y and +-z pairs and one x neighbour, at addresses fixed for
-// the launch, and the pass's random words are drawn while the barrier before
-// it is waited for.  ni a multiple of 4, or open boundaries (a padding slot
-// reads as the zero of a missing neighbour).
+// with the unit loop, 64^3 6.5 against 7.1): the block in registers
+// (resident.cuh), and the pass's random words drawn while the barrier before it
+// is waited for.
 template <bool P>
 struct OwnUnit {
   const ResidentArgs& A;
-  uint32_t g, u, o0;             // unit, its slot, parity of colour 0's sites in the row
-  uint32_t yp, ym, zp, zm;       // slots of the neighbour pairs
-  uint32_t xm, xp;               // the x neighbours outside the block: below, above
-  bool has, hyp, hym, hzp, hzm, hxm, hxp;
-  bool v[4];                     // sites 4q .. 4q+3 inside the lattice
-  float4 n[2][2];
+  OwnBlock<P> B;
   Ctr4 words;
 
-  __device__ __forceinline__ explicit OwnUnit(const ResidentArgs& a) : A(a) {
-    const LatticeView& L = A.L;
-    g = blockIdx.x * blockDim.x + threadIdx.x;
-    has = g < A.G.units;
-    const uint32_t hx = (uint32_t)L.hx, nj = (uint32_t)L.nj, nk = (uint32_t)L.nk;
-    const uint32_t plane = hx * nj;
-    const uint32_t row = A.G.by_Q.div(g), q = g - row * A.G.Q;
-    const uint32_t k = A.G.by_nj.div(row), j = row - k * nj;
-    o0 = (j + k) & 1u;
-    u = 2 * g;
-    hyp = P || j + 1 < nj;
-    hym = P || j > 0;
-    hzp = P || k + 1 < nk;
-    hzm = P || k > 0;
-    hxm = P || q > 0;
-    hxp = P || q + 1 < A.G.Q;
-    yp = j + 1 < nj ? u + hx : u - (nj - 1) * hx;
-    ym = j > 0 ? u - hx : u + (nj - 1) * hx;
-    zp = k + 1 < nk ? u + plane : u - (nk - 1) * plane;
-    zm = k > 0 ? u - plane : u + (nk - 1) * plane;
-    xm = q > 0 ? u - 1 : u + hx - 1;
-    xp = q + 1 < A.G.Q ? u + 2 : u - 2 * q;
-#pragma unroll
-    for (int t = 0; t < 4; ++t) v[t] = has && 4 * q + t < (uint32_t)L.ni;
-    n[0][0] = n[0][1] = n[1][0] = n[1][1] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (has) {
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const UnitSlots s = ld_unit(L.col[c] + u);
-        n[c][0] = s.a;
-        n[c][1] = s.b;
-      }
-    }
-  }
+  __device__ __forceinline__ explicit OwnUnit(const ResidentArgs& a) : A(a), B(a.L, a.G) {}
 
   // The random words of the next pass (colour C, step): independent of the
   // lattice, so they are drawn before the wait.
   template <int C>
   __device__ __forceinline__ void draw(uint32_t step) {
-    words = philox4x32_10({{g, step, A.replica, (uint32_t)C}}, A.keys);
+    words = philox4x32_10({{B.g, step, A.replica, (uint32_t)C}}, A.keys);
     asm volatile("" : "+r"(words.v[0]), "+r"(words.v[1]), "+r"(words.v[2]), "+r"(words.v[3]));
   }
 
@@ -185,25 +128,14 @@ struct OwnUnit {
     using T = PhaseOf<PHASE>;
     constexpr int C = T::C;
     nacc = nflip = 0;
-    if (!has) return;
-    const float4* oth = A.L.col[C ^ 1];
-    const bool odd = (o0 ^ C) != 0;  // sites 4q+1, 4q+3 rather than 4q, 4q+2
+    if (!B.has) return;
     Nbrs nb0, nb1;
-    nbr_units<kLoadCoherentOrdered>(hyp, oth + yp, nb0.b[2], nb1.b[2]);
-    nbr_units<kLoadCoherentOrdered>(hym, oth + ym, nb0.b[3], nb1.b[3]);
-    nbr_units<kLoadCoherentOrdered>(hzp, oth + zp, nb0.b[4], nb1.b[4]);
-    nbr_units<kLoadCoherentOrdered>(hzm, oth + zm, nb0.b[5], nb1.b[5]);
-    float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (odd ? hxp : hxm) e = ld4_other<kLoadCoherentOrdered>(oth + (odd ? xp : xm));
-    const float4 xa = n[C ^ 1][0], xb = n[C ^ 1][1];
-    nb0.b[0] = odd ? xb : xa;
-    nb0.b[1] = odd ? xa : e;
-    nb1.b[0] = odd ? e : xb;
-    nb1.b[1] = odd ? xb : xa;
+    B.template neighbours<C>(A.L, nb0, nb1);
+    const bool odd = B.template odd<C>();
     unit_trials_drawn<T::flip_before, T::dir, T::flip_after>(
-        n[C][0], n[C][1], nb0, nb1, odd ? v[1] : v[0], odd ? v[3] : v[2], unit_randoms(words), d,
-        A.cp, nacc, nflip);
-    st_unit(A.L.col[C] + u, n[C][0], n[C][1]);
+        B.n[C][0], B.n[C][1], nb0, nb1, odd ? B.v[1] : B.v[0], odd ? B.v[3] : B.v[2],
+        unit_randoms(words), d, A.cp, nacc, nflip);
+    st_unit(A.L.col[C] + B.u, B.n[C][0], B.n[C][1]);
   }
 };
 
@@ -229,32 +161,6 @@ __device__ __forceinline__ unsigned long long cta_counts(ResidentShared& S, unsi
     }
     v = (unsigned long long)a | ((unsigned long long)f << kCountBits);
   }
-  return v;
-}
-
-// Thread 0 of every CTA adds the CTA's counts and arrival to the pass's word
-// (release: the CTA's stores, ordered before it by the CTA barrier, are
-// visible to whoever acquires the word) ...
-__device__ __forceinline__ void grid_arrive(unsigned long long* w, unsigned long long counts,
-                                            uint32_t nct) {
-  if (nct == 1) return;
-  const unsigned long long add = counts + (1ull << kArriveShift);
-  asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(w), "l"(add) : "memory");
-}
-
-// ... and waits until every CTA has (acquire).  Returns the word, or the CTA's
-// own counts of a grid of one CTA; ok = false if the wait ran out.
-__device__ __forceinline__ unsigned long long grid_wait(unsigned long long* w,
-                                                        unsigned long long counts, uint32_t nct,
-                                                        uint32_t limit, bool& ok) {
-  if (nct == 1) return counts;
-  unsigned long long v;
-  uint32_t polls = 0;
-  do {
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(w) : "memory");
-    if ((uint32_t)(v >> kArriveShift) == nct) return v;
-  } while (++polls < limit);
-  ok = false;
   return v;
 }
 
@@ -335,14 +241,13 @@ __device__ __forceinline__ void resident_sweeps(const ResidentArgs& A, ResidentS
   unsigned long long v = cta_counts(S, 0, nf, true);
   if (!lead) return;
   // the CTA that completes the closing pass's word has the flip count and
-  // writes the control block; nobody waits for this word, so it also clears
-  // all three for the next launch
+  // writes the control block
   if (nct > 1) {
     const unsigned long long old =
         atomicAdd(A.words + slot * kWordStride, v + (1ull << kArriveShift));
     if ((uint32_t)(old >> kArriveShift) != nct - 1) return;
     v += old;
-    for (int w = 0; w < 3; ++w) A.words[w * kWordStride] = 0;
+    clear_words(A.words);
   }
   nflip += v >> kCountBits & kCountMask;
   ctl->d = d;
@@ -374,37 +279,12 @@ const ResidentKernel kResident[2][4] = {
     {resident_sweeps_kernel<true, 0>, resident_sweeps_kernel<true, 1>,
      resident_sweeps_kernel<true, 2>, resident_sweeps_kernel<true, 3>}};
 
-std::mutex g_res_mutex;
-int g_res_sms[64];
-
-int resident_sms() {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) dev = 0;
-  std::lock_guard<std::mutex> lk(g_res_mutex);
-  if (!g_res_sms[dev]) {
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    g_res_sms[dev] = sms > 0 ? sms : 148;
-  }
-  return g_res_sms[dev];
-}
-
 }  // namespace
 
-// Lattice of a pass's counts in 26 bits (fewer than 2^27 sites).
+// A pass's counts fit 26 bits (fewer than 2^27 sites).
 bool resident_fits(const LatticeView& L) {
   return 2 * (uint64_t)make_geom(L).units < (1ull << kCountBits);
 }
-
-namespace {
-
-// One unit per thread: see OwnUnit.
-bool one_unit_each(const LatticeView& L, uint32_t units) {
-  return units <= (uint32_t)resident_sms() * kResThreads && (L.ni % 4 == 0 || !L.periodic);
-}
-
-}  // namespace
 
 // Against a launch per pass: always where a thread holds one unit.  Beyond
 // that the barrier still saves about 1 us per pass, but the loops' coherent
@@ -423,15 +303,10 @@ cudaError_t launch_resident_sweeps(const LatticeView& L, const Coupling& cp, uin
   ResidentArgs A;
   A.L = L;
   A.G = make_geom(L);
-  const uint32_t sms = (uint32_t)resident_sms();
   const bool full = L.ni % 4 == 0;
   const bool own = one_unit_each(L, A.G.units);
-  // Up to 256 units (two warps per scheduler) one CTA, whose barrier is its
-  // own; else the units spread over the SMs in CTAs of whole warps.
-  const uint32_t share = A.G.units <= 256 ? A.G.units : (A.G.units + sms - 1) / sms;
-  const uint32_t block = std::min<uint32_t>(kResThreads, (share + 31) / 32 * 32);
-  const uint32_t ctas =
-      std::min((A.G.units + block - 1) / block, sms * (uint32_t)(kResThreads / block));
+  uint32_t block, ctas;
+  resident_shape(A.G.units, block, ctas);
   const uint32_t ncols = A.G.Q * (uint32_t)L.nj;
   uint32_t seg = 0;
   if (full && !own)
@@ -445,16 +320,7 @@ cudaError_t launch_resident_sweeps(const LatticeView& L, const Coupling& cp, uin
   A.words = words;
   A.nsweeps = nsweeps;
   A.wait_limit = kWaitLimit;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ctas);
-  cfg.blockDim = dim3(block);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kResident[L.periodic ? 1 : 0][form], A);
+  return launch_cooperative(kResident[L.periodic ? 1 : 0][form], ctas, block, stream, A);
 }
 
 }  // namespace chll

@@ -1,0 +1,181 @@
+// What the resident launches share: many passes over one lattice in one
+// cooperative launch whose CTAs meet at a grid barrier between passes (the
+// sweeps of resident.cu, the gradient quench of adjoint.cu).
+#pragma once
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <atomic>
+
+#include "chll_common.cuh"
+#include "chll_physics.cuh"
+#include "sweep.cuh"
+#include "sweep_unit.cuh"
+
+namespace chll {
+
+constexpr int kResThreads = 512;  // most threads per CTA, and per SM (128 registers each)
+constexpr uint32_t kWaitLimit = 1u << 22;  // polls of the word before a wait gives up
+
+// One word per pass, three in rotation, 128 bytes apart: director accepts in
+// bits 0-25, flips in bits 26-51, arrived CTAs in bits 52-63.  The word of pass
+// q is cleared by the first CTA once the barrier of pass q + 1 is through --
+// every CTA has then read it for the last time -- and that CTA's release at
+// pass q + 2 puts the clear before any arrival at pass q + 3, its next use.
+constexpr int kWordStride = 16;
+constexpr int kCountBits = 26;
+constexpr unsigned long long kCountMask = (1ull << kCountBits) - 1;
+constexpr int kArriveShift = 2 * kCountBits;
+
+// Thread 0 of every CTA adds the CTA's counts and arrival to the pass's word
+// (release: the CTA's stores, ordered before it by the CTA barrier, are
+// visible to whoever acquires the word) ...
+__device__ __forceinline__ void grid_arrive(unsigned long long* w, unsigned long long counts,
+                                            uint32_t nct) {
+  if (nct == 1) return;
+  const unsigned long long add = counts + (1ull << kArriveShift);
+  asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(w), "l"(add) : "memory");
+}
+
+// ... and waits until every CTA has (acquire).  Returns the word, or the CTA's
+// own counts of a grid of one CTA; ok = false if the wait ran out.
+__device__ __forceinline__ unsigned long long grid_wait(unsigned long long* w,
+                                                        unsigned long long counts, uint32_t nct,
+                                                        uint32_t limit, bool& ok) {
+  if (nct == 1) return counts;
+  unsigned long long v;
+  uint32_t polls = 0;
+  do {
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(w) : "memory");
+    if ((uint32_t)(v >> kArriveShift) == nct) return v;
+  } while (++polls < limit);
+  ok = false;
+  return v;
+}
+
+// Thread 0 of the CTA that arrives last at the launch's last word: nobody waits
+// for that one, so all three can be cleared for the next launch.
+__device__ __forceinline__ void clear_words(unsigned long long* words) {
+  for (int w = 0; w < 3; ++w) words[w * kWordStride] = 0;
+}
+
+// One unit per thread: the thread keeps both colours' unit g (the 4-site x-block
+// q of row (j, k)) in registers for the whole launch.  The other colour's pair
+// then is the x-row pair of walk_task, so a pass loads the +-y and +-z pairs and
+// one x neighbour, at addresses fixed for the launch.  ni a multiple of 4, or
+// open boundaries (a padding slot reads as the zero of a missing neighbour).
+template <bool P>
+struct OwnBlock {
+  uint32_t g, u, o0;        // unit, its slot, parity of colour 0's sites in the row
+  uint32_t yp, ym, zp, zm;  // slots of the neighbour pairs
+  uint32_t xm, xp;          // the x neighbours outside the block: below, above
+  bool has, hyp, hym, hzp, hzm, hxm, hxp;
+  bool v[4];                // sites 4q .. 4q+3 inside the lattice
+  float4 n[2][2];           // [colour][slot of the pair]
+
+  __device__ __forceinline__ OwnBlock(const LatticeView& L, const SweepGeom& G) {
+    g = blockIdx.x * blockDim.x + threadIdx.x;
+    has = g < G.units;
+    const uint32_t hx = (uint32_t)L.hx, nj = (uint32_t)L.nj, nk = (uint32_t)L.nk;
+    const uint32_t plane = hx * nj;
+    const uint32_t row = G.by_Q.div(g), q = g - row * G.Q;
+    const uint32_t k = G.by_nj.div(row), j = row - k * nj;
+    o0 = (j + k) & 1u;
+    u = 2 * g;
+    hyp = P || j + 1 < nj;
+    hym = P || j > 0;
+    hzp = P || k + 1 < nk;
+    hzm = P || k > 0;
+    hxm = P || q > 0;
+    hxp = P || q + 1 < G.Q;
+    yp = j + 1 < nj ? u + hx : u - (nj - 1) * hx;
+    ym = j > 0 ? u - hx : u + (nj - 1) * hx;
+    zp = k + 1 < nk ? u + plane : u - (nk - 1) * plane;
+    zm = k > 0 ? u - plane : u + (nk - 1) * plane;
+    xm = q > 0 ? u - 1 : u + hx - 1;
+    xp = q + 1 < G.Q ? u + 2 : u - 2 * q;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) v[t] = has && 4 * q + t < (uint32_t)L.ni;
+    n[0][0] = n[0][1] = n[1][0] = n[1][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (has) {
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const UnitSlots s = ld_unit(L.col[c] + u);
+        n[c][0] = s.a;
+        n[c][1] = s.b;
+      }
+    }
+  }
+
+  // Colour C's sites are 4q+1, 4q+3 rather than 4q, 4q+2.
+  template <int C>
+  __device__ __forceinline__ bool odd() const {
+    return (o0 ^ C) != 0;
+  }
+
+  // The neighbours of colour C's two sites; has only.
+  template <int C>
+  __device__ __forceinline__ void neighbours(const LatticeView& L, Nbrs& nb0, Nbrs& nb1) const {
+    const float4* oth = L.col[C ^ 1];
+    const bool o = odd<C>();
+    nbr_units<kLoadCoherentOrdered>(hyp, oth + yp, nb0.b[2], nb1.b[2]);
+    nbr_units<kLoadCoherentOrdered>(hym, oth + ym, nb0.b[3], nb1.b[3]);
+    nbr_units<kLoadCoherentOrdered>(hzp, oth + zp, nb0.b[4], nb1.b[4]);
+    nbr_units<kLoadCoherentOrdered>(hzm, oth + zm, nb0.b[5], nb1.b[5]);
+    float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (o ? hxp : hxm) e = ld4_other<kLoadCoherentOrdered>(oth + (o ? xp : xm));
+    const float4 xa = n[C ^ 1][0], xb = n[C ^ 1][1];
+    nb0.b[0] = o ? xb : xa;
+    nb0.b[1] = o ? xa : e;
+    nb1.b[0] = o ? e : xb;
+    nb1.b[1] = o ? xb : xa;
+  }
+};
+
+// Streaming multiprocessors of the current device (kResThreads threads of a
+// resident launch each).
+inline uint32_t resident_sms() {
+  static std::atomic<int> cache[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::atomic<int>& slot = cache[dev & 63];
+  int n = slot.load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    if (n <= 0) n = 148;
+    slot.store(n, std::memory_order_relaxed);
+  }
+  return (uint32_t)n;
+}
+
+// Whether OwnBlock holds the lattice.
+inline bool one_unit_each(const LatticeView& L, uint32_t units) {
+  return units <= resident_sms() * kResThreads && (L.ni % 4 == 0 || !L.periodic);
+}
+
+// Threads per CTA and CTAs: up to 256 units (two warps per scheduler) one CTA,
+// whose barrier is its own; else the units spread over the SMs in CTAs of whole
+// warps.
+inline void resident_shape(uint32_t units, uint32_t& block, uint32_t& ctas) {
+  const uint32_t sms = resident_sms();
+  const uint32_t share = units <= 256 ? units : (units + sms - 1) / sms;
+  block = std::min<uint32_t>(kResThreads, (share + 31) / 32 * 32);
+  ctas = std::min((units + block - 1) / block, sms * (uint32_t)(kResThreads / block));
+}
+
+template <class KERNEL, class ARGS>
+cudaError_t launch_cooperative(KERNEL kernel, uint32_t ctas, uint32_t block, cudaStream_t stream,
+                               const ARGS& args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(block);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args);
+}
+
+}  // namespace chll

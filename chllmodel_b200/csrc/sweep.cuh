@@ -99,6 +99,14 @@ int energy_grad_max_blocks();
 void launch_quench_pass(const LatticeView& L, const CouplingD& cd, float eta, int colour,
                         cudaStream_t stream);
 
+// adjoint.cu: nsteps quench steps (a pass of colour 0, then 1) in one
+// cooperative launch; words as launch_resident_sweeps.  quench_resident_pays:
+// faster than the passes' launches.
+bool quench_resident_pays(const LatticeView& L);
+cudaError_t launch_quench_resident(const LatticeView& L, const CouplingD& cd, float eta,
+                                   Control* ctl, unsigned long long* words, int nsteps,
+                                   cudaStream_t stream);
+
 // analysis.cu: shell correlations over natural-order float4 sites and a zero
 // site behind them (offsets {di, dj, dk}, chunks {first, end, shell} of at most
 // kCorrChunk offsets of one shell; out = [sum (n.n')^2 per shell, sum s s' per

@@ -173,6 +173,13 @@ class Lattice:
         """nsteps of zero-temperature tangent gradient descent (asynchronous)."""
         check(self._L.chll_lattice_quench(self._h, ct.byref(cp), float(eta), int(nsteps)))
 
+    def energy_sums(self, cp: Coupling) -> np.ndarray:
+        """E, dE/deps, dE/dK, dE/dh without the gradient."""
+        out4 = np.zeros(4, np.float64)
+        check(self._L.chll_lattice_energy_grad(self._h, ct.byref(cp), None, 0,
+                                               out4.ctypes.data_as(ct.c_void_p)))
+        return out4
+
     def energy_grad(self, cp: Coupling, project: bool = False, grad_ptr: int | None = None):
         """Returns (grad (N,4) host array or None if grad_ptr given, out4)."""
         out4 = np.zeros(4, np.float64)
