@@ -15,6 +15,7 @@
 #include <cstdarg>
 #include <cstddef>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -162,6 +163,7 @@ struct chll_lattice {
   unsigned long long* words = nullptr;  // meeting words of the resident sweeps
   double* rows = nullptr;
   int rows_cap = 0;
+  double* host_rows = nullptr;  // pinned, of run()'s lattice
   double* out4 = nullptr;
   void* staging = nullptr;
   size_t staging_bytes = 0;
@@ -537,6 +539,39 @@ void print_row(long long step, const double* row) {
   std::fflush(stdout);
 }
 
+// Host memory of one run's rows.
+constexpr long long kPinnedRows = 4096;  // 512 KB kept per lattice
+
+struct RowBuffer {
+  double* p = nullptr;
+  bool pinned_here = false, plain_here = false;
+
+  cudaError_t reserve(chll_lattice* L, long long rows, bool pinned) {
+    if (rows <= 0) return cudaSuccess;
+    if (!pinned) {
+      p = (double*)std::malloc(sizeof(double) * chll::kRowLen * (size_t)rows);
+      plain_here = p != nullptr;
+      return p ? cudaSuccess : cudaErrorMemoryAllocation;
+    }
+    if (rows > kPinnedRows) {
+      const cudaError_t e = cudaMallocHost(&p, sizeof(double) * chll::kRowLen * rows);
+      pinned_here = e == cudaSuccess;
+      return e;
+    }
+    if (!L->host_rows) {
+      const cudaError_t e =
+          cudaMallocHost(&L->host_rows, sizeof(double) * chll::kRowLen * kPinnedRows);
+      if (e != cudaSuccess) return e;
+    }
+    p = L->host_rows;
+    return cudaSuccess;
+  }
+  ~RowBuffer() {
+    if (pinned_here) cudaFreeHost(p);
+    if (plain_here) std::free(p);
+  }
+};
+
 // Shared body of run() and chll_run_ex().
 int run_impl(const chll_run_config& cfg, int nstart, int nstop, int nout, double* nx, double* ny,
              double* nz, int* s, int ni, int nj, int nk, int* msteps, double* m, double* rows16,
@@ -565,10 +600,12 @@ int run_impl(const chll_run_config& cfg, int nstart, int nstop, int nout, double
   CHLL_TRY(set_control_impl(L, cfg.d, nstart, cfg.adapt_until));
   if (cfg.verbose && nstart == 1) print_header();
 
-  double* host_rows = nullptr;
-  if (rows > 0) {
-    CHLL_CUDA_TRY(cudaMallocHost(&host_rows, sizeof(double) * chll::kRowLen * rows));
-  }
+  // Rows come back as they complete where they are printed, into pinned memory
+  // (the lattice's own up to kPinnedRows; allocating and freeing it took 0.5 to
+  // 6 ms per call), else all together at the end.
+  RowBuffer buffer;
+  CHLL_CUDA_TRY(buffer.reserve(L, rows, cfg.verbose));
+  double* const host_rows = buffer.p;
   std::vector<cudaEvent_t> events;
   std::vector<long long> row_step;
   long long printed = 0, r = 0, dropped = 0;
@@ -580,7 +617,7 @@ int run_impl(const chll_run_config& cfg, int nstart, int nstop, int nout, double
         cudaEventSynchronize(events[printed]);
       else if (cudaEventQuery(events[printed]) != cudaSuccess)
         break;
-      if (cfg.verbose) print_row(row_step[printed], host_rows + printed * chll::kRowLen);
+      print_row(row_step[printed], host_rows + printed * chll::kRowLen);
       ++printed;
     }
   };
@@ -596,12 +633,14 @@ int run_impl(const chll_run_config& cfg, int nstart, int nstop, int nout, double
         double* drow = L->rows + r * chll::kRowLen;
         rc = observe_impl(L, make_coupling_d(cc), drow, end);
         if (rc != CHLL_OK) break;
-        cudaEvent_t ev;
-        cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-        cudaMemcpyAsync(host_rows + r * chll::kRowLen, drow, sizeof(double) * chll::kRowLen,
-                        cudaMemcpyDeviceToHost, L->stream);
-        cudaEventRecord(ev, L->stream);
-        events.push_back(ev);
+        if (cfg.verbose) {
+          cudaEvent_t ev;
+          cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+          cudaMemcpyAsync(host_rows + r * chll::kRowLen, drow, sizeof(double) * chll::kRowLen,
+                          cudaMemcpyDeviceToHost, L->stream);
+          cudaEventRecord(ev, L->stream);
+          events.push_back(ev);
+        }
         row_step.push_back(end);
         ++r;
       } else {
@@ -609,12 +648,15 @@ int run_impl(const chll_run_config& cfg, int nstart, int nstop, int nout, double
       }
     }
     istep = end + 1;
-    flush_rows(false);
+    if (cfg.verbose) flush_rows(false);
   }
+  if (rc == CHLL_OK && !cfg.verbose && r > 0)
+    cudaMemcpyAsync(host_rows, L->rows, sizeof(double) * chll::kRowLen * r, cudaMemcpyDeviceToHost,
+                    L->stream);
   cudaError_t e = cudaStreamSynchronize(L->stream);
   if (rc == CHLL_OK && e != cudaSuccess)
     rc = fail(CHLL_ECUDA, "run: %s", cudaGetErrorString(e));
-  if (rc == CHLL_OK) flush_rows(true);
+  if (rc == CHLL_OK && cfg.verbose) flush_rows(true);
   for (auto ev : events) cudaEventDestroy(ev);
 
   if (rc == CHLL_OK) rc = download_f64_impl(L, nx, ny, nz, s);
@@ -633,7 +675,6 @@ int run_impl(const chll_run_config& cfg, int nstart, int nstop, int nout, double
       if (rows16) std::memcpy(rows16 + q * chll::kRowLen, hr, sizeof(double) * chll::kRowLen);
     }
   }
-  if (host_rows) cudaFreeHost(host_rows);
   if (rc == CHLL_OK && dropped)
     rc = fail(CHLL_ERANGE,
               "run: %lld measurement steps did not fit in the %lld rows of msteps/m "
@@ -751,6 +792,7 @@ void chll_lattice_destroy(chll_lattice* L) {
   cudaFree(L->tickets);
   cudaFree(L->words);
   cudaFree(L->rows);
+  if (L->host_rows) cudaFreeHost(L->host_rows);
   cudaFree(L->out4);
   cudaFree(L->staging);
   cudaFree(L->grad);
