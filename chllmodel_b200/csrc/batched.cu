@@ -552,6 +552,7 @@ struct chll_batch {
   chll::ReplicaDesc* d_desc = nullptr;
   chll::ReplicaState* d_state = nullptr;
   int2* d_cta_replica = nullptr;  // per wave and CTA: its group's replicas
+  size_t cta_replica_cap = 0;
   double* d_partials = nullptr;
   void* staging = nullptr;
   size_t staging_bytes = 0;
@@ -714,9 +715,13 @@ int shape_launch(chll_batch* B) {
   }
   B->grid = budget;
   B->nwaves = (int)waves.size();
-  if (B->d_cta_replica) cudaFree(B->d_cta_replica);
-  B->d_cta_replica = nullptr;
-  BATCH_CUDA(cudaMalloc(&B->d_cta_replica, sizeof(int2) * map.size()));
+  if (B->cta_replica_cap < map.size()) {  // kept from shape to shape (the tuner tries dozens)
+    if (B->d_cta_replica) cudaFree(B->d_cta_replica);
+    B->d_cta_replica = nullptr;
+    B->cta_replica_cap = 0;
+    BATCH_CUDA(cudaMalloc(&B->d_cta_replica, sizeof(int2) * map.size()));
+    B->cta_replica_cap = map.size();
+  }
   BATCH_CUDA(cudaMemcpyAsync(B->d_cta_replica, map.data(), sizeof(int2) * map.size(),
                              cudaMemcpyHostToDevice, B->stream));
   BATCH_CUDA(cudaMemcpyAsync(B->d_desc, B->desc.data(), sizeof(chll::ReplicaDesc) * B->n,
@@ -1237,10 +1242,15 @@ int chll_batch_autotune(chll_batch* B, int trial_sweeps, int* best_threads, int*
   // replicas sharing the grid); each block size at its two highest
   // occupancies (lower occupancies were never faster on this kernel).  Trials
   // measure every 10 sweeps like a production run.
+  // A wave size that holds the whole batch is the one-wave launch again and is
+  // not timed twice, nor is pairing a batch of one.
   const long long kWaveOptions[] = {0ll, 40ll << 20, 64ll << 20, 96ll << 20};
+  long long state_bytes = 0;
+  for (size_t pc : B->per_colour) state_bytes += (long long)(2 * pc * sizeof(float4));
   for (int pair : {1, 0})
   for (long long wb : kWaveOptions)
   for (int threads : {128, 256, 512}) {
+    if (wb >= state_bytes || (pair && B->n == 1)) continue;
     const int occ = occupancy_of(threads);
     for (int c = std::max(1, occ - 1); c <= occ && rc == CHLL_OK; ++c) {
       if (c * threads > 2048) break;
