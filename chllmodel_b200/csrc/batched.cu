@@ -71,9 +71,7 @@ struct ReplicaDesc {
 struct ReplicaState {
   double d;
   long long step;
-  unsigned long long cnt[4];  // director counts by step parity [0,1], flips [2,3]
-  unsigned int bar_count;
-  unsigned int bar_gen;
+  unsigned long long nflip;  // flips of a sweep that ends with its closing pass
   unsigned int status;
   unsigned int pad;
   float paccept, faccept;
@@ -83,80 +81,111 @@ struct ReplicaState {
 
 constexpr int kMomLen = 16;  // chll_batch_moments row
 
+// Threads per CTA are 128, 256 or 512: 128 registers each, so 512 per SM.
+constexpr int kMaxThreads = 512;
+
 
 // Group barrier of one replica's CTAs, split in two so that a CTA can do
-// other work between arriving and waiting (a second replica's pass).
-// group_arrive: every thread of the CTA has finished the phase; thread 0
-// publishes the CTA's writes (fence) and counts itself in, the last CTA of
-// the group advancing the generation word.  Returns, in thread 0, the
-// generation to wait past.
-__device__ unsigned int group_arrive(ReplicaState* st, int nct) {
-  __syncthreads();
-  unsigned int gen = 0;
-  if (threadIdx.x == 0 && nct > 1) {
-    gen = *(volatile unsigned int*)&st->bar_gen;
-    __threadfence();
-    const unsigned int arrived = atomicAdd(&st->bar_count, 1u);
-    if (arrived == (unsigned int)nct - 1) {
-      st->bar_count = 0;
-      __threadfence();
-      atomicAdd(&st->bar_gen, 1u);
-    }
-  }
-  return gen;
-}
+// other work between arriving and waiting (a second replica's pass).  A meeting
+// is one 64-bit word -- the CTAs' director accepts in bits 0-39, their arrivals
+// above -- that thread 0 of each CTA adds to (release) and polls (acquire), so
+// the wait ends with the pass's count.  Three words in rotation, as the resident
+// sweeps' (resident.cuh): the group's first CTA clears a word one meeting later,
+// and the CTA that completes a launch's last meeting, which nobody waits for,
+// clears all three.  The form before it had two fences, an arrival counter and a
+// generation word per meeting, added the counts apart and read them back, and
+// every pass read its replica's descriptor from L2 again (it is in shared memory
+// now).  us per sweep, then and now: one 32^3 replica 11.3 and 7.6, 4 of 64^3 21.6
+// and 17.2, 16 of 48^3 28.2 and 23.6, 64 of 64^3 190 and 178, the 64-replica grid
+// of 32^3, 48^3 and 64^3 110.5 and 102.
+constexpr int kMeetShift = 40;
+constexpr unsigned long long kMeetCount = (1ull << kMeetShift) - 1;
+constexpr int kMeetStride = 16;  // words 128 bytes apart
+constexpr size_t kMeetWords = 3 * kMeetStride;  // per replica
 
-// Waits until the generation moved past `gen` (every CTA of the group
-// arrived).  Every wait is bounded: after `limit` polls it sets the replica's
-// status word.  Returns false, in every thread, if the status word is set (a
-// wait gave up here or in another CTA of the group).
-__device__ bool group_wait(ReplicaState* st, int nct, unsigned int gen,
-                           unsigned long long limit) {
-  __shared__ int s_ok;
-  if (threadIdx.x == 0) {
-    volatile unsigned int* genp = &st->bar_gen;
-    volatile unsigned int* statp = &st->status;
-    if (nct > 1) {
-      unsigned long long it = 0;
-      while (*genp == gen) {
-        if (*statp) break;
-        if (++it > limit) {
-          atomicOr(&st->status, 1u);
-          break;
-        }
-        if (it > 64) __nanosleep(32);
-      }
-      __threadfence();
-    }
-    s_ok = *statp == 0;
-  }
-  __syncthreads();
-  return s_ok != 0;
-}
+// One replica as seen by one CTA of its group: where it is in its sweeps.
+struct RepCtx {
+  const ReplicaDesc* D;      // in shared memory
+  ReplicaState* st;
+  unsigned long long* words;
+  int rank, nct, which;      // which: 0 or 1, the replica's place in its group
+  int slot;                  // word of the next meeting
+  double d;
+  long long step;
+  bool pending;              // colour-0 flips of the previous sweep still to run
+  float paccept;             // thread 0
+  unsigned long long nacc;   // thread 0: director accepts of the sweep so far
+};
 
-// CTA sums of three counts, valid in thread 0.
-template <int THREADS>
-__device__ __forceinline__ void cta_sum3(unsigned int& a, unsigned int& b, unsigned int& c) {
-  __shared__ unsigned int s_w[3][THREADS / 32];
-  a = __reduce_add_sync(0xffffffffu, a);
-  b = __reduce_add_sync(0xffffffffu, b);
-  c = __reduce_add_sync(0xffffffffu, c);
+struct GroupShared {
+  alignas(16) uint32_t desc_words[2][sizeof(ReplicaDesc) / 4];
+  unsigned int cnt[2][2][kMaxThreads / 32];  // [which][accepts, flips][warp]
+  double d[2];
+  int ok[2];
+  double m[kMaxThreads / 32][kObsMoments];  // a measurement's warp sums
+};
+
+// Every thread of the CTA: the pass is done; its counts (flips only where they
+// are wanted) and the arrival go out.  Returns the word's value before this CTA
+// in thread 0 if LAST (the launch's last meeting), with the others' writes
+// acquired.
+template <bool LAST>
+__device__ __forceinline__ unsigned long long meet_arrive(RepCtx& c, GroupShared& S,
+                                                          unsigned int na, unsigned int nf,
+                                                          bool flips) {
+  const int warp = threadIdx.x >> 5;
+  na = __reduce_add_sync(0xffffffffu, na);
+  if (flips) nf = __reduce_add_sync(0xffffffffu, nf);
   if ((threadIdx.x & 31) == 0) {
-    s_w[0][threadIdx.x >> 5] = a;
-    s_w[1][threadIdx.x >> 5] = b;
-    s_w[2][threadIdx.x >> 5] = c;
+    S.cnt[c.which][0][warp] = na;
+    if (flips) S.cnt[c.which][1][warp] = nf;
   }
-  __syncthreads();
+  __syncthreads();  // the CTA's stores before thread 0's release
+  unsigned long long before = 0;
   if (threadIdx.x == 0) {
-    a = b = c = 0;
-    for (int w = 0; w < THREADS / 32; ++w) {
-      a += s_w[0][w];
-      b += s_w[1][w];
-      c += s_w[2][w];
+    unsigned long long a = 0, f = 0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
+      a += S.cnt[c.which][0][w];
+      if (flips) f += S.cnt[c.which][1][w];
     }
+    if (f) atomicAdd(&c.st->nflip, f);
+    unsigned long long* const word = c.words + c.slot * kMeetStride;
+    const unsigned long long add = a + (1ull << kMeetShift);
+    if (c.nct == 1)
+      c.nacc += a;
+    else if (LAST)
+      asm volatile("atom.acq_rel.gpu.global.add.u64 %0, [%1], %2;"
+                   : "=l"(before)
+                   : "l"(word), "l"(add)
+                   : "memory");
+    else
+      asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(word), "l"(add) : "memory");
   }
-  __syncthreads();
+  return before;
 }
+
+// Waits until every CTA of the group has arrived; adds the meeting's count to
+// c.nacc (thread 0).  Every wait is bounded: after `limit` polls it sets the
+// replica's status word.  Thread 0 of each CTA returns false if the status word
+// is set (a wait gave up here or in another CTA of the group).
+__device__ __forceinline__ bool meet_wait(RepCtx& c, unsigned long long limit) {
+  unsigned long long* const word = c.words + c.slot * kMeetStride;
+  if (c.nct > 1) {
+    unsigned long long v, polls = 0;
+    for (;;) {
+      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(word) : "memory");
+      if ((int)(v >> kMeetShift) == c.nct) break;
+      if (++polls >= limit) atomicOr(&c.st->status, 1u);
+      if ((polls >= limit || polls % 64 == 0) && *(volatile unsigned int*)&c.st->status)
+        return false;
+    }
+    c.nacc += v & kMeetCount;
+    if (c.rank == 0) c.words[(c.slot == 0 ? 2 : c.slot - 1) * kMeetStride] = 0;
+  }
+  return true;
+}
+
+__device__ __forceinline__ void meet_next(RepCtx& c) { c.slot = c.slot == 2 ? 0 : c.slot + 1; }
 
 // The other colour is read through the coherent path (sweep_unit.cuh
 // ld_other): it was written by other CTAs of the group earlier in this launch.
@@ -165,7 +194,9 @@ constexpr int kCoherent = kLoadCoherent;
 // One fused pass (sweep.cuh FusedPhase) of a replica by its CTA group: the
 // group's CTAs walk the replica's units grid-stride with the plain kernels'
 // unit_step, so the chain is the one the replica follows alone.
-template <int PHASE, bool PERIODIC, bool FULL, int THREADS>
+// KERNEL only gives each kernel its own copy (ptxas 12.9 fails on kernels that
+// share these functions).
+template <int PHASE, bool PERIODIC, bool FULL, int KERNEL>
 __device__ __noinline__ void group_loop(const ReplicaDesc& D, int rank, int nct,
                                            uint32_t step, float d, unsigned int& nacc,
                                            unsigned int& nflip) {
@@ -182,35 +213,35 @@ __device__ __noinline__ void group_loop(const ReplicaDesc& D, int rank, int nct,
   const Coupling cp = D.cp;
   const PhiloxKeys key = philox_keys(D.key0, D.key1);
   const uint32_t replica = D.replica;
-  const uint32_t stride = (uint32_t)nct * THREADS;
+  const uint32_t stride = (uint32_t)nct * blockDim.x;
   if (FULL && D.W.seg > 0) {
     const WalkGeom W = D.W;
-    for (uint32_t t = (uint32_t)rank * THREADS + threadIdx.x; t < W.ntasks; t += stride)
+    for (uint32_t t = (uint32_t)rank * blockDim.x + threadIdx.x; t < W.ntasks; t += stride)
       walk_task<C, PERIODIC, PERIODIC, FLIP_BEFORE, DIR, FLIP_AFTER, kCoherent>(
           L, W, t, step, d, cp, key, replica, nacc, nflip);
     return;
   }
   const uint32_t plane = (uint32_t)L.hx * (uint32_t)L.nj;
   const uint32_t per_colour = plane * (uint32_t)L.nk;
-  for (uint32_t g = (uint32_t)rank * THREADS + threadIdx.x; g < G.units; g += stride) {
+  for (uint32_t g = (uint32_t)rank * blockDim.x + threadIdx.x; g < G.units; g += stride) {
     if (g + stride < G.units) prefetch_unit<C>(L, g + stride, plane, per_colour);
     unit_step<C, PERIODIC, PERIODIC, FLIP_BEFORE, DIR, FLIP_AFTER, FULL, kCoherent>(
         L, G, g, step, d, cp, key, replica, nacc, nflip);
   }
 }
 
-template <int PHASE, int THREADS>
+template <int PHASE, int KERNEL>
 __device__ __forceinline__ void group_pass(const ReplicaDesc& D, int rank, int nct,
                                            uint32_t step, float d, unsigned int& nacc,
                                            unsigned int& nflip) {
   // a replica whose ni is a multiple of 4 has no padding slots
   const bool full = D.L.ni % 4 == 0;
   if (D.L.periodic) {
-    if (full) group_loop<PHASE, true, true, THREADS>(D, rank, nct, step, d, nacc, nflip);
-    else group_loop<PHASE, true, false, THREADS>(D, rank, nct, step, d, nacc, nflip);
+    if (full) group_loop<PHASE, true, true, KERNEL>(D, rank, nct, step, d, nacc, nflip);
+    else group_loop<PHASE, true, false, KERNEL>(D, rank, nct, step, d, nacc, nflip);
   } else {
-    if (full) group_loop<PHASE, false, true, THREADS>(D, rank, nct, step, d, nacc, nflip);
-    else group_loop<PHASE, false, false, THREADS>(D, rank, nct, step, d, nacc, nflip);
+    if (full) group_loop<PHASE, false, true, KERNEL>(D, rank, nct, step, d, nacc, nflip);
+    else group_loop<PHASE, false, false, KERNEL>(D, rank, nct, step, d, nacc, nflip);
   }
 }
 
@@ -218,26 +249,25 @@ __device__ __forceinline__ void group_pass(const ReplicaDesc& D, int rank, int n
 // partial sums into its slot (slot = 2 * CTA + which replica of its group).
 // Kept out of line: it runs once per measurement and its FP64 registers would
 // otherwise crowd the sweep loop.
-template <int THREADS>
+template <int KERNEL>
 __device__ __noinline__ void measure_partials(const ReplicaDesc& D, int rank, int nct,
-                                              double* __restrict__ slot) {
+                                              GroupShared& S, double* __restrict__ slot) {
   double m[kObsMoments];
 #pragma unroll
   for (int t = 0; t < kObsMoments; ++t) m[t] = 0.0;
   const uint64_t total = 2ull * D.M.per_colour;  // < 2^32
-  for (uint64_t e = (uint64_t)rank * THREADS + threadIdx.x; e < total;
-       e += (uint64_t)nct * THREADS)
+  for (uint64_t e = (uint64_t)rank * blockDim.x + threadIdx.x; e < total;
+       e += (uint64_t)nct * blockDim.x)
     site_moments<false>(D.L, D.M, D.cd, (uint32_t)e, m);
-  __shared__ double s_m[THREADS / 32][kObsMoments];
 #pragma unroll
   for (int t = 0; t < kObsMoments; ++t) {
     const double v = warp_sum_d(m[t]);
-    if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5][t] = v;
+    if ((threadIdx.x & 31) == 0) S.m[threadIdx.x >> 5][t] = v;
   }
   __syncthreads();
   if (threadIdx.x < kObsMoments) {
     double v = 0.0;
-    for (int w = 0; w < THREADS / 32; ++w) v += s_m[w][threadIdx.x];
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += S.m[w][threadIdx.x];
     slot[threadIdx.x] = v;
   }
 }
@@ -246,9 +276,10 @@ __device__ __noinline__ void measure_partials(const ReplicaDesc& D, int rank, in
 // moment per thread in CTA order, and accumulates e = E/N, eta = sum(s)/N and
 // S into the replica's state block.  L2 loads (the partials come from other
 // SMs; the barrier's fences made them visible there).
+template <int KERNEL>
 __device__ __noinline__ void measure_sum(const ReplicaDesc& D, ReplicaState* st, int nct,
-                                         const double* __restrict__ first_slot) {
-  __shared__ double s_tot[kObsMoments];
+                                         GroupShared& S, const double* __restrict__ first_slot) {
+  double* const s_tot = S.m[0];
   if (threadIdx.x < kObsMoments) {
     double v = 0.0;
     for (int c = 0; c < nct; ++c) v += __ldcg(first_slot + (size_t)c * 2 * kObsMoments +
@@ -279,179 +310,153 @@ __device__ __noinline__ void measure_sum(const ReplicaDesc& D, ReplicaState* st,
   __syncthreads();
 }
 
-// One replica as seen by one CTA of its group: where it is in its sweeps.
-struct RepCtx {
-  const ReplicaDesc* D;
-  ReplicaState* st;
-  int rank, nct, which;  // which: 0 or 1, the replica's place in its group
-  double d;
-  long long step;
-  bool pending;          // colour-0 flips of the previous sweep still to run
-  unsigned int gen;      // generation of the last arrival at the group barrier
-  unsigned int na, nf_prev, nf;
-};
-
-__device__ __forceinline__ void ctx_init(RepCtx& c, const ReplicaDesc* descs,
-                                         ReplicaState* states, int rep, int which) {
-  c.D = descs + rep;
-  c.st = states + rep;
-  c.rank = (int)blockIdx.x - c.D->cta_first;
-  c.nct = c.D->cta_count;
-  c.which = which;
-  c.d = c.st->d;
-  c.step = c.st->step;
-  c.pending = false;
-  c.gen = 0;
+// Thread 0 of the CTA that completes a launch's last meeting: the replica's
+// control values, and the words cleared for the next launch.
+__device__ __forceinline__ void close_run(RepCtx& c) {
+  const unsigned long long nf = atomicExch(&c.st->nflip, 0ull);
+  c.st->d = c.d;
+  c.st->step = c.step;
+  c.st->paccept = c.paccept;
+  c.st->faccept = (float)nf / (float)c.D->nsites;
+  if (c.nct > 1)
+    for (int w = 0; w < 3; ++w) c.words[w * kMeetStride] = 0;
 }
 
 // The fused two-pass sweep of the plain kernels (sweep.cu): pass A = the
 // previous sweep's colour-0 flips (when pending) + colour-0 director trials,
 // pass B = colour-1 director trials + colour-1 flips, and a colour-0 flip
-// pass F closes the sweep before a measurement and after the last sweep.
-// Counts: director accepts of step t in cnt[t&1], flips of step t in
-// cnt[2 + (t&1)].  Each phase below ends where the group must meet; the
-// caller arrives at the group barrier after it and waits before the next.
-
-template <int THREADS>
-__device__ __forceinline__ void phase_a(RepCtx& c) {
-  c.na = c.nf_prev = c.nf = 0;
-  if (c.pending)
-    group_pass<kFusedA, THREADS>(*c.D, c.rank, c.nct, (uint32_t)c.step, (float)c.d, c.na,
-                                 c.nf_prev);
-  else
-    group_pass<kFusedA0, THREADS>(*c.D, c.rank, c.nct, (uint32_t)c.step, (float)c.d, c.na,
-                                  c.nf_prev);
-}
-
-template <int THREADS>
-__device__ __forceinline__ void phase_b(RepCtx& c) {
-  group_pass<kFusedB, THREADS>(*c.D, c.rank, c.nct, (uint32_t)c.step, (float)c.d, c.na, c.nf);
-}
-
-template <int THREADS>
-__device__ __forceinline__ void phase_f(RepCtx& c) {
-  group_pass<kFusedF, THREADS>(*c.D, c.rank, c.nct, (uint32_t)c.step + 1u, (float)c.d, c.na,
-                               c.nf);
-}
-
-// The CTA's counts of the sweep into the replica's counters.
-template <int THREADS>
-__device__ __forceinline__ void phase_counts(RepCtx& c) {
-  unsigned int na = c.na, nfp = c.nf_prev, nf = c.nf;
-  cta_sum3<THREADS>(na, nfp, nf);
-  if (threadIdx.x == 0) {
-    const int par = (int)(c.step & 1);
-    if (na) atomicAdd(&c.st->cnt[par], (unsigned long long)na);
-    if (nfp) atomicAdd(&c.st->cnt[2 + (par ^ 1)], (unsigned long long)nfp);
-    if (nf) atomicAdd(&c.st->cnt[2 + par], (unsigned long long)nf);
-  }
-}
-
-// After the count barrier: every CTA of the group derives the same new d
-// from the group's count (chll_mod.f90:83-90).  The counters read here are
-// reset by the group's first CTA for their next use, which no CTA reaches
-// before it passes the next barrier.
-__device__ __forceinline__ void phase_d(RepCtx& c, bool flush) {
-  __shared__ double s_d[2];
-  if (threadIdx.x == 0) {
-    ReplicaState* st = c.st;
-    const int par = (int)(c.step & 1);
-    const float n3 = (float)c.D->nsites;
-    const unsigned long long na_all = *((volatile unsigned long long*)&st->cnt[par]);
-    const float pa = (float)na_all / n3;
-    s_d[c.which] = (c.step < c.D->adapt_until) ? adapt_d(c.d, pa) : c.d;
-    if (c.rank == 0) {
-      st->cnt[par ^ 1] = 0;
-      st->paccept = pa;
-      if (c.pending) {  // flips of step-1 are complete (chll_mod.f90:93)
-        st->faccept = (float)*((volatile unsigned long long*)&st->cnt[2 + (par ^ 1)]) / n3;
-        st->cnt[2 + (par ^ 1)] = 0;
-      }
-      if (flush) {
-        st->faccept = (float)*((volatile unsigned long long*)&st->cnt[2 + par]) / n3;
-        st->cnt[2 + par] = 0;
-      }
-    }
+// pass F closes the sweep before a measurement and after the last sweep.  Only
+// a sweep that F closes needs its flips counted (faccept, chll_mod.f90:93): B's
+// and F's go to the replica's nflip.
+//
+// All sweeps of the one or two replicas of this CTA's group.  With two, the
+// CTA alternates them phase by phase: after arriving at one replica's meeting it
+// runs the other replica's phase, and only then waits, so a wait for the group's
+// slowest CTA overlaps useful work.  Each replica follows exactly the chain it
+// follows alone.  Returns false if a group's status word was set (a wait gave
+// up).
+template <int NREP>
+__device__ bool run_group(const ReplicaDesc* __restrict__ descs,
+                          ReplicaState* __restrict__ states, unsigned long long* words,
+                          GroupShared& S, int2 reps, double* __restrict__ partials,
+                          int nsweeps, int measure_every, int measure_from,
+                          unsigned long long limit) {
+  RepCtx c[NREP];
+  const int nrep = NREP == 2 && reps.y >= 0 ? 2 : 1;
+  __syncthreads();  // the descriptors of the wave before are no longer read
+  for (int r = 0; r < nrep; ++r) {
+    const int rep = r ? reps.y : reps.x;
+    const uint32_t* from = reinterpret_cast<const uint32_t*>(descs + rep);
+    for (uint32_t w = threadIdx.x; w < sizeof(ReplicaDesc) / 4; w += blockDim.x)
+      S.desc_words[r][w] = from[w];
   }
   __syncthreads();
-  c.d = s_d[c.which];
-  c.pending = !flush;
-  ++c.step;
-}
-
-// All sweeps of the one or two replicas of this CTA's group.  With two, the
-// CTA alternates them phase by phase: after arriving at one replica's group
-// barrier it runs the other replica's phase, and only then waits, so a wait
-// for the group's slowest CTA overlaps useful work.  Each replica follows
-// exactly the chain it follows alone.  Returns false if a group's status
-// word was set (a barrier wait gave up).
-template <int THREADS>
-__device__ bool run_group(const ReplicaDesc* __restrict__ descs,
-                          ReplicaState* __restrict__ states, int2 reps,
-                          double* __restrict__ partials, int nsweeps, int measure_every,
-                          int measure_from, unsigned long long limit) {
-  RepCtx c[2];
-  const int nrep = reps.y >= 0 ? 2 : 1;
-  ctx_init(c[0], descs, states, reps.x, 0);
-  if (nrep == 2) ctx_init(c[1], descs, states, reps.y, 1);
-#define CHLL_EACH(body)                 \
+  for (int r = 0; r < nrep; ++r) {
+    RepCtx& x = c[r];
+    const int rep = r ? reps.y : reps.x;
+    x.D = reinterpret_cast<const ReplicaDesc*>(S.desc_words[r]);
+    x.st = states + rep;
+    x.words = words + (size_t)rep * kMeetWords;
+    x.rank = (int)blockIdx.x - x.D->cta_first;
+    x.nct = x.D->cta_count;
+    x.which = r;
+    x.slot = 0;
+    x.d = x.st->d;
+    x.step = x.st->step;
+    x.pending = false;
+    x.nacc = 0;
+    if (threadIdx.x == 0) S.ok[r] = x.st->status == 0;
+  }
+  __syncthreads();
+  if (!S.ok[0] || (nrep == 2 && !S.ok[1])) return false;  // an earlier wait gave up
+#define CHLL_EACH(...)                  \
   for (int r = 0; r < nrep; ++r) {      \
     RepCtx& x = c[r];                   \
-    body;                               \
+    __VA_ARGS__;                        \
   }
-#define CHLL_WAIT() \
-  if (!group_wait(x.st, x.nct, x.gen, limit)) return false
-#define CHLL_ARRIVE() x.gen = group_arrive(x.st, x.nct)
+// thread 0 waits and does `then`; every thread goes on with what it left
+#define CHLL_WAIT(...)                  \
+  if (threadIdx.x == 0) {               \
+    S.ok[r] = meet_wait(x, limit);      \
+    __VA_ARGS__;                        \
+  }                                     \
+  meet_next(x);                         \
+  __syncthreads();                      \
+  if (!S.ok[r]) return false
   for (int s = 0; s < nsweeps; ++s) {
     const int done = s + 1;
     const bool measure =
         measure_every > 0 && done >= measure_from && done % measure_every == 0;
-    const bool flush = measure || done == nsweeps;
+    const bool last = done == nsweeps;
+    const bool flush = measure || last;
+    unsigned int na, nf;
     CHLL_EACH({
-      phase_a<THREADS>(x);
-      CHLL_ARRIVE();
+      na = nf = 0;
+      if (x.pending)
+        group_pass<kFusedA, NREP>(*x.D, x.rank, x.nct, (uint32_t)x.step, (float)x.d, na, nf);
+      else
+        group_pass<kFusedA0, NREP>(*x.D, x.rank, x.nct, (uint32_t)x.step, (float)x.d, na, nf);
+      meet_arrive<false>(x, S, na, 0, false);
     });
     CHLL_EACH({
-      CHLL_WAIT();
-      phase_b<THREADS>(x);
-      if (!flush) phase_counts<THREADS>(x);
-      CHLL_ARRIVE();
+      CHLL_WAIT({});
+      na = nf = 0;
+      group_pass<kFusedB, NREP>(*x.D, x.rank, x.nct, (uint32_t)x.step, (float)x.d, na, nf);
+      meet_arrive<false>(x, S, na, nf, flush);
     });
-    if (flush) {
-      CHLL_EACH({
-        CHLL_WAIT();
-        phase_f<THREADS>(x);
-        phase_counts<THREADS>(x);
-        CHLL_ARRIVE();
+    CHLL_EACH({
+      // every CTA of the group derives the same new d from the group's count
+      // (chll_mod.f90:83-90)
+      CHLL_WAIT({
+        x.paccept = (float)x.nacc / (float)x.D->nsites;
+        S.d[r] = x.step < x.D->adapt_until ? adapt_d(x.d, x.paccept) : x.d;
+        x.nacc = 0;
       });
-    }
-    CHLL_EACH({
-      CHLL_WAIT();
-      phase_d(x, flush);
-      if (measure) {  // FP64 measurement of the completed sweep
-        measure_partials<THREADS>(*x.D, x.rank, x.nct,
-                                  partials + ((size_t)blockIdx.x * 2 + x.which) * kObsMoments);
-        CHLL_ARRIVE();
+      x.d = S.d[r];
+      x.pending = !flush;
+      ++x.step;
+      if (flush) {
+        na = nf = 0;
+        group_pass<kFusedF, NREP>(*x.D, x.rank, x.nct, (uint32_t)x.step, (float)x.d, na, nf);
+        if (!last || measure) meet_arrive<false>(x, S, 0, nf, true);
+        else {
+          const unsigned long long before = meet_arrive<true>(x, S, 0, nf, true);
+          if (threadIdx.x == 0 && (int)(before >> kMeetShift) == x.nct - 1) close_run(x);
+        }
       }
     });
     if (measure) {
       CHLL_EACH({
-        CHLL_WAIT();
-        if (x.rank == 0)
-          measure_sum(*x.D, x.st, x.nct,
-                      partials + ((size_t)x.D->cta_first * 2 + x.which) * kObsMoments);
+        CHLL_WAIT({ x.nacc = 0; });
+        // FP64 measurement of the completed sweep
+        measure_partials<NREP>(*x.D, x.rank, x.nct, S,
+                         partials + ((size_t)blockIdx.x * 2 + x.which) * kObsMoments);
+        const double* const first =
+            partials + ((size_t)x.D->cta_first * 2 + x.which) * kObsMoments;
+        if (last) {
+          const unsigned long long before = meet_arrive<true>(x, S, 0, 0, false);
+          if (threadIdx.x == 0) S.ok[r] = (int)(before >> kMeetShift) == x.nct - 1;
+          __syncthreads();
+          if (S.ok[r]) {
+            measure_sum<NREP>(*x.D, x.st, x.nct, S, first);
+            if (threadIdx.x == 0) close_run(x);
+          }
+          __syncthreads();
+        } else {
+          meet_arrive<false>(x, S, 0, 0, false);
+        }
       });
+      if (!last)
+        CHLL_EACH({
+          CHLL_WAIT({ x.nacc = 0; if (x.rank == 0) x.st->nflip = 0; });
+          if (x.rank == 0)
+            measure_sum<NREP>(*x.D, x.st, x.nct, S,
+                        partials + ((size_t)x.D->cta_first * 2 + x.which) * kObsMoments);
+        });
     }
   }
 #undef CHLL_EACH
 #undef CHLL_WAIT
-#undef CHLL_ARRIVE
-  if (threadIdx.x == 0)
-    for (int r = 0; r < nrep; ++r)
-      if (c[r].rank == 0) {
-        c[r].st->d = c[r].d;
-        c[r].st->step = c[r].step;
-      }
   return true;
 }
 
@@ -460,16 +465,18 @@ __device__ bool run_group(const ReplicaDesc* __restrict__ descs,
 // ({-1, -1}: idle in this wave).  Waves hold replicas whose state together
 // fits the wave size, so each wave's sweeps can run from L2; CTAs move to
 // their next wave as soon as their group is done.
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS, 512 / THREADS)
+template <bool PAIRED>
+__global__ void __launch_bounds__(kMaxThreads, 1)
     batch_kernel(const ReplicaDesc* __restrict__ descs, ReplicaState* __restrict__ states,
-                 const int2* __restrict__ cta_map, int nwaves, double* __restrict__ partials,
-                 int nsweeps, int measure_every, int measure_from, unsigned long long limit) {
+                 unsigned long long* words, const int2* __restrict__ cta_map, int nwaves,
+                 double* __restrict__ partials, int nsweeps, int measure_every, int measure_from,
+                 unsigned long long limit) {
+  __shared__ GroupShared S;
   for (int w = 0; w < nwaves; ++w) {
     const int2 reps = cta_map[(size_t)w * gridDim.x + blockIdx.x];
     if (reps.x < 0) continue;
-    if (!run_group<THREADS>(descs, states, reps, partials, nsweeps, measure_every,
-                            measure_from, limit))
+    if (!run_group<PAIRED ? 2 : 1>(descs, states, words, S, reps, partials, nsweeps, measure_every,
+                                   measure_from, limit))
       return;
   }
 }
@@ -508,16 +515,10 @@ __global__ void controls_to_states(const Control* __restrict__ ctl,
 namespace chll {
 namespace {
 
-using BatchKernel = void (*)(const ReplicaDesc*, ReplicaState*, const int2*, int, double*, int,
-                             int, int, unsigned long long);
+using BatchKernel = void (*)(const ReplicaDesc*, ReplicaState*, unsigned long long*, const int2*,
+                             int, double*, int, int, int, unsigned long long);
 
-BatchKernel kernel_for(int threads) {
-  switch (threads) {
-    case 128: return batch_kernel<128>;
-    case 512: return batch_kernel<512>;
-    default: return batch_kernel<256>;
-  }
-}
+BatchKernel kernel_for(bool paired) { return paired ? batch_kernel<true> : batch_kernel<false>; }
 
 int fail(int code, const char* fmt, ...) {
   char buf[512];
@@ -551,6 +552,7 @@ struct chll_batch {
   size_t slots = 0;
   chll::ReplicaDesc* d_desc = nullptr;
   chll::ReplicaState* d_state = nullptr;
+  unsigned long long* d_words = nullptr;  // kMeetWords per replica, zero between launches
   int2* d_cta_replica = nullptr;  // per wave and CTA: its group's replicas
   size_t cta_replica_cap = 0;
   double* d_partials = nullptr;
@@ -593,9 +595,9 @@ namespace {
 
 using chll::fail;
 
-int occupancy_of(int threads) {
+int occupancy_of(int threads, bool paired) {
   int n = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, chll::kernel_for(threads), threads, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, chll::kernel_for(paired), threads, 0);
   return n;
 }
 
@@ -626,7 +628,7 @@ int shape_launch(chll_batch* B) {
   if (B->shape_threads == B->threads && B->shape_ctas == B->ctas_per_sm &&
       B->shape_wave_bytes == B->wave_bytes && B->shape_pair == B->pair && B->grid > 0)
     return CHLL_OK;
-  const int occ = occupancy_of(B->threads);
+  const int occ = occupancy_of(B->threads, B->pair);
   if (occ <= 0) return fail(CHLL_ECUDA, "batch: kernel with %d threads cannot run", B->threads);
   const int per_sm = std::min(B->ctas_per_sm > 0 ? std::min(B->ctas_per_sm, occ) : occ,
                               chll::kMaxCtasPerSm);
@@ -745,8 +747,8 @@ int launch_batch(chll_batch* B, cudaStream_t s, int nsweeps, int every, int from
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  BATCH_CUDA(cudaLaunchKernelEx(&cfg, chll::kernel_for(B->threads),
-                                (const chll::ReplicaDesc*)B->d_desc, B->d_state,
+  BATCH_CUDA(cudaLaunchKernelEx(&cfg, chll::kernel_for(B->pair),
+                                (const chll::ReplicaDesc*)B->d_desc, B->d_state, B->d_words,
                                 (const int2*)B->d_cta_replica, B->nwaves, B->d_partials, nsweeps,
                                 every, from,
                                 B->limit));
@@ -971,10 +973,20 @@ int chll_batch_create(const chll_replica_spec* specs, int n, chll_batch** out) {
   if ((e = cudaStreamCreateWithFlags(&B->capture_stream, cudaStreamNonBlocking)))
     return bail(e, "stream");
   B->stream = B->own_stream;
+  // Threads per CTA until set_tuning or the tuner says otherwise: 128 for
+  // replicas of different sizes, whose groups then share every SM four by four
+  // and fill each other's waits (the 64-replica grid 93.4 against 102.1 us per
+  // sweep, 20 replicas of 16^3 to 54^3 19.1 against 21.6), 256 for equal ones (64 of
+  // 32^3 25.5 against 26.6, 64 of 64^3 178 against 182).
+  for (int r = 1; r < n; ++r)
+    if (B->per_colour[r] != B->per_colour[0]) B->threads = 128;
   if ((e = cudaMalloc(&B->lat, slots * sizeof(float4)))) return bail(e, "lattices");
   if ((e = cudaMemsetAsync(B->lat, 0, slots * sizeof(float4), B->stream))) return bail(e, "memset");
   if ((e = cudaMalloc(&B->d_desc, sizeof(chll::ReplicaDesc) * n))) return bail(e, "descriptors");
   if ((e = cudaMalloc(&B->d_state, sizeof(chll::ReplicaState) * n))) return bail(e, "states");
+  const size_t word_bytes = sizeof(unsigned long long) * chll::kMeetWords * n;
+  if ((e = cudaMalloc(&B->d_words, word_bytes))) return bail(e, "meeting words");
+  if ((e = cudaMemsetAsync(B->d_words, 0, word_bytes, B->stream))) return bail(e, "memset");
   if ((e = cudaMalloc(&B->d_partials,
                       sizeof(double) * chll::kObsMoments * B->sms * chll::kMaxCtasPerSm * 2)))
     return bail(e, "partials");
@@ -1034,6 +1046,7 @@ void chll_batch_destroy(chll_batch* B) {
   cudaFree(B->lat);
   cudaFree(B->d_desc);
   cudaFree(B->d_state);
+  cudaFree(B->d_words);
   cudaFree(B->d_cta_replica);
   cudaFree(B->d_partials);
   cudaFree(B->staging);
@@ -1251,7 +1264,7 @@ int chll_batch_autotune(chll_batch* B, int trial_sweeps, int* best_threads, int*
   for (long long wb : kWaveOptions)
   for (int threads : {128, 256, 512}) {
     if (wb >= state_bytes || (pair && B->n == 1)) continue;
-    const int occ = occupancy_of(threads);
+    const int occ = occupancy_of(threads, pair);
     for (int c = std::max(1, occ - 1); c <= occ && rc == CHLL_OK; ++c) {
       if (c * threads > 2048) break;
       B->threads = threads;

@@ -1,0 +1,53 @@
+"""The batch's meetings: groups of one and of many CTAs, paired and single, in
+one wave and several, with and without measurements, run after run -- every
+replica equal to the same lattice swept alone, control values included."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("threads,paired,wave_bytes", [
+    (None, False, 0), (128, True, 0), (256, False, 0), (512, True, 0), (128, False, 1 << 20),
+    (256, True, 3 << 20),
+])
+def test_replicas_follow_their_lattices(threads, paired, wave_bytes):
+    from chllmodel_b200.batched import Batch, replica
+    from chllmodel_b200.lattice import Lattice, coupling
+    from chllmodel_b200.observables import B_D, B_FACCEPT, B_NMEAS, B_PACCEPT, B_STEP
+
+    specs = [replica(8, kT=0.5, K=0.9, g=0.1, seed=3, replica=0),
+             replica(40, 36, 44, kT=0.7, K=0.5, seed=4, replica=1),
+             replica(30, 18, 10, kT=0.3, K=1.0, seed=5, replica=2, boundary="open"),
+             replica(64, kT=1.1, K=1.0, g=0.3, seed=(7 << 33) + 1, replica=3),
+             replica(5, 3, 7, kT=0.4, K=0.2, seed=6, replica=4, boundary="open")]
+    runs = ((7, 3), (1, 1), (5, 0), (6, 3))  # sweeps, measured every
+    with Batch(specs) as b:
+        if threads:
+            b.set_tuning(threads, 0, wave_bytes, paired, False)
+        b.init_random()
+        for n, every in runs:
+            b.run(n, every)
+        m = b.moments()
+        states = [b.download_f4(r) for r in range(len(specs))]
+    for r, sp in enumerate(specs):
+        lat = Lattice(sp["ni"], sp["nj"], sp["nk"], boundary=sp["boundary"])
+        lat.set_kernel("fused")
+        lat.init_random(sp["seed"], sp["replica"])
+        lat.set_control(sp["d"], step=1)
+        cp = coupling(sp["kT"], sp["K"], sp["g"], sp["eps"])
+        rows = []
+        for n, every in runs:
+            for i in range(n):
+                lat.sweep(cp, 1, seed=sp["seed"], replica=sp["replica"])
+                if every and (i + 1) % every == 0:
+                    rows.append(lat.observe(cp))
+        assert np.array_equal(states[r], lat.download_f4())
+        ctl = lat.control()
+        assert m[r, B_NMEAS] == len(rows)
+        assert (m[r, B_D], m[r, B_STEP]) == (ctl["d"], ctl["step"])
+        assert (m[r, B_PACCEPT], m[r, B_FACCEPT]) == (ctl["paccept"], ctl["faccept"])
+        e = np.array([row[5] for row in rows]) / lat.nsites
+        # FP64 sums of the same terms in another order
+        assert m[r, 1] == pytest.approx(e.sum(), rel=1e-11, abs=1e-11)
+        lat.close()
