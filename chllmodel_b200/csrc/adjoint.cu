@@ -503,10 +503,11 @@ __device__ __forceinline__ float quench_dot(float x0, float y0, float x1, float 
 // One bond's dE/dn_i (bond_grad) added to g.
 template <int AXIS, bool SECOND>
 __device__ __forceinline__ void quench_bond(const float4& n, const float4& b, float m2eps, float sk,
-                                            float g[3]) {
+                                            float g[3], bool second = SECOND) {
   constexpr int p = (AXIS + 1) % 3, q = (AXIS + 2) % 3;
   const float nv[3] = {n.x, n.y, n.z}, bv[3] = {b.x, b.y, b.z};
-  const float c = quench_dot<SECOND>(n.x, b.x, n.y, b.y, n.z, b.z);
+  const float c = SECOND || second ? quench_dot<true>(n.x, b.x, n.y, b.y, n.z, b.z)
+                                   : quench_dot<false>(n.x, b.x, n.y, b.y, n.z, b.z);
   const float X = fmaf(nv[p], bv[q], -__fmul_rn(nv[q], bv[p]));
   const float a = __fmul_rn(m2eps, c);
   const float w = __fmul_rn(sk, __fmul_rn(0.5f, __fadd_rn(n.w, b.w)));
@@ -523,11 +524,11 @@ __device__ __forceinline__ void quench_bond(const float4& n, const float4& b, fl
 // tangent-projected energy gradient, n <- normalise(n - eta (I - n n^T) dE/dn),
 // with the neighbours nb (+x, -x, +y, -y, +z, -z) held fixed.  Which product of a
 // bond's dot product is rounded on its own differs between the boundaries and,
-// for -z, between a unit's sites (SITE 0, 1): the roundings this quench has
-// always had.
-template <bool P, int SITE>
+// for -z, between a unit's sites (second: the unit's second one): the roundings
+// this quench has always had.
+template <bool P>
 __device__ __forceinline__ float4 quench_site(float4 n, const Nbrs& nb, const Coupling& cp,
-                                              float eta) {
+                                              float eta, bool second) {
   const float m2eps = __fmul_rn(-2.f, cp.eps);
   float g[3] = {0.f, 0.f, 0.f};
   quench_bond<0, true>(n, nb.b[0], m2eps, -cp.K, g);
@@ -535,7 +536,7 @@ __device__ __forceinline__ float4 quench_site(float4 n, const Nbrs& nb, const Co
   quench_bond<1, P>(n, nb.b[2], m2eps, -cp.K, g);
   quench_bond<1, P>(n, nb.b[3], m2eps, cp.K, g);
   quench_bond<2, P>(n, nb.b[4], m2eps, -cp.K, g);
-  quench_bond<2, P || SITE == 1>(n, nb.b[5], m2eps, cp.K, g);
+  quench_bond<2, P>(n, nb.b[5], m2eps, cp.K, g, second);
   const float nn = quench_dot<true>(n.x, n.x, n.y, n.y, n.z, n.z);
   const float gn = __fdiv_rn(quench_dot<true>(g[0], n.x, g[1], n.y, g[2], n.z), nn);
   const float x = fmaf(-eta, fmaf(-gn, n.x, g[0]), n.x);
@@ -559,8 +560,8 @@ __global__ void __launch_bounds__(kGradThreads) quench_pass_kernel(LatticeView L
        g += gridDim.x * kGradThreads) {
     UnitNbhd U;
     gather_unit<C, PERIODIC, PERIODIC>(L, G, g, U);
-    if (U.v0) U.n0 = quench_site<PERIODIC, 0>(U.n0, U.nb0, cp, eta);
-    if (U.v1) U.n1 = quench_site<PERIODIC, 1>(U.n1, U.nb1, cp, eta);
+    if (U.v0) U.n0 = quench_site<PERIODIC>(U.n0, U.nb0, cp, eta, false);
+    if (U.v1) U.n1 = quench_site<PERIODIC>(U.n1, U.nb1, cp, eta, true);
     st_unit(U.cen, U.n0, U.n1);
   }
 }
@@ -578,31 +579,39 @@ struct QuenchArgs {
   int nsteps;
 };
 
-template <bool P, bool OWN>
+// FORM: 0 the unit loop, 1 one unit per thread, 2 one site of each colour.
+template <bool P, int FORM>
 __global__ void __launch_bounds__(kResThreads, 1)
     quench_resident_kernel(const __grid_constant__ QuenchArgs A) {
   __shared__ int s_ok;
   if (A.ctl->status) return;  // an earlier wait ran out: the words are not to be trusted
   const bool lead = threadIdx.x == 0;
-  OwnBlock<P> B(A.L, A.G);
+  std::conditional_t<FORM == 2, OwnSite<P>, OwnBlock<P>> B(A.L, A.G);
   uint32_t slot = 0;
   auto pass = [&](auto colour) {
     constexpr int C = decltype(colour)::value;
-    if (OWN) {
+    if constexpr (FORM == 2) {
+      if (!B.has) return;
+      Nbrs nb;
+      B.template neighbours<C>(A.L, nb);
+      if (B.template valid<C>())
+        B.n[C] = quench_site<P>(B.n[C], nb, A.cp, A.eta, (B.h & 1u) != 0);
+      B.template store<C>(A.L);
+    } else if constexpr (FORM == 1) {
       if (!B.has) return;
       Nbrs nb0, nb1;
       B.template neighbours<C>(A.L, nb0, nb1);
       const bool odd = B.template odd<C>();
-      if (odd ? B.v[1] : B.v[0]) B.n[C][0] = quench_site<P, 0>(B.n[C][0], nb0, A.cp, A.eta);
-      if (odd ? B.v[3] : B.v[2]) B.n[C][1] = quench_site<P, 1>(B.n[C][1], nb1, A.cp, A.eta);
+      if (odd ? B.v[1] : B.v[0]) B.n[C][0] = quench_site<P>(B.n[C][0], nb0, A.cp, A.eta, false);
+      if (odd ? B.v[3] : B.v[2]) B.n[C][1] = quench_site<P>(B.n[C][1], nb1, A.cp, A.eta, true);
       st_unit(A.L.col[C] + B.u, B.n[C][0], B.n[C][1]);
     } else {
       for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < A.G.units;
            g += gridDim.x * blockDim.x) {
         UnitNbhd U;
         gather_unit<C, P, P, false, kLoadCoherentOrdered>(A.L, A.G, g, U);
-        if (U.v0) U.n0 = quench_site<P, 0>(U.n0, U.nb0, A.cp, A.eta);
-        if (U.v1) U.n1 = quench_site<P, 1>(U.n1, U.nb1, A.cp, A.eta);
+        if (U.v0) U.n0 = quench_site<P>(U.n0, U.nb0, A.cp, A.eta, false);
+        if (U.v1) U.n1 = quench_site<P>(U.n1, U.nb1, A.cp, A.eta, true);
         st_unit(U.cen, U.n0, U.n1);
       }
     }
@@ -699,14 +708,16 @@ cudaError_t launch_quench_resident(const LatticeView& L, const CouplingD& cd, fl
   A.ctl = ctl;
   A.words = words;
   A.nsteps = nsteps;
+  const int form = one_site_each(L, A.G.units) ? 2 : (one_unit_each(L, A.G.units) ? 1 : 0);
   uint32_t block, ctas;
-  resident_shape(A.G.units, block, ctas);
-  const bool own = one_unit_each(L, A.G.units);
-  auto kernel = L.periodic ? (own ? quench_resident_kernel<true, true>
-                                  : quench_resident_kernel<true, false>)
-                           : (own ? quench_resident_kernel<false, true>
-                                  : quench_resident_kernel<false, false>);
-  return launch_cooperative(kernel, ctas, block, stream, A);
+  resident_shape(form == 2 ? 2 * A.G.units : A.G.units, block, ctas);
+  using Kernel = void (*)(const QuenchArgs);
+  static const Kernel kernels[2][3] = {
+      {quench_resident_kernel<false, 0>, quench_resident_kernel<false, 1>,
+       quench_resident_kernel<false, 2>},
+      {quench_resident_kernel<true, 0>, quench_resident_kernel<true, 1>,
+       quench_resident_kernel<true, 2>}};
+  return launch_cooperative(kernels[L.periodic ? 1 : 0][form], ctas, block, stream, A);
 }
 
 cudaError_t launch_natural_grad(int ni, int nj, int nk, int periodic, const float* n,

@@ -6,20 +6,20 @@
 // units, and as a launch of its own it takes 3.3 us, most of it the grid's
 // start and drain, the read of the control block and the count epilogue.
 // Here a pass is its loads (L2: the lattice was written by other SMs a pass
-// earlier), one unit's serial trial arithmetic, and the barrier: about 0.75 us
-// for the barrier of 128 CTAs and 1.1 us for the arithmetic of a single warp
-// per scheduler (8^3 in one CTA, where the barrier is the CTA's own, runs a
-// sweep in 2.3 us; 16^3 on 32 CTAs in 4.5).  So the units are spread over all
-// SMs, as few warps on each as there can be: threads per CTA come from
-// units / SMs.  The form that this one replaces kept the chunk in one cluster
+// earlier), one site's or unit's serial trial arithmetic, and the barrier, about
+// 0.8 us of 128 CTAs (8^3 in one CTA, where the barrier is the CTA's own, runs a
+// sweep in 2.0 us; 16^3 on 64 CTAs in 4.1).  So the sites are spread over all SMs,
+// as few warps on each as there can be: a thread holds one site of each colour
+// while that fits (37 k units), then one unit, then several, and the threads per
+// CTA come from their number per SM.  The form that this one replaces kept the chunk in one cluster
 // of 16 CTAs with the hardware cluster barrier: its barrier was cheaper, but 16
 // SMs had to issue every instruction of the pass.  us per sweep on one B200
 // (periodic, kT 0.5, K 0.5):
 //
 //   edge                    8     16    24    32    48    64    96    128   200
-//   passes launched each   5.4   6.3   6.4   6.5   6.9   8.1   15.0  26.6  85.2
+//   passes launched each   5.5   4.8   6.4   6.5   6.9   8.1   15.0  26.6  85.2
 //   one cluster            3.5   5.4   5.5   5.6  14.5
-//   this form              2.3   4.5   4.6   4.7   5.1   6.5   13.6  24.6  79.9
+//   this form              2.0   4.1   4.2   4.2   4.7   6.5   13.6  24.6  79.9
 //
 // The barrier and the counts are one 64-bit word per pass: a CTA adds its
 // accept counts and its arrival with one release reduction and polls the
@@ -136,6 +136,44 @@ struct OwnUnit {
         B.n[C][0], B.n[C][1], nb0, nb1, odd ? B.v[1] : B.v[0], odd ? B.v[3] : B.v[2],
         unit_randoms(words), d, A.cp, nacc, nflip);
     st_unit(A.L.col[C] + B.u, B.n[C][0], B.n[C][1]);
+  }
+};
+
+// The same with a site of each colour per thread.
+template <bool P>
+struct OwnSiteUnit {
+  const ResidentArgs& A;
+  OwnSite<P> B;
+  Ctr4 words;
+
+  __device__ __forceinline__ explicit OwnSiteUnit(const ResidentArgs& a) : A(a), B(a.L, a.G) {}
+
+  template <int C>
+  __device__ __forceinline__ void draw(uint32_t step) {
+    words = philox4x32_10({{B.g, step, A.replica, (uint32_t)C}}, A.keys);
+    asm volatile("" : "+r"(words.v[0]), "+r"(words.v[1]), "+r"(words.v[2]), "+r"(words.v[3]));
+  }
+
+  template <int PHASE>
+  __device__ __forceinline__ void pass(uint32_t, float d, unsigned int& nacc,
+                                       unsigned int& nflip) {
+    using T = PhaseOf<PHASE>;
+    constexpr int C = T::C;
+    nacc = nflip = 0;
+    if (!B.has) return;
+    Nbrs nb;
+    B.template neighbours<C>(A.L, nb);
+    // this site's numbers of the unit's call first; the second site is not there
+    UnitRandoms u = unit_randoms(words);
+    const bool second = (B.h & 1u) != 0;
+    u.acc[0] = second ? u.acc[1] : u.acc[0];
+    u.ang[0] = second ? u.ang[1] : u.ang[0];
+    u.flip[0] = second ? u.flip[1] : u.flip[0];
+    float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+    unit_trials_drawn<T::flip_before, T::dir, T::flip_after>(B.n[C], none, nb, nb,
+                                                             B.template valid<C>(), false, u, d,
+                                                             A.cp, nacc, nflip);
+    B.template store<C>(A.L);
   }
 };
 
@@ -264,7 +302,9 @@ template <bool P, int FORM>
 __global__ void __launch_bounds__(kResThreads, 1)
     resident_sweeps_kernel(const __grid_constant__ ResidentArgs A) {
   __shared__ ResidentShared S;
-  if (FORM == 3)
+  if (FORM == 4)
+    resident_sweeps<OwnSiteUnit<P>>(A, S);
+  else if (FORM == 3)
     resident_sweeps<OwnUnit<P>>(A, S);
   else
     resident_sweeps<SharedUnits<P, FORM>>(A, S);
@@ -272,12 +312,14 @@ __global__ void __launch_bounds__(kResThreads, 1)
 
 using ResidentKernel = void (*)(const ResidentArgs);
 // [periodic][form]: 0 unit loop with padding checks, 1 unit loop, 2 column
-// walk, 3 one unit per thread
-const ResidentKernel kResident[2][4] = {
+// walk, 3 one unit per thread, 4 one site of each colour per thread
+const ResidentKernel kResident[2][5] = {
     {resident_sweeps_kernel<false, 0>, resident_sweeps_kernel<false, 1>,
-     resident_sweeps_kernel<false, 2>, resident_sweeps_kernel<false, 3>},
+     resident_sweeps_kernel<false, 2>, resident_sweeps_kernel<false, 3>,
+     resident_sweeps_kernel<false, 4>},
     {resident_sweeps_kernel<true, 0>, resident_sweeps_kernel<true, 1>,
-     resident_sweeps_kernel<true, 2>, resident_sweeps_kernel<true, 3>}};
+     resident_sweeps_kernel<true, 2>, resident_sweeps_kernel<true, 3>,
+     resident_sweeps_kernel<true, 4>}};
 
 }  // namespace
 
@@ -305,14 +347,15 @@ cudaError_t launch_resident_sweeps(const LatticeView& L, const Coupling& cp, uin
   A.G = make_geom(L);
   const bool full = L.ni % 4 == 0;
   const bool own = one_unit_each(L, A.G.units);
+  const bool site = one_site_each(L, A.G.units);
   uint32_t block, ctas;
-  resident_shape(A.G.units, block, ctas);
+  resident_shape(site ? 2 * A.G.units : A.G.units, block, ctas);
   const uint32_t ncols = A.G.Q * (uint32_t)L.nj;
   uint32_t seg = 0;
   if (full && !own)
     walk_pass_cost(A.G.units, ncols, (uint32_t)L.nk, true, ctas * block, -1, &seg);
   A.W = make_walk(A.G, L, seg ? seg : 1);
-  const int form = own ? 3 : (seg ? 2 : (full ? 1 : 0));
+  const int form = site ? 4 : (own ? 3 : (seg ? 2 : (full ? 1 : 0)));
   A.cp = cp;
   A.keys = philox_keys(key0, key1);
   A.replica = replica;
