@@ -8,7 +8,7 @@
 // Here a pass is its loads (L2: the lattice was written by other SMs a pass
 // earlier), one site's or unit's serial trial arithmetic, and the barrier, about
 // 0.8 us of 128 CTAs (8^3 in one CTA, where the barrier is the CTA's own, runs a
-// sweep in 2.0 us; 16^3 on 64 CTAs in 4.1).  So the sites are spread over all SMs,
+// sweep in 1.9 us; 16^3 on 64 CTAs in 3.9).  So the sites are spread over all SMs,
 // as few warps on each as there can be: a thread holds one site of each colour
 // while that fits (37 k units), then one unit, then several, and the threads per
 // CTA come from their number per SM.  The form that this one replaces kept the chunk in one cluster
@@ -17,9 +17,9 @@
 // (periodic, kT 0.5, K 0.5):
 //
 //   edge                    8     16    24    32    48    64    96    128   200
-//   passes launched each   5.5   4.8   6.4   6.5   6.9   8.1   15.0  26.6  85.2
+//   passes launched each   5.5   4.6   6.4   6.5   6.6   8.1   15.0  26.9  85.6
 //   one cluster            3.5   5.4   5.5   5.6  14.5
-//   this form              2.0   4.1   4.2   4.2   4.7   6.5   13.6  24.6  79.9
+//   this form              1.9   3.9   4.0   4.0   4.6   6.3   13.5  24.6  79.5
 //
 // The barrier and the counts are one 64-bit word per pass: a CTA adds its
 // accept counts and its arrival with one release reduction and polls the
@@ -48,12 +48,14 @@ struct ResidentArgs {
   Control* ctl;
   unsigned long long* words;
   int nsweeps;
-  uint32_t wait_limit;
 };
 
 struct ResidentShared {
   unsigned int cnt[2][kResThreads / 32];
   double d;
+  long long step;
+  unsigned long long nacc, nflip;
+  float paccept;
   int ok;
 };
 
@@ -203,97 +205,99 @@ __device__ __forceinline__ unsigned long long cta_counts(ResidentShared& S, unsi
 }
 
 // The chunk: A0 B (A B)... F with the grid barrier after every pass but the
-// last.
+// last.  The control values live in shared memory, thread 0's to change: kept in
+// registers across the passes they cost the unit loops theirs.
 template <class UNITS>
 __device__ __forceinline__ void resident_sweeps(const ResidentArgs& A, ResidentShared& S) {
   Control* ctl = A.ctl;
   if (ctl->status) return;  // an earlier wait ran out: the words are not to be trusted
-  const uint32_t nct = gridDim.x;
-  const bool lead = threadIdx.x == 0;
-  double d = ctl->d;
-  long long step = ctl->step;
-  const long long adapt_until = ctl->adapt_until;
-  const float n3 = (float)ctl->nsites;  // chll_mod.f90:83,93
-  unsigned long long nacc = ctl->nacc, nflip = ctl->nflip;  // left open by single passes
-  float paccept = 0.f;
-  bool ok = true;
+  if (threadIdx.x == 0) {
+    S.d = ctl->d;
+    S.step = ctl->step;
+    S.nacc = ctl->nacc;  // left open by single passes
+    S.nflip = ctl->nflip;
+    S.ok = 1;
+  }
+  uint32_t step = (uint32_t)ctl->step;
   uint32_t slot = 0;  // word of the pass
   unsigned int na, nf;
   UNITS units(A);
-  units.template draw<0>((uint32_t)step);
+  units.template draw<0>(step);
+  __syncthreads();
+  // thread 0: this pass's word, complete; the word before it cleared
+  auto wait = [&](unsigned long long v) {
+    bool ok = true;
+    v = grid_wait(A.words + slot * kWordStride, v, gridDim.x, kWaitLimit, ok);
+    if (blockIdx.x == 0) A.words[(slot == 0 ? 2 : slot - 1) * kWordStride] = 0;
+    S.nacc += v & kCountMask;
+    S.ok = ok;
+    return v;
+  };
   for (int s = 0; s < A.nsweeps; ++s) {
     const bool last = s == A.nsweeps - 1;
     if (s)
-      units.template pass<kFusedA>((uint32_t)step, (float)d, na, nf);
+      units.template pass<kFusedA>(step, (float)S.d, na, nf);
     else
-      units.template pass<kFusedA0>((uint32_t)step, (float)d, na, nf);
+      units.template pass<kFusedA0>(step, (float)S.d, na, nf);
     unsigned long long v = cta_counts(S, na, nf, false);
-    if (lead) grid_arrive(A.words + slot * kWordStride, v, nct);
-    units.template draw<1>((uint32_t)step);
-    if (lead) {
-      v = grid_wait(A.words + slot * kWordStride, v, nct, A.wait_limit, ok);
-      nacc += v & kCountMask;
-      if (blockIdx.x == 0) A.words[(slot == 0 ? 2 : slot - 1) * kWordStride] = 0;
-      S.ok = ok;
-    }
+    if (threadIdx.x == 0) grid_arrive(A.words + slot * kWordStride, v, gridDim.x);
+    units.template draw<1>(step);
+    if (threadIdx.x == 0) wait(v);
     slot = slot == 2 ? 0 : slot + 1;
     __syncthreads();
     if (!S.ok) break;
-    units.template pass<kFusedB>((uint32_t)step, (float)d, na, nf);
+    units.template pass<kFusedB>(step, (float)S.d, na, nf);
     v = cta_counts(S, na, nf, last);
-    if (lead) grid_arrive(A.words + slot * kWordStride, v, nct);
-    units.template draw<0>((uint32_t)step + 1u);
-    if (lead) {
+    if (threadIdx.x == 0) grid_arrive(A.words + slot * kWordStride, v, gridDim.x);
+    units.template draw<0>(step + 1u);
+    if (threadIdx.x == 0) {
       // both outcomes of adapt_d ahead of the wait
-      double dn = adapt_d(d, 0.f), up = adapt_d(d, 1.f);
+      double dn = adapt_d(S.d, 0.f), up = adapt_d(S.d, 1.f);
       asm volatile("" : "+d"(dn), "+d"(up));
-      v = grid_wait(A.words + slot * kWordStride, v, nct, A.wait_limit, ok);
-      nacc += v & kCountMask;
-      if (blockIdx.x == 0) A.words[(slot == 0 ? 2 : slot - 1) * kWordStride] = 0;
+      v = wait(v);
       // the control update that closes the director count (fused_close)
-      paccept = (float)nacc / n3;
-      if (step < adapt_until) {
-        if ((double)paccept < 0.4) d = dn;
-        else if ((double)paccept > 0.6) d = up;
+      const float pa = (float)S.nacc / (float)ctl->nsites;  // chll_mod.f90:83
+      S.paccept = pa;
+      if (S.step < ctl->adapt_until) {
+        if ((double)pa < 0.4) S.d = dn;
+        else if ((double)pa > 0.6) S.d = up;
       }
+      ++S.step;
       if (last) {
-        if (s) nflip = 0;  // closed by this sweep's pass A
-        nflip += v >> kCountBits & kCountMask;
+        // earlier flips were closed by this sweep's pass A
+        S.nflip = (s ? 0ull : S.nflip) + (v >> kCountBits & kCountMask);
       } else {
-        nacc = 0;
+        S.nacc = 0;
       }
-      S.d = d;
-      S.ok = ok;
     }
     slot = slot == 2 ? 0 : slot + 1;
     ++step;
     __syncthreads();
     if (!S.ok) break;
-    d = S.d;
   }
   if (!S.ok) {
-    if (lead) atomicOr(&ctl->status, 4u);
+    if (threadIdx.x == 0) atomicOr(&ctl->status, 4u);
     return;
   }
-  units.template pass<kFusedF>((uint32_t)step, (float)d, na, nf);
+  units.template pass<kFusedF>(step, (float)S.d, na, nf);
   unsigned long long v = cta_counts(S, 0, nf, true);
-  if (!lead) return;
+  if (threadIdx.x != 0) return;
   // the CTA that completes the closing pass's word has the flip count and
   // writes the control block
-  if (nct > 1) {
+  if (gridDim.x > 1) {
     const unsigned long long old =
         atomicAdd(A.words + slot * kWordStride, v + (1ull << kArriveShift));
-    if ((uint32_t)(old >> kArriveShift) != nct - 1) return;
+    if ((uint32_t)(old >> kArriveShift) != gridDim.x - 1) return;
     v += old;
     clear_words(A.words);
   }
-  nflip += v >> kCountBits & kCountMask;
-  ctl->d = d;
-  ctl->step = step;
-  ctl->paccept = paccept;
-  ctl->nacc_last = (long long)nacc;
+  const unsigned long long nflip = S.nflip + (v >> kCountBits & kCountMask);
+  ctl->d = S.d;
+  ctl->step = S.step;
+  ctl->paccept = S.paccept;
+  ctl->nacc_last = (long long)S.nacc;
   ctl->nacc = 0;
-  ctl->faccept = (float)nflip / n3;
+  ctl->faccept = (float)nflip / (float)ctl->nsites;  // chll_mod.f90:93
   ctl->nflip_last = (long long)nflip;
   ctl->nflip = 0;
 }
@@ -330,13 +334,15 @@ bool resident_fits(const LatticeView& L) {
 
 // Against a launch per pass: always where a thread holds one unit.  Beyond
 // that the barrier still saves about 1 us per pass, but the loops' coherent
-// loads cost the units more than the read-only ones do: with periodic
-// boundaries and unpadded rows it pays up to 200^3 (2 M units; 79.9 against
-// 85.2 us, but 174.7 against 164.6 at 256^3), with open boundaries or padded
-// rows it does not (128^3 open 28.4 against 27.1, 102^3 open 19.5 against 17.7).
+// loads cost the units more than the read-only ones do.  With unpadded rows it
+// pays up to 256^3 (4 M units) periodic (128^3 24.6 against 26.9 us, 200^3 79.5
+// against 85.6, 256^3 161 against 164) and 200^3 (2 M units) open (128^3 26.0
+// against 27.2, 200^3 83.6 against 87.2, 256^3 183 against 180); with padded rows
+// it does not (130^3 open 31.1 against 29.7, 150 x 125 x 101 28.1 against 27.2).
 bool resident_pays(const LatticeView& L) {
   const uint32_t units = make_geom(L).units;
-  return one_unit_each(L, units) || (L.periodic && L.ni % 4 == 0 && units <= (1u << 21));
+  return one_unit_each(L, units) ||
+         (L.ni % 4 == 0 && units <= (L.periodic ? 1u << 22 : 1u << 21));
 }
 
 cudaError_t launch_resident_sweeps(const LatticeView& L, const Coupling& cp, uint32_t key0,
@@ -362,7 +368,6 @@ cudaError_t launch_resident_sweeps(const LatticeView& L, const Coupling& cp, uin
   A.ctl = ctl;
   A.words = words;
   A.nsweeps = nsweeps;
-  A.wait_limit = kWaitLimit;
   return launch_cooperative(kResident[L.periodic ? 1 : 0][form], ctas, block, stream, A);
 }
 

@@ -70,14 +70,14 @@ class Lattice:
 
     def set_kernel(self, kind: str) -> None:
         """Sweep form: 'auto' ('resident' where it is the faster one: up to
-        one unit of two sites per GPU thread, about 66^3, and periodic lattices
-        up to 200^3; else 'fused'),
+        one unit of two sites per GPU thread, about 66^3, and lattices of rows
+        of a multiple of 4 sites up to 256^3 periodic, 200^3 open; else 'fused'),
         'fused' (two passes per sweep),
         'direct' (the reference's four half-sweeps, neighbours from global
         memory), 'staged' (four half-sweeps from shared-memory row tiles) or
         'resident' (the fused passes of a whole chunk in one cooperative
-        launch; lattices of 2^27 sites and more take the fused passes).  All give the same chain bit for
-        bit."""
+        launch; lattices of 2^27 sites and more take the fused passes).  All
+        give the same chain bit for bit."""
         code = {"auto": 0, "direct": 1, "staged": 2, "fused": 3, "resident": 4}[kind]
         check(self._L.chll_lattice_set_kernel(self._h, code))
 
