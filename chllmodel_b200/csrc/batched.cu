@@ -652,9 +652,10 @@ int shape_launch(chll_batch* B) {
           placed = true;
         }
       }
-    } else if (!waves.empty() && (int)waves[0].size() < budget) {
-      waves[0].push_back(r);
-      wave_load[0] += bytes;
+    } else if (!waves.empty() && (int)waves.back().size() < budget) {
+      // more replicas than CTAs fill wave after wave
+      waves.back().push_back(r);
+      wave_load.back() += bytes;
       placed = true;
     }
     if (!placed) {
@@ -1247,30 +1248,31 @@ int chll_batch_autotune(chll_batch* B, int trial_sweeps, int* best_threads, int*
   BATCH_CUDA(cudaEventCreate(&e0));
   BATCH_CUDA(cudaEventCreate(&e1));
   double best = 1e300;
-  int bt = keep_threads, bc = keep_ctas, bp = keep_pair;
+  int bt = keep_threads, bc = keep_ctas;
   int rc = CHLL_OK;
   long long bw = B->wave_bytes;
   // Candidates: one wave, or waves of 40, 64 or 96 MiB of state (a wave that
   // fits in the 126 MB L2 runs its sweeps from L2, at the price of fewer
   // replicas sharing the grid); each block size at its two highest
   // occupancies (lower occupancies were never faster on this kernel).  Trials
-  // measure every 10 sweeps like a production run.
-  // A wave size that holds the whole batch is the one-wave launch again and is
-  // not timed twice, nor is pairing a batch of one.
+  // measure every 10 sweeps like a production run.  A wave size that holds the
+  // whole batch is the one-wave launch again and is not timed twice.  Pairing and
+  // the pooled passes are not tried: over 21 sets, 2 to 1300 replicas of 8^3 to
+  // 256^3, the best paired shape took 1.01 to 2 times the best single one and the
+  // pooled passes 1.1 to 4 times (their trials were two thirds of the tuning time).
   const long long kWaveOptions[] = {0ll, 40ll << 20, 64ll << 20, 96ll << 20};
   long long state_bytes = 0;
   for (size_t pc : B->per_colour) state_bytes += (long long)(2 * pc * sizeof(float4));
-  for (int pair : {1, 0})
+  B->pair = 0;
   for (long long wb : kWaveOptions)
   for (int threads : {128, 256, 512}) {
-    if (wb >= state_bytes || (pair && B->n == 1)) continue;
-    const int occ = occupancy_of(threads, pair);
+    if (wb >= state_bytes) continue;
+    const int occ = occupancy_of(threads, false);
     for (int c = std::max(1, occ - 1); c <= occ && rc == CHLL_OK; ++c) {
       if (c * threads > 2048) break;
       B->threads = threads;
       B->ctas_per_sm = c;
       B->wave_bytes = wb;
-      B->pair = pair;
       rc = shape_launch(B);
       if (rc != CHLL_OK) break;
       cudaMemcpyAsync(B->lat, B->snap_lat, B->slots * sizeof(float4), cudaMemcpyDeviceToDevice,
@@ -1292,49 +1294,15 @@ int chll_batch_autotune(chll_batch* B, int trial_sweeps, int* best_threads, int*
       cudaEventElapsedTime(&ms, e0, e1);
       if (std::getenv("CHLL_TUNE_VERBOSE"))
         std::fprintf(stderr,
-                     "chll batch tune: pairs %d threads %d ctas/SM %d wave %lld MiB waves %d: "
-                     "%.3f ms\n",
-                     pair, threads, c, wb >> 20, B->nwaves, ms);
+                     "chll batch tune: threads %d ctas/SM %d wave %lld MiB waves %d: %.3f ms\n",
+                     threads, c, wb >> 20, B->nwaves, ms);
       if (ms < best) {
         best = ms;
         bt = threads;
         bc = c;
         bw = wb;
-        bp = pair;
       }
     }
-  }
-  // the pooled passes (pooled.cu): no launch shape to choose; timed on the
-  // second of two trials (the first captures the chunk graph)
-  int bpool = 0;
-  if (rc == CHLL_OK) {
-    B->pooled = 1;
-    for (int trial = 0; trial < 2 && rc == CHLL_OK; ++trial) {
-      cudaMemcpyAsync(B->lat, B->snap_lat, B->slots * sizeof(float4), cudaMemcpyDeviceToDevice,
-                      B->stream);
-      cudaMemcpyAsync(B->d_state, B->snap_state, sizeof(chll::ReplicaState) * B->n,
-                      cudaMemcpyDeviceToDevice, B->stream);
-      cudaEventRecord(e0, B->stream);
-      rc = pool_run(B, trial_sweeps, 10, 0);
-      cudaEventRecord(e1, B->stream);
-      if (rc != CHLL_OK) break;
-      cudaError_t e = cudaEventSynchronize(e1);
-      if (e != cudaSuccess) {
-        rc = fail(CHLL_ECUDA, "batch_autotune: %s", cudaGetErrorString(e));
-        break;
-      }
-      float ms = 0.f;
-      cudaEventElapsedTime(&ms, e0, e1);
-      if (trial == 1) {
-        if (std::getenv("CHLL_TUNE_VERBOSE"))
-          std::fprintf(stderr, "chll batch tune: pooled passes: %.3f ms\n", ms);
-        if (ms < best) {
-          best = ms;
-          bpool = 1;
-        }
-      }
-    }
-    B->pooled = 0;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -1354,8 +1322,6 @@ int chll_batch_autotune(chll_batch* B, int trial_sweeps, int* best_threads, int*
   B->threads = bt;
   B->ctas_per_sm = bc;
   B->wave_bytes = bw;
-  B->pair = bp;
-  B->pooled = bpool;
   if (best_threads) *best_threads = bt;
   if (best_ctas) *best_ctas = bc;
   if (best_ms) *best_ms = best;

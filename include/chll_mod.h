@@ -253,15 +253,14 @@ int chll_batch_info(chll_batch* b, int64_t* total_sites, int32_t* nreplicas, int
  * fit).  Each replica gets CTAs in proportion to its sites. */
 int chll_batch_set_tuning(chll_batch* b, int threads, int ctas_per_sm);
 /* Replicas run in waves whose float4 state together stays within wave_bytes
- * (0, the default: all replicas in one wave), largest first; each wave gets
- * the whole co-resident grid, in the same launch. */
+ * (0, the default: one wave, or as many as the replicas need at one CTA each),
+ * largest first; each wave gets the whole co-resident grid, in the same launch. */
 int chll_batch_set_wave_bytes(chll_batch* b, int64_t wave_bytes);
 /* pooled = 1: chll_batch_run sweeps the replicas as pooled passes -- one
  * launch per fused pass over all replicas' units, cut into equal blocks per
  * CTA, the next pass launched as a programmatic dependent (CUDA graphs of
  * measurement-interval chunks) -- instead of the persistent launch with
- * software group barriers; 0 (the default unless chll_batch_autotune chose
- * it): the persistent launch.  The chains are the same either way; the
+ * software group barriers; 0 (the default): the persistent launch.  The chains are the same either way; the
  * launch shape, waves and pairing apply to the persistent launch only.  No
  * counterpart in the reference, which has no batched launch. */
 int chll_batch_set_pooled(chll_batch* b, int pooled);
@@ -269,9 +268,8 @@ int chll_batch_get_pooled(chll_batch* b, int* pooled);
 /* pair = 1: the replicas of a wave are grouped two by two, by size, and each
  * group's CTAs alternate the two replicas' passes, so a wait at one
  * replica's group barrier overlaps the other replica's pass; 0 (the
- * default): one replica per group.  The chains are the same either way;
- * chll_batch_autotune tries both.  No counterpart in the reference, which
- * has no batched launch. */
+ * default): one replica per group.  The chains are the same either way.  No
+ * counterpart in the reference, which has no batched launch. */
 int chll_batch_set_pairing(chll_batch* b, int pair);
 int chll_batch_get_pairing(chll_batch* b, int* pair);
 /* How many polls a replica group's barrier wait makes before it gives up
@@ -285,8 +283,9 @@ int chll_batch_set_wait_limit(chll_batch* b, uint64_t polls);
 int chll_batch_get_tuning(chll_batch* b, int32_t* threads, int32_t* ctas_per_sm,
                           int64_t* wave_bytes, int32_t* nwaves);
 /* Times every launch shape (threads, CTAs per SM, wave size) for trial_sweeps
- * sweeps from a snapshot of the current state, keeps the fastest and restores
- * the state. */
+ * sweeps from a snapshot of the current state, keeps the fastest (of the
+ * persistent launch with single groups; pairing and pooled passes are never the
+ * fastest and are turned off) and restores the state. */
 int chll_batch_autotune(chll_batch* b, int trial_sweeps, int* best_threads, int* best_ctas,
                         double* best_ms);
 

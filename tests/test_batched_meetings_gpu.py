@@ -51,3 +51,28 @@ def test_replicas_follow_their_lattices(threads, paired, wave_bytes):
         # FP64 sums of the same terms in another order
         assert m[r, 1] == pytest.approx(e.sum(), rel=1e-11, abs=1e-11)
         lat.close()
+
+
+@pytest.mark.parametrize("threads", [128, 512])
+def test_more_replicas_than_ctas(threads):
+    """A batch of more replicas than the grid has CTAs fills wave after wave."""
+    from chllmodel_b200.batched import Batch, replica
+    from chllmodel_b200.lattice import Lattice, coupling
+
+    specs = [replica(4, 4, 2 + 2 * (i % 3), kT=0.5, K=0.7, seed=i, replica=i) for i in range(700)]
+    with Batch(specs) as b:
+        b.set_tuning(threads)
+        b.init_random()
+        b.run(5, 5)
+        grid = b.info()["grid"]
+        assert b.tuning()["waves"] == -(-len(specs) // grid)
+        m = b.moments()
+        assert np.all(m[:, 12] == 6) and np.all(m[:, 15] == 0)
+        for r in (0, 299, 699):
+            sp = specs[r]
+            lat = Lattice(sp["ni"], sp["nj"], sp["nk"], boundary="periodic")
+            lat.init_random(sp["seed"], sp["replica"])
+            lat.set_control(0.1, step=1)
+            lat.sweep(coupling(0.5, 0.7), 5, seed=sp["seed"], replica=sp["replica"])
+            assert np.array_equal(b.download_f4(r), lat.download_f4())
+            lat.close()
