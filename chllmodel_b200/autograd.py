@@ -66,7 +66,7 @@ class LatticeEnergy(torch.autograd.Function):
     def backward(ctx, g_out):
         grad_n, d_couplings = ctx.saved_tensors
         g = g_out.to(torch.float64)
-        gn = (g.to(grad_n.dtype) * grad_n) if ctx.needs_input_grad[0] else None
+        gn = (g * grad_n) if ctx.needs_input_grad[0] else None
         ge = gk = gh = None
         if any(ctx.needs_input_grad[2:5]):
             gc = g * d_couplings

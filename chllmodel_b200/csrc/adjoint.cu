@@ -287,7 +287,6 @@ struct NaturalGeom {
   uint32_t plane;      // ni * nj, columns
   uint32_t cols;       // columns rounded up to whole warps
   uint32_t seg, nseg;  // planes per task, tasks per column
-  int periodic;
 };
 
 struct Site64 {
@@ -298,9 +297,11 @@ __device__ __forceinline__ Site64 to64(const float4& v) {
   return {(double)v.x, (double)v.y, (double)v.z, (double)v.w};
 }
 
+// Site e of fewer than 2^32: 32-bit indices, widened once per address.
 __device__ __forceinline__ float4 natural_site(const float* __restrict__ n,
-                                               const float* __restrict__ s, size_t e) {
-  return make_float4(__ldg(n + 3 * e), __ldg(n + 3 * e + 1), __ldg(n + 3 * e + 2), __ldg(s + e));
+                                               const float* __restrict__ s, uint32_t e) {
+  const float* const p = n + 3ull * e;
+  return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(s + e));
 }
 
 // One forward bond's FP64 terms: acc[0] the sum of 1 - c^2, acc[1] that of
@@ -319,15 +320,18 @@ __device__ __forceinline__ void bond_sums64(const Site64& n, const Site64& b, do
 // (-2 eps c + w X) b + (w c) (b x e_a) with w = sigma K sbar, in half the
 // instructions of bond_grad's term by term form (m2eps = -2 eps, kw = sigma
 // K / 2).  Adds the second part to g and returns the first one's coefficient,
-// so that the smaller parts are summed before the larger ones.
-template <int AXIS>
-__device__ __forceinline__ float bond_grad_part(const float4& n, const float4& b, float m2eps,
-                                                float kw, float& gx, float& gy, float& gz) {
+// so that the smaller parts are summed before the larger ones.  A bond that is
+// not there (has) has zero coefficients.
+template <int AXIS, bool ALWAYS>
+__device__ __forceinline__ float bond_grad_part(const float4& n, const float4& b, bool has,
+                                                float m2eps, float kw, float& gx, float& gy,
+                                                float& gz) {
   const float c = n.x * b.x + n.y * b.y + n.z * b.z;
   const float X = AXIS == 0 ? n.y * b.z - n.z * b.y
                 : AXIS == 1 ? n.z * b.x - n.x * b.z
                             : n.x * b.y - n.y * b.x;
-  const float w = kw * (n.w + b.w), q = w * c;
+  const float w = kw * (n.w + b.w);
+  const float q = ALWAYS || has ? w * c : 0.f;
   if (AXIS == 0) {
     gy += q * b.z;
     gz -= q * b.y;
@@ -338,7 +342,8 @@ __device__ __forceinline__ float bond_grad_part(const float4& n, const float4& b
     gx += q * b.y;
     gy -= q * b.x;
   }
-  return w * X + m2eps * c;
+  const float p = w * X + m2eps * c;
+  return ALWAYS || has ? p : 0.f;
 }
 
 __device__ __forceinline__ void add_scaled(float p, const float4& b, float& gx, float& gy,
@@ -348,14 +353,14 @@ __device__ __forceinline__ void add_scaled(float p, const float4& b, float& gx, 
   gz += p * b.z;
 }
 
-template <bool GRAD>
+// A neighbour that is not there is read as the site itself, so that no load is
+// conditional, and its bond left out.
+template <bool GRAD, bool PER>
 __global__ void __launch_bounds__(kGradThreads)
     natural_grad_kernel(NaturalGeom G, const float* __restrict__ n, const float* __restrict__ s,
                         CouplingD cd, float* __restrict__ grad, int project,
                         double* __restrict__ partials) {
   const float m2eps = -2.f * (float)cd.eps, kw = 0.5f * (float)cd.K;
-  const bool per = G.periodic;
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t ntasks = (uint64_t)G.cols * G.nseg;
   double acc[3] = {0.0, 0.0, 0.0};  // bond_sums64's two, then the sum of s
@@ -363,57 +368,63 @@ __global__ void __launch_bounds__(kGradThreads)
        t += (uint64_t)gridDim.x * kGradThreads) {
     // whole warps share a segment: the same planes in every lane
     const uint32_t sg = (uint32_t)(t / G.cols);
-    const uint32_t p = (uint32_t)(t - (uint64_t)sg * G.cols);
-    const bool has = p < G.plane;
+    const uint32_t p0 = (uint32_t)(t - (uint64_t)sg * G.cols);
+    const bool has = p0 < G.plane;
+    const uint32_t p = has ? p0 : G.plane - 1;
     const uint32_t j = p / G.ni, i = p - j * G.ni;
     const uint32_t k0 = sg * G.seg, k1 = min(k0 + G.seg, G.nk);
-    const bool hxp = has && (per || i + 1 < G.ni), hxm = has && (per || i > 0);
-    const bool hyp = has && (per || j + 1 < G.nj), hym = has && (per || j > 0);
+    const bool hxp = PER || i + 1 < G.ni, hxm = PER || i > 0;
+    const bool hyp = PER || j + 1 < G.nj, hym = PER || j > 0;
     // columns of the in-plane neighbours
-    const uint32_t cxp = i + 1 < G.ni ? p + 1 : p - i;
-    const uint32_t cxm = i > 0 ? p - 1 : p + (G.ni - 1);
-    const uint32_t cyp = j + 1 < G.nj ? p + G.ni : i;
-    const uint32_t cym = j > 0 ? p - G.ni : p + (G.nj - 1) * G.ni;
+    const uint32_t cxp = i + 1 < G.ni ? p + 1 : (PER ? p - i : p);
+    const uint32_t cxm = i > 0 ? p - 1 : (PER ? p + (G.ni - 1) : p);
+    const uint32_t cyp = j + 1 < G.nj ? p + G.ni : (PER ? i : p);
+    const uint32_t cym = j > 0 ? p - G.ni : (PER ? p + (G.nj - 1) * G.ni : p);
     // whose x neighbours are not in the lanes beside
-    const bool lxp = hxp && (lane == 31 || i + 1 == G.ni);
-    const bool lxm = hxm && (lane == 0 || i == 0);
-    size_t base = (size_t)k0 * G.plane;  // first site of the plane
-    float4 c = has ? natural_site(n, s, base + p) : zero;
-    float4 zm = zero;
-    if (GRAD && has && (per || k0 > 0))
-      zm = natural_site(n, s, (k0 > 0 ? base - G.plane : (size_t)(G.nk - 1) * G.plane) + p);
+    const bool lxp = lane == 31 || p0 + 1 >= G.plane || i + 1 == G.ni;
+    const bool lxm = lane == 0 || i == 0;
+    const uint32_t last = (G.nk - 1) * G.plane;  // first site of the last plane
+    uint32_t base = k0 * G.plane;                // of this plane
+    float4 c = natural_site(n, s, base + p);
+    float4 zm = c;
+    if (GRAD)
+      zm = natural_site(n, s, (k0 > 0 ? base - G.plane : (PER ? last : base)) + p);
     Site64 c64 = to64(c);
     for (uint32_t k = k0; k < k1; ++k, base += G.plane) {
-      const bool hzp = has && (per || k + 1 < G.nk);
+      const bool hzp = PER || k + 1 < G.nk, hzm = PER || k > 0;
+      if (k + 2 < G.nk) {  // the plane after the next: the lines no thread has read yet
+        const uint32_t e = base + 2 * G.plane + p;
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(n + 3ull * e));
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(s + e));
+      }
       const float4 zp =
-          hzp ? natural_site(n, s, (k + 1 < G.nk ? base + G.plane : 0) + p) : zero;
-      const float4 yp = hyp ? natural_site(n, s, base + cyp) : zero;
-      const float4 ym = GRAD && hym ? natural_site(n, s, base + cym) : zero;
-      float4 xp, xm = zero;
+          natural_site(n, s, (k + 1 < G.nk ? base + G.plane : (PER ? 0u : base)) + p);
+      const float4 yp = natural_site(n, s, base + cyp);
+      float4 ym = yp;
+      if (GRAD) ym = natural_site(n, s, base + cym);
+      float4 xp, xm = c;
       xp.x = __shfl_down_sync(0xffffffffu, c.x, 1);
       xp.y = __shfl_down_sync(0xffffffffu, c.y, 1);
       xp.z = __shfl_down_sync(0xffffffffu, c.z, 1);
       xp.w = __shfl_down_sync(0xffffffffu, c.w, 1);
       if (lxp) xp = natural_site(n, s, base + cxp);
-      if (!hxp) xp = zero;
       if (GRAD) {
         xm.x = __shfl_up_sync(0xffffffffu, c.x, 1);
         xm.y = __shfl_up_sync(0xffffffffu, c.y, 1);
         xm.z = __shfl_up_sync(0xffffffffu, c.z, 1);
         xm.w = __shfl_up_sync(0xffffffffu, c.w, 1);
         if (lxm) xm = natural_site(n, s, base + cxm);
-        if (!hxm) xm = zero;
       }
       const Site64 zp64 = to64(zp);
       if (has) {
         if (GRAD) {
           float gx = 0.f, gy = 0.f, gz = 0.f;
-          const float pxp = bond_grad_part<0>(c, xp, m2eps, -kw, gx, gy, gz);
-          const float pxm = bond_grad_part<0>(c, xm, m2eps, kw, gx, gy, gz);
-          const float pyp = bond_grad_part<1>(c, yp, m2eps, -kw, gx, gy, gz);
-          const float pym = bond_grad_part<1>(c, ym, m2eps, kw, gx, gy, gz);
-          const float pzp = bond_grad_part<2>(c, zp, m2eps, -kw, gx, gy, gz);
-          const float pzm = bond_grad_part<2>(c, zm, m2eps, kw, gx, gy, gz);
+          const float pxp = bond_grad_part<0, PER>(c, xp, hxp, m2eps, -kw, gx, gy, gz);
+          const float pxm = bond_grad_part<0, PER>(c, xm, hxm, m2eps, kw, gx, gy, gz);
+          const float pyp = bond_grad_part<1, PER>(c, yp, hyp, m2eps, -kw, gx, gy, gz);
+          const float pym = bond_grad_part<1, PER>(c, ym, hym, m2eps, kw, gx, gy, gz);
+          const float pzp = bond_grad_part<2, PER>(c, zp, hzp, m2eps, -kw, gx, gy, gz);
+          const float pzm = bond_grad_part<2, PER>(c, zm, hzm, m2eps, kw, gx, gy, gz);
           add_scaled(pxp, xp, gx, gy, gz);
           add_scaled(pxm, xm, gx, gy, gz);
           add_scaled(pyp, yp, gx, gy, gz);
@@ -427,7 +438,7 @@ __global__ void __launch_bounds__(kGradThreads)
             gy -= gn * c.y;
             gz -= gn * c.z;
           }
-          float* out = grad + 3 * (base + p);
+          float* out = grad + 3ull * (base + p);
           out[0] = gx;
           out[1] = gy;
           out[2] = gz;
@@ -726,15 +737,14 @@ cudaError_t launch_natural_grad(int ni, int nj, int nk, int periodic, const floa
                                 cudaStream_t stream) {
   static std::atomic<int> resident[2][16];
   const uint32_t ctas = (uint32_t)std::min(
-      kGradMaxBlocks, grad ? resident_ctas(natural_grad_kernel<true>, resident[1])
-                           : resident_ctas(natural_grad_kernel<false>, resident[0]));
+      kGradMaxBlocks, grad ? resident_ctas(natural_grad_kernel<true, false>, resident[1])
+                           : resident_ctas(natural_grad_kernel<false, false>, resident[0]));
   NaturalGeom G;
   G.ni = (uint32_t)ni;
   G.nj = (uint32_t)nj;
   G.nk = (uint32_t)nk;
   G.plane = G.ni * G.nj;
   G.cols = (G.plane + 31) / 32 * 32;
-  G.periodic = periodic;
   // Planes per task: the fewest steps on the busiest thread, a task's first
   // loads counted as half a step.
   double best = 1e300;
@@ -750,12 +760,10 @@ cudaError_t launch_natural_grad(int ni, int nj, int nk, int periodic, const floa
   G.nseg = (G.nk + G.seg - 1) / G.seg;
   const uint64_t need = ((uint64_t)G.cols * G.nseg + kGradThreads - 1) / kGradThreads;
   const uint32_t blocks = (uint32_t)std::min<uint64_t>(need, ctas);
-  if (grad)
-    natural_grad_kernel<true><<<blocks, kGradThreads, 0, stream>>>(G, n, s, cd, grad, project,
-                                                                   partials);
-  else
-    natural_grad_kernel<false><<<blocks, kGradThreads, 0, stream>>>(G, n, s, cd, nullptr, 0,
-                                                                    partials);
+  auto kernel = grad ? (periodic ? natural_grad_kernel<true, true> : natural_grad_kernel<true, false>)
+                     : (periodic ? natural_grad_kernel<false, true>
+                                 : natural_grad_kernel<false, false>);
+  kernel<<<blocks, kGradThreads, 0, stream>>>(G, n, s, cd, grad, project, partials);
   // scheduled while the kernel before it drains
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(1);
