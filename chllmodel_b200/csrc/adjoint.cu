@@ -719,7 +719,7 @@ cudaError_t launch_quench_resident(const LatticeView& L, const CouplingD& cd, fl
   A.ctl = ctl;
   A.words = words;
   A.nsteps = nsteps;
-  const int form = one_site_each(L, A.G.units) ? 2 : (one_unit_each(L, A.G.units) ? 1 : 0);
+  const int form = one_site_each(A.G.units) ? 2 : (one_unit_each(L, A.G.units) ? 1 : 0);
   uint32_t block, ctas;
   resident_shape(form == 2 ? 2 * A.G.units : A.G.units, block, ctas);
   using Kernel = void (*)(const QuenchArgs);

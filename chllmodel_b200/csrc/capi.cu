@@ -161,6 +161,7 @@ struct chll_lattice {
   double* partials = nullptr;
   unsigned int* tickets = nullptr;  // [0] observables, [1] gradient
   unsigned long long* words = nullptr;  // meeting words of the resident sweeps
+  void* xch = nullptr;  // published sites of the resident sweeps without a barrier
   double* rows = nullptr;
   int rows_cap = 0;
   double* host_rows = nullptr;  // pinned, of run()'s lattice
@@ -312,9 +313,12 @@ int sweep_impl(chll_lattice* L, const Coupling& cp, uint64_t seed, uint32_t rep,
   const DeviceGuard on(L->device);
   if (runs_resident(L)) {
     for (int done = 0; done < nsweeps; done += kResidentChunk) {
-      const cudaError_t e = chll::launch_resident_sweeps(
-          L->view(), cp, k0, k1, rep, L->ctl, L->words, std::min(kResidentChunk, nsweeps - done),
-          L->stream);
+      const int n = std::min(kResidentChunk, nsweeps - done);
+      const cudaError_t e =
+          L->xch ? chll::launch_flow_sweeps(L->view(), cp, k0, k1, rep, L->ctl, L->words, L->xch, n,
+                                            L->stream)
+                 : chll::launch_resident_sweeps(L->view(), cp, k0, k1, rep, L->ctl, L->words, n,
+                                                L->stream);
       if (e != cudaSuccess)
         return fail(CHLL_ECUDA, "resident sweep launch: %s", cudaGetErrorString(e));
     }
@@ -491,8 +495,16 @@ int create_impl(int ni, int nj, int nk, int boundary, chll_lattice** out, int sl
     return bail(e, "partials");
   if ((e = cudaMalloc(&L->tickets, 2 * sizeof(unsigned int))) != cudaSuccess)
     return bail(e, "tickets");
-  if ((e = cudaMalloc(&L->words, chll::kResidentWordBytes)) != cudaSuccess)
+  if ((e = cudaMalloc(&L->words, chll::kResidentAllocBytes)) != cudaSuccess)
     return bail(e, "meeting words");
+  if ((e = cudaMemsetAsync(L->words, 0, chll::kResidentAllocBytes, L->stream)) != cudaSuccess)
+    return bail(e, "memset");
+  if (!L->slab && chll::flow_pays(L->view())) {  // at most 2.4 MB
+    if ((e = cudaMalloc(&L->xch, chll::flow_bytes(L->view()))) != cudaSuccess)
+      return bail(e, "published sites");
+    if ((e = cudaMemsetAsync(L->xch, 0, chll::flow_bytes(L->view()), L->stream)) != cudaSuccess)
+      return bail(e, "memset");
+  }
   if ((e = cudaMalloc(&L->out4, 4 * sizeof(double) + chll::kRowLen * sizeof(double))) !=
       cudaSuccess)
     return bail(e, "result buffer");
@@ -791,6 +803,7 @@ void chll_lattice_destroy(chll_lattice* L) {
   cudaFree(L->partials);
   cudaFree(L->tickets);
   cudaFree(L->words);
+  cudaFree(L->xch);
   cudaFree(L->rows);
   if (L->host_rows) cudaFreeHost(L->host_rows);
   cudaFree(L->out4);

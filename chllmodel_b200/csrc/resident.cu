@@ -7,19 +7,19 @@
 // start and drain, the read of the control block and the count epilogue.
 // Here a pass is its loads (L2: the lattice was written by other SMs a pass
 // earlier), one site's or unit's serial trial arithmetic, and the barrier, about
-// 0.8 us of 128 CTAs (8^3 in one CTA, where the barrier is the CTA's own, runs a
-// sweep in 1.9 us; 16^3 on 64 CTAs in 3.9).  So the sites are spread over all SMs,
-// as few warps on each as there can be: a thread holds one site of each colour
-// while that fits (37 k units), then one unit, then several, and the threads per
-// CTA come from their number per SM.  The form that this one replaces kept the chunk in one cluster
-// of 16 CTAs with the hardware cluster barrier: its barrier was cheaper, but 16
-// SMs had to issue every instruction of the pass.  us per sweep on one B200
-// (periodic, kT 0.5, K 0.5):
+// 0.8 us of 128 CTAs.  So the sites are spread over all SMs, as few warps on each
+// as there can be: a thread holds one site of each colour while that fits (37 k
+// units), then one unit, then several, and the threads per CTA come from their
+// number per SM.  Lattices of a site per thread and more than one CTA leave the
+// barrier out (flow.cu, which sweeps take there).  us per sweep on one B200
+// (periodic, kT 0.5, K 0.5; one cluster: a form of 16 CTAs with the hardware
+// cluster barrier, whose 16 SMs had to issue every instruction of the pass):
 //
 //   edge                    8     16    24    32    48    64    96    128   200
 //   passes launched each   5.5   4.6   6.4   6.5   6.6   8.1   15.0  26.9  85.6
 //   one cluster            3.5   5.4   5.5   5.6  14.5
 //   this form              1.9   3.9   4.0   4.0   4.6   6.3   13.5  24.6  79.5
+//   flow.cu                      2.9   3.0   2.8   3.4
 //
 // The barrier and the counts are one 64-bit word per pass: a CTA adds its
 // accept counts and its arrival with one release reduction and polls the
@@ -332,7 +332,8 @@ bool resident_fits(const LatticeView& L) {
   return 2 * (uint64_t)make_geom(L).units < (1ull << kCountBits);
 }
 
-// Against a launch per pass: always where a thread holds one unit.  Beyond
+// Against a launch per pass: always where a thread holds one site of each colour
+// or one unit (50^3 periodic 3.8 against 7.5 us, 64^3 6.3 against 8.1).  Beyond
 // that the barrier still saves about 1 us per pass, but the loops' coherent
 // loads cost the units more than the read-only ones do.  With unpadded rows it
 // pays up to 256^3 (4 M units) periodic (128^3 24.6 against 26.9 us, 200^3 79.5
@@ -341,7 +342,7 @@ bool resident_fits(const LatticeView& L) {
 // it does not (130^3 open 31.1 against 29.7, 150 x 125 x 101 28.1 against 27.2).
 bool resident_pays(const LatticeView& L) {
   const uint32_t units = make_geom(L).units;
-  return one_unit_each(L, units) ||
+  return one_site_each(units) || one_unit_each(L, units) ||
          (L.ni % 4 == 0 && units <= (L.periodic ? 1u << 22 : 1u << 21));
 }
 
@@ -353,12 +354,12 @@ cudaError_t launch_resident_sweeps(const LatticeView& L, const Coupling& cp, uin
   A.G = make_geom(L);
   const bool full = L.ni % 4 == 0;
   const bool own = one_unit_each(L, A.G.units);
-  const bool site = one_site_each(L, A.G.units);
+  const bool site = one_site_each(A.G.units);
   uint32_t block, ctas;
   resident_shape(site ? 2 * A.G.units : A.G.units, block, ctas);
   const uint32_t ncols = A.G.Q * (uint32_t)L.nj;
   uint32_t seg = 0;
-  if (full && !own)
+  if (full && !own && !site)
     walk_pass_cost(A.G.units, ncols, (uint32_t)L.nk, true, ctas * block, -1, &seg);
   A.W = make_walk(A.G, L, seg ? seg : 1);
   const int form = site ? 4 : (own ? 3 : (seg ? 2 : (full ? 1 : 0)));

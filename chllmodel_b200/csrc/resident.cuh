@@ -149,13 +149,15 @@ struct OwnSite {
   bool v[2];                // sites 2h, 2h+1 of the row inside the lattice
   float4 n[2];              // [colour]
 
-  __device__ __forceinline__ OwnSite(const LatticeView& L, const SweepGeom& G) {
-    h = blockIdx.x * blockDim.x + threadIdx.x;
+  __device__ __forceinline__ OwnSite(const LatticeView& L, const SweepGeom& G)
+      : OwnSite(L, G, blockIdx.x * blockDim.x + threadIdx.x) {}
+  __device__ __forceinline__ OwnSite(const LatticeView& L, const SweepGeom& G, uint32_t slot) {
+    h = slot;
     g = h >> 1;
-    has = g < G.units;
     const uint32_t hx = (uint32_t)L.hx, nj = (uint32_t)L.nj, nk = (uint32_t)L.nk;
-    const uint32_t plane = hx * nj;
+    const uint32_t plane = hx * nj, wide = P ? (uint32_t)L.ni / 2 : hx;
     const uint32_t row = G.by_Q.div(g), r = h - row * hx;
+    has = g < G.units && r < wide;  // periodic: a padding slot is nobody's neighbour
     const uint32_t k = G.by_nj.div(row), j = row - k * nj;
     o0 = (j + k) & 1u;
     hyp = P || j + 1 < nj;
@@ -163,13 +165,13 @@ struct OwnSite {
     hzp = P || k + 1 < nk;
     hzm = P || k > 0;
     hxm = P || r > 0;
-    hxp = P || r + 1 < hx;
+    hxp = P || r + 1 < wide;
     yp = j + 1 < nj ? h + hx : h - (nj - 1) * hx;
     ym = j > 0 ? h - hx : h + (nj - 1) * hx;
     zp = k + 1 < nk ? h + plane : h - (nk - 1) * plane;
     zm = k > 0 ? h - plane : h + (nk - 1) * plane;
-    xm = r > 0 ? h - 1 : h + hx - 1;
-    xp = r + 1 < hx ? h + 1 : h - r;
+    xm = r > 0 ? h - 1 : h + wide - 1;
+    xp = r + 1 < wide ? h + 1 : h - r;
     v[0] = has && 2 * r < (uint32_t)L.ni;
     v[1] = has && 2 * r + 1 < (uint32_t)L.ni;
     n[0] = n[1] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -228,22 +230,24 @@ inline uint32_t resident_sms() {
   return (uint32_t)n;
 }
 
-// Whether OwnBlock (OwnSite) holds the lattice: a unit (site) per thread.
+// Whether OwnBlock (OwnSite) holds the lattice: a unit (site of each colour) per
+// thread.  An OwnSite wraps a padded row, an OwnBlock does not.
 inline bool one_unit_each(const LatticeView& L, uint32_t units) {
   return units <= resident_sms() * kResThreads && (L.ni % 4 == 0 || !L.periodic);
 }
-inline bool one_site_each(const LatticeView& L, uint32_t units) {
-  return one_unit_each(L, 2 * units);
+inline bool one_site_each(uint32_t units, uint32_t per_sm = kResThreads) {
+  return 2 * units <= resident_sms() * per_sm;
 }
 
 // Threads per CTA and CTAs for `items` threads: up to 256 one CTA (two warps per
 // scheduler), whose barrier is its own; else spread over the SMs in CTAs of whole
 // warps.
-inline void resident_shape(uint32_t items, uint32_t& block, uint32_t& ctas) {
+inline void resident_shape(uint32_t items, uint32_t& block, uint32_t& ctas,
+                           uint32_t per_sm = kResThreads) {
   const uint32_t sms = resident_sms();
   const uint32_t share = items <= 256 ? items : (items + sms - 1) / sms;
-  block = std::min<uint32_t>(kResThreads, (share + 31) / 32 * 32);
-  ctas = std::min((items + block - 1) / block, sms * (uint32_t)(kResThreads / block));
+  block = std::min<uint32_t>(per_sm, (share + 31) / 32 * 32);
+  ctas = std::min((items + block - 1) / block, sms * (per_sm / block));
 }
 
 template <class KERNEL, class ARGS>

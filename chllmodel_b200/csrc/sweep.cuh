@@ -51,12 +51,25 @@ void launch_control_update(Control* ctl, int phase, cudaStream_t stream);
 // of device memory, zero before the first launch (a launch leaves them zero).
 // resident_fits: the lattice's counts fit the words; resident_pays: the form
 // is faster than the fused passes' launches.
-constexpr size_t kResidentWordBytes = 3 * 128;
+// The words' memory is kResidentAllocBytes: behind them flow.cu's sweep number.
+constexpr size_t kResidentWordBytes = 3 * 128, kResidentAllocBytes = 4 * 128;
 bool resident_fits(const LatticeView& L);
 bool resident_pays(const LatticeView& L);
 cudaError_t launch_resident_sweeps(const LatticeView& L, const Coupling& cp, uint32_t key0,
                                    uint32_t key1, uint32_t replica, Control* ctl,
                                    unsigned long long* words, int nsweeps, cudaStream_t stream);
+
+// flow.cu: the same for small lattices, threads waiting for their neighbours'
+// sites instead of the grid.  xch: flow_bytes of device memory, zero before the
+// first launch; it and the words' sweep number are left alone between launches.
+bool flow_pays(const LatticeView& L);
+inline size_t flow_bytes(const LatticeView& L) {
+  return 2 * (size_t)L.hx * L.nj * L.nk * sizeof(float4);
+}
+cudaError_t launch_flow_sweeps(const LatticeView& L, const Coupling& cp, uint32_t key0,
+                               uint32_t key1, uint32_t replica, Control* ctl,
+                               unsigned long long* words, void* xch, int nsweeps,
+                               cudaStream_t stream);
 
 // layout.cu: natural-order (F-order, i fastest) <-> red/black float4.
 void launch_pack_f64(const LatticeView& L, const double* nx, const double* ny, const double* nz,
