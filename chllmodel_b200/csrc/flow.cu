@@ -32,15 +32,20 @@
 // has been used), so nothing is cleared on the way.
 //
 // us per sweep on one B200 (kT 0.5, K 0.5, d adapted): the barrier form, this one
-// with the count in the site warps and no guess, and this one:
+// with the count in the site warps and no guess, and its two further steps:
 //
 //   periodic         16^3   32^3   40^3   48^3    open  30x18x10  33x31x17  48^3
 //   barrier          3.92   4.03   4.49   4.59          4.06      4.20      4.84
 //   neighbours       3.30   3.29   3.59   3.88          3.35      3.49      3.93
 //   control warp     2.86   2.84   3.18   3.42          3.03      3.30      3.48
+//   proposal first   2.64   2.74   2.91   3.27          2.75      2.96      3.39
 //
-// (30^3, which had a launch per pass before: 7.0 and 3.1.)  What is left of a pass,
-// 1.4 us, is a store's way to L2 and a load's back, and one site's serial trials.
+// (30^3, which had a launch per pass before: 7.0 and 3.1.)  Proposal first: what a
+// trial does not need its neighbours for is done while they are on their way, and
+// its acceptance is worked out for both outcomes of the trial before it.  What is
+// left of a pass, 1.2 us with d fixed and 1.35 while it is adapted, is a store's way
+// to L2 and a load's back and the bond sums.  Several polls in flight do not shorten
+// it (32^3 with d fixed 2.43 against 2.36 us; the count's polls 2.73 against 2.70).
 //
 // Units, counters, arithmetic and control block are the fused form's bit for bit.
 // Every wait is bounded; one that runs out sets the status word.
@@ -119,15 +124,27 @@ struct FlowSite {
   const FlowArgs& A;
   OwnSite<P> B;
   float mag[2][5];  // [colour]: |s| of that colour's site's neighbours +y, -y, +z, -z and x
-  Ctr4 words;
+  float ang, acc, flip;  // the next trials' random numbers (UnitRandoms)
+  float mx, my, mz;      // the proposed director
 
   __device__ __forceinline__ explicit FlowSite(const FlowArgs& a)
       : A(a), B(a.L, a.G, blockIdx.x * (blockDim.x - 32) + threadIdx.x) {}
 
+  // What colour C's next trials do not need the neighbours for.
   template <int C>
-  __device__ __forceinline__ void draw(uint32_t step) {
-    words = philox4x32_10({{B.g, step, A.replica, (uint32_t)C}}, A.keys);
-    asm volatile("" : "+r"(words.v[0]), "+r"(words.v[1]), "+r"(words.v[2]), "+r"(words.v[3]));
+  __device__ __forceinline__ void draw(uint32_t step, float d) {
+    const UnitRandoms u =
+        unit_randoms(philox4x32_10({{B.g, step, A.replica, (uint32_t)C}}, A.keys));
+    const bool second = (B.h & 1u) != 0;
+    ang = second ? u.ang[1] : u.ang[0];
+    acc = second ? u.acc[1] : u.acc[0];
+    flip = second ? u.flip[1] : u.flip[0];
+    propose<C>(d);
+    asm volatile("" : "+f"(ang), "+f"(acc), "+f"(flip), "+f"(mx), "+f"(my), "+f"(mz));
+  }
+  template <int C>
+  __device__ __forceinline__ void propose(float d) {
+    propose_director(B.n[C].x, B.n[C].y, B.n[C].z, d, ang, mx, my, mz);
   }
 
   // The neighbours of colour C's site from the lattice, their magnitudes kept.
@@ -182,18 +199,46 @@ struct FlowSite {
     nb.b[1] = o ? B.n[C ^ 1] : v[4];
   }
 
+  // unit_trials_drawn of one site, its operations; a trial's acceptance is worked
+  // out for both outcomes of the trial before it.
   template <int C, bool FLIP_BEFORE, bool DIR, bool FLIP_AFTER>
-  __device__ __forceinline__ void trial(const Nbrs& nb, float d, unsigned int& nacc,
-                                        unsigned int& nflip) {
+  __device__ __forceinline__ void trial(const Nbrs& nb, unsigned int& nacc, unsigned int& nflip) {
     if (!B.has) return;
-    UnitRandoms u = unit_randoms(words);
-    const bool second = (B.h & 1u) != 0;
-    u.acc[0] = second ? u.acc[1] : u.acc[0];
-    u.ang[0] = second ? u.ang[1] : u.ang[0];
-    u.flip[0] = second ? u.flip[1] : u.flip[0];
-    float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
-    unit_trials_drawn<FLIP_BEFORE, DIR, FLIP_AFTER>(B.n[C], none, nb, nb, B.template valid<C>(),
-                                                    false, u, d, A.cp, nacc, nflip);
+    float4& n = B.n[C];
+    const Coupling& cp = A.cp;
+    const bool v = B.template valid<C>();
+    BondSums o, m;
+    if (DIR)
+      bond_sums2(n.x, n.y, n.z, mx, my, mz, nb, o, m);
+    else
+      o = bond_sums(n.x, n.y, n.z, nb);
+    bool moved = false;
+    if (DIR) moved = metropolis(director_dE(o, m, n.w, cp), acc, cp.inv_kT);
+    if (FLIP_BEFORE) {
+      const bool f = v && metropolis(flip_dE(o.c, n.w, cp), flip, cp.inv_kT);
+      if (DIR) {
+        const bool other = metropolis(director_dE(o, m, -n.w, cp), acc, cp.inv_kT);
+        moved = f ? other : moved;
+      }
+      if (f) n.w = -n.w;
+      nflip += (unsigned int)f;
+    }
+    if (DIR) {
+      moved = v && moved;
+      if (moved) {
+        n.x = mx;
+        n.y = my;
+        n.z = mz;
+      }
+      nacc += (unsigned int)moved;
+    }
+    if (FLIP_AFTER) {
+      const bool stay = metropolis(flip_dE(o.c, n.w, cp), flip, cp.inv_kT);
+      const bool f =
+          v && (DIR && moved ? metropolis(flip_dE(m.c, n.w, cp), flip, cp.inv_kT) : stay);
+      if (f) n.w = -n.w;
+      nflip += (unsigned int)f;
+    }
   }
 
   template <int C>
@@ -308,45 +353,44 @@ __device__ __forceinline__ void site_warps(const FlowArgs& A, FlowShared& S, int
   Nbrs nb;
   F.template first<1>(nb);
   F.template first<0>(nb);
-  F.template draw<0>(step);
   float d = S.d, guess = d;
+  F.template draw<0>(step, d);
   unsigned int na, nf = 0, none = 0;
   for (int s = 0; s < A.nsweeps; ++s) {
     const bool last = s == A.nsweeps - 1;
     na = nf = 0;
     if (s) {
-      const bool check = s <= nadapt;
-      if (!check) guess = d;
       F.template wait<0>(base + (uint32_t)s, S, nb);
       const float4 n = F.B.n[0];
-      F.template trial<0, true, true, false>(nb, guess, na, none);
-      if (check) {
+      F.template trial<0, true, true, false>(nb, na, none);
+      if (s <= nadapt) {
         bar_wait(kBarStep);
         d = S.d;
         if (d != guess) {
           F.B.n[0] = n;
           na = 0;
-          F.template trial<0, true, true, false>(nb, d, na, none);
+          F.template propose<0>(d);
+          F.template trial<0, true, true, false>(nb, na, none);
         }
-        guess = S.guess;
+        guess = s < nadapt ? S.guess : d;
       }
     } else {
-      F.template trial<0, false, true, false>(nb, d, na, none);
+      F.template trial<0, false, true, false>(nb, na, none);
     }
     F.template publish<0>(base + (uint32_t)s + 1u);
-    F.template draw<1>(step);
+    F.template draw<1>(step, d);
     F.template wait<1>(base + (uint32_t)s + 1u, S, nb);
-    F.template trial<1, false, true, true>(nb, d, na, nf);
+    F.template trial<1, false, true, true>(nb, na, nf);
     F.template publish<1>(base + (uint32_t)s + 1u);
     if (s < nadapt || last) {
       put_count(S.cnt[s & 1], na);
       bar_arrive(kBarCounts);
     }
     ++step;
-    F.template draw<0>(step);
+    F.template draw<0>(step, guess);
   }
   F.template wait<0>(base + (uint32_t)A.nsweeps, S, nb);
-  F.template trial<0, true, false, false>(nb, d, none, nf);  // with B's flips: the sweep's
+  F.template trial<0, true, false, false>(nb, none, nf);  // with B's flips: the sweep's
   if (F.B.has && !S.lost) {
     F.B.template store<0>(A.L);
     F.B.template store<1>(A.L);

@@ -19,7 +19,7 @@
 //   passes launched each   5.5   4.6   6.4   6.5   6.6   8.1   15.0  26.9  85.6
 //   one cluster            3.5   5.4   5.5   5.6  14.5
 //   this form              1.9   3.9   4.0   4.0   4.6   6.3   13.5  24.6  79.5
-//   flow.cu                      2.9   3.0   2.8   3.4
+//   flow.cu                      2.6   2.7   2.7   3.3
 //
 // The barrier and the counts are one 64-bit word per pass: a CTA adds its
 // accept counts and its arrival with one release reduction and polls the
@@ -333,7 +333,7 @@ bool resident_fits(const LatticeView& L) {
 }
 
 // Against a launch per pass: always where a thread holds one site of each colour
-// or one unit (50^3 periodic 3.8 against 7.5 us, 64^3 6.3 against 8.1).  Beyond
+// or one unit (50^3 periodic 3.7 against 7.5 us, 64^3 6.3 against 8.1).  Beyond
 // that the barrier still saves about 1 us per pass, but the loops' coherent
 // loads cost the units more than the read-only ones do.  With unpadded rows it
 // pays up to 256^3 (4 M units) periodic (128^3 24.6 against 26.9 us, 200^3 79.5
