@@ -578,8 +578,8 @@ __global__ void __launch_bounds__(kGradThreads) quench_pass_kernel(LatticeView L
 }
 
 // The same steps in one cooperative launch (resident.cuh): a step is a pass of
-// each colour with the grid barrier after it.  A launch per pass costs a small
-// lattice about 4 us, most of it the launch; a pass here takes 2.9 at 64^3.
+// each colour with a barrier after it.  For lattices of one CTA, whose barrier is
+// the CTA's own, and for those of more units than threads.
 struct QuenchArgs {
   LatticeView L;
   SweepGeom G;
@@ -590,32 +590,28 @@ struct QuenchArgs {
   int nsteps;
 };
 
-// FORM: 0 the unit loop, 1 one unit per thread, 2 one site of each colour.
-template <bool P, int FORM>
+struct NoOwn {
+  __device__ __forceinline__ NoOwn(const LatticeView&, const SweepGeom&) {}
+};
+
+// SITE: one site of each colour per thread (one CTA); else the unit loop.
+template <bool P, bool SITE>
 __global__ void __launch_bounds__(kResThreads, 1)
     quench_resident_kernel(const __grid_constant__ QuenchArgs A) {
   __shared__ int s_ok;
   if (A.ctl->status) return;  // an earlier wait ran out: the words are not to be trusted
   const bool lead = threadIdx.x == 0;
-  std::conditional_t<FORM == 2, OwnSite<P>, OwnBlock<P>> B(A.L, A.G);
+  std::conditional_t<SITE, OwnSite<P>, NoOwn> B(A.L, A.G);
   uint32_t slot = 0;
   auto pass = [&](auto colour) {
     constexpr int C = decltype(colour)::value;
-    if constexpr (FORM == 2) {
+    if constexpr (SITE) {
       if (!B.has) return;
       Nbrs nb;
       B.template neighbours<C>(A.L, nb);
       if (B.template valid<C>())
         B.n[C] = quench_site<P>(B.n[C], nb, A.cp, A.eta, (B.h & 1u) != 0);
       B.template store<C>(A.L);
-    } else if constexpr (FORM == 1) {
-      if (!B.has) return;
-      Nbrs nb0, nb1;
-      B.template neighbours<C>(A.L, nb0, nb1);
-      const bool odd = B.template odd<C>();
-      if (odd ? B.v[1] : B.v[0]) B.n[C][0] = quench_site<P>(B.n[C][0], nb0, A.cp, A.eta, false);
-      if (odd ? B.v[3] : B.v[2]) B.n[C][1] = quench_site<P>(B.n[C][1], nb1, A.cp, A.eta, true);
-      st_unit(A.L.col[C] + B.u, B.n[C][0], B.n[C][1]);
     } else {
       for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < A.G.units;
            g += gridDim.x * blockDim.x) {
@@ -651,6 +647,195 @@ __global__ void __launch_bounds__(kResThreads, 1)
   if (lead && gridDim.x > 1) {
     const unsigned long long old = atomicAdd(A.words + slot * kWordStride, 1ull << kArriveShift);
     if ((uint32_t)(old >> kArriveShift) == gridDim.x - 1) clear_words(A.words);
+  }
+}
+
+// The same without the grid barrier, for lattices of up to a site of each colour
+// (N = 1) or a unit (N = 2) per thread: a thread waits for its neighbours' sites,
+// as flow.cu's sweeps.  Those of its own CTA, most of an x-y neighbourhood, come
+// through shared memory and a CTA barrier; the others are published words.  What
+// bounds a pass is a word's way to L2 and back, and beyond a site per thread the
+// words' bandwidth.  us per step on one B200, with the grid barrier and here:
+//
+//   periodic   16^3   30^3   32^3   48^3   64^3    open  33x31x17  48^3   65x63x61
+//   barrier    3.41   4.13   3.49   3.95   5.49          3.58      4.14   5.77
+//   here       1.82   1.94   1.78   2.08   4.35          2.20      2.33   4.72
+//
+// (64 registers, for 1024 threads per SM and a site each at 64^3: 18.8 us there and
+// 7.5 at 32^3, as the spills wait behind the polls.)
+struct QuenchFlowArgs {
+  QuenchArgs Q;
+  uint4* xch;
+  uint32_t* epoch;
+  uint32_t per_colour;
+};
+
+__device__ __forceinline__ float4 as_site(const uint4& w) {
+  return make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z),
+                     __uint_as_float(w.w));
+}
+__device__ __forceinline__ uint4 as_word(const float4& n) {
+  return make_uint4(__float_as_uint(n.x), __float_as_uint(n.y), __float_as_uint(n.z),
+                    __float_as_uint(n.w));
+}
+
+template <bool P, int N>
+struct QuenchFlow {
+  using Own = std::conditional_t<N == 1, OwnSite<P>, OwnBlock<P>>;
+  const QuenchFlowArgs& A;
+  float4 (&sites)[2][N * kResThreads];
+  volatile int& lost;
+  Own B;
+
+  __device__ __forceinline__ QuenchFlow(const QuenchFlowArgs& a, float4 (&s)[2][N * kResThreads],
+                                        volatile int& l)
+      : A(a), sites(s), lost(l), B(a.Q.L, a.Q.G) {}
+
+  __device__ __forceinline__ uint32_t slot() const {
+    if constexpr (N == 1) return B.h;
+    else return B.u;
+  }
+  template <int C>
+  __device__ __forceinline__ float4& own(int t) {
+    if constexpr (N == 1) return B.n[C];
+    else return B.n[C][t];
+  }
+
+  // The neighbours of colour C's sites, the other CTAs' as published with `tag`.
+  template <int C>
+  __device__ __forceinline__ void neighbours(uint32_t tag, Nbrs (&nb)[N]) {
+    const uint4* const words = A.xch + (C ? 0u : A.per_colour);
+    const uint32_t first = blockIdx.x * blockDim.x * N, span = blockDim.x * N;
+    const bool o = B.template odd<C>();
+    const uint32_t at[5] = {B.yp, B.ym, B.zp, B.zm, o ? B.xp : B.xm};
+    const bool in[5] = {B.hyp, B.hym, B.hzp, B.hzm, o ? B.hxp : B.hxm};
+    bool open[5];
+    uint4 w[5][N];
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const uint32_t l = at[i] - first;
+      open[i] = in[i] && l >= span;
+#pragma unroll
+      for (int t = 0; t < (i < 4 ? N : 1); ++t)
+        w[i][t] = in[i] && l < span ? as_word(sites[C ^ 1][l + t]) : make_uint4(0, 0, 0, 0);
+    }
+    uint32_t polls = 0;
+    bool again;
+    do {
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+#pragma unroll
+        for (int t = 0; t < (i < 4 ? N : 1); ++t)
+          if (open[i]) w[i][t] = ld_word(words + at[i] + t);
+      }
+      again = false;
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        bool there = true;
+#pragma unroll
+        for (int t = 0; t < (i < 4 ? N : 1); ++t)
+          there = there && ((w[i][t].w ^ tag) & kTagMask) == 0;
+        if (there) open[i] = false;
+        again = again || open[i];
+      }
+      if (again && ++polls % 1024 == 0) {
+        if (polls >= kWaitLimit || *(volatile unsigned int*)&A.Q.ctl->status) lost = 1;
+        again = !lost;  // a lost launch runs to its end without waiting
+      }
+    } while (again);
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {  // a published site's chirality: it does not change
+      if (in[i] && at[i] - first >= span) {
+#pragma unroll
+        for (int t = 0; t < (i < 4 ? N : 1); ++t)
+          w[i][t].w = __float_as_uint(A.Q.L.col[C ^ 1][at[i] + t].w);
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) nb[t].b[2 + i] = as_site(w[i][t]);
+    }
+    const float4 e = as_site(w[4][0]), xa = own<C ^ 1>(0);
+    if constexpr (N == 1) {
+      nb[0].b[0] = o ? e : xa;
+      nb[0].b[1] = o ? xa : e;
+    } else {
+      const float4 xb = own<C ^ 1>(1);
+      nb[0].b[0] = o ? xb : xa;
+      nb[0].b[1] = o ? xa : e;
+      nb[1].b[0] = o ? e : xb;
+      nb[1].b[1] = o ? xb : xa;
+    }
+  }
+
+  // Colour 0's first neighbours, from the lattice.
+  __device__ __forceinline__ void start(Nbrs (&nb)[N]) {
+    if constexpr (N == 1) B.template neighbours<0>(A.Q.L, nb[0]);
+    else B.template neighbours<0>(A.Q.L, nb[0], nb[1]);
+  }
+
+  template <int C>
+  __device__ __forceinline__ void move(uint32_t tag, const Nbrs (&nb)[N]) {
+    if (B.has) {
+#pragma unroll
+      for (int t = 0; t < N; ++t) {
+        float4& n = own<C>(t);
+        const bool second = N == 1 ? (slot() & 1u) != 0 : t == 1;
+        if (N == 1 ? (B.template odd<C>() ? B.v[1] : B.v[0])
+                   : (B.template odd<C>() ? B.v[N * t + 1] : B.v[N * t]))
+          n = quench_site<P>(n, nb[t], A.Q.cp, A.Q.eta, second);
+        st_word(A.xch + (C ? A.per_colour : 0u) + slot() + t, n, tag);
+        sites[C][threadIdx.x * N + t] = n;
+      }
+    }
+    __syncthreads();
+  }
+
+  template <int C>
+  __device__ __forceinline__ void store() {
+    if constexpr (N == 1) B.template store<C>(A.Q.L);
+    else st_unit(A.Q.L.col[C] + B.u, B.n[C][0], B.n[C][1]);
+  }
+};
+
+template <bool P, int N>
+__global__ void __launch_bounds__(kResThreads, 1)
+    quench_flow_kernel(const __grid_constant__ QuenchFlowArgs A) {
+  __shared__ float4 sites[2][N * kResThreads];
+  __shared__ volatile int s_lost;
+  Control* const ctl = A.Q.ctl;
+  const uint32_t base = *(volatile uint32_t*)A.epoch;
+  if (threadIdx.x == 0) s_lost = *(volatile unsigned int*)&ctl->status ? 1 : 0;
+  __syncthreads();
+  const bool stale = s_lost;  // an earlier wait ran out: the words are not to be trusted
+  __syncthreads();
+  if (stale) return;
+  QuenchFlow<P, N> F(A, sites, s_lost);
+  const bool has = F.B.has;
+  for (int s = 0; s < A.Q.nsteps; ++s) {
+    Nbrs nb[N];
+    if (has) {
+      if (s)
+        F.template neighbours<0>(base + (uint32_t)s, nb);
+      else
+        F.start(nb);
+    }
+    F.template move<0>(base + (uint32_t)s + 1u, nb);
+    if (has) F.template neighbours<1>(base + (uint32_t)s + 1u, nb);
+    F.template move<1>(base + (uint32_t)s + 1u, nb);
+  }
+  if (has && !s_lost) {
+    F.template store<0>();
+    F.template store<1>();
+  }
+  if (threadIdx.x != 0) return;
+  if (s_lost) {
+    atomicOr(&ctl->status, 4u);
+    atomicAdd(A.epoch, (uint32_t)A.Q.nsteps + 2u);  // what was published is never read again
+  } else if (atomicAdd(A.Q.words, 1ull) == gridDim.x - 1) {
+    *A.epoch = base + (uint32_t)A.Q.nsteps;
+    *A.Q.words = 0;
   }
 }
 
@@ -700,13 +885,20 @@ void launch_quench_pass(const LatticeView& L, const CouplingD& cd, float eta, in
   }
 }
 
-// Against a launch per pass, us per step (periodic): 8^3 1.5 and 7.5, 48^3 4.6 and
-// 8.4, 64^3 5.7 and 8.4, 96^3 12.7 and 16.6, 128^3 24.6 and 25.0; from 160^3 on the
-// launches win (45.2 and 41.3: their loads are the read-only ones).
+// Sites (1) or a unit (2) per thread of quench_flow_kernel; 0: not that form.
+int quench_flow_sites(const LatticeView& L) {
+  const uint32_t units = make_geom(L).units;
+  if (2 * units <= 256) return 0;
+  return one_site_each(units) ? 1 : (one_unit_each(L, units) ? 2 : 0);
+}
+
+// Against a launch per pass, us per step (periodic): 8^3 1.5 and 7.5, 64^3 4.4 and
+// 8.4, 96^3 12.7 and 16.6, 128^3 24.6 and 25.0; from 160^3 on the launches win (45.2
+// and 41.3: their loads are the read-only ones).
 bool quench_resident_pays(const LatticeView& L) { return make_geom(L).units <= (1u << 19); }
 
 cudaError_t launch_quench_resident(const LatticeView& L, const CouplingD& cd, float eta,
-                                   Control* ctl, unsigned long long* words, int nsteps,
+                                   Control* ctl, unsigned long long* words, void* xch, int nsteps,
                                    cudaStream_t stream) {
   QuenchArgs A;
   A.L = L;
@@ -719,16 +911,28 @@ cudaError_t launch_quench_resident(const LatticeView& L, const CouplingD& cd, fl
   A.ctl = ctl;
   A.words = words;
   A.nsteps = nsteps;
-  const int form = one_site_each(A.G.units) ? 2 : (one_unit_each(L, A.G.units) ? 1 : 0);
+  if (const int n = quench_flow_sites(L)) {
+    QuenchFlowArgs F;
+    F.Q = A;
+    F.xch = static_cast<uint4*>(xch);
+    F.epoch = reinterpret_cast<uint32_t*>(words + 3 * kWordStride);
+    F.per_colour = 2 * A.G.units;
+    using Kernel = void (*)(const QuenchFlowArgs);
+    static const Kernel kernels[2][2] = {
+        {quench_flow_kernel<false, 1>, quench_flow_kernel<false, 2>},
+        {quench_flow_kernel<true, 1>, quench_flow_kernel<true, 2>}};
+    uint32_t threads, grid;
+    resident_shape(n == 1 ? 2 * A.G.units : A.G.units, threads, grid);
+    return launch_cooperative(kernels[L.periodic ? 1 : 0][n - 1], grid, threads, stream, F);
+  }
+  const bool site = 2 * A.G.units <= 256;
   uint32_t block, ctas;
-  resident_shape(form == 2 ? 2 * A.G.units : A.G.units, block, ctas);
+  resident_shape(site ? 2 * A.G.units : A.G.units, block, ctas);
   using Kernel = void (*)(const QuenchArgs);
-  static const Kernel kernels[2][3] = {
-      {quench_resident_kernel<false, 0>, quench_resident_kernel<false, 1>,
-       quench_resident_kernel<false, 2>},
-      {quench_resident_kernel<true, 0>, quench_resident_kernel<true, 1>,
-       quench_resident_kernel<true, 2>}};
-  return launch_cooperative(kernels[L.periodic ? 1 : 0][form], ctas, block, stream, A);
+  static const Kernel kernels[2][2] = {
+      {quench_resident_kernel<false, false>, quench_resident_kernel<false, true>},
+      {quench_resident_kernel<true, false>, quench_resident_kernel<true, true>}};
+  return launch_cooperative(kernels[L.periodic ? 1 : 0][site ? 1 : 0], ctas, block, stream, A);
 }
 
 cudaError_t launch_natural_grad(int ni, int nj, int nk, int periodic, const float* n,

@@ -161,7 +161,7 @@ struct chll_lattice {
   double* partials = nullptr;
   unsigned int* tickets = nullptr;  // [0] observables, [1] gradient
   unsigned long long* words = nullptr;  // meeting words of the resident sweeps
-  void* xch = nullptr;  // published sites of the resident sweeps without a barrier
+  void* xch = nullptr;  // published sites of flow.cu and the quench, behind lat
   double* rows = nullptr;
   int rows_cap = 0;
   double* host_rows = nullptr;  // pinned, of run()'s lattice
@@ -315,7 +315,8 @@ int sweep_impl(chll_lattice* L, const Coupling& cp, uint64_t seed, uint32_t rep,
     for (int done = 0; done < nsweeps; done += kResidentChunk) {
       const int n = std::min(kResidentChunk, nsweeps - done);
       const cudaError_t e =
-          L->xch ? chll::launch_flow_sweeps(L->view(), cp, k0, k1, rep, L->ctl, L->words, L->xch, n,
+          chll::flow_pays(L->view())
+              ? chll::launch_flow_sweeps(L->view(), cp, k0, k1, rep, L->ctl, L->words, L->xch, n,
                                             L->stream)
                  : chll::launch_resident_sweeps(L->view(), cp, k0, k1, rep, L->ctl, L->words, n,
                                                 L->stream);
@@ -482,8 +483,12 @@ int create_impl(int ni, int nj, int nk, int boundary, chll_lattice** out, int sl
   if ((e = cudaStreamCreateWithFlags(&L->capture_stream, cudaStreamNonBlocking)) != cudaSuccess)
     return bail(e, "stream");
   L->stream = L->own_stream;
-  if ((e = cudaMalloc(&L->lat, 2 * L->per_colour * sizeof(float4))) != cudaSuccess)
-    return bail(e, "lattice allocation");
+  // small lattices: the published sites behind the lattice (at most 4.8 MB)
+  const size_t lat_bytes = 2 * L->per_colour * sizeof(float4);
+  const bool publishes = !L->slab && chll::quench_flow_sites(L->view());
+  const size_t all_bytes = lat_bytes + (publishes ? chll::flow_bytes(L->view()) : 0);
+  if ((e = cudaMalloc(&L->lat, all_bytes)) != cudaSuccess) return bail(e, "lattice allocation");
+  if (publishes) L->xch = reinterpret_cast<char*>(L->lat) + lat_bytes;
   if (!chll::unit_view_aligned(L->store_view()) || !chll::unit_view_aligned(L->view())) {
     chll_lattice_destroy(L);
     return fail(CHLL_ECUDA, "lattice allocation is not 32-byte aligned");
@@ -499,19 +504,12 @@ int create_impl(int ni, int nj, int nk, int boundary, chll_lattice** out, int sl
     return bail(e, "meeting words");
   if ((e = cudaMemsetAsync(L->words, 0, chll::kResidentAllocBytes, L->stream)) != cudaSuccess)
     return bail(e, "memset");
-  if (!L->slab && chll::flow_pays(L->view())) {  // at most 2.4 MB
-    if ((e = cudaMalloc(&L->xch, chll::flow_bytes(L->view()))) != cudaSuccess)
-      return bail(e, "published sites");
-    if ((e = cudaMemsetAsync(L->xch, 0, chll::flow_bytes(L->view()), L->stream)) != cudaSuccess)
-      return bail(e, "memset");
-  }
   if ((e = cudaMalloc(&L->out4, 4 * sizeof(double) + chll::kRowLen * sizeof(double))) !=
       cudaSuccess)
     return bail(e, "result buffer");
   if ((e = cudaMemsetAsync(L->tickets, 0, 2 * sizeof(unsigned int), L->stream)) != cudaSuccess)
     return bail(e, "memset");
-  if ((e = cudaMemsetAsync(L->lat, 0, 2 * L->per_colour * sizeof(float4), L->stream)) !=
-      cudaSuccess)
+  if ((e = cudaMemsetAsync(L->lat, 0, all_bytes, L->stream)) != cudaSuccess)
     return bail(e, "memset");
   *out = L;
   if (set_control_impl(L, 0.1, 1, 10000) != CHLL_OK) {
@@ -803,7 +801,6 @@ void chll_lattice_destroy(chll_lattice* L) {
   cudaFree(L->partials);
   cudaFree(L->tickets);
   cudaFree(L->words);
-  cudaFree(L->xch);
   cudaFree(L->rows);
   if (L->host_rows) cudaFreeHost(L->host_rows);
   cudaFree(L->out4);
@@ -1011,7 +1008,8 @@ int chll_lattice_quench(chll_lattice* L, const chll_coupling* c, double eta, int
   if (chll::quench_resident_pays(v)) {
     for (int done = 0; done < nsteps; done += kResidentChunk) {
       const cudaError_t e = chll::launch_quench_resident(
-          v, cd, (float)eta, L->ctl, L->words, std::min(kResidentChunk, nsteps - done), L->stream);
+          v, cd, (float)eta, L->ctl, L->words, L->xch, std::min(kResidentChunk, nsteps - done),
+          L->stream);
       if (e != cudaSuccess) return fail(CHLL_ECUDA, "quench launch: %s", cudaGetErrorString(e));
     }
     return ok();

@@ -95,29 +95,8 @@ __device__ __forceinline__ void bar_wait(int id) {
   asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(blockDim.x) : "memory");
 }
 
-constexpr uint32_t kTagMask = 0x7fffffffu;
 constexpr int kUseShift = 52;  // count words: director accepts or flips below, arrivals above
 constexpr unsigned long long kSumMask = (1ull << kUseShift) - 1;
-
-__device__ __forceinline__ uint4 ld_word(const uint4* p) {
-  unsigned long long lo, hi;
-  asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0,%1}, t;\n\t}"
-               : "=l"(lo), "=l"(hi)
-               : "l"(p)
-               : "memory");
-  return make_uint4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32));
-}
-
-__device__ __forceinline__ void st_word(uint4* p, const float4& n, uint32_t tag) {
-  const uint32_t w = (__float_as_uint(n.w) & 0x80000000u) | (tag & kTagMask);
-  const unsigned long long lo = (unsigned long long)__float_as_uint(n.x) |
-                                ((unsigned long long)__float_as_uint(n.y) << 32);
-  const unsigned long long hi =
-      (unsigned long long)__float_as_uint(n.z) | ((unsigned long long)w << 32);
-  asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1,%2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}"
-               ::"l"(p), "l"(lo), "l"(hi)
-               : "memory");
-}
 
 template <bool P>
 struct FlowSite {

@@ -136,10 +136,8 @@ struct OwnBlock {
 // thread: slot h of both colour arrays.  In the row, colour C's site has the other
 // colour's slot h as one x neighbour (+x where its parity is even) and slot h - 1
 // or h + 1 as the other; the slots h of the rows beside are its y and z
-// neighbours.  Half of OwnBlock's serial arithmetic per pass: sweeps of 32^3 4.2
-// against 4.7 us, 48^3 4.7 against 5.1, quench steps of 48^3 4.1 against 4.6.  (1024
-// threads per SM at 64 registers would hold 64^3: quench steps 5.5 against 5.7 us,
-// but 6.1 against 6.0 open, and 8^3 1.4 against 1.3.)
+// neighbours.  Half of OwnBlock's serial arithmetic per pass: with the grid barrier
+// sweeps of 32^3 4.2 against 4.7 us, 48^3 4.7 against 5.1.
 template <bool P>
 struct OwnSite {
   uint32_t h, g, o0;        // slot, unit, parity of colour 0's site in the row
@@ -213,6 +211,31 @@ struct OwnSite {
                  : "memory");
   }
 };
+
+// A site as published to the threads of other CTAs: the director, and the
+// chirality's sign beside a number.  One 128-bit access of device scope, so a
+// reader that finds the number it waits for has the whole site.
+constexpr uint32_t kTagMask = 0x7fffffffu;
+
+__device__ __forceinline__ uint4 ld_word(const uint4* p) {
+  unsigned long long lo, hi;
+  asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0,%1}, t;\n\t}"
+               : "=l"(lo), "=l"(hi)
+               : "l"(p)
+               : "memory");
+  return make_uint4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32));
+}
+
+__device__ __forceinline__ void st_word(uint4* p, const float4& n, uint32_t tag) {
+  const uint32_t w = (__float_as_uint(n.w) & 0x80000000u) | (tag & kTagMask);
+  const unsigned long long lo = (unsigned long long)__float_as_uint(n.x) |
+                                ((unsigned long long)__float_as_uint(n.y) << 32);
+  const unsigned long long hi =
+      (unsigned long long)__float_as_uint(n.z) | ((unsigned long long)w << 32);
+  asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1,%2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}"
+               ::"l"(p), "l"(lo), "l"(hi)
+               : "memory");
+}
 
 // Streaming multiprocessors of the current device (kResThreads threads of a
 // resident launch each).

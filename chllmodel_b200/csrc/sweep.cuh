@@ -116,8 +116,9 @@ void launch_quench_pass(const LatticeView& L, const CouplingD& cd, float eta, in
 // cooperative launch; words as launch_resident_sweeps.  quench_resident_pays:
 // faster than the passes' launches.
 bool quench_resident_pays(const LatticeView& L);
+int quench_flow_sites(const LatticeView& L);  // nonzero: launch_quench_resident uses xch
 cudaError_t launch_quench_resident(const LatticeView& L, const CouplingD& cd, float eta,
-                                   Control* ctl, unsigned long long* words, int nsteps,
+                                   Control* ctl, unsigned long long* words, void* xch, int nsteps,
                                    cudaStream_t stream);
 
 // analysis.cu: shell correlations over natural-order float4 sites and a zero

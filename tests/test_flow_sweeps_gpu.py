@@ -44,3 +44,29 @@ def test_flow_equals_fused(shape, boundary):
     for (state, control), (got, got_control) in zip(*out):
         assert np.array_equal(state, got)
         assert control == got_control
+
+
+@pytest.mark.parametrize("shape,boundary", [((12, 10, 9), "open"), ((30, 18, 10), "periodic"),
+                                            ((64, 74, 32), "periodic")])  # a unit per thread
+def test_sweeps_and_quench_take_turns(shape, boundary):
+    """Both count on one sweep number; a lattice that sweeps by single passes in
+    between, and one that is new for every turn, go the same way."""
+    from chllmodel_b200.lattice import Lattice, coupling
+
+    cp = coupling(0.3, 0.9, 0.2)
+    turns = ((5, 3), (1, 2), (4, 1), (2, 8))
+    ends = []
+    for mode in ("auto", "fused", "new"):
+        lat = Lattice(*shape, boundary=boundary)
+        lat.set_kernel("fused" if mode == "fused" else "auto")
+        lat.init_random(4)
+        for i, (sweeps, steps) in enumerate(turns):
+            if mode == "new" and i:
+                state, lat = lat.download_f4(), Lattice(*shape, boundary=boundary)
+                lat.upload_f4(state)
+            lat.set_control(0.1, step=1, adapt_until=3)
+            lat.sweep(cp, sweeps, seed=6)
+            lat.quench(cp, 0.05, steps)
+        ends.append(lat.download_f4())
+    assert np.array_equal(ends[0], ends[1])
+    assert np.array_equal(ends[0], ends[2])
