@@ -32,20 +32,25 @@
 // has been used), so nothing is cleared on the way.
 //
 // us per sweep on one B200 (kT 0.5, K 0.5, d adapted): the barrier form, this one
-// with the count in the site warps and no guess, and its two further steps:
+// with the count in the site warps and no guess, and its three further steps:
 //
 //   periodic         16^3   32^3   40^3   48^3    open  30x18x10  33x31x17  48^3
 //   barrier          3.92   4.03   4.49   4.59          4.06      4.20      4.84
 //   neighbours       3.30   3.29   3.59   3.88          3.35      3.49      3.93
 //   control warp     2.86   2.84   3.18   3.42          3.03      3.30      3.48
 //   proposal first   2.64   2.74   2.91   3.27          2.75      2.96      3.39
+//   aligned          2.61   2.60   2.86   3.17          2.69      2.87      3.34
 //
-// (30^3, which had a launch per pass before: 7.0 and 3.1.)  Proposal first: what a
+// (30^3, which had a launch per pass before: 7.0 and 2.9.)  Proposal first: what a
 // trial does not need its neighbours for is done while they are on their way, and
 // its acceptance is worked out for both outcomes of the trial before it.  What is
-// left of a pass, 1.2 us with d fixed and 1.35 while it is adapted, is a store's way
-// to L2 and a load's back and the bond sums.  Several polls in flight do not shorten
-// it (32^3 with d fixed 2.43 against 2.36 us; the count's polls 2.73 against 2.70).
+// left of a pass, 1.2 us with d fixed and 1.3 while it is adapted, is a store's way to
+// L2 and a load's back, and more than that the dependent instructions of one site's
+// trials, 470 per warp and pass on one warp per scheduler (issue active 18%, waits on
+// fixed latencies twice those on loads).  Several polls in flight do not shorten it
+// (32^3 with d fixed 2.43 against 2.36 us; the count's polls 2.73 against 2.70), and
+// exchanging a CTA's own sites through shared memory, as the quench does, takes as
+// long (2.67 against 2.60 us).
 //
 // Units, counters, arithmetic and control block are the fused form's bit for bit.
 // Every wait is bounded; one that runs out sets the status word.
@@ -83,16 +88,17 @@ struct FlowShared {
 };
 
 // Named barriers between the site warps and the control warp: the sites' counts
-// are in shared memory, the next step size is, and the last counts are.
+// are in shared memory, the next step size is, and the last counts are.  Aligned:
+// every warp is together there (the other form cost 0.1 us per sweep at 32^3).
 enum FlowBarrier : int { kBarCounts = 1, kBarStep = 2, kBarEnd = 3 };
 
 __device__ __forceinline__ void bar_arrive(int id) {
   __syncwarp();
-  asm volatile("barrier.cta.arrive %0, %1;" ::"r"(id), "r"(blockDim.x) : "memory");
+  asm volatile("barrier.cta.arrive.aligned %0, %1;" ::"r"(id), "r"(blockDim.x) : "memory");
 }
 __device__ __forceinline__ void bar_wait(int id) {
   __syncwarp();
-  asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(blockDim.x) : "memory");
+  asm volatile("barrier.cta.sync.aligned %0, %1;" ::"r"(id), "r"(blockDim.x) : "memory");
 }
 
 constexpr int kUseShift = 52;  // count words: director accepts or flips below, arrivals above

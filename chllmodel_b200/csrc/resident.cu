@@ -19,7 +19,7 @@
 //   passes launched each   5.5   4.6   6.4   6.5   6.6   8.1   15.0  26.9  85.6
 //   one cluster            3.5   5.4   5.5   5.6  14.5
 //   this form              1.9   3.9   4.0   4.0   4.6   6.3   13.5  24.6  79.5
-//   flow.cu                      2.6   2.7   2.7   3.3
+//   flow.cu                      2.6   2.6   2.6   3.2
 //
 // The barrier and the counts are one 64-bit word per pass: a CTA adds its
 // accept counts and its arrival with one release reduction and polls the
