@@ -659,7 +659,10 @@ __global__ void __launch_bounds__(kResThreads, 1)
 //
 //   periodic   16^3   30^3   32^3   48^3   64^3    open  33x31x17  48^3   65x63x61
 //   barrier    3.41   4.13   3.49   3.95   5.49          3.58      4.14   5.77
-//   here       1.82   1.94   1.78   2.08   4.35          2.20      2.33   4.72
+//   here       1.81   1.96   1.78   2.11   4.25          2.18      2.25   4.44
+//
+// (With the z neighbours' chiralities loaded in every pass, 16 bytes apart, as the
+// other remote ones' still are: 64^3 4.35, 65x63x61 4.72.)
 //
 // (64 registers, for 1024 threads per SM and a site each at 64^3: 18.8 us there and
 // 7.5 at 32^3, as the spills wait behind the polls.)
@@ -686,10 +689,20 @@ struct QuenchFlow {
   float4 (&sites)[2][N * kResThreads];
   volatile int& lost;
   Own B;
+  float zs[2][2][N];  // [colour][+z, -z]: the neighbours' chiralities, which do not change
 
   __device__ __forceinline__ QuenchFlow(const QuenchFlowArgs& a, float4 (&s)[2][N * kResThreads],
                                         volatile int& l)
-      : A(a), sites(s), lost(l), B(a.Q.L, a.Q.G) {}
+      : A(a), sites(s), lost(l), B(a.Q.L, a.Q.G) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+#pragma unroll
+      for (int t = 0; t < N; ++t) {
+        zs[c][0][t] = B.has && B.hzp ? A.Q.L.col[c ^ 1][B.zp + t].w : 0.f;
+        zs[c][1][t] = B.has && B.hzm ? A.Q.L.col[c ^ 1][B.zm + t].w : 0.f;
+      }
+    }
+  }
 
   __device__ __forceinline__ uint32_t slot() const {
     if constexpr (N == 1) return B.h;
@@ -744,8 +757,13 @@ struct QuenchFlow {
       }
     } while (again);
 #pragma unroll
-    for (int i = 0; i < 5; ++i) {  // a published site's chirality: it does not change
-      if (in[i] && at[i] - first >= span) {
+    for (int t = 0; t < N; ++t) {
+      w[2][t].w = __float_as_uint(zs[C][0][t]);
+      w[3][t].w = __float_as_uint(zs[C][1][t]);
+    }
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {  // the other published sites are a CTA's border rows
+      if (i != 2 && i != 3 && in[i] && at[i] - first >= span) {
 #pragma unroll
         for (int t = 0; t < (i < 4 ? N : 1); ++t)
           w[i][t].w = __float_as_uint(A.Q.L.col[C ^ 1][at[i] + t].w);
@@ -892,7 +910,7 @@ int quench_flow_sites(const LatticeView& L) {
   return one_site_each(units) ? 1 : (one_unit_each(L, units) ? 2 : 0);
 }
 
-// Against a launch per pass, us per step (periodic): 8^3 1.5 and 7.5, 64^3 4.4 and
+// Against a launch per pass, us per step (periodic): 8^3 1.1 and 7.5, 64^3 4.3 and
 // 8.4, 96^3 12.7 and 16.6, 128^3 24.6 and 25.0; from 160^3 on the launches win (45.2
 // and 41.3: their loads are the read-only ones).
 bool quench_resident_pays(const LatticeView& L) { return make_geom(L).units <= (1u << 19); }
