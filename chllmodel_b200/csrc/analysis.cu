@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(32)
 // plane and by px between even and odd planes.  With pz = 0 the run has two
 // bins, kept in registers; with px = 0 the lanes of a row share their bin, summed
 // in the warp first (else 32 lanes add to one shared word in turn).  256^3 along
-// (1, 1, 1): 54 us (73 with one site per thread and its index divisions, 41 for
+// (1, 1, 1): 46 us (73 with one site per thread and its index divisions, 41 for
 // the read of the state alone).
 __global__ void __launch_bounds__(256)
     projection_kernel(LatticeView L, uint32_t seg, uint32_t ntasks, int px, int py, int pz,
@@ -339,7 +339,13 @@ void launch_shell_corr(const float4* site, int ni, int nj, int nk, const int4* o
 void launch_projection(const LatticeView& L, int px, int py, int pz, long long m0, int nbins,
                        unsigned long long* hist, cudaStream_t stream) {
   const uint32_t cols = 2 * (uint32_t)L.hx * (uint32_t)L.nj, nk = (uint32_t)L.nk;
-  const uint32_t ctas = (uint32_t)device_sms() * 4, threads = ctas * 256;
+  // Six CTAs per SM, or as many as the bins leave room for: the loads of four planes
+  // are all a thread has in flight.  With four, a whole call for 100 wave numbers took
+  // 155 us at 320^3 along (1, -1, 2) and 97 at 256^3 along (0, 0, 1), with six 124 and
+  // 85; eight are no better (126 and 79 to 86), and 96^3 takes 40 us with any.
+  const uint32_t room = (227u << 10) / ((uint32_t)nbins * (uint32_t)sizeof(int) + 1024);
+  const uint32_t ctas = (uint32_t)device_sms() * std::max(1u, std::min(6u, room));
+  const uint32_t threads = ctas * 256;
   // planes per task: enough tasks for the resident threads, runs as long as that
   // leaves them
   const uint32_t nseg = std::min(nk, std::max(1u, threads / cols));
