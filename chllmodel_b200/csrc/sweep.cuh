@@ -10,11 +10,11 @@ namespace chll {
 // stream capture) and one half-sweep (pass = kPassDir0..kPassSpin1).
 void sweep_prepare();
 // Sweep form: the two-pass fused sweep, the fused passes of a chunk in one
-// cooperative launch (resident.cu; auto picks it where resident_pays, else the
-// fused sweep), or the reference's four
-// half-sweeps with the direct kernel or the staged kernel (shared-memory
-// tiles by bulk copies).  All give the same chain.  Single half-sweeps
-// (chll_lattice_pass) use the direct kernel unless staged is chosen.
+// cooperative launch (flow.cu or resident.cu; auto picks it where resident_pays,
+// else the fused sweep), or the reference's four half-sweeps with the direct
+// kernel or the staged kernel (shared-memory tiles by bulk copies).  All give the
+// same chain.  Single half-sweeps (chll_lattice_pass) use the direct kernel unless
+// staged is chosen.
 enum SweepKernel : int {
   kSweepAuto = 0,
   kSweepDirect = 1,
@@ -113,8 +113,8 @@ void launch_quench_pass(const LatticeView& L, const CouplingD& cd, float eta, in
                         cudaStream_t stream);
 
 // adjoint.cu: nsteps quench steps (a pass of colour 0, then 1) in one
-// cooperative launch; words as launch_resident_sweeps.  quench_resident_pays:
-// faster than the passes' launches.
+// cooperative launch; words as launch_resident_sweeps, xch as launch_flow_sweeps.
+// quench_resident_pays: faster than the passes' launches.
 bool quench_resident_pays(const LatticeView& L);
 int quench_flow_sites(const LatticeView& L);  // nonzero: launch_quench_resident uses xch
 cudaError_t launch_quench_resident(const LatticeView& L, const CouplingD& cd, float eta,

@@ -70,13 +70,16 @@ class Lattice:
 
     def set_kernel(self, kind: str) -> None:
         """Sweep form: 'auto' ('resident' where it is the faster one: up to
-        one unit of two sites per GPU thread, about 66^3, and lattices of rows
-        of a multiple of 4 sites up to 256^3 periodic, 200^3 open; else 'fused'),
+        one unit of two sites per GPU thread, about 66^3 (periodic rows that are
+        not a multiple of 4 sites: one site of each colour, about 53^3), and
+        lattices of rows of a multiple of 4 sites up to 256^3 periodic, 200^3
+        open; else 'fused'),
         'fused' (two passes per sweep),
         'direct' (the reference's four half-sweeps, neighbours from global
         memory), 'staged' (four half-sweeps from shared-memory row tiles) or
         'resident' (the fused passes of a whole chunk in one cooperative
-        launch; lattices of 2^27 sites and more take the fused passes).  All
+        launch, whose threads wait for the grid between passes or, up to about
+        52^3, for their neighbours' sites; lattices of 2^27 sites and more take the fused passes).  All
         give the same chain bit for bit."""
         code = {"auto": 0, "direct": 1, "staged": 2, "fused": 3, "resident": 4}[kind]
         check(self._L.chll_lattice_set_kernel(self._h, code))

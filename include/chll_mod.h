@@ -132,8 +132,9 @@ void chll_lattice_destroy(chll_lattice* lat);
  * stream). */
 int chll_lattice_set_stream(chll_lattice* lat, void* stream);
 /* Sweep form: 0 auto (4 where it is the faster one -- lattices of at most one
- * unit of two sites per GPU thread, about 66^3, and of rows of a multiple of 4
- * sites up to 256^3 periodic, 200^3 open -- else 3), 1 the reference's four
+ * unit of two sites per GPU thread, about 66^3 (periodic rows that are not a
+ * multiple of 4 sites: one site of each colour, about 53^3), and of rows of a
+ * multiple of 4 sites up to 256^3 periodic, 200^3 open -- else 3), 1 the reference's four
  * half-sweeps per step with
  * neighbours read from global memory, 2 the four half-sweeps with row tiles
  * staged in shared memory by bulk copies, 3 the fused two-pass sweep (each
