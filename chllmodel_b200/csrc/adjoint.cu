@@ -659,13 +659,15 @@ __global__ void __launch_bounds__(kResThreads, 1)
 //
 //   periodic   16^3   30^3   32^3   48^3   64^3    open  33x31x17  48^3   65x63x61
 //   barrier    3.41   4.13   3.49   3.95   5.49          3.58      4.14   5.77
-//   here       1.81   1.96   1.78   2.11   4.25          2.18      2.25   4.44
+//   here       1.81   1.96   1.78   2.11   3.58          2.18      2.25   4.44
 //
 // (With the z neighbours' chiralities loaded in every pass, 16 bytes apart, as the
-// other remote ones' still are: 64^3 4.35, 65x63x61 4.72.)
-//
-// (64 registers, for 1024 threads per SM and a site each at 64^3: 18.8 us there and
-// 7.5 at 32^3, as the spills wait behind the polls.)
+// other remote ones' still are, a unit each: 64^3 4.35 against 4.25, 65x63x61 4.72.)
+// T threads per SM: 512 with 128 registers, and periodic up to 896 with 72, where a
+// site each is still faster than a unit each though 100 bytes spill.  Spills wait
+// behind the polls: a form with a kilobyte of them took 18.8 us at 64^3.
+constexpr int kQuenchWide = 896;  // threads of 72 registers per SM
+
 struct QuenchFlowArgs {
   QuenchArgs Q;
   uint4* xch;
@@ -682,16 +684,16 @@ __device__ __forceinline__ uint4 as_word(const float4& n) {
                     __float_as_uint(n.w));
 }
 
-template <bool P, int N>
+template <bool P, int N, int T>
 struct QuenchFlow {
   using Own = std::conditional_t<N == 1, OwnSite<P>, OwnBlock<P>>;
   const QuenchFlowArgs& A;
-  float4 (&sites)[2][N * kResThreads];
+  float4 (&sites)[2][N * T];
   volatile int& lost;
   Own B;
   float zs[2][2][N];  // [colour][+z, -z]: the neighbours' chiralities, which do not change
 
-  __device__ __forceinline__ QuenchFlow(const QuenchFlowArgs& a, float4 (&s)[2][N * kResThreads],
+  __device__ __forceinline__ QuenchFlow(const QuenchFlowArgs& a, float4 (&s)[2][N * T],
                                         volatile int& l)
       : A(a), sites(s), lost(l), B(a.Q.L, a.Q.G) {
 #pragma unroll
@@ -817,10 +819,10 @@ struct QuenchFlow {
   }
 };
 
-template <bool P, int N>
-__global__ void __launch_bounds__(kResThreads, 1)
+template <bool P, int N, int T>
+__global__ void __launch_bounds__(T, 1)
     quench_flow_kernel(const __grid_constant__ QuenchFlowArgs A) {
-  __shared__ float4 sites[2][N * kResThreads];
+  __shared__ float4 sites[2][N * T];
   __shared__ volatile int s_lost;
   Control* const ctl = A.Q.ctl;
   const uint32_t base = *(volatile uint32_t*)A.epoch;
@@ -829,7 +831,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
   const bool stale = s_lost;  // an earlier wait ran out: the words are not to be trusted
   __syncthreads();
   if (stale) return;
-  QuenchFlow<P, N> F(A, sites, s_lost);
+  QuenchFlow<P, N, T> F(A, sites, s_lost);
   const bool has = F.B.has;
   for (int s = 0; s < A.Q.nsteps; ++s) {
     Nbrs nb[N];
@@ -903,14 +905,19 @@ void launch_quench_pass(const LatticeView& L, const CouplingD& cd, float eta, in
   }
 }
 
-// Sites (1) or a unit (2) per thread of quench_flow_kernel; 0: not that form.
+// Sites (1) or a unit (2) per thread of quench_flow_kernel; 0: not that form.  With
+// kQuenchWide threads per SM a site each takes periodic lattices up to 64^3 (3.58
+// against 4.25 us with a unit each, 56^3 2.82 against 3.70, and 54^3, whose rows are
+// padded, 3.0 against the unit loop's 5.4); the open kernel spills more there and is
+// slower (4.6 against 4.3).
 int quench_flow_sites(const LatticeView& L) {
   const uint32_t units = make_geom(L).units;
   if (2 * units <= 256) return 0;
-  return one_site_each(units) ? 1 : (one_unit_each(L, units) ? 2 : 0);
+  if (one_site_each(units, L.periodic ? kQuenchWide : kResThreads)) return 1;
+  return one_unit_each(L, units) ? 2 : 0;
 }
 
-// Against a launch per pass, us per step (periodic): 8^3 1.1 and 7.5, 64^3 4.3 and
+// Against a launch per pass, us per step (periodic): 8^3 1.1 and 7.5, 64^3 3.6 and
 // 8.4, 96^3 12.7 and 16.6, 128^3 24.6 and 25.0; from 160^3 on the launches win (45.2
 // and 41.3: their loads are the read-only ones).
 bool quench_resident_pays(const LatticeView& L) { return make_geom(L).units <= (1u << 19); }
@@ -936,12 +943,17 @@ cudaError_t launch_quench_resident(const LatticeView& L, const CouplingD& cd, fl
     F.epoch = reinterpret_cast<uint32_t*>(words + 3 * kWordStride);
     F.per_colour = 2 * A.G.units;
     using Kernel = void (*)(const QuenchFlowArgs);
-    static const Kernel kernels[2][2] = {
-        {quench_flow_kernel<false, 1>, quench_flow_kernel<false, 2>},
-        {quench_flow_kernel<true, 1>, quench_flow_kernel<true, 2>}};
+    const bool wide = n == 1 && !one_site_each(A.G.units);
+    const Kernel kernel =
+        wide ? quench_flow_kernel<true, 1, kQuenchWide>
+             : (n == 1 ? (L.periodic ? quench_flow_kernel<true, 1, kResThreads>
+                                     : quench_flow_kernel<false, 1, kResThreads>)
+                       : (L.periodic ? quench_flow_kernel<true, 2, kResThreads>
+                                     : quench_flow_kernel<false, 2, kResThreads>));
     uint32_t threads, grid;
-    resident_shape(n == 1 ? 2 * A.G.units : A.G.units, threads, grid);
-    return launch_cooperative(kernels[L.periodic ? 1 : 0][n - 1], grid, threads, stream, F);
+    resident_shape(n == 1 ? 2 * A.G.units : A.G.units, threads, grid,
+                   wide ? kQuenchWide : kResThreads);
+    return launch_cooperative(kernel, grid, threads, stream, F);
   }
   const bool site = 2 * A.G.units <= 256;
   uint32_t block, ctas;

@@ -1,4 +1,4 @@
-"""The quench's forms: one unit per thread, the unit loop and a launch per pass
+"""The quench's forms: one site or unit per thread, the unit loop and a launch per pass
 follow the same steps, and each step is the FP64 one to rounding."""
 import numpy as np
 import pytest
@@ -27,7 +27,9 @@ def _tiled(shape, copies, steps):
 
 
 @pytest.mark.parametrize("shape,copies", [((64, 64, 32), (1, 2, 4, 18)),   # 32,768 .. 589,824 units
-                                          ((30, 18, 10), (1, 3, 440))])    # padded rows
+                                          ((64, 74, 32), (1, 2)),  # 75,776 and 151,552 slots
+                                          ((62, 74, 28), (1, 2)),  # padded: 66,304, 132,608
+                                          ((30, 18, 10), (1, 3, 30, 440))])  # padded rows
 def test_forms_agree(shape, copies):
     """A lattice repeated along z stays a repetition: every copy equals the
     smallest lattice's run, whatever form its size takes."""
