@@ -1226,7 +1226,7 @@ int chll_batch_set_tuning(chll_batch* B, int threads, int ctas_per_sm) {
   return chll::record_ok();
 }
 
-// Tries every (threads, CTAs per SM) shape that fits for `trial_sweeps`
+// Tries the (threads, CTAs per SM) shapes that can be the fastest for `trial_sweeps`
 // sweeps from a snapshot of the current state, keeps the fastest, and
 // restores the snapshot.
 int chll_batch_autotune(chll_batch* B, int trial_sweeps, int* best_threads, int* best_ctas,
@@ -1253,8 +1253,8 @@ int chll_batch_autotune(chll_batch* B, int trial_sweeps, int* best_threads, int*
   long long bw = B->wave_bytes;
   // Candidates: one wave, or waves of 40, 64 or 96 MiB of state (a wave that
   // fits in the 126 MB L2 runs its sweeps from L2, at the price of fewer
-  // replicas sharing the grid); each block size at its two highest
-  // occupancies (lower occupancies were never faster on this kernel).  Trials
+  // replicas sharing the grid); each block size at its highest
+  // occupancy or its two highest (lower ones were never faster on this kernel).  Trials
   // measure every 10 sweeps like a production run.  A wave size that holds the
   // whole batch is the one-wave launch again and is not timed twice.  Pairing and
   // the pooled passes are not tried: over 21 sets, 2 to 1300 replicas of 8^3 to
@@ -1263,12 +1263,20 @@ int chll_batch_autotune(chll_batch* B, int trial_sweeps, int* best_threads, int*
   const long long kWaveOptions[] = {0ll, 40ll << 20, 64ll << 20, 96ll << 20};
   long long state_bytes = 0;
   for (size_t pc : B->per_colour) state_bytes += (long long)(2 * pc * sizeof(float4));
+  // The second highest occupancy only where there are few units per thread (four,
+  // with 512 threads per SM) or many replicas: over 114 sets (1 to 400 replicas of
+  // 8^3 to 128^3, 25 of them mixed) it was the fastest by more than 1% for 32, with
+  // at most 2.3 units per thread or 400 replicas, and never for the 46 that leave it
+  // out here.  These trials are the slowest ones: tuning 16 x 48^3 takes 1.55 ms without
+  // them, 2.3 with.
+  const bool full_only =
+      B->slots / 4 > 4ull * 512 * (size_t)B->sms && B->n <= B->sms;
   B->pair = 0;
   for (long long wb : kWaveOptions)
   for (int threads : {128, 256, 512}) {
     if (wb >= state_bytes) continue;
     const int occ = occupancy_of(threads, false);
-    for (int c = std::max(1, occ - 1); c <= occ && rc == CHLL_OK; ++c) {
+    for (int c = std::max(1, full_only ? occ : occ - 1); c <= occ && rc == CHLL_OK; ++c) {
       if (c * threads > 2048) break;
       B->threads = threads;
       B->ctas_per_sm = c;

@@ -283,8 +283,8 @@ int chll_batch_get_pairing(chll_batch* b, int* pair);
 int chll_batch_set_wait_limit(chll_batch* b, uint64_t polls);
 int chll_batch_get_tuning(chll_batch* b, int32_t* threads, int32_t* ctas_per_sm,
                           int64_t* wave_bytes, int32_t* nwaves);
-/* Times every launch shape (threads, CTAs per SM, wave size) for trial_sweeps
- * sweeps from a snapshot of the current state, keeps the fastest (of the
+/* Times the launch shapes (threads, CTAs per SM, wave size) that can be the
+ * fastest for this batch for trial_sweeps sweeps from a snapshot of the current state, keeps the fastest (of the
  * persistent launch with single groups; pairing and pooled passes are never the
  * fastest and are turned off) and restores the state. */
 int chll_batch_autotune(chll_batch* b, int trial_sweeps, int* best_threads, int* best_ctas,

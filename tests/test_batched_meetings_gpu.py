@@ -76,3 +76,26 @@ def test_more_replicas_than_ctas(threads):
             lat.sweep(coupling(0.5, 0.7), 5, seed=sp["seed"], replica=sp["replica"])
             assert np.array_equal(b.download_f4(r), lat.download_f4())
             lat.close()
+
+
+@pytest.mark.parametrize("size,count", [(48, 10), (48, 11), (8, 148), (20, 149)])
+def test_tuned_batches_keep_their_state(size, count):
+    """Either side of the sizes whose lower occupancies are tried: the tuner
+    leaves states and control values as they were, and the run follows its lattice."""
+    from chllmodel_b200.batched import Batch, replica
+    from chllmodel_b200.lattice import Lattice, coupling
+
+    with Batch([replica(size, kT=0.6, K=0.8, seed=r, replica=r) for r in range(count)]) as b:
+        b.init_random()
+        before = b.download_f4(count - 1)
+        tuned = b.autotune(trial_sweeps=2, cache=False)
+        assert np.array_equal(before, b.download_f4(count - 1))
+        assert tuned["ctas_per_sm"] >= 1
+        b.run(3, 0)
+        after = b.download_f4(count - 1)
+    lat = Lattice(size, size, size, boundary="periodic")
+    lat.init_random(count - 1, count - 1)
+    lat.set_control(0.1, step=1)
+    lat.sweep(coupling(0.6, 0.8), 3, seed=count - 1, replica=count - 1)
+    assert np.array_equal(after, lat.download_f4())
+    lat.close()
