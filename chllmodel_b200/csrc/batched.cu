@@ -614,6 +614,12 @@ double pass_cost(const chll::ReplicaDesc& D, uint32_t threads, uint32_t* seg) {
                               seg);
 }
 
+// The captured launch of run_impl.
+void drop_graph(chll_batch* B) {
+  if (B->graph) cudaGraphExecDestroy(B->graph);
+  B->graph = nullptr;
+}
+
 // Splits the replicas into waves whose float4 state together stays within
 // wave_bytes (0: one wave), largest replicas first, and gives every replica of
 // a wave CTAs in proportion to its units (at least one, at most one per
@@ -719,6 +725,7 @@ int shape_launch(chll_batch* B) {
   B->grid = budget;
   B->nwaves = (int)waves.size();
   if (B->cta_replica_cap < map.size()) {  // kept from shape to shape (the tuner tries dozens)
+    drop_graph(B);  // it holds the map's address
     if (B->d_cta_replica) cudaFree(B->d_cta_replica);
     B->d_cta_replica = nullptr;
     B->cta_replica_cap = 0;
@@ -875,8 +882,7 @@ int run_impl(chll_batch* B, int nsweeps, int every, int from) {
   if (!(B->graph && B->g_sweeps == nsweeps && B->g_every == every && B->g_from == from &&
         B->g_grid == B->grid && B->g_threads == B->threads && B->g_waves == B->wave_bytes &&
         B->g_limit == B->limit && B->g_pair == B->pair)) {
-    if (B->graph) cudaGraphExecDestroy(B->graph);
-    B->graph = nullptr;
+    drop_graph(B);
     cudaGraph_t g = nullptr;
     BATCH_CUDA(cudaStreamBeginCapture(B->capture_stream, cudaStreamCaptureModeThreadLocal));
     rc = launch_batch(B, B->capture_stream, nsweeps, every, from);
@@ -1038,7 +1044,7 @@ void chll_batch_destroy(chll_batch* B) {
   if (!B) return;
   if (B->own_stream) cudaStreamSynchronize(B->own_stream);
   if (B->stream && B->stream != B->own_stream) cudaStreamSynchronize(B->stream);
-  if (B->graph) cudaGraphExecDestroy(B->graph);
+  drop_graph(B);
   for (cudaGraphExec_t g : B->pool_graph)
     if (g) cudaGraphExecDestroy(g);
   cudaFree(B->d_ctl);
