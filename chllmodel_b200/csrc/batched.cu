@@ -639,6 +639,7 @@ int shape_launch(chll_batch* B) {
   const int per_sm = std::min(B->ctas_per_sm > 0 ? std::min(B->ctas_per_sm, occ) : occ,
                               chll::kMaxCtasPerSm);
   const int budget = B->sms * per_sm;
+  B->grid = 0;  // no shape until this one is whole: a failure below leaves none behind
   // waves, largest first
   std::vector<int> order(B->n);
   for (int r = 0; r < B->n; ++r) order[r] = r;
@@ -722,7 +723,6 @@ int shape_launch(chll_batch* B) {
       for (int c = 0; c < cnt[t]; ++c) map[w * (size_t)budget + next++] = groups[t];
     }
   }
-  B->grid = budget;
   B->nwaves = (int)waves.size();
   if (B->cta_replica_cap < map.size()) {  // kept from shape to shape (the tuner tries dozens)
     drop_graph(B);  // it holds the map's address
@@ -737,6 +737,7 @@ int shape_launch(chll_batch* B) {
   BATCH_CUDA(cudaMemcpyAsync(B->d_desc, B->desc.data(), sizeof(chll::ReplicaDesc) * B->n,
                              cudaMemcpyHostToDevice, B->stream));
   BATCH_CUDA(cudaStreamSynchronize(B->stream));
+  B->grid = budget;
   B->shape_threads = B->threads;
   B->shape_ctas = B->ctas_per_sm;
   B->shape_wave_bytes = B->wave_bytes;

@@ -49,6 +49,6 @@ def _run(exe, *args):
     assert r.returncode == 0, r.stdout + r.stderr
 
 
-@pytest.mark.parametrize("what", ["larger_map", "tuned"])
+@pytest.mark.parametrize("what", ["larger_map", "tuned", "no_memory", "no_copy"])
 def test_batch_launches_only_allocated_memory(program, what):
     _run(program("batch_map", "batched.cu", "capi.cu"), what)
