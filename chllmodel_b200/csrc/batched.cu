@@ -1247,13 +1247,34 @@ int chll_batch_autotune(chll_batch* B, int trial_sweeps, int* best_threads, int*
                              cudaMemcpyDeviceToDevice, B->stream));
   BATCH_CUDA(cudaMemcpyAsync(B->snap_state, B->d_state, sizeof(chll::ReplicaState) * B->n,
                              cudaMemcpyDeviceToDevice, B->stream));
+  // The snapshot back, and with its status words the meetings': a trial whose wait
+  // gave up leaves arrivals in them.
+  auto restore = [&]() -> int {
+    BATCH_CUDA(cudaMemcpyAsync(B->lat, B->snap_lat, B->slots * sizeof(float4),
+                               cudaMemcpyDeviceToDevice, B->stream));
+    BATCH_CUDA(cudaMemcpyAsync(B->d_state, B->snap_state, sizeof(chll::ReplicaState) * B->n,
+                               cudaMemcpyDeviceToDevice, B->stream));
+    BATCH_CUDA(cudaMemsetAsync(B->d_words, 0,
+                               sizeof(unsigned long long) * chll::kMeetWords * B->n, B->stream));
+    return CHLL_OK;
+  };
+  std::vector<chll::ReplicaState> after(B->n);
+  // whether every sweep of the trial was run
+  auto complete = [&](bool* all) -> int {
+    BATCH_CUDA(cudaMemcpyAsync(after.data(), B->d_state, sizeof(chll::ReplicaState) * B->n,
+                               cudaMemcpyDeviceToHost, B->stream));
+    BATCH_CUDA(cudaStreamSynchronize(B->stream));
+    *all = true;
+    for (const chll::ReplicaState& st : after) *all = *all && st.status == 0;
+    return CHLL_OK;
+  };
+  cudaEvent_t e0, e1;
+  BATCH_CUDA(cudaEventCreate(&e0));
+  BATCH_CUDA(cudaEventCreate(&e1));
   const int keep_threads = B->threads, keep_ctas = B->ctas_per_sm, keep_pair = B->pair,
             keep_pooled = B->pooled;
   B->pooled = 0;
   const long long keep_waves = B->wave_bytes;
-  cudaEvent_t e0, e1;
-  BATCH_CUDA(cudaEventCreate(&e0));
-  BATCH_CUDA(cudaEventCreate(&e1));
   double best = 1e300;
   int bt = keep_threads, bc = keep_ctas;
   int rc = CHLL_OK;
@@ -1289,12 +1310,8 @@ int chll_batch_autotune(chll_batch* B, int trial_sweeps, int* best_threads, int*
       B->ctas_per_sm = c;
       B->wave_bytes = wb;
       rc = shape_launch(B);
-      if (rc != CHLL_OK) break;
-      cudaMemcpyAsync(B->lat, B->snap_lat, B->slots * sizeof(float4), cudaMemcpyDeviceToDevice,
-                      B->stream);
-      cudaMemcpyAsync(B->d_state, B->snap_state, sizeof(chll::ReplicaState) * B->n,
-                      cudaMemcpyDeviceToDevice, B->stream);
-      rc = launch_batch(B, B->stream, 1, 0, 0);  // warm-up
+      if (rc == CHLL_OK) rc = restore();
+      if (rc == CHLL_OK) rc = launch_batch(B, B->stream, 1, 0, 0);  // warm-up
       if (rc != CHLL_OK) break;
       cudaEventRecord(e0, B->stream);
       rc = launch_batch(B, B->stream, trial_sweeps, 10, 0);
@@ -1307,6 +1324,10 @@ int chll_batch_autotune(chll_batch* B, int trial_sweeps, int* best_threads, int*
       }
       float ms = 0.f;
       cudaEventElapsedTime(&ms, e0, e1);
+      bool all = false;
+      rc = complete(&all);
+      if (rc != CHLL_OK) break;
+      if (!all) continue;  // a launch that gave up is not timed
       if (std::getenv("CHLL_TUNE_VERBOSE"))
         std::fprintf(stderr,
                      "chll batch tune: threads %d ctas/SM %d wave %lld MiB waves %d: %.3f ms\n",
@@ -1321,11 +1342,11 @@ int chll_batch_autotune(chll_batch* B, int trial_sweeps, int* best_threads, int*
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  cudaMemcpyAsync(B->lat, B->snap_lat, B->slots * sizeof(float4), cudaMemcpyDeviceToDevice,
-                  B->stream);
-  cudaMemcpyAsync(B->d_state, B->snap_state, sizeof(chll::ReplicaState) * B->n,
-                  cudaMemcpyDeviceToDevice, B->stream);
-  BATCH_CUDA(cudaStreamSynchronize(B->stream));
+  if (rc == CHLL_OK && best == 1e300)
+    rc = fail(CHLL_EDEVICE, "batch_autotune: a replica group barrier timed out in every trial");
+  const cudaError_t e = restore() == CHLL_OK ? cudaStreamSynchronize(B->stream) : cudaErrorUnknown;
+  if (e != cudaSuccess && rc == CHLL_OK)
+    rc = fail(CHLL_ECUDA, "batch_autotune: restoring the state: %s", cudaGetErrorString(e));
   if (rc != CHLL_OK) {
     B->threads = keep_threads;
     B->ctas_per_sm = keep_ctas;

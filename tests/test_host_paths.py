@@ -52,3 +52,7 @@ def _run(exe, *args):
 @pytest.mark.parametrize("what", ["larger_map", "tuned", "no_memory", "no_copy"])
 def test_batch_launches_only_allocated_memory(program, what):
     _run(program("batch_map", "batched.cu", "capi.cu"), what)
+
+
+def test_tuner_and_trials_that_give_up(program):
+    _run(program("batch_lost", "batched.cu", "capi.cu"))
