@@ -151,13 +151,22 @@ struct DeviceGuard {
   }
 };
 
+// A lattice's control block and, behind it, the results that come back with it in
+// one copy.
+struct ControlResults {
+  Control ctl;
+  double out4[4];
+  double row[chll::kRowLen];
+};
+
 struct chll_lattice {
   int ni = 0, nj = 0, nk = 0, hx = 0, periodic = 0;
   long long nsites = 0;
   size_t per_colour = 0;
   int device = 0;
   float4* lat = nullptr;
-  Control* ctl = nullptr;
+  ControlResults* results = nullptr;
+  Control* ctl = nullptr;  // results->ctl
   double* partials = nullptr;
   unsigned int* tickets = nullptr;  // [0] observables, [1] gradient
   unsigned long long* words = nullptr;  // meeting words of the resident sweeps
@@ -165,7 +174,6 @@ struct chll_lattice {
   double* rows = nullptr;
   int rows_cap = 0;
   double* host_rows = nullptr;  // pinned, of run()'s lattice
-  double* out4 = nullptr;
   void* staging = nullptr;
   size_t staging_bytes = 0;
   float4* grad = nullptr;
@@ -175,6 +183,10 @@ struct chll_lattice {
   std::vector<GraphEntry> graphs;
   uint64_t use_clock = 0;
   int kernel = chll::kSweepAuto;
+  // Launches whose waits can give up (and then set the status word) have been made
+  // since the word was last read; some of them into a caller's graph, whose
+  // replays are not seen here.
+  bool unread_waits = false, captured_waits = false;
   // z-slab of a larger lattice: global planes z0 .. z0+nk-1 of nk_global,
   // stored as planes 2 .. nk+1 of nk+3 (plane 1 and nk+2 are the halos,
   // plane 0 keeps the storage checkerboard equal to the global one).
@@ -235,6 +247,37 @@ void drop_graphs(chll_lattice* L) {
   for (auto& g : L->graphs)
     if (g.exec) cudaGraphExecDestroy(g.exec);
   L->graphs.clear();
+}
+
+// Before a launch whose waits can give up.
+void note_waits(chll_lattice* L) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(L->stream, &st) != cudaSuccess) cudaGetLastError();
+  if (st != cudaStreamCaptureStatusNone) L->captured_waits = true;
+  L->unread_waits = true;
+}
+
+// The status word as read from the device: a set one is an error of the call that
+// read it, and of those after it until set_control clears it.
+int report_status(chll_lattice* L, unsigned int status) {
+  L->unread_waits = status != 0 || L->captured_waits;
+  if (status)
+    return fail(CHLL_EDEVICE,
+                "device status word 0x%x: a wait gave up and the state is not usable (load one and "
+                "set the control block again)",
+                status);
+  return CHLL_OK;
+}
+
+// The end of a synchronising call: waits for the stream and reports a wait that
+// gave up.  The word is read only where one can have.
+int finish(chll_lattice* L) {
+  unsigned int status = 0;
+  if (L->unread_waits)
+    CHLL_CUDA_TRY(cudaMemcpyAsync(&status, &L->ctl->status, sizeof(status),
+                                  cudaMemcpyDeviceToHost, L->stream));
+  CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
+  return L->unread_waits ? report_status(L, status) : CHLL_OK;
 }
 
 // Returns an executable graph of `nsweeps` steps for this coupling and key,
@@ -311,7 +354,9 @@ int sweep_impl(chll_lattice* L, const Coupling& cp, uint64_t seed, uint32_t rep,
   if (nsweeps <= 0) return CHLL_OK;
   const uint32_t k0 = seed_lo(seed), k1 = seed_hi(seed);
   const DeviceGuard on(L->device);
-  if (runs_resident(L)) {
+  const bool resident = runs_resident(L);
+  if (resident || L->kernel == chll::kSweepStaged) note_waits(L);
+  if (resident) {
     for (int done = 0; done < nsweeps; done += kResidentChunk) {
       const int n = std::min(kResidentChunk, nsweeps - done);
       const cudaError_t e =
@@ -407,6 +452,7 @@ int set_control_impl(chll_lattice* L, double d, long long step, long long adapt_
   // the new block's status is clear: so are the words a failed wait left
   CHLL_CUDA_TRY(cudaMemsetAsync(L->words, 0, chll::kResidentWordBytes, L->stream));
   CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
+  L->unread_waits = L->captured_waits;
   return CHLL_OK;
 }
 
@@ -493,7 +539,9 @@ int create_impl(int ni, int nj, int nk, int boundary, chll_lattice** out, int sl
     chll_lattice_destroy(L);
     return fail(CHLL_ECUDA, "lattice allocation is not 32-byte aligned");
   }
-  if ((e = cudaMalloc(&L->ctl, sizeof(Control))) != cudaSuccess) return bail(e, "control");
+  if ((e = cudaMalloc(&L->results, sizeof(ControlResults))) != cudaSuccess)
+    return bail(e, "control");
+  L->ctl = &L->results->ctl;
   const int pb = std::max(chll::observables_max_blocks() * chll::kObsMoments,
                           chll::energy_grad_max_blocks() * 4);
   if ((e = cudaMalloc(&L->partials, sizeof(double) * pb)) != cudaSuccess)
@@ -504,9 +552,6 @@ int create_impl(int ni, int nj, int nk, int boundary, chll_lattice** out, int sl
     return bail(e, "meeting words");
   if ((e = cudaMemsetAsync(L->words, 0, chll::kResidentAllocBytes, L->stream)) != cudaSuccess)
     return bail(e, "memset");
-  if ((e = cudaMalloc(&L->out4, 4 * sizeof(double) + chll::kRowLen * sizeof(double))) !=
-      cudaSuccess)
-    return bail(e, "result buffer");
   if ((e = cudaMemsetAsync(L->tickets, 0, 2 * sizeof(unsigned int), L->stream)) != cudaSuccess)
     return bail(e, "memset");
   if ((e = cudaMemsetAsync(L->lat, 0, all_bytes, L->stream)) != cudaSuccess)
@@ -669,13 +714,14 @@ int run_impl(const chll_run_config& cfg, int nstart, int nstop, int nout, double
   if (rc == CHLL_OK && cfg.verbose) flush_rows(true);
   for (auto ev : events) cudaEventDestroy(ev);
 
-  if (rc == CHLL_OK) rc = download_f64_impl(L, nx, ny, nz, s);
+  Control c;
   if (rc == CHLL_OK) {
-    Control c;
     e = cudaMemcpy(&c, L->ctl, sizeof(c), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) rc = fail(CHLL_ECUDA, "run: %s", cudaGetErrorString(e));
-    else if (d_out) *d_out = c.d;
+    else rc = report_status(L, c.status);  // the caller's arrays keep what they held
   }
+  if (rc == CHLL_OK) rc = download_f64_impl(L, nx, ny, nz, s);
+  if (rc == CHLL_OK && d_out) *d_out = c.d;
   if (rc == CHLL_OK) {
     for (long long q = 0; q < r; ++q) {
       const double* hr = host_rows + q * chll::kRowLen;
@@ -797,13 +843,12 @@ void chll_lattice_destroy(chll_lattice* L) {
   if (L->own_stream) cudaStreamSynchronize(L->own_stream);
   if (L->stream && L->stream != L->own_stream) cudaStreamSynchronize(L->stream);
   cudaFree(L->lat);
-  cudaFree(L->ctl);
+  cudaFree(L->results);
   cudaFree(L->partials);
   cudaFree(L->tickets);
   cudaFree(L->words);
   cudaFree(L->rows);
   if (L->host_rows) cudaFreeHost(L->host_rows);
-  cudaFree(L->out4);
   cudaFree(L->staging);
   cudaFree(L->grad);
   if (L->own_stream) cudaStreamDestroy(L->own_stream);
@@ -833,7 +878,7 @@ int chll_lattice_set_stream(chll_lattice* L, void* stream) {
 
 int chll_lattice_sync(chll_lattice* L) {
   if (!L) return fail(CHLL_EINVAL, "null lattice");
-  CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
+  CHLL_TRY(finish(L));
   return ok();
 }
 
@@ -858,6 +903,7 @@ int chll_lattice_upload_f64(chll_lattice* L, const double* nx, const double* ny,
 int chll_lattice_download_f64(chll_lattice* L, double* nx, double* ny, double* nz, int* s) {
   if (!L) return fail(CHLL_EINVAL, "null lattice");
   CHLL_TRY(download_f64_impl(L, nx, ny, nz, s));
+  CHLL_TRY(finish(L));
   return ok();
 }
 
@@ -890,7 +936,7 @@ int chll_lattice_download_f4(chll_lattice* L, float* xyzs) {
                                   L->stream));
   }
   CHLL_CUDA_TRY(cudaGetLastError());
-  CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
+  CHLL_TRY(finish(L));
   return ok();
 }
 
@@ -916,7 +962,7 @@ int chll_lattice_get_control(chll_lattice* L, double* d, int64_t* step, double* 
   Control c;
   CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
   CHLL_CUDA_TRY(cudaMemcpy(&c, L->ctl, sizeof(c), cudaMemcpyDeviceToHost));
-  if (c.status) return fail(CHLL_EDEVICE, "device status word 0x%x", c.status);
+  CHLL_TRY(report_status(L, c.status));
   if (d) *d = c.d;
   if (step) *step = c.step;
   if (paccept) *paccept = c.paccept;
@@ -954,9 +1000,11 @@ int chll_lattice_pass(chll_lattice* L, const chll_coupling* c, uint64_t seed, ui
   if (pass >= 4)
     chll::launch_fused_pass(L->view(), make_coupling(*c), seed_lo(seed), seed_hi(seed), replica,
                             L->ctl, pass - 4, L->stream);
-  else
+  else {
+    if (L->kernel == chll::kSweepStaged) note_waits(L);
     chll::launch_sweep_pass(L->view(), make_coupling(*c), seed_lo(seed), seed_hi(seed),
                             replica, L->ctl, pass, L->stream, L->kernel);
+  }
   CHLL_CUDA_TRY(cudaGetLastError());
   return ok();
 }
@@ -984,17 +1032,19 @@ int chll_lattice_read_rows(chll_lattice* L, double* rows16, int first, int count
   CHLL_CUDA_TRY(cudaMemcpyAsync(rows16, L->rows + (size_t)first * chll::kRowLen,
                                 sizeof(double) * chll::kRowLen * count, cudaMemcpyDeviceToHost,
                                 L->stream));
-  CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
+  CHLL_TRY(finish(L));
   return ok();
 }
 
 int chll_lattice_observe(chll_lattice* L, const chll_coupling* c, double* row16) {
   if (!L || !c || !row16) return fail(CHLL_EINVAL, "observe: null argument");
-  double* drow = L->out4 + 4;
-  CHLL_TRY(observe_impl(L, make_coupling_d(*c), drow, chll::kStepOfControl));
-  CHLL_CUDA_TRY(cudaMemcpyAsync(row16, drow, sizeof(double) * chll::kRowLen,
-                                cudaMemcpyDeviceToHost, L->stream));
+  CHLL_TRY(observe_impl(L, make_coupling_d(*c), L->results->row, chll::kStepOfControl));
+  ControlResults back;
+  CHLL_CUDA_TRY(cudaMemcpyAsync(&back, L->results, sizeof(back), cudaMemcpyDeviceToHost,
+                                L->stream));
   CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
+  CHLL_TRY(report_status(L, back.ctl.status));
+  std::memcpy(row16, back.row, sizeof(back.row));
   return ok();
 }
 
@@ -1006,6 +1056,7 @@ int chll_lattice_quench(chll_lattice* L, const chll_coupling* c, double eta, int
   const chll::CouplingD cd = make_coupling_d(*c);
   const DeviceGuard on(L->device);
   if (chll::quench_resident_pays(v)) {
+    note_waits(L);
     for (int done = 0; done < nsteps; done += kResidentChunk) {
       const cudaError_t e = chll::launch_quench_resident(
           v, cd, (float)eta, L->ctl, L->words, L->xch, std::min(kResidentChunk, nsteps - done),
@@ -1029,7 +1080,7 @@ int chll_lattice_energy_grad(chll_lattice* L, const chll_coupling* c, float* gra
   const size_t total = 2 * L->per_colour;
   if (grad && !L->grad) CHLL_CUDA_TRY(cudaMalloc(&L->grad, total * sizeof(float4)));
   chll::launch_energy_grad(L->view(), make_coupling_d(*c), grad ? L->grad : nullptr, project,
-                           L->partials, &L->tickets[1], L->out4, L->stream);
+                           L->partials, &L->tickets[1], L->results->out4, L->stream);
   CHLL_CUDA_TRY(cudaGetLastError());
   if (grad) {
     LatticeView gv = L->view();
@@ -1046,10 +1097,16 @@ int chll_lattice_energy_grad(chll_lattice* L, const chll_coupling* c, float* gra
     }
     CHLL_CUDA_TRY(cudaGetLastError());
   }
-  if (out4)
-    CHLL_CUDA_TRY(cudaMemcpyAsync(out4, L->out4, 4 * sizeof(double), cudaMemcpyDeviceToHost,
-                                  L->stream));
+  if (!out4) {
+    CHLL_TRY(finish(L));
+    return ok();
+  }
+  ControlResults back;
+  CHLL_CUDA_TRY(cudaMemcpyAsync(&back, L->results, offsetof(ControlResults, row),
+                                cudaMemcpyDeviceToHost, L->stream));
   CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
+  CHLL_TRY(report_status(L, back.ctl.status));
+  std::memcpy(out4, back.out4, sizeof(back.out4));
   return ok();
 }
 
@@ -1138,7 +1195,7 @@ int chll_lattice_shell_corr(chll_lattice* L, int nshells, int wrap, double* gn, 
   CHLL_CUDA_TRY(cudaGetLastError());
   CHLL_CUDA_TRY(cudaMemcpyAsync(out.data(), d_part + (size_t)blocks * width, width * sizeof(double),
                                 cudaMemcpyDeviceToHost, L->stream));
-  CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
+  CHLL_TRY(finish(L));
   const double s_mean = out[2 * R] / N;
   for (int r = 0; r < R; ++r) {
     const double w = r == 0 ? 1.0 : 2.0;  // shells >= 1 hold d and -d
@@ -1198,7 +1255,7 @@ int chll_lattice_projection(chll_lattice* L, const int* plane, long long* hist,
   CHLL_TRY(project(L, plane, lo, nb, (unsigned long long*)L->staging));
   CHLL_CUDA_TRY(cudaMemcpyAsync(hist, L->staging, (size_t)nb * sizeof(long long),
                                 cudaMemcpyDeviceToHost, L->stream));
-  CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
+  CHLL_TRY(finish(L));
   return ok();
 }
 
@@ -1223,7 +1280,7 @@ int chll_lattice_structure_factor(chll_lattice* L, const int* plane, const doubl
   CHLL_CUDA_TRY(cudaGetLastError());
   CHLL_CUDA_TRY(cudaMemcpyAsync(sf, d_sf, nkv * sizeof(double), cudaMemcpyDeviceToHost,
                                 L->stream));
-  CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
+  CHLL_TRY(finish(L));
   return ok();
 }
 

@@ -161,7 +161,13 @@ int chll_lattice_download_f4(chll_lattice* lat, float* xyzs);
  * planes, halos included; its own planes start 2*hx*nj float4 in. */
 int chll_lattice_storage(chll_lattice* lat, void** colour0, void** colour1, int64_t* per_colour,
                          int32_t* hx);
-/* Device control block: d, step, adaptation limit. */
+/* Device control block: d, step, adaptation limit.  Its status word is set when a
+ * bounded wait of a sweep or quench launch gave up (seconds without progress, as
+ * on a stalled GPU): the launches after it do nothing, and every call that waits
+ * for the stream -- sync, downloads, rows, observables, adjoint, analyses,
+ * get_control, and run / chll_run_ex, which then leave the caller's arrays alone
+ * -- returns CHLL_EDEVICE until set_control writes a new block.  The lattice's
+ * state is not usable after that: load one. */
 int chll_lattice_set_control(chll_lattice* lat, double d, int64_t step, int64_t adapt_until);
 int chll_lattice_get_control(chll_lattice* lat, double* d, int64_t* step, double* paccept,
                              double* faccept);

@@ -33,9 +33,9 @@ def program(tmp_path_factory):
         return str(o)
 
     def build(name, *sources):
-        exe = out / name
+        exe = out / os.path.splitext(name)[0]
         objs = [obj(os.path.join(CSRC, s)) for s in sources]
-        objs += [obj(os.path.join(FAKE, f)) for f in ("fake_cuda.cpp", name + ".cpp")]
+        objs += [obj(os.path.join(FAKE, f)) for f in ("fake_cuda.cpp", name)]
         # launchers of the other sources are not reached
         subprocess.run(["g++", "-o", str(exe), *objs, "-Wl,--unresolved-symbols=ignore-all"],
                        check=True)
@@ -51,8 +51,12 @@ def _run(exe, *args):
 
 @pytest.mark.parametrize("what", ["larger_map", "tuned", "no_memory", "no_copy"])
 def test_batch_launches_only_allocated_memory(program, what):
-    _run(program("batch_map", "batched.cu", "capi.cu"), what)
+    _run(program("batch_map.cpp", "batched.cu", "capi.cu"), what)
 
 
 def test_tuner_and_trials_that_give_up(program):
-    _run(program("batch_lost", "batched.cu", "capi.cu"))
+    _run(program("batch_lost.cpp", "batched.cu", "capi.cu"))
+
+
+def test_a_wait_that_gave_up_is_reported(program):
+    _run(program("lattice_lost.cu", "capi.cu"))
