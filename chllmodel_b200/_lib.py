@@ -33,7 +33,8 @@ EXPORTS = (
     "chll_lattice_energy_grad", "chll_lattice_reserve_rows", "chll_lattice_measure",
     "chll_lattice_read_rows", "chll_energy_grad_noalloc",
     "chll_energy_grad_natural", "chll_lattice_quench",
-    "chll_lattice_set_kernel", "chll_lattice_shell_corr", "chll_lattice_projection",
+    "chll_lattice_set_kernel", "chll_lattice_set_wait_limit", "chll_lattice_shell_corr",
+    "chll_lattice_projection",
     "chll_lattice_structure_factor",
     "chll_lattice_create_slab", "chll_lattice_slab_plane", "chll_lattice_counters",
     "chll_lattice_control_update", "chll_lattice_slab_set_peers", "chll_lattice_slab_push",
@@ -160,6 +161,8 @@ def _declare(L: ct.CDLL) -> None:
     L.chll_lattice_energy_grad.argtypes = [vp, P(Coupling), vp, i32, vp]
     L.chll_lattice_set_kernel.argtypes = [vp, i32]
     L.chll_lattice_set_kernel.restype = i32
+    L.chll_lattice_set_wait_limit.argtypes = [vp, ct.c_uint64]
+    L.chll_lattice_set_wait_limit.restype = i32
     L.chll_lattice_quench.argtypes = [vp, P(Coupling), dbl, i32]
     L.chll_lattice_quench.restype = i32
     L.chll_lattice_create_slab.argtypes = [i32, i32, i32, i32, i32, i32, P(vp)]

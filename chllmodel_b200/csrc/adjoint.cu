@@ -588,6 +588,7 @@ struct QuenchArgs {
   Control* ctl;
   unsigned long long* words;
   int nsteps;
+  uint32_t first_poll;
 };
 
 struct NoOwn {
@@ -595,7 +596,7 @@ struct NoOwn {
 };
 
 // SITE: one site of each colour per thread (one CTA); else the unit loop.
-template <bool P, bool SITE>
+template <bool P, bool SITE, bool LIMITED>
 __global__ void __launch_bounds__(kResThreads, 1)
     quench_resident_kernel(const __grid_constant__ QuenchArgs A) {
   __shared__ int s_ok;
@@ -629,7 +630,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
     if (lead) {
       bool ok = true;
       grid_arrive(A.words + slot * kWordStride, 0, gridDim.x);
-      grid_wait(A.words + slot * kWordStride, 0, gridDim.x, kWaitLimit, ok);
+      grid_wait(A.words + slot * kWordStride, 0, gridDim.x, LIMITED ? A.first_poll : 0u, ok);
       if (blockIdx.x == 0) A.words[(slot == 0 ? 2 : slot - 1) * kWordStride] = 0;
       if (!ok) atomicOr(&A.ctl->status, 4u);
       s_ok = ok;
@@ -684,7 +685,7 @@ __device__ __forceinline__ uint4 as_word(const float4& n) {
                     __float_as_uint(n.w));
 }
 
-template <bool P, int N, int T>
+template <bool P, int N, int T, bool LIMITED>
 struct QuenchFlow {
   using Own = std::conditional_t<N == 1, OwnSite<P>, OwnBlock<P>>;
   const QuenchFlowArgs& A;
@@ -734,7 +735,7 @@ struct QuenchFlow {
       for (int t = 0; t < (i < 4 ? N : 1); ++t)
         w[i][t] = in[i] && l < span ? as_word(sites[C ^ 1][l + t]) : make_uint4(0, 0, 0, 0);
     }
-    uint32_t polls = 0;
+    uint32_t polls = LIMITED ? A.Q.first_poll : 0u;
     bool again;
     do {
 #pragma unroll
@@ -754,7 +755,7 @@ struct QuenchFlow {
         again = again || open[i];
       }
       if (again && ++polls % 1024 == 0) {
-        if (polls >= kWaitLimit || *(volatile unsigned int*)&A.Q.ctl->status) lost = 1;
+        if (polls >= kWaitPolls || *(volatile unsigned int*)&A.Q.ctl->status) lost = 1;
         again = !lost;  // a lost launch runs to its end without waiting
       }
     } while (again);
@@ -819,7 +820,7 @@ struct QuenchFlow {
   }
 };
 
-template <bool P, int N, int T>
+template <bool P, int N, int T, bool LIMITED>
 __global__ void __launch_bounds__(T, 1)
     quench_flow_kernel(const __grid_constant__ QuenchFlowArgs A) {
   __shared__ float4 sites[2][N * T];
@@ -831,7 +832,7 @@ __global__ void __launch_bounds__(T, 1)
   const bool stale = s_lost;  // an earlier wait ran out: the words are not to be trusted
   __syncthreads();
   if (stale) return;
-  QuenchFlow<P, N, T> F(A, sites, s_lost);
+  QuenchFlow<P, N, T, LIMITED> F(A, sites, s_lost);
   const bool has = F.B.has;
   for (int s = 0; s < A.Q.nsteps; ++s) {
     Nbrs nb[N];
@@ -857,6 +858,28 @@ __global__ void __launch_bounds__(T, 1)
     *A.epoch = base + (uint32_t)A.Q.nsteps;
     *A.Q.words = 0;
   }
+}
+
+using QuenchKernel = void (*)(const QuenchArgs);
+template <bool LIMITED>
+QuenchKernel quench_resident(bool periodic, bool site) {
+  if (site)
+    return periodic ? quench_resident_kernel<true, true, LIMITED>
+                    : quench_resident_kernel<false, true, LIMITED>;
+  return periodic ? quench_resident_kernel<true, false, LIMITED>
+                  : quench_resident_kernel<false, false, LIMITED>;
+}
+
+// n: sites (1) or a unit (2) per thread.
+using QuenchFlowKernel = void (*)(const QuenchFlowArgs);
+template <bool LIMITED>
+QuenchFlowKernel quench_flow(bool periodic, int n, bool wide) {
+  if (wide) return quench_flow_kernel<true, 1, kQuenchWide, LIMITED>;
+  if (n == 1)
+    return periodic ? quench_flow_kernel<true, 1, kResThreads, LIMITED>
+                    : quench_flow_kernel<false, 1, kResThreads, LIMITED>;
+  return periodic ? quench_flow_kernel<true, 2, kResThreads, LIMITED>
+                  : quench_flow_kernel<false, 2, kResThreads, LIMITED>;
 }
 
 // CTAs of `kernel` (kGradThreads threads) resident on the current device, one
@@ -924,7 +947,7 @@ bool quench_resident_pays(const LatticeView& L) { return make_geom(L).units <= (
 
 cudaError_t launch_quench_resident(const LatticeView& L, const CouplingD& cd, float eta,
                                    Control* ctl, unsigned long long* words, void* xch, int nsteps,
-                                   cudaStream_t stream) {
+                                   uint32_t wait_limit, cudaStream_t stream) {
   QuenchArgs A;
   A.L = L;
   A.G = make_geom(L);
@@ -936,20 +959,16 @@ cudaError_t launch_quench_resident(const LatticeView& L, const CouplingD& cd, fl
   A.ctl = ctl;
   A.words = words;
   A.nsteps = nsteps;
+  A.first_poll = first_poll(wait_limit);
   if (const int n = quench_flow_sites(L)) {
     QuenchFlowArgs F;
     F.Q = A;
     F.xch = static_cast<uint4*>(xch);
     F.epoch = reinterpret_cast<uint32_t*>(words + 3 * kWordStride);
     F.per_colour = 2 * A.G.units;
-    using Kernel = void (*)(const QuenchFlowArgs);
     const bool wide = n == 1 && !one_site_each(A.G.units);
-    const Kernel kernel =
-        wide ? quench_flow_kernel<true, 1, kQuenchWide>
-             : (n == 1 ? (L.periodic ? quench_flow_kernel<true, 1, kResThreads>
-                                     : quench_flow_kernel<false, 1, kResThreads>)
-                       : (L.periodic ? quench_flow_kernel<true, 2, kResThreads>
-                                     : quench_flow_kernel<false, 2, kResThreads>));
+    const auto kernel = A.first_poll ? quench_flow<true>(L.periodic, n, wide)
+                                     : quench_flow<false>(L.periodic, n, wide);
     uint32_t threads, grid;
     resident_shape(n == 1 ? 2 * A.G.units : A.G.units, threads, grid,
                    wide ? kQuenchWide : kResThreads);
@@ -958,11 +977,9 @@ cudaError_t launch_quench_resident(const LatticeView& L, const CouplingD& cd, fl
   const bool site = 2 * A.G.units <= 256;
   uint32_t block, ctas;
   resident_shape(site ? 2 * A.G.units : A.G.units, block, ctas);
-  using Kernel = void (*)(const QuenchArgs);
-  static const Kernel kernels[2][2] = {
-      {quench_resident_kernel<false, false>, quench_resident_kernel<false, true>},
-      {quench_resident_kernel<true, false>, quench_resident_kernel<true, true>}};
-  return launch_cooperative(kernels[L.periodic ? 1 : 0][site ? 1 : 0], ctas, block, stream, A);
+  return launch_cooperative(A.first_poll ? quench_resident<true>(L.periodic, site)
+                                         : quench_resident<false>(L.periodic, site),
+                            ctas, block, stream, A);
 }
 
 cudaError_t launch_natural_grad(int ni, int nj, int nk, int periodic, const float* n,

@@ -187,6 +187,7 @@ struct chll_lattice {
   // since the word was last read; some of them into a caller's graph, whose
   // replays are not seen here.
   bool unread_waits = false, captured_waits = false;
+  uint32_t wait_limit = chll::kWaitPolls;
   // z-slab of a larger lattice: global planes z0 .. z0+nk-1 of nk_global,
   // stored as planes 2 .. nk+1 of nk+3 (plane 1 and nk+2 are the halos,
   // plane 0 keeps the storage checkerboard equal to the global one).
@@ -362,9 +363,9 @@ int sweep_impl(chll_lattice* L, const Coupling& cp, uint64_t seed, uint32_t rep,
       const cudaError_t e =
           chll::flow_pays(L->view())
               ? chll::launch_flow_sweeps(L->view(), cp, k0, k1, rep, L->ctl, L->words, L->xch, n,
-                                            L->stream)
-                 : chll::launch_resident_sweeps(L->view(), cp, k0, k1, rep, L->ctl, L->words, n,
-                                                L->stream);
+                                         L->wait_limit, L->stream)
+              : chll::launch_resident_sweeps(L->view(), cp, k0, k1, rep, L->ctl, L->words, n,
+                                             L->wait_limit, L->stream);
       if (e != cudaSuccess)
         return fail(CHLL_ECUDA, "resident sweep launch: %s", cudaGetErrorString(e));
     }
@@ -876,6 +877,13 @@ int chll_lattice_set_stream(chll_lattice* L, void* stream) {
   return ok();
 }
 
+int chll_lattice_set_wait_limit(chll_lattice* L, uint64_t polls) {
+  if (!L || polls == 0)
+    return fail(CHLL_EINVAL, "set_wait_limit: need a lattice and polls >= 1");
+  L->wait_limit = (uint32_t)std::min<uint64_t>(polls, chll::kWaitPolls);
+  return ok();
+}
+
 int chll_lattice_sync(chll_lattice* L) {
   if (!L) return fail(CHLL_EINVAL, "null lattice");
   CHLL_TRY(finish(L));
@@ -1060,7 +1068,7 @@ int chll_lattice_quench(chll_lattice* L, const chll_coupling* c, double eta, int
     for (int done = 0; done < nsteps; done += kResidentChunk) {
       const cudaError_t e = chll::launch_quench_resident(
           v, cd, (float)eta, L->ctl, L->words, L->xch, std::min(kResidentChunk, nsteps - done),
-          L->stream);
+          L->wait_limit, L->stream);
       if (e != cudaSuccess) return fail(CHLL_ECUDA, "quench launch: %s", cudaGetErrorString(e));
     }
     return ok();

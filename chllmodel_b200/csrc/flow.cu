@@ -75,6 +75,7 @@ struct FlowArgs {
   uint4* xch;                 // a word per slot of both colours
   uint32_t per_colour;
   int nsweeps;
+  uint32_t first_poll;
 };
 
 struct FlowShared {
@@ -104,7 +105,7 @@ __device__ __forceinline__ void bar_wait(int id) {
 constexpr int kUseShift = 52;  // count words: director accepts or flips below, arrivals above
 constexpr unsigned long long kSumMask = (1ull << kUseShift) - 1;
 
-template <bool P>
+template <bool P, bool LIMITED>
 struct FlowSite {
   const FlowArgs& A;
   OwnSite<P> B;
@@ -153,7 +154,7 @@ struct FlowSite {
     float4 v[5];
 #pragma unroll
     for (int i = 0; i < 5; ++i) v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    uint32_t polls = 0;
+    uint32_t polls = LIMITED ? A.first_poll : 0u;
     bool again;
     do {
       uint4 w[5];
@@ -174,7 +175,7 @@ struct FlowSite {
         }
       }
       if (again && ++polls % 1024 == 0) {
-        if (polls >= kWaitLimit || *(volatile unsigned int*)&A.ctl->status) S.lost = 1;
+        if (polls >= kWaitPolls || *(volatile unsigned int*)&A.ctl->status) S.lost = 1;
         again = !S.lost;  // a lost launch runs to its end without waiting
       }
     } while (again);
@@ -240,6 +241,7 @@ __device__ __forceinline__ void put_count(unsigned int (&part)[kResThreads / 32]
 }
 
 // The last warp of a CTA: counts out, step sizes back.  One lane of it works.
+template <bool LIMITED>
 __device__ __forceinline__ void control_warp(const FlowArgs& A, FlowShared& S, int nadapt,
                                              uint32_t base) {
   Control* const ctl = A.ctl;
@@ -274,12 +276,12 @@ __device__ __forceinline__ void control_warp(const FlowArgs& A, FlowShared& S, i
       ++uses;
       if (!last) {
         unsigned long long v;
-        uint32_t polls = 0;
+        uint32_t polls = LIMITED ? A.first_poll : 0u;
         for (;;) {
           asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(word) : "memory");
           if (complete(v)) break;
           if (++polls % 1024 == 0) {
-            if (polls >= kWaitLimit || *(volatile unsigned int*)&ctl->status) S.lost = 1;
+            if (polls >= kWaitPolls || *(volatile unsigned int*)&ctl->status) S.lost = 1;
             if (S.lost) break;
           }
         }
@@ -331,10 +333,10 @@ __device__ __forceinline__ void control_warp(const FlowArgs& A, FlowShared& S, i
 // The other warps.  A sweep's first trials are made with the step size that the
 // last change's rule gives again, while the count is on its way; where it turns
 // out otherwise they are made anew.
-template <bool P>
+template <bool P, bool LIMITED>
 __device__ __forceinline__ void site_warps(const FlowArgs& A, FlowShared& S, int nadapt,
                                            uint32_t base, uint32_t step) {
-  FlowSite<P> F(A);
+  FlowSite<P, LIMITED> F(A);
   Nbrs nb;
   F.template first<1>(nb);
   F.template first<0>(nb);
@@ -384,7 +386,7 @@ __device__ __forceinline__ void site_warps(const FlowArgs& A, FlowShared& S, int
   bar_arrive(kBarEnd);
 }
 
-template <bool P>
+template <bool P, bool LIMITED>
 __global__ void __launch_bounds__(kResThreads, 1)
     flow_sweeps_kernel(const __grid_constant__ FlowArgs A) {
   __shared__ FlowShared S;
@@ -406,9 +408,9 @@ __global__ void __launch_bounds__(kResThreads, 1)
   __syncthreads();
   if (stale) return;
   if ((threadIdx.x >> 5) + 1 == blockDim.x >> 5)
-    control_warp(A, S, nadapt, base);
+    control_warp<LIMITED>(A, S, nadapt, base);
   else
-    site_warps<P>(A, S, nadapt, base, step);
+    site_warps<P, LIMITED>(A, S, nadapt, base, step);
 }
 
 constexpr uint32_t kFlowSites = kResThreads - 32;  // site threads per SM beside the control warp
@@ -427,7 +429,7 @@ bool flow_pays(const LatticeView& L) {
 cudaError_t launch_flow_sweeps(const LatticeView& L, const Coupling& cp, uint32_t key0,
                                uint32_t key1, uint32_t replica, Control* ctl,
                                unsigned long long* words, void* xch, int nsweeps,
-                               cudaStream_t stream) {
+                               uint32_t wait_limit, cudaStream_t stream) {
   FlowArgs A;
   A.L = L;
   A.G = make_geom(L);
@@ -440,10 +442,15 @@ cudaError_t launch_flow_sweeps(const LatticeView& L, const Coupling& cp, uint32_
   A.xch = static_cast<uint4*>(xch);
   A.per_colour = 2 * A.G.units;
   A.nsweeps = nsweeps;
+  A.first_poll = first_poll(wait_limit);
   uint32_t block, ctas;
   resident_shape(2 * A.G.units, block, ctas, kFlowSites);
-  return launch_cooperative(L.periodic ? flow_sweeps_kernel<true> : flow_sweeps_kernel<false>,
-                            ctas, block + 32, stream, A);
+  using Kernel = void (*)(const FlowArgs);
+  static const Kernel kernels[2][2] = {
+      {flow_sweeps_kernel<false, false>, flow_sweeps_kernel<false, true>},
+      {flow_sweeps_kernel<true, false>, flow_sweeps_kernel<true, true>}};
+  return launch_cooperative(kernels[L.periodic ? 1 : 0][A.first_poll ? 1 : 0], ctas, block + 32,
+                            stream, A);
 }
 
 }  // namespace chll

@@ -48,6 +48,7 @@ struct ResidentArgs {
   Control* ctl;
   unsigned long long* words;
   int nsweeps;
+  uint32_t first_poll;
 };
 
 struct ResidentShared {
@@ -207,7 +208,7 @@ __device__ __forceinline__ unsigned long long cta_counts(ResidentShared& S, unsi
 // The chunk: A0 B (A B)... F with the grid barrier after every pass but the
 // last.  The control values live in shared memory, thread 0's to change: kept in
 // registers across the passes they cost the unit loops theirs.
-template <class UNITS>
+template <class UNITS, bool LIMITED>
 __device__ __forceinline__ void resident_sweeps(const ResidentArgs& A, ResidentShared& S) {
   Control* ctl = A.ctl;
   if (ctl->status) return;  // an earlier wait ran out: the words are not to be trusted
@@ -227,7 +228,7 @@ __device__ __forceinline__ void resident_sweeps(const ResidentArgs& A, ResidentS
   // thread 0: this pass's word, complete; the word before it cleared
   auto wait = [&](unsigned long long v) {
     bool ok = true;
-    v = grid_wait(A.words + slot * kWordStride, v, gridDim.x, kWaitLimit, ok);
+    v = grid_wait(A.words + slot * kWordStride, v, gridDim.x, LIMITED ? A.first_poll : 0u, ok);
     if (blockIdx.x == 0) A.words[(slot == 0 ? 2 : slot - 1) * kWordStride] = 0;
     S.nacc += v & kCountMask;
     S.ok = ok;
@@ -302,28 +303,32 @@ __device__ __forceinline__ void resident_sweeps(const ResidentArgs& A, ResidentS
   ctl->nflip = 0;
 }
 
-template <bool P, int FORM>
+template <bool P, int FORM, bool LIMITED>
 __global__ void __launch_bounds__(kResThreads, 1)
     resident_sweeps_kernel(const __grid_constant__ ResidentArgs A) {
   __shared__ ResidentShared S;
   if (FORM == 4)
-    resident_sweeps<OwnSiteUnit<P>>(A, S);
+    resident_sweeps<OwnSiteUnit<P>, LIMITED>(A, S);
   else if (FORM == 3)
-    resident_sweeps<OwnUnit<P>>(A, S);
+    resident_sweeps<OwnUnit<P>, LIMITED>(A, S);
   else
-    resident_sweeps<SharedUnits<P, FORM>>(A, S);
+    resident_sweeps<SharedUnits<P, FORM>, LIMITED>(A, S);
 }
 
 using ResidentKernel = void (*)(const ResidentArgs);
-// [periodic][form]: 0 unit loop with padding checks, 1 unit loop, 2 column
-// walk, 3 one unit per thread, 4 one site of each colour per thread
-const ResidentKernel kResident[2][5] = {
-    {resident_sweeps_kernel<false, 0>, resident_sweeps_kernel<false, 1>,
-     resident_sweeps_kernel<false, 2>, resident_sweeps_kernel<false, 3>,
-     resident_sweeps_kernel<false, 4>},
-    {resident_sweeps_kernel<true, 0>, resident_sweeps_kernel<true, 1>,
-     resident_sweeps_kernel<true, 2>, resident_sweeps_kernel<true, 3>,
-     resident_sweeps_kernel<true, 4>}};
+template <bool LIMITED>
+ResidentKernel resident_kernel(int periodic, int form) {
+  // [periodic][form]: 0 unit loop with padding checks, 1 unit loop, 2 column
+  // walk, 3 one unit per thread, 4 one site of each colour per thread
+  static const ResidentKernel kernels[2][5] = {
+      {resident_sweeps_kernel<false, 0, LIMITED>, resident_sweeps_kernel<false, 1, LIMITED>,
+       resident_sweeps_kernel<false, 2, LIMITED>, resident_sweeps_kernel<false, 3, LIMITED>,
+       resident_sweeps_kernel<false, 4, LIMITED>},
+      {resident_sweeps_kernel<true, 0, LIMITED>, resident_sweeps_kernel<true, 1, LIMITED>,
+       resident_sweeps_kernel<true, 2, LIMITED>, resident_sweeps_kernel<true, 3, LIMITED>,
+       resident_sweeps_kernel<true, 4, LIMITED>}};
+  return kernels[periodic][form];
+}
 
 }  // namespace
 
@@ -348,7 +353,8 @@ bool resident_pays(const LatticeView& L) {
 
 cudaError_t launch_resident_sweeps(const LatticeView& L, const Coupling& cp, uint32_t key0,
                                    uint32_t key1, uint32_t replica, Control* ctl,
-                                   unsigned long long* words, int nsweeps, cudaStream_t stream) {
+                                   unsigned long long* words, int nsweeps, uint32_t wait_limit,
+                                   cudaStream_t stream) {
   ResidentArgs A;
   A.L = L;
   A.G = make_geom(L);
@@ -369,7 +375,11 @@ cudaError_t launch_resident_sweeps(const LatticeView& L, const Coupling& cp, uin
   A.ctl = ctl;
   A.words = words;
   A.nsweeps = nsweeps;
-  return launch_cooperative(kResident[L.periodic ? 1 : 0][form], ctas, block, stream, A);
+  A.first_poll = first_poll(wait_limit);
+  const int periodic = L.periodic ? 1 : 0;
+  return launch_cooperative(A.first_poll ? resident_kernel<true>(periodic, form)
+                                         : resident_kernel<false>(periodic, form),
+                            ctas, block, stream, A);
 }
 
 }  // namespace chll

@@ -52,12 +52,16 @@ void launch_control_update(Control* ctl, int phase, cudaStream_t stream);
 // resident_fits: the lattice's counts fit the words; resident_pays: the form
 // is faster than the fused passes' launches.
 // The words' memory is kResidentAllocBytes: behind them flow.cu's sweep number.
+// wait_limit, here and below: polls that a wait makes before it gives up and sets
+// the control block's status word; at most kWaitPolls.
+constexpr uint32_t kWaitPolls = 1u << 22;
 constexpr size_t kResidentWordBytes = 3 * 128, kResidentAllocBytes = 4 * 128;
 bool resident_fits(const LatticeView& L);
 bool resident_pays(const LatticeView& L);
 cudaError_t launch_resident_sweeps(const LatticeView& L, const Coupling& cp, uint32_t key0,
                                    uint32_t key1, uint32_t replica, Control* ctl,
-                                   unsigned long long* words, int nsweeps, cudaStream_t stream);
+                                   unsigned long long* words, int nsweeps, uint32_t wait_limit,
+                                   cudaStream_t stream);
 
 // flow.cu: the same for small lattices, threads waiting for their neighbours'
 // sites instead of the grid.  xch: flow_bytes of device memory, zero before the
@@ -69,7 +73,7 @@ inline size_t flow_bytes(const LatticeView& L) {
 cudaError_t launch_flow_sweeps(const LatticeView& L, const Coupling& cp, uint32_t key0,
                                uint32_t key1, uint32_t replica, Control* ctl,
                                unsigned long long* words, void* xch, int nsweeps,
-                               cudaStream_t stream);
+                               uint32_t wait_limit, cudaStream_t stream);
 
 // layout.cu: natural-order (F-order, i fastest) <-> red/black float4.
 void launch_pack_f64(const LatticeView& L, const double* nx, const double* ny, const double* nz,
@@ -119,7 +123,7 @@ bool quench_resident_pays(const LatticeView& L);
 int quench_flow_sites(const LatticeView& L);  // nonzero: launch_quench_resident uses xch
 cudaError_t launch_quench_resident(const LatticeView& L, const CouplingD& cd, float eta,
                                    Control* ctl, unsigned long long* words, void* xch, int nsteps,
-                                   cudaStream_t stream);
+                                   uint32_t wait_limit, cudaStream_t stream);
 
 // analysis.cu: shell correlations over natural-order float4 sites and a zero
 // site behind them (offsets {di, dj, dk}, chunks {first, end, shell} of at most

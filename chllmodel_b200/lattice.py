@@ -84,6 +84,11 @@ class Lattice:
         code = {"auto": 0, "direct": 1, "staged": 2, "fused": 3, "resident": 4}[kind]
         check(self._L.chll_lattice_set_kernel(self._h, code))
 
+    def set_wait_limit(self, polls: int) -> None:
+        """Polls a wait of a resident sweep or quench launch makes before it gives
+        up and sets the status word (default and at most 2^22)."""
+        check(self._L.chll_lattice_set_wait_limit(self._h, int(polls)))
+
     def sync(self) -> None:
         check(self._L.chll_lattice_sync(self._h))
 

@@ -146,6 +146,10 @@ int chll_lattice_set_stream(chll_lattice* lat, void* stream);
  * and more take the launches of 3).  All give the same chain bit for bit.  chll_lattice_pass runs the staged kernel under 2 and the direct kernel
  * otherwise. */
 int chll_lattice_set_kernel(chll_lattice* lat, int kernel);
+/* How many polls a wait of the resident sweep launches and of the quench makes
+ * before it gives up (default and at most 2^22, seconds of waiting; >= 1) and sets
+ * the status word (chll_lattice_set_control).  No counterpart in the reference. */
+int chll_lattice_set_wait_limit(chll_lattice* lat, uint64_t polls);
 int chll_lattice_sync(chll_lattice* lat);
 /* Random initial state: directors uniform on the sphere, s = +-1 with p=1/2. */
 int chll_lattice_init_random(chll_lattice* lat, uint64_t seed, uint32_t replica);

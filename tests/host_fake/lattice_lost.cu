@@ -40,17 +40,17 @@ int energy_grad_max_blocks() { return 8; }
 int observables_max_blocks() { return 8; }
 int shell_corr_blocks(int) { return 8; }
 cudaError_t launch_flow_sweeps(const LatticeView&, const Coupling&, uint32_t, uint32_t, uint32_t,
-                               Control* ctl, unsigned long long*, void*, int n, cudaStream_t) {
+                               Control* ctl, unsigned long long*, void*, int n, uint32_t, cudaStream_t) {
   launch(ctl, n);
   return cudaSuccess;
 }
 cudaError_t launch_resident_sweeps(const LatticeView&, const Coupling&, uint32_t, uint32_t, uint32_t,
-                                   Control* ctl, unsigned long long*, int n, cudaStream_t) {
+                                   Control* ctl, unsigned long long*, int n, uint32_t, cudaStream_t) {
   launch(ctl, n);
   return cudaSuccess;
 }
 cudaError_t launch_quench_resident(const LatticeView&, const CouplingD&, float, Control* ctl,
-                                   unsigned long long*, void*, int, cudaStream_t) {
+                                   unsigned long long*, void*, int, uint32_t, cudaStream_t) {
   launch(ctl, 0);
   return cudaSuccess;
 }
