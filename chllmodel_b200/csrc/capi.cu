@@ -690,12 +690,17 @@ int run_impl(const chll_run_config& cfg, int nstart, int nstop, int nout, double
         rc = observe_impl(L, make_coupling_d(cc), drow, end);
         if (rc != CHLL_OK) break;
         if (cfg.verbose) {
-          cudaEvent_t ev;
-          cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-          cudaMemcpyAsync(host_rows + r * chll::kRowLen, drow, sizeof(double) * chll::kRowLen,
-                          cudaMemcpyDeviceToHost, L->stream);
-          cudaEventRecord(ev, L->stream);
-          events.push_back(ev);
+          cudaEvent_t ev = nullptr;
+          cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+          if (e == cudaSuccess) events.push_back(ev);
+          if (e == cudaSuccess)
+            e = cudaMemcpyAsync(host_rows + r * chll::kRowLen, drow, sizeof(double) * chll::kRowLen,
+                                cudaMemcpyDeviceToHost, L->stream);
+          if (e == cudaSuccess) e = cudaEventRecord(ev, L->stream);
+          if (e != cudaSuccess) {
+            rc = fail(CHLL_ECUDA, "run: row of step %lld: %s", end, cudaGetErrorString(e));
+            break;
+          }
         }
         row_step.push_back(end);
         ++r;
@@ -706,10 +711,12 @@ int run_impl(const chll_run_config& cfg, int nstart, int nstop, int nout, double
     istep = end + 1;
     if (cfg.verbose) flush_rows(false);
   }
+  cudaError_t e = cudaSuccess;
   if (rc == CHLL_OK && !cfg.verbose && r > 0)
-    cudaMemcpyAsync(host_rows, L->rows, sizeof(double) * chll::kRowLen * r, cudaMemcpyDeviceToHost,
-                    L->stream);
-  cudaError_t e = cudaStreamSynchronize(L->stream);
+    e = cudaMemcpyAsync(host_rows, L->rows, sizeof(double) * chll::kRowLen * r,
+                        cudaMemcpyDeviceToHost, L->stream);
+  const cudaError_t drained = cudaStreamSynchronize(L->stream);
+  if (e == cudaSuccess) e = drained;
   if (rc == CHLL_OK && e != cudaSuccess)
     rc = fail(CHLL_ECUDA, "run: %s", cudaGetErrorString(e));
   if (rc == CHLL_OK && cfg.verbose) flush_rows(true);

@@ -1,6 +1,7 @@
 // A wait that gave up (a launch that sets the control block's status word) is
 // reported by every call that waits for the lattice's stream, and by run(), until
-// set_control; run() leaves the caller's arrays alone.
+// set_control; run() leaves the caller's arrays alone.  With an argument: copies of a
+// run that fail.
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -111,7 +112,40 @@ static void calls(chll_lattice* L, const chll_coupling* c, int sites, int want, 
   }
 }
 
-int main() {
+// Every copy of a run that fails is reported.
+static void run_copies() {
+  const int edge = 12, sites = edge * edge * edge;
+  chll_run_config cfg;
+  std::memset(&cfg, 0, sizeof(cfg));
+  cfg.kT = cfg.K = cfg.eps = 1.0;
+  cfg.d = 0.1;
+  std::vector<double> x(sites), y(sites), z(sites), m(5 * 2), rows(2 * 16);
+  std::vector<int> s(sites), steps(2);
+  double d;
+  for (int verbose : {0, 1}) {
+    cfg.verbose = verbose;
+    int nth = 0;
+    do {
+      fake::fail_copy = ++nth;
+      const int rc = chll_run_ex(&cfg, 1, 20, 10, x.data(), y.data(), z.data(), s.data(), edge, edge,
+                                 edge, steps.data(), m.data(), rows.data(), &d);
+      const int want = fake::fail_copy ? CHLL_OK : CHLL_ECUDA;
+      if (rc != want) {
+        std::printf("wrong: run gives %d where copy %d of it fails\n", rc, nth);
+        ++bad;
+      }
+    } while (!fake::fail_copy);
+    fake::fail_copy = 0;
+    expect(nth > 10, "copies of a run");
+  }
+}
+
+int main(int argc, char**) {
+  if (argc > 1) {
+    run_copies();
+    std::printf("%d wrong\n", bad);
+    return bad != 0;
+  }
   const chll_coupling c = {0.5, 1.0, 0.0, 1.0};
   for (int edge : {8, 12}) {
     const int sites = edge * edge * edge;

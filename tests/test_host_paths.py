@@ -60,3 +60,7 @@ def test_tuner_and_trials_that_give_up(program):
 
 def test_a_wait_that_gave_up_is_reported(program):
     _run(program("lattice_lost.cu", "capi.cu"))
+
+
+def test_copies_of_a_run_that_fail_are_reported(program):
+    _run(program("lattice_lost.cu", "capi.cu"), "copies")
