@@ -998,16 +998,7 @@ cudaError_t launch_natural_grad(int ni, int nj, int nk, int periodic, const floa
   G.cols = (G.plane + 31) / 32 * 32;
   // Planes per task: the fewest steps on the busiest thread, a task's first
   // loads counted as half a step.
-  double best = 1e300;
-  for (uint32_t seg = 1; seg <= G.nk; ++seg) {
-    const uint64_t tasks = (uint64_t)G.cols * ((G.nk + seg - 1) / seg);
-    const uint64_t threads = (uint64_t)ctas * kGradThreads;
-    const double cost = (double)((tasks + threads - 1) / threads) * (seg + 0.5);
-    if (cost < best) {
-      best = cost;
-      G.seg = seg;
-    }
-  }
+  G.seg = cheapest_segment(G.cols, G.nk, (uint64_t)ctas * kGradThreads, 0.5);
   G.nseg = (G.nk + G.seg - 1) / G.seg;
   const uint64_t need = ((uint64_t)G.cols * G.nseg + kGradThreads - 1) / kGradThreads;
   const uint32_t blocks = (uint32_t)std::min<uint64_t>(need, ctas);

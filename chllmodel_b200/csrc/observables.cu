@@ -283,16 +283,8 @@ void launch_observables(const LatticeView& L, const MomentGeom& M, const Couplin
   // Planes per task: the fewest steps on the busiest thread, a task's first
   // block counted as a third of a step.
   const uint32_t threads = (uint32_t)obs_ctas() * kObsThreads, nk = (uint32_t)L.nk;
-  double best = 1e300;
-  for (uint32_t seg = 1; seg <= nk; ++seg) {
-    const uint64_t tasks = (uint64_t)W.ncols * ((nk + seg - 1) / seg);
-    const double cost = (double)((tasks + threads - 1) / threads) * (seg + 0.33);
-    if (cost < best) {
-      best = cost;
-      W.seg = seg;
-      W.ntasks = (uint32_t)tasks;
-    }
-  }
+  W.seg = cheapest_segment(W.ncols, nk, threads, 0.33);
+  W.ntasks = W.ncols * ((nk + W.seg - 1) / W.seg);
   const uint32_t need = (W.ntasks + kObsThreads - 1) / kObsThreads;
   const uint32_t blocks = std::min(need, (uint32_t)obs_ctas());
   kObs[L.periodic ? 1 : 0][L.ni % 4 ? 1 : 0]<<<blocks, kObsThreads, 0, stream>>>(

@@ -381,12 +381,14 @@ __host__ inline double walk_pass_cost(uint32_t units, uint32_t ncols, uint32_t p
   double best = (double)((units + threads - 1) / (threads ? threads : 1));
   *seg = 0;
   if (!full || force_seg == 0 || ncols == 0) return best;
-  for (uint32_t s = 2; s <= planes; ++s) {
-    if (force_seg > 0 && s != (uint32_t)force_seg) continue;
+  const bool forced = force_seg > 0;
+  if (forced && (force_seg < 2 || (uint32_t)force_seg > planes)) return best;
+  for (uint32_t s = forced ? (uint32_t)force_seg : 2u; s && s <= planes;
+       s = forced ? 0u : next_segment(planes, s)) {
     const uint64_t tasks = (uint64_t)ncols * ((planes + s - 1) / s);
     const double cost =
         (double)((tasks + threads - 1) / threads) * ((double)s * kWalkStep + kWalkPrime);
-    if (cost < best || force_seg > 0) {
+    if (cost < best || forced) {
       best = cost;
       *seg = s;
     }

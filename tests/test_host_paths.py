@@ -64,3 +64,7 @@ def test_a_wait_that_gave_up_is_reported(program):
 
 def test_copies_of_a_run_that_fail_are_reported(program):
     _run(program("lattice_lost.cu", "capi.cu"), "copies")
+
+
+def test_segment_lengths(program):
+    _run(program("segments.cu"))
