@@ -351,7 +351,7 @@ void launch_projection(const LatticeView& L, int px, int py, int pz, long long m
   const uint32_t nseg = std::min(nk, std::max(1u, threads / cols));
   const uint32_t seg = (nk + nseg - 1) / nseg;
   const uint32_t ntasks = cols * ((nk + seg - 1) / seg);
-  const uint32_t need = (ntasks + 255) / 256;
+  const uint32_t need = (uint32_t)(((uint64_t)ntasks + 255) / 256);  // ntasks < 2^32
   projection_kernel<<<std::min(need, ctas), 256, (size_t)nbins * sizeof(int), stream>>>(
       L, seg, ntasks, px, py, pz, m0, nbins, hist);
 }

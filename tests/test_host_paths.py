@@ -68,3 +68,7 @@ def test_copies_of_a_run_that_fail_are_reported(program):
 
 def test_segment_lengths(program):
     _run(program("segments.cu"))
+
+
+def test_projection_of_the_largest_planes(program):
+    _run(program("projection_grid.cpp", "analysis.cu"))
