@@ -167,7 +167,8 @@ class Batch:
                 "waves": n.value, "paired": bool(p.value), "pooled": bool(q.value)}
 
     def autotune(self, trial_sweeps=20, cache=None) -> dict:
-        """Times every launch shape on this replica set and keeps the fastest.
+        """Times the launch shapes that can be the fastest for this replica set and
+        keeps the fastest (single groups, one persistent launch).
         With `cache` (a JSON path) the choice is stored per GPU and size mix."""
         key = self._tune_key()
         if cache and os.path.exists(cache):

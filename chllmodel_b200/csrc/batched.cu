@@ -7,8 +7,9 @@
 // scripts/g_field0.5.py:24-31).
 //
 // Layout: each replica keeps the plain lattice layout (two red/black float4
-// colour arrays) in one shared allocation, and a ReplicaState block holds its
-// d, step, accept counters, barrier words and FP64 measurement accumulators.
+// colour arrays) in one shared allocation; a ReplicaState block holds its d, step,
+// flip count, status and FP64 measurement accumulators, and three words of their own
+// its group's meetings.
 //
 // Schedule: the launch is sized to the co-resident CTA count (cooperative
 // launch), and every group of one replica (or, with pairing, two of
@@ -17,11 +18,11 @@
 // kernels' code (the column walk or the grid-stride unit loop, as the cost
 // model picks for the group's thread count), so a replica's chain is
 // bit-identical to the same replica run alone.  Between passes the group
-// meets at a software barrier in global memory (arrive counter + generation
-// word), split into arrive and wait so that a paired group runs the other
-// replica's pass in between.  Every wait is bounded: on timeout the CTA sets
-// the replica's status word and returns, and so do the others at their next
-// barrier, so a fault ends the launch instead of hanging it.  The pooled
+// meets at a word in global memory (the CTAs' accepts and arrivals), split into
+// arrive and wait so that a paired group runs the other replica's pass in between.
+// Every wait is bounded: on timeout the CTA sets the replica's status word and
+// returns, and so do the others at their next meeting, so a fault ends the launch
+// instead of hanging it.  The pooled
 // passes of pooled.cu are the alternative schedule (chll_batch_set_pooled).
 //
 // Measurements every `measure_every` sweeps (from sweep `measure_from`):
@@ -258,7 +259,7 @@ __device__ __noinline__ void measure_partials(const ReplicaDesc& D, int rank, in
   const uint64_t total = 2ull * D.M.per_colour;  // < 2^32
   for (uint64_t e = (uint64_t)rank * blockDim.x + threadIdx.x; e < total;
        e += (uint64_t)nct * blockDim.x)
-    site_moments<false>(D.L, D.M, D.cd, (uint32_t)e, m);
+    site_moments(D.L, D.M, D.cd, (uint32_t)e, m);
 #pragma unroll
   for (int t = 0; t < kObsMoments; ++t) {
     const double v = warp_sum_d(m[t]);

@@ -1,12 +1,11 @@
-// FP64 moments of one lattice site, shared by the observables kernel
-// (observables.cu) and the batched kernel's measurements (batched.cu).
+// FP64 moments of a lattice: their order, and one site's, as the batch's
+// measurements take them (batched.cu, pooled.cu; a single lattice's measurement row
+// comes from observables.cu, which also fills acc[1]).
 //
 // Per site (FP64 arithmetic on the FP32 state), added into acc[0..8]:
 //   acc[0] total energy with the lattice's boundary, each bond once
 //          (+x, +y, +z) plus the field term;
-//   acc[1] the reference etot() sum (chll_mod.f90:414-456): x and y
-//          periodic, z open, and the +y dot product's x component read from
-//          the diagonal neighbour (ip1,jp1,k) exactly as chll_mod.f90:438;
+//   acc[1] the reference's etot() sum (observables.cu only);
 //   acc[2] s;  acc[3..8] nx*nx, ny*ny, nz*nz, nx*ny, nx*nz, ny*nz.
 #pragma once
 #include <cmath>
@@ -60,9 +59,6 @@ __device__ __forceinline__ double fwd_bond(double eps, double K, double dot, dou
 }
 
 // Storage slot e of the concatenated colour arrays (colour = e >= per_colour).
-// REF_ETOT: also the reference etot() column acc[1] (measurement rows); the
-// batched moments leave it out.
-template <bool REF_ETOT>
 __device__ __forceinline__ void site_moments(const LatticeView& L, const MomentGeom& M,
                                              const CouplingD& cp, uint32_t e,
                                              double acc[kObsMoments]) {
@@ -96,16 +92,8 @@ __device__ __forceinline__ void site_moments(const LatticeView& L, const MomentG
 
   const bool has_xp = L.periodic || (i + 1 < L.ni);
   const bool has_yp = L.periodic || (j + 1 < L.nj);
-  const bool ref_zp = M.kglob0 + k + 1 < M.nkg;  // z is open in etot
-  const bool has_zp = L.periodic || ref_zp;
+  const bool has_zp = L.periodic || M.kglob0 + k + 1 < M.nkg;
   acc[0] += (has_xp ? bx : 0.0) + (has_yp ? by : 0.0) + (has_zp ? bz : 0.0) - g * s;
-
-  if (REF_ETOT) {
-    const float4 T = site_at(L, ip, jp, k);  // diagonal read of chll_mod.f90:438
-    const double dyt = nx * (double)T.x + ny * Y.y + nz * Y.z;
-    const double byt = fwd_bond(eps, K, dyt, cy, s, Y.w);
-    acc[1] += bx + byt + (ref_zp ? bz : 0.0) - g * s;
-  }
 
   acc[2] += s;
   acc[3] += nx * nx;

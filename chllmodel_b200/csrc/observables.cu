@@ -1,5 +1,7 @@
 // FP64 observables of one red/black lattice and the reference measurement
-// row: the moments that moments.cuh defines per site.
+// row: the sums that moments.cuh lists, and the reference's etot()
+// (chll_mod.f90:414-456): x and y periodic, z open, and the +y dot product's x
+// component read from the diagonal neighbour (ip1, jp1, k) as chll_mod.f90:438.
 //
 // A thread walks a column of 4-site x-blocks (both colours' units at one slot)
 // over a run of planes.  Its four sites are converted to FP64 once and serve as

@@ -135,7 +135,7 @@ __device__ __forceinline__ void pool_moment_segment(const PoolEntry& E, uint32_t
 #pragma unroll
   for (int t = 0; t < kObsMoments; ++t) m[t] = 0.0;
   for (uint32_t e = lo + threadIdx.x; e < hi; e += kPoolThreads)
-    site_moments<false>(E.L, E.M, E.cd, e, m);
+    site_moments(E.L, E.M, E.cd, e, m);
   __shared__ double s_m[kPoolThreads / 32][kObsMoments];
 #pragma unroll
   for (int t = 0; t < kObsMoments; ++t) {
