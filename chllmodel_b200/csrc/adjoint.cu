@@ -632,7 +632,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
       grid_arrive(A.words + slot * kWordStride, 0, gridDim.x);
       grid_wait(A.words + slot * kWordStride, 0, gridDim.x, LIMITED ? A.first_poll : 0u, ok);
       if (blockIdx.x == 0) A.words[(slot == 0 ? 2 : slot - 1) * kWordStride] = 0;
-      if (!ok) atomicOr(&A.ctl->status, 4u);
+      if (!ok) set_status(A.ctl, 4u);
       s_ok = ok;
     }
     slot = slot == 2 ? 0 : slot + 1;
@@ -852,7 +852,7 @@ __global__ void __launch_bounds__(T, 1)
   }
   if (threadIdx.x != 0) return;
   if (s_lost) {
-    atomicOr(&ctl->status, 4u);
+    set_status(ctl, 4u);
     atomicAdd(A.epoch, (uint32_t)A.Q.nsteps + 2u);  // what was published is never read again
   } else if (atomicAdd(A.Q.words, 1ull) == gridDim.x - 1) {
     *A.epoch = base + (uint32_t)A.Q.nsteps;

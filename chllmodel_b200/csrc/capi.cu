@@ -151,13 +151,43 @@ struct DeviceGuard {
   }
 };
 
-// A lattice's control block and, behind it, the results that come back with it in
-// one copy.
-struct ControlResults {
-  Control ctl;
-  double out4[4];
-  double row[chll::kRowLen];
+// Host words that device code can set, one per lattice: a launch whose wait gives up
+// sets its lattice's word beside the control block's status, so that the calls that
+// wait for the stream find it without a copy (a copy of the status word took them 8
+// to 13 us).  Words come from pinned pages that stay (an allocation takes 0.5 to 6
+// ms) and are used again.
+class HostWords {
+ public:
+  cudaError_t take(unsigned int** word) {
+    std::lock_guard<std::mutex> lk(mutex_);
+    if (free_.empty()) {
+      unsigned int* page = nullptr;
+      const cudaError_t e = cudaHostAlloc(&page, kPage * sizeof(unsigned int),
+                                          cudaHostAllocPortable | cudaHostAllocMapped);
+      if (e != cudaSuccess) return e;
+      for (int w = kPage; w-- > 0;) free_.push_back(page + w);
+    }
+    *word = free_.back();
+    free_.pop_back();
+    **word = 0;
+    return cudaSuccess;
+  }
+  void give(unsigned int* word) {
+    if (!word) return;
+    std::lock_guard<std::mutex> lk(mutex_);
+    free_.push_back(word);
+  }
+
+ private:
+  static constexpr int kPage = 1024;
+  std::mutex mutex_;
+  std::vector<unsigned int*> free_;
 };
+
+HostWords& host_words() {
+  static HostWords* const words = new HostWords;  // lattices may outlive static objects
+  return *words;
+}
 
 struct chll_lattice {
   int ni = 0, nj = 0, nk = 0, hx = 0, periodic = 0;
@@ -165,8 +195,8 @@ struct chll_lattice {
   size_t per_colour = 0;
   int device = 0;
   float4* lat = nullptr;
-  ControlResults* results = nullptr;
-  Control* ctl = nullptr;  // results->ctl
+  Control* ctl = nullptr;
+  unsigned int* host_status = nullptr;  // nonzero: a wait has given up (HostWords)
   double* partials = nullptr;
   unsigned int* tickets = nullptr;  // [0] observables, [1] gradient
   unsigned long long* words = nullptr;  // meeting words of the resident sweeps
@@ -174,6 +204,7 @@ struct chll_lattice {
   double* rows = nullptr;
   int rows_cap = 0;
   double* host_rows = nullptr;  // pinned, of run()'s lattice
+  double* out4 = nullptr;
   void* staging = nullptr;
   size_t staging_bytes = 0;
   float4* grad = nullptr;
@@ -183,10 +214,6 @@ struct chll_lattice {
   std::vector<GraphEntry> graphs;
   uint64_t use_clock = 0;
   int kernel = chll::kSweepAuto;
-  // Launches whose waits can give up (and then set the status word) have been made
-  // since the word was last read; some of them into a caller's graph, whose
-  // replays are not seen here.
-  bool unread_waits = false, captured_waits = false;
   uint32_t wait_limit = chll::kWaitPolls;
   // z-slab of a larger lattice: global planes z0 .. z0+nk-1 of nk_global,
   // stored as planes 2 .. nk+1 of nk+3 (plane 1 and nk+2 are the halos,
@@ -250,18 +277,9 @@ void drop_graphs(chll_lattice* L) {
   L->graphs.clear();
 }
 
-// Before a launch whose waits can give up.
-void note_waits(chll_lattice* L) {
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(L->stream, &st) != cudaSuccess) cudaGetLastError();
-  if (st != cudaStreamCaptureStatusNone) L->captured_waits = true;
-  L->unread_waits = true;
-}
-
-// The status word as read from the device: a set one is an error of the call that
-// read it, and of those after it until set_control clears it.
-int report_status(chll_lattice* L, unsigned int status) {
-  L->unread_waits = status != 0 || L->captured_waits;
+// A status word that is set is an error of every call that looks at it, until
+// set_control clears it.
+int report_status(unsigned int status) {
   if (status)
     return fail(CHLL_EDEVICE,
                 "device status word 0x%x: a wait gave up and the state is not usable (load one and "
@@ -271,14 +289,10 @@ int report_status(chll_lattice* L, unsigned int status) {
 }
 
 // The end of a synchronising call: waits for the stream and reports a wait that
-// gave up.  The word is read only where one can have.
+// gave up.
 int finish(chll_lattice* L) {
-  unsigned int status = 0;
-  if (L->unread_waits)
-    CHLL_CUDA_TRY(cudaMemcpyAsync(&status, &L->ctl->status, sizeof(status),
-                                  cudaMemcpyDeviceToHost, L->stream));
   CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
-  return L->unread_waits ? report_status(L, status) : CHLL_OK;
+  return report_status(*(volatile unsigned int*)L->host_status);
 }
 
 // Returns an executable graph of `nsweeps` steps for this coupling and key,
@@ -355,9 +369,7 @@ int sweep_impl(chll_lattice* L, const Coupling& cp, uint64_t seed, uint32_t rep,
   if (nsweeps <= 0) return CHLL_OK;
   const uint32_t k0 = seed_lo(seed), k1 = seed_hi(seed);
   const DeviceGuard on(L->device);
-  const bool resident = runs_resident(L);
-  if (resident || L->kernel == chll::kSweepStaged) note_waits(L);
-  if (resident) {
+  if (runs_resident(L)) {
     for (int done = 0; done < nsweeps; done += kResidentChunk) {
       const int n = std::min(kResidentChunk, nsweeps - done);
       const cudaError_t e =
@@ -449,11 +461,12 @@ int set_control_impl(chll_lattice* L, double d, long long step, long long adapt_
   c.adapt_until = adapt_until;
   c.nsites = L->ctl_sites;
   c.deferred = L->slab;
+  c.host_status = L->host_status;
   CHLL_CUDA_TRY(cudaMemcpyAsync(L->ctl, &c, sizeof(c), cudaMemcpyHostToDevice, L->stream));
   // the new block's status is clear: so are the words a failed wait left
   CHLL_CUDA_TRY(cudaMemsetAsync(L->words, 0, chll::kResidentWordBytes, L->stream));
   CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
-  L->unread_waits = L->captured_waits;
+  *(volatile unsigned int*)L->host_status = 0;
   return CHLL_OK;
 }
 
@@ -540,9 +553,8 @@ int create_impl(int ni, int nj, int nk, int boundary, chll_lattice** out, int sl
     chll_lattice_destroy(L);
     return fail(CHLL_ECUDA, "lattice allocation is not 32-byte aligned");
   }
-  if ((e = cudaMalloc(&L->results, sizeof(ControlResults))) != cudaSuccess)
-    return bail(e, "control");
-  L->ctl = &L->results->ctl;
+  if ((e = cudaMalloc(&L->ctl, sizeof(Control))) != cudaSuccess) return bail(e, "control");
+  if ((e = host_words().take(&L->host_status)) != cudaSuccess) return bail(e, "status word");
   const int pb = std::max(chll::observables_max_blocks() * chll::kObsMoments,
                           chll::energy_grad_max_blocks() * 4);
   if ((e = cudaMalloc(&L->partials, sizeof(double) * pb)) != cudaSuccess)
@@ -553,6 +565,9 @@ int create_impl(int ni, int nj, int nk, int boundary, chll_lattice** out, int sl
     return bail(e, "meeting words");
   if ((e = cudaMemsetAsync(L->words, 0, chll::kResidentAllocBytes, L->stream)) != cudaSuccess)
     return bail(e, "memset");
+  if ((e = cudaMalloc(&L->out4, 4 * sizeof(double) + chll::kRowLen * sizeof(double))) !=
+      cudaSuccess)
+    return bail(e, "result buffer");
   if ((e = cudaMemsetAsync(L->tickets, 0, 2 * sizeof(unsigned int), L->stream)) != cudaSuccess)
     return bail(e, "memset");
   if ((e = cudaMemsetAsync(L->lat, 0, all_bytes, L->stream)) != cudaSuccess)
@@ -726,7 +741,7 @@ int run_impl(const chll_run_config& cfg, int nstart, int nstop, int nout, double
   if (rc == CHLL_OK) {
     e = cudaMemcpy(&c, L->ctl, sizeof(c), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) rc = fail(CHLL_ECUDA, "run: %s", cudaGetErrorString(e));
-    else rc = report_status(L, c.status);  // the caller's arrays keep what they held
+    else rc = report_status(c.status);  // the caller's arrays keep what they held
   }
   if (rc == CHLL_OK) rc = download_f64_impl(L, nx, ny, nz, s);
   if (rc == CHLL_OK && d_out) *d_out = c.d;
@@ -851,12 +866,14 @@ void chll_lattice_destroy(chll_lattice* L) {
   if (L->own_stream) cudaStreamSynchronize(L->own_stream);
   if (L->stream && L->stream != L->own_stream) cudaStreamSynchronize(L->stream);
   cudaFree(L->lat);
-  cudaFree(L->results);
+  cudaFree(L->ctl);
+  host_words().give(L->host_status);
   cudaFree(L->partials);
   cudaFree(L->tickets);
   cudaFree(L->words);
   cudaFree(L->rows);
   if (L->host_rows) cudaFreeHost(L->host_rows);
+  cudaFree(L->out4);
   cudaFree(L->staging);
   cudaFree(L->grad);
   if (L->own_stream) cudaStreamDestroy(L->own_stream);
@@ -977,7 +994,7 @@ int chll_lattice_get_control(chll_lattice* L, double* d, int64_t* step, double* 
   Control c;
   CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
   CHLL_CUDA_TRY(cudaMemcpy(&c, L->ctl, sizeof(c), cudaMemcpyDeviceToHost));
-  CHLL_TRY(report_status(L, c.status));
+  CHLL_TRY(report_status(c.status));
   if (d) *d = c.d;
   if (step) *step = c.step;
   if (paccept) *paccept = c.paccept;
@@ -1015,11 +1032,9 @@ int chll_lattice_pass(chll_lattice* L, const chll_coupling* c, uint64_t seed, ui
   if (pass >= 4)
     chll::launch_fused_pass(L->view(), make_coupling(*c), seed_lo(seed), seed_hi(seed), replica,
                             L->ctl, pass - 4, L->stream);
-  else {
-    if (L->kernel == chll::kSweepStaged) note_waits(L);
+  else
     chll::launch_sweep_pass(L->view(), make_coupling(*c), seed_lo(seed), seed_hi(seed),
                             replica, L->ctl, pass, L->stream, L->kernel);
-  }
   CHLL_CUDA_TRY(cudaGetLastError());
   return ok();
 }
@@ -1053,13 +1068,11 @@ int chll_lattice_read_rows(chll_lattice* L, double* rows16, int first, int count
 
 int chll_lattice_observe(chll_lattice* L, const chll_coupling* c, double* row16) {
   if (!L || !c || !row16) return fail(CHLL_EINVAL, "observe: null argument");
-  CHLL_TRY(observe_impl(L, make_coupling_d(*c), L->results->row, chll::kStepOfControl));
-  ControlResults back;
-  CHLL_CUDA_TRY(cudaMemcpyAsync(&back, L->results, sizeof(back), cudaMemcpyDeviceToHost,
-                                L->stream));
-  CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
-  CHLL_TRY(report_status(L, back.ctl.status));
-  std::memcpy(row16, back.row, sizeof(back.row));
+  double* drow = L->out4 + 4;
+  CHLL_TRY(observe_impl(L, make_coupling_d(*c), drow, chll::kStepOfControl));
+  CHLL_CUDA_TRY(cudaMemcpyAsync(row16, drow, sizeof(double) * chll::kRowLen,
+                                cudaMemcpyDeviceToHost, L->stream));
+  CHLL_TRY(finish(L));
   return ok();
 }
 
@@ -1071,7 +1084,6 @@ int chll_lattice_quench(chll_lattice* L, const chll_coupling* c, double eta, int
   const chll::CouplingD cd = make_coupling_d(*c);
   const DeviceGuard on(L->device);
   if (chll::quench_resident_pays(v)) {
-    note_waits(L);
     for (int done = 0; done < nsteps; done += kResidentChunk) {
       const cudaError_t e = chll::launch_quench_resident(
           v, cd, (float)eta, L->ctl, L->words, L->xch, std::min(kResidentChunk, nsteps - done),
@@ -1095,7 +1107,7 @@ int chll_lattice_energy_grad(chll_lattice* L, const chll_coupling* c, float* gra
   const size_t total = 2 * L->per_colour;
   if (grad && !L->grad) CHLL_CUDA_TRY(cudaMalloc(&L->grad, total * sizeof(float4)));
   chll::launch_energy_grad(L->view(), make_coupling_d(*c), grad ? L->grad : nullptr, project,
-                           L->partials, &L->tickets[1], L->results->out4, L->stream);
+                           L->partials, &L->tickets[1], L->out4, L->stream);
   CHLL_CUDA_TRY(cudaGetLastError());
   if (grad) {
     LatticeView gv = L->view();
@@ -1112,16 +1124,10 @@ int chll_lattice_energy_grad(chll_lattice* L, const chll_coupling* c, float* gra
     }
     CHLL_CUDA_TRY(cudaGetLastError());
   }
-  if (!out4) {
-    CHLL_TRY(finish(L));
-    return ok();
-  }
-  ControlResults back;
-  CHLL_CUDA_TRY(cudaMemcpyAsync(&back, L->results, offsetof(ControlResults, row),
-                                cudaMemcpyDeviceToHost, L->stream));
-  CHLL_CUDA_TRY(cudaStreamSynchronize(L->stream));
-  CHLL_TRY(report_status(L, back.ctl.status));
-  std::memcpy(out4, back.out4, sizeof(back.out4));
+  if (out4)
+    CHLL_CUDA_TRY(cudaMemcpyAsync(out4, L->out4, 4 * sizeof(double), cudaMemcpyDeviceToHost,
+                                  L->stream));
+  CHLL_TRY(finish(L));
   return ok();
 }
 

@@ -254,6 +254,7 @@ struct Control {
   int deferred;              // nonzero: passes only count; the epilogue runs apart
                              // (a slab, whose counts are summed over ranks first)
   int pad;
+  unsigned int* host_status;  // pinned host memory, or null: set with status
 };
 
 // Row written by the observables kernel (FP64).  Columns 0-4 are the

@@ -297,7 +297,7 @@ __device__ __forceinline__ void control_warp(const FlowArgs& A, FlowShared& S, i
   bar_wait(kBarEnd);
   if (!lead) return;
   if (S.lost) {
-    atomicOr(&ctl->status, 4u);
+    set_status(ctl, 4u);
     atomicAdd(A.epoch, (uint32_t)A.nsweeps + 2u);  // what was published is never read again
     return;
   }

@@ -277,7 +277,7 @@ __device__ __forceinline__ void resident_sweeps(const ResidentArgs& A, ResidentS
     if (!S.ok) break;
   }
   if (!S.ok) {
-    if (threadIdx.x == 0) atomicOr(&ctl->status, 4u);
+    if (threadIdx.x == 0) set_status(ctl, 4u);
     return;
   }
   units.template pass<kFusedF>(step, (float)S.d, na, nf);

@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(kThreads, 2)
       T, L, reinterpret_cast<float4*>(smem), smem_addr(&bars[0]), smem_addr(&bars[1]), uses0,
       uses1, blockIdx.x, gridDim.x, (uint32_t)step, d, cp, key0, key1, replica, kWaitLimit,
       &timed_out);
-  if (timed_out && threadIdx.x == 0) atomicOr(&ctl->status, 2u);
+  if (timed_out && threadIdx.x == 0) set_status(ctl, 2u);
   pass_epilogue<DIRECTOR, C>(ctl, accepted, step);
 }
 

@@ -16,6 +16,12 @@
 
 namespace chll {
 
+// A wait that gave up: the status word, and the host's copy of it.
+__device__ __forceinline__ void set_status(Control* ctl, unsigned int bits) {
+  atomicOr(&ctl->status, bits);
+  if (ctl->host_status) *(volatile unsigned int*)ctl->host_status = bits;
+}
+
 struct SweepGeom {
   uint32_t Q;      // units (4-site blocks) per row = hx/2
   uint32_t first;  // first unit updated (0, or a slab's first interior plane)

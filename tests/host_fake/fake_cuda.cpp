@@ -137,10 +137,6 @@ cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) {
   captured.clear();
   return cudaSuccess;
 }
-cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* s) {
-  *s = cudaStreamCaptureStatusNone;
-  return cudaSuccess;
-}
 cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) {
   capturing = false;
   *g = reinterpret_cast<cudaGraph_t>(new FakeGraph{captured});

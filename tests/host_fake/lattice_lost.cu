@@ -24,10 +24,12 @@ static void expect(bool ok, const char* what) {
 
 static void launch(chll::Control* ctl, int n) {
   if (ctl->status) return;
-  if (lose)
+  if (lose) {
     ctl->status = 4;
-  else
+    *ctl->host_status = 4;
+  } else {
     ctl->step += n;
+  }
 }
 
 namespace chll {
