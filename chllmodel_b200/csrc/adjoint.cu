@@ -498,9 +498,9 @@ __global__ void __launch_bounds__(kGradThreads)
 }
 
 // Every product and sum of a quench step is an explicit fmaf / __fmul_rn /
-// __fadd_rn, so that the pass kernel and the resident form round alike: a quench
-// amplifies a rounding along the lattice's soft modes, and its energies are
-// compared to ten digits.
+// __fadd_rn, so that the pass kernel and the resident forms round alike: a quench
+// amplifies a rounding along the lattice's soft modes, and forms that contracted
+// differently would end in different states of one lattice.
 
 // x0 y0 + x1 y1 + x2 y2; SECOND: the second product is the rounded one of the
 // first two.
@@ -535,8 +535,9 @@ __device__ __forceinline__ void quench_bond(const float4& n, const float4& b, fl
 // tangent-projected energy gradient, n <- normalise(n - eta (I - n n^T) dE/dn),
 // with the neighbours nb (+x, -x, +y, -y, +z, -z) held fixed.  Which product of a
 // bond's dot product is rounded on its own differs between the boundaries and,
-// for -z, between a unit's sites (second: the unit's second one): the roundings
-// this quench has always had.
+// for -z, between a unit's sites (second: the unit's second one).  The physics does
+// not ask for it: these are the roundings of the pass kernel as it was first
+// compiled, kept so that a quench still ends in the state it ended in before.
 template <bool P>
 __device__ __forceinline__ float4 quench_site(float4 n, const Nbrs& nb, const Coupling& cp,
                                               float eta, bool second) {
@@ -941,7 +942,7 @@ int quench_flow_sites(const LatticeView& L) {
 }
 
 // Against a launch per pass, us per step (periodic): 8^3 1.1 and 7.5, 64^3 3.6 and
-// 8.4, 96^3 12.7 and 16.6, 128^3 24.6 and 25.0; from 160^3 on the launches win (45.2
+// 8.4, 96^3 12.4 and 16.6, 128^3 24.4 and 25.0; from 160^3 on the launches win (45.2
 // and 41.3: their loads are the read-only ones).
 bool quench_resident_pays(const LatticeView& L) { return make_geom(L).units <= (1u << 19); }
 

@@ -16,9 +16,9 @@
 // cluster barrier, whose 16 SMs had to issue every instruction of the pass):
 //
 //   edge                    8     16    24    32    48    64    96    128   200
-//   passes launched each   5.5   4.6   6.4   6.5   6.6   8.1   15.0  26.9  85.6
+//   passes launched each   5.8   5.8   6.4   6.6   6.9   7.9   14.2  25.6  84.8
 //   one cluster            3.5   5.4   5.5   5.6  14.5
-//   this form              1.9   3.9   4.0   4.0   4.6   6.3   13.5  24.6  79.5
+//   this form              1.9   3.9   4.0   4.0   4.6   6.1   12.4  23.2  78.6
 //   flow.cu                      2.6   2.6   2.6   3.2
 //
 // The barrier and the counts are one 64-bit word per pass: a CTA adds its
@@ -338,12 +338,13 @@ bool resident_fits(const LatticeView& L) {
 }
 
 // Against a launch per pass: always where a thread holds one site of each colour
-// or one unit (50^3 periodic 3.7 against 7.5 us, 64^3 6.3 against 8.1).  Beyond
+// or one unit (50^3 periodic 3.7 against 7.5 us, 64^3 6.1 against 7.9).  Beyond
 // that the barrier still saves about 1 us per pass, but the loops' coherent
 // loads cost the units more than the read-only ones do.  With unpadded rows it
-// pays up to 256^3 (4 M units) periodic (128^3 24.6 against 26.9 us, 200^3 79.5
-// against 85.6, 256^3 161 against 164) and 200^3 (2 M units) open (128^3 26.0
-// against 27.2, 200^3 83.6 against 87.2, 256^3 183 against 180); with padded rows
+// pays up to 256^3 (4 M units) periodic (128^3 23.2 against 25.6 us, 200^3 78.6
+// against 84.8, 256^3 167 against 175) and 200^3 (2 M units) open (128^3 24.6
+// against 26.0, 176^3 56.4 against 60.1, 200^3 81.3 against 84.9, 256^3 180 against
+// 178; 192^3 alone loses, 82.6 against 81.1); with padded rows
 // it does not (130^3 open 31.1 against 29.7, 150 x 125 x 101 28.1 against 27.2).
 bool resident_pays(const LatticeView& L) {
   const uint32_t units = make_geom(L).units;

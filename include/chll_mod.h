@@ -134,16 +134,19 @@ int chll_lattice_set_stream(chll_lattice* lat, void* stream);
 /* Sweep form: 0 auto (4 where it is the faster one -- lattices of at most one
  * unit of two sites per GPU thread, about 66^3 (periodic rows that are not a
  * multiple of 4 sites: one site of each colour, about 53^3), and of rows of a
- * multiple of 4 sites up to 256^3 periodic, 200^3 open -- else 3), 1 the reference's four
- * half-sweeps per step with
- * neighbours read from global memory, 2 the four half-sweeps with row tiles
- * staged in shared memory by bulk copies, 3 the fused two-pass sweep (each
- * pass reads and writes every site once; the colour-0 flips of a step run at
- * the start of the next step's first pass, and after the last step), 4 the
- * fused passes of a whole chunk of steps in one cooperative launch whose CTAs
- * meet at a grid barrier between passes (small lattices, where a pass is
- * mostly launch and grid latency; refused for a slab; lattices of 2^27 sites
- * and more take the launches of 3).  All give the same chain bit for bit.  chll_lattice_pass runs the staged kernel under 2 and the direct kernel
+ * multiple of 4 sites up to 256^3 periodic, 200^3 open -- else 3), 1 the
+ * reference's four half-sweeps per step with neighbours read from global memory,
+ * 2 the four half-sweeps with row tiles staged in shared memory by bulk copies, 3
+ * the fused two-pass sweep (each pass reads and writes every site once; the
+ * colour-0 flips of a step run at the start of the next step's first pass, and
+ * after the last step), 4 the fused passes of a whole chunk of steps in one
+ * cooperative launch whose CTAs meet at a grid barrier between passes, or, up to
+ * about 52^3, wait for their neighbours' sites (small lattices, where a pass is
+ * mostly launch and grid latency; refused for a slab; lattices of 2^27 sites and
+ * more take the launches of 3).  All give the same chain bit for bit.  A launch of
+ * 4 fills the GPU from about 48^3 on: lattices that sweep at once, each on its own
+ * stream, then run one after the other, where the launches of 3 overlap.
+ * chll_lattice_pass runs the staged kernel under 2 and the direct kernel
  * otherwise. */
 int chll_lattice_set_kernel(chll_lattice* lat, int kernel);
 /* How many polls a wait of the resident sweep launches and of the quench makes
@@ -177,7 +180,8 @@ int chll_lattice_get_control(chll_lattice* lat, double* d, int64_t* step, double
                              double* faccept);
 /* nsweeps full steps from the control block's step, in the form chosen by
  * chll_lattice_set_kernel; every call ends with all trials of its last step
- * done.  Consecutive calls with the same count replay one captured CUDA graph. */
+ * done.  The launches of a pass each are captured as a CUDA graph, which
+ * consecutive calls with the same count replay. */
 int chll_lattice_sweep(chll_lattice* lat, const chll_coupling* c, uint64_t seed,
                        uint32_t replica, int nsweeps);
 /* One pass.  The reference's half-sweeps: 0/1 director trials on colour 0/1,
@@ -271,9 +275,10 @@ int chll_batch_set_wave_bytes(chll_batch* b, int64_t wave_bytes);
  * launch per fused pass over all replicas' units, cut into equal blocks per
  * CTA, the next pass launched as a programmatic dependent (CUDA graphs of
  * measurement-interval chunks) -- instead of the persistent launch with
- * software group barriers; 0 (the default): the persistent launch.  The chains are the same either way; the
- * launch shape, waves and pairing apply to the persistent launch only.  No
- * counterpart in the reference, which has no batched launch. */
+ * software group barriers; 0 (the default): the persistent launch.  The chains
+ * are the same either way; the launch shape, waves and pairing apply to the
+ * persistent launch only.  No counterpart in the reference, which has no batched
+ * launch. */
 int chll_batch_set_pooled(chll_batch* b, int pooled);
 int chll_batch_get_pooled(chll_batch* b, int* pooled);
 /* pair = 1: the replicas of a wave are grouped two by two, by size, and each
@@ -294,9 +299,10 @@ int chll_batch_set_wait_limit(chll_batch* b, uint64_t polls);
 int chll_batch_get_tuning(chll_batch* b, int32_t* threads, int32_t* ctas_per_sm,
                           int64_t* wave_bytes, int32_t* nwaves);
 /* Times the launch shapes (threads, CTAs per SM, wave size) that can be the
- * fastest for this batch for trial_sweeps sweeps from a snapshot of the current state, keeps the fastest (of the
- * persistent launch with single groups; pairing and pooled passes are never the
- * fastest and are turned off) and restores the state. */
+ * fastest for this batch for trial_sweeps sweeps from a snapshot of the current
+ * state, keeps the fastest (of the persistent launch with single groups; pairing
+ * and pooled passes are never the fastest and are turned off) and restores the
+ * state.  A trial whose wait gave up is left out; CHLL_EDEVICE if all did. */
 int chll_batch_autotune(chll_batch* b, int trial_sweeps, int* best_threads, int* best_ctas,
                         double* best_ms);
 
